@@ -378,20 +378,26 @@ static int forward_pass(const moba_problem_t* p, int64_t sel_rs, const void* q, 
     return (events && events[i]) ? cudaEventRecord((cudaEvent_t)events[i], st) : cudaSuccess;
   };
   if (first && (e = mark(0)) != cudaSuccess) return (int)e;
-  if ((e = cudaMemsetAsync(w.list_counts, 0, w.zero_bytes, st)) != cudaSuccess) return (int)e;
+  // the counters are cleared by the chunk-mean kernel where one runs
+  if ((r.hist <= 0 || opt.means_ready) &&
+      (e = cudaMemsetAsync(w.list_counts, 0, w.zero_bytes, st)) != cudaSuccess)
+    return (int)e;
   const __nv_bfloat16* qb = static_cast<const __nv_bfloat16*>(q);
   const __nv_bfloat16* kb = static_cast<const __nv_bfloat16*>(k);
   if (r.hist > 0) {
     int32_t* sel = selected_out ? selected_out : w.selected;
     __nv_bfloat16* means = opt.means_ext ? opt.means_ext : w.means;
     if (!opt.means_ready &&
-        (e = launch_chunk_means_range(r, opt.means_ext ? opt.means_from : 0, r.slots, kb, cu, means, st)) != cudaSuccess)
+        (e = launch_chunk_means_range(r, opt.means_ext ? opt.means_from : 0, r.slots, kb, cu, means, st, w.list_counts,
+                                      (int64_t)(w.zero_bytes / sizeof(int32_t)))) != cudaSuccess)
       return (int)e;
     if (last && (e = mark(1)) != cudaSuccess) return (int)e;
-    if ((e = launch_gate_topk(r, qb, means, cu, sel, w.list_counts, st)) != cudaSuccess) return (int)e;
+    // the gating kernel ends with the prefix sums over the lists it counted
+    const ListScan scan{w.list_counts, w.list_offsets, w.tile_prefix, w.cursors, r.lists,
+                        tile_rows_of(p->attend_impl, p->head_dim, p->chunk_size)};
+    if ((e = launch_gate_topk(r, qb, means, cu, sel, w.list_counts, st, &scan, w.status + 1)) != cudaSuccess) return (int)e;
     if (last && (e = mark(2)) != cudaSuccess) return (int)e;
-    if ((e = launch_compact(r, cu, sel, w.list_counts, w.list_offsets, w.tile_prefix, w.cursors, w.row_list,
-                            w.partial_lse, tile_rows_of(p->attend_impl, p->head_dim, p->chunk_size), st)) != cudaSuccess)
+    if ((e = launch_scatter(r, cu, sel, w.list_offsets, w.cursors, w.row_list, w.partial_lse, st)) != cudaSuccess)
       return (int)e;
   } else if (last) {
     if ((e = mark(1)) != cudaSuccess || (e = mark(2)) != cudaSuccess) return (int)e;

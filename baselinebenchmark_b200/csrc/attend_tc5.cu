@@ -355,9 +355,6 @@ attend_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
       mbar_init(smem_u32(&c.item_ready[i]), 1);
     }
     c.abort = 0;
-    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
-    c.own = own_slot_range(p, a.cu);
-    c.n_items = c.n_routed + own_item_count(c.own.n, p.Hq, p.C, 2 * kTileM);
     fence_barrier_init();
     prefetch_tmap(&tmap_k);
     prefetch_tmap(&tmap_v);
@@ -365,6 +362,13 @@ attend_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
   if (warp == 1) {
     tmem_alloc(smem_u32(&c.tmem_slot), kTmemCols);
     tmem_relinquish();
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (threadIdx.x == 0) {
+    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
+    c.own = own_slot_range(p, a.cu);
+    c.n_items = c.n_routed + own_item_count(c.own.n, p.Hq, p.C, 2 * kTileM);
   }
   if (p.hist > 0) fill_prefix_cache(c, a.tile_prefix, p.lists, kThreads);
   tc_fence_before();
@@ -661,9 +665,6 @@ attend_tc5_wide_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_
       mbar_init(smem_u32(&c.item_ready[i]), 1);
     }
     c.abort = 0;
-    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
-    c.own = own_slot_range(p, a.cu);
-    c.n_items = c.n_routed + own_item_count(c.own.n, p.Hq, p.C, kTileM);
     fence_barrier_init();
     prefetch_tmap(&tmap_k);
     prefetch_tmap(&tmap_v);
@@ -671,6 +672,13 @@ attend_tc5_wide_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_
   if (warp == 1) {
     tmem_alloc(smem_u32(&c.tmem_slot), kTmemCols);
     tmem_relinquish();
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (threadIdx.x == 0) {
+    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
+    c.own = own_slot_range(p, a.cu);
+    c.n_items = c.n_routed + own_item_count(c.own.n, p.Hq, p.C, kTileM);
   }
   if (p.hist > 0) fill_prefix_cache(c, a.tile_prefix, p.lists, kThreads);
   tc_fence_before();
@@ -964,9 +972,6 @@ attend_tc5_small_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
     mbar_init(smem_u32(&c.item_ready[0]), 1);
     mbar_init(smem_u32(&c.item_ready[1]), 1);
     c.abort = 0;
-    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
-    c.own = own_slot_range(p, a.cu);
-    c.n_items = c.n_routed + own_item_count(c.own.n, p.Hq, p.C, kTileM);
     fence_barrier_init();
     prefetch_tmap(&tmap_k);
     prefetch_tmap(&tmap_v);
@@ -974,6 +979,13 @@ attend_tc5_small_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
   if (warp == 5) {
     tmem_alloc(smem_u32(&c.tmem_slot), kCols);
     tmem_relinquish();
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (threadIdx.x == 0) {
+    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
+    c.own = own_slot_range(p, a.cu);
+    c.n_items = c.n_routed + own_item_count(c.own.n, p.Hq, p.C, kTileM);
   }
   if (p.hist > 0) fill_prefix_cache(c, a.tile_prefix, p.lists, kSmallThreads);
   tc_fence_before();
@@ -1272,11 +1284,9 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
                             : (p.fp16 ? attend_tc5_small_kernel<true, 64> : attend_tc5_small_kernel<false, 64>);
     e = cudaFuncSetAttribute(small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmemBytes);
     if (e != cudaSuccess) return e;
-    small<<<2 * sms, kSmallThreads, kSmallSmemBytes, st>>>(p, mk, mv, args);
-    return cudaGetLastError();
+    return launch_pdl(small, dim3(2 * sms), kSmallThreads, kSmallSmemBytes, st, p, mk, mv, args);
   }
-  kernel<<<sms, kThreads, kSmemBytes, st>>>(p, mk, mv, args);
-  return cudaGetLastError();
+  return launch_pdl(kernel, dim3(sms), kThreads, kSmemBytes, st, p, mk, mv, args);
 }
 
 }  // namespace moba

@@ -56,7 +56,13 @@ cudaError_t launch_chunk_metadata(const Params& p, const int32_t* cu, int32_t* c
 template <bool kHalf, int D>
 __global__ void __launch_bounds__(kMeanLanes * (D / 8))
 chunk_mean_kernel(Params p, int slot_begin, const __nv_bfloat16* __restrict__ k, const int32_t* __restrict__ cu,
-                  __nv_bfloat16* __restrict__ means) {
+                  __nv_bfloat16* __restrict__ means, int32_t* __restrict__ zero, int64_t zero_words) {
+  pdl_wait();
+  pdl_trigger();
+  // the counters that the kernels behind this one add to
+  for (int64_t i = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < zero_words;
+       i += (int64_t)gridDim.x * gridDim.y * blockDim.x)
+    zero[i] = 0;
   const int slot = slot_begin + blockIdx.x, hk = blockIdx.y;
   const int b = slot / p.mc, j = slot - b * p.mc;
   const Slot sl = slot_of(cu, b, j, p.C);
@@ -110,20 +116,22 @@ chunk_mean_kernel(Params p, int slot_begin, const __nv_bfloat16* __restrict__ k,
 
 // Means of the slots [slot_begin, slot_end) only (context-parallel ranks compute those of their own chunks).
 cudaError_t launch_chunk_means_range(const Params& p, int slot_begin, int slot_end, const __nv_bfloat16* k,
-                                     const int32_t* cu, __nv_bfloat16* means, cudaStream_t st) {
-  if (slot_end <= slot_begin) return cudaSuccess;
+                                     const int32_t* cu, __nv_bfloat16* means, cudaStream_t st, int32_t* zero,
+                                     int64_t zero_words) {
+  if (slot_end <= slot_begin)
+    return zero_words > 0 ? cudaMemsetAsync(zero, 0, (size_t)zero_words * sizeof(int32_t), st) : cudaSuccess;
   dim3 grid(slot_end - slot_begin, p.Hkv);
 #define MOBA_MEANS(HALF, DIM) \
-  chunk_mean_kernel<HALF, DIM><<<grid, kMeanLanes * (DIM / 8), 0, st>>>(p, slot_begin, k, cu, means)
+  return launch_pdl(chunk_mean_kernel<HALF, DIM>, grid, kMeanLanes * (DIM / 8), 0, st, p, slot_begin, k, cu, means, zero, \
+                    zero_words)
   switch (p.D) {
-    case 64:  if (p.fp16) MOBA_MEANS(true, 64);  else MOBA_MEANS(false, 64);  break;
-    case 96:  if (p.fp16) MOBA_MEANS(true, 96);  else MOBA_MEANS(false, 96);  break;
-    case 128: if (p.fp16) MOBA_MEANS(true, 128); else MOBA_MEANS(false, 128); break;
-    case 256: if (p.fp16) MOBA_MEANS(true, 256); else MOBA_MEANS(false, 256); break;
+    case 64:  if (p.fp16) MOBA_MEANS(true, 64);  else MOBA_MEANS(false, 64);
+    case 96:  if (p.fp16) MOBA_MEANS(true, 96);  else MOBA_MEANS(false, 96);
+    case 128: if (p.fp16) MOBA_MEANS(true, 128); else MOBA_MEANS(false, 128);
+    case 256: if (p.fp16) MOBA_MEANS(true, 256); else MOBA_MEANS(false, 256);
     default: return cudaErrorInvalidValue;
   }
 #undef MOBA_MEANS
-  return cudaGetLastError();
 }
 
 cudaError_t launch_chunk_means(const Params& p, const __nv_bfloat16* k, const int32_t* cu,
@@ -338,7 +346,8 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
                  int tokens_per_cta, int nt, int list_len, int nbuf, int cnt_in_smem,
                  const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ means,
                  const int32_t* __restrict__ cu, int32_t* __restrict__ selected,
-                 int32_t* __restrict__ list_counts, int32_t* __restrict__ stats, int flags) {
+                 int32_t* __restrict__ list_counts, int32_t* __restrict__ stats, int flags, const ListScan scan,
+                 int32_t* __restrict__ ticket) {
   extern __shared__ unsigned char gate_smem_raw[];
   constexpr int kNBlk = (D + 63) / 64;                 // 64-dim blocks of a row
   const int hist = p.hist;
@@ -374,6 +383,8 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
   }
   if (cnt_in_smem)
     for (int i = tid; i < p.mc; i += kGateThreads) cnt_s[i] = 0;       // every tile leaves them at zero again
+  pdl_wait();
+  pdl_trigger();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -796,6 +807,20 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
     ++n;
   }
 
+  // the CTA that finishes last turns the counts of all into the offsets of the lists
+  if (ticket != nullptr) {
+    int* scratch = reinterpret_cast<int*>(c.exact);           // no row is being ranked any more
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) scratch[0] = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+    __syncthreads();
+    const bool last = scratch[0] != 0;
+    __syncthreads();
+    if (last) {
+      __threadfence();
+      scan_lists<kGateThreads, 8>(scan, scratch);
+    }
+  }
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, (uint32_t)nt);
@@ -844,7 +869,7 @@ bool gate_topk_fits(const Params& p) { return p.hist <= 0 || gate_launch_config(
 
 cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* means,
                                    const int32_t* cu, int32_t* selected, int32_t* list_counts, int32_t* stats,
-                                   int flags, cudaStream_t st) {
+                                   int flags, cudaStream_t st, const ListScan* scan, int32_t* ticket) {
   int tokens_per_cta = kGateRows / p.G;
   if (tokens_per_cta < 1) return cudaErrorInvalidConfiguration;
   const GateLaunch g = gate_launch_config(p);
@@ -854,7 +879,7 @@ cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, cons
       !make_tile_map(&mm, p.fp16 != 0, p.D, means, p.slots, p.Hkv, (int64_t)p.Hkv * p.D, p.D, 1, g.nt))
     return cudaErrorNotSupported;
   typedef void (*Kernel)(Params, CUtensorMap, CUtensorMap, int, int, int, int, int, const __nv_bfloat16*,
-                         const __nv_bfloat16*, const int32_t*, int32_t*, int32_t*, int32_t*, int);
+                         const __nv_bfloat16*, const int32_t*, int32_t*, int32_t*, int32_t*, int, ListScan, int32_t*);
   Kernel kernel = nullptr;
   const int w = g.list_len <= 8 ? 8 : (g.list_len <= 16 ? 16 : (g.list_len <= 32 ? 32 : 0));
 #define MOBA_GATE_W(HALF, DIM)                                                                       \
@@ -890,15 +915,15 @@ cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, cons
   if (resident < 1) resident = 1;
   int64_t grid = (int64_t)sms * resident;
   if (grid > n_tiles) grid = n_tiles;
-  kernel<<<(int)grid, kGateThreads, g.smem, st>>>(p, mq, mm, tokens_per_cta, g.nt, g.list_len, g.nbuf, g.cnt_in_smem, q,
-                                                  means, cu, selected, list_counts, stats, flags);
-  return cudaGetLastError();
+  return launch_pdl(kernel, dim3((unsigned)grid), kGateThreads, g.smem, st, p, mq, mm, tokens_per_cta, g.nt, g.list_len,
+                    g.nbuf, g.cnt_in_smem, q, means, cu, selected, list_counts, stats, flags, scan ? *scan : ListScan{},
+                    scan ? ticket : nullptr);
 }
 
 cudaError_t launch_gate_topk(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* means,
                              const int32_t* cu, int32_t* selected, int32_t* list_counts,
-                             cudaStream_t st) {
-  return launch_gate_topk_stats(p, q, means, cu, selected, list_counts, nullptr, 0, st);
+                             cudaStream_t st, const ListScan* scan, int32_t* ticket) {
+  return launch_gate_topk_stats(p, q, means, cu, selected, list_counts, nullptr, 0, st, scan, ticket);
 }
 
 }  // namespace moba

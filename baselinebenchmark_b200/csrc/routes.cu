@@ -21,47 +21,11 @@ namespace moba {
 // ---------------------------------------------------------------------------
 constexpr int kScanThreads = 1024;
 
-__global__ void __launch_bounds__(kScanThreads)
-scan_lists_kernel(int64_t lists, int tile_rows, const int32_t* __restrict__ counts,
-                  int32_t* __restrict__ offsets, int32_t* __restrict__ tile_prefix,
-                  int32_t* __restrict__ cursors) {
-  __shared__ int warp_rows[32], warp_tiles[32];
-  __shared__ int carry_rows, carry_tiles;
-  if (threadIdx.x == 0) { carry_rows = 0; carry_tiles = 0; }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int64_t base = 0; base < lists; base += kScanThreads) {
-    const int64_t l = base + threadIdx.x;
-    const int n = l < lists ? counts[l] : 0;
-    const int t = (n + tile_rows - 1) / tile_rows;
-    int xr = n, xt = t;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int yr = __shfl_up_sync(0xffffffffu, xr, o);
-      const int yt = __shfl_up_sync(0xffffffffu, xt, o);
-      if (lane >= o) { xr += yr; xt += yt; }
-    }
-    if (lane == 31) { warp_rows[warp] = xr; warp_tiles[warp] = xt; }
-    __syncthreads();
-    if (warp == 0) {
-      int wr = warp_rows[lane], wt = warp_tiles[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int yr = __shfl_up_sync(0xffffffffu, wr, o);
-        const int yt = __shfl_up_sync(0xffffffffu, wt, o);
-        if (lane >= o) { wr += yr; wt += yt; }
-      }
-      warp_rows[lane] = wr; warp_tiles[lane] = wt;            // inclusive over warps
-    }
-    __syncthreads();
-    const int pre_r = carry_rows + (warp ? warp_rows[warp - 1] : 0) + xr - n;
-    const int pre_t = carry_tiles + (warp ? warp_tiles[warp - 1] : 0) + xt - t;
-    if (l < lists) { offsets[l] = pre_r; tile_prefix[l] = pre_t; cursors[l] = 0; }
-    __syncthreads();
-    if (threadIdx.x == 0) { carry_rows += warp_rows[31]; carry_tiles += warp_tiles[31]; }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) { offsets[lists] = carry_rows; tile_prefix[lists] = carry_tiles; }
+__global__ void __launch_bounds__(kScanThreads) scan_lists_kernel(const ListScan a) {
+  pdl_wait();
+  pdl_trigger();
+  __shared__ int scratch[2 * kScanThreads / 32];
+  scan_lists<kScanThreads, 1>(a, scratch);
 }
 
 // ---------------------------------------------------------------------------
@@ -76,6 +40,8 @@ __global__ void __launch_bounds__(kScatterThreads)
 scatter_routes_kernel(Params p, const int32_t* __restrict__ cu, const int32_t* __restrict__ selected,
                       const int32_t* __restrict__ offsets, int32_t* __restrict__ cursors,
                       int32_t* __restrict__ row_list, float2* __restrict__ partial_lse) {
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ int32_t sm[];
   int32_t* cnt_s = sm;               // [mc] rows of this CTA per list, then running index
   int32_t* base_s = sm + p.mc;       // [mc] first position reserved for this CTA
@@ -124,16 +90,23 @@ cudaError_t launch_compact(const Params& p, const int32_t* cu, const int32_t* se
                            const int32_t* list_counts, int32_t* list_offsets, int32_t* tile_prefix,
                            int32_t* cursors, int32_t* row_list, float2* partial_lse, int tile_rows,
                            cudaStream_t st) {
-  scan_lists_kernel<<<1, kScanThreads, 0, st>>>(p.lists, tile_rows, list_counts, list_offsets, tile_prefix, cursors);
-  cudaError_t e = cudaGetLastError();
+  const ListScan scan{list_counts, list_offsets, tile_prefix, cursors, p.lists, tile_rows};
+  const cudaError_t e = launch_pdl(scan_lists_kernel, dim3(1), kScanThreads, 0, st, scan);
   if (e != cudaSuccess) return e;
+  return launch_scatter(p, cu, selected, list_offsets, cursors, row_list, partial_lse, st);
+}
+
+cudaError_t launch_scatter(const Params& p, const int32_t* cu, const int32_t* selected, const int32_t* list_offsets,
+                           int32_t* cursors, int32_t* row_list, float2* partial_lse, cudaStream_t st) {
   const size_t smem = (size_t)p.mc * 2 * sizeof(int32_t);
   if (smem > 200 * 1024) return cudaErrorInvalidConfiguration;
-  e = cudaFuncSetAttribute(scatter_routes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(scatter_routes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
   dim3 grid(window_tiles(p, kScatterTokens), p.Hkv, p.B);
-  scatter_routes_kernel<<<grid, kScatterThreads, smem, st>>>(p, cu, selected, list_offsets, cursors, row_list, partial_lse);
-  return cudaGetLastError();
+  return launch_pdl(scatter_routes_kernel, grid, kScatterThreads, smem, st, p, cu, selected, list_offsets, cursors,
+                    row_list, partial_lse);
 }
 
 // ---------------------------------------------------------------------------
@@ -152,6 +125,8 @@ template <bool kHalf, int D>
 __global__ void __launch_bounds__(kMergeThreads, 5)
 merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __restrict__ partial_lse,
              const int32_t* __restrict__ status, __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out) {
+  pdl_wait();
+  pdl_trigger();
   constexpr int kLanes = D / 8;                  // lanes per partial row
   constexpr int kGroups = 32 / kLanes;
   constexpr int kAhead = 4;                      // partial rows a group has in flight
@@ -247,16 +222,16 @@ cudaError_t launch_merge(const Params& p, const __half* partial_out, const float
   int64_t blocks = (p.rows + (kMergeThreads / 32) - 1) / (kMergeThreads / 32);
   if (blocks > 148 * 64) blocks = 148 * 64;
 #define MOBA_MERGE(HALF, DIM) \
-  merge_kernel<HALF, DIM><<<(int)blocks, kMergeThreads, 0, st>>>(p, partial_out, partial_lse, status, out, lse_out)
+  return launch_pdl(merge_kernel<HALF, DIM>, dim3((unsigned)blocks), kMergeThreads, 0, st, p, partial_out, partial_lse, \
+                    status, out, lse_out)
   switch (p.D) {
-    case 64:  if (p.fp16) MOBA_MERGE(true, 64);  else MOBA_MERGE(false, 64);  break;
-    case 96:  if (p.fp16) MOBA_MERGE(true, 96);  else MOBA_MERGE(false, 96);  break;
-    case 128: if (p.fp16) MOBA_MERGE(true, 128); else MOBA_MERGE(false, 128); break;
-    case 256: if (p.fp16) MOBA_MERGE(true, 256); else MOBA_MERGE(false, 256); break;
+    case 64:  if (p.fp16) MOBA_MERGE(true, 64);  else MOBA_MERGE(false, 64);
+    case 96:  if (p.fp16) MOBA_MERGE(true, 96);  else MOBA_MERGE(false, 96);
+    case 128: if (p.fp16) MOBA_MERGE(true, 128); else MOBA_MERGE(false, 128);
+    case 256: if (p.fp16) MOBA_MERGE(true, 256); else MOBA_MERGE(false, 256);
     default: return cudaErrorInvalidValue;
   }
 #undef MOBA_MERGE
-  return cudaGetLastError();
 }
 
 }  // namespace moba
