@@ -110,81 +110,93 @@ cudaError_t launch_scatter(const Params& p, const int32_t* cu, const int32_t* se
 }
 
 // ---------------------------------------------------------------------------
-// merge: one warp per (token, head) row.
+// merge: D / 8 lanes (rounded up to a power of two) per (token, head) row, so a warp combines one row
+// at head dim 256, two at 128 and 96, four at 64.
 //   lse_tot = log sum_j exp(lse_j);  out = sum_j O_j * exp(lse_j - lse_tot)
 // (exponentials through ex2.approx: relative error 2^-22, far below the rounding of the output)
+// Bound by HBM by bytes, in practice by issue slots: a whole warp per row spent as many instructions on
+// reducing a handful of LSEs and adding its groups' sums as on the partial rows.  Measured against
+// that: 13311 tokens x 16 heads, head_dim 64, 8 partials 98 -> 60 us; 32768 x 32, head_dim 128 500 -> 417 us;
+// 19456 x 32, 3 partials 277 -> 224 us.
 // ---------------------------------------------------------------------------
 constexpr int kMergeThreads = 256;
 
-// A partial row is D/8 pieces of eight fp16 values (16 bytes), one per lane: 32 / (D/8) rows fit
-// one load instruction of the warp (2 at head dim 128 and 96, 4 at 64, 1 at 256), so the lanes form
-// that many groups, group g takes the partials g, g + groups, ... of the row, four of them in
-// flight at a time, and the groups' sums are added at the end.
+// A partial row is D/8 pieces of eight fp16 values (16 bytes), one per lane of the row's lanes, which
+// take the partials of the row in turn, kMergeAhead of them in flight.  No sum crosses the
+// lanes but the two reductions over the LSEs.
+// Two or more rows a warp: eight loads in flight at three CTAs per SM (80 registers); one row a warp: four at four.
+template <int D> constexpr int kMergeAhead = D == 256 ? 4 : 8;
+template <int D> constexpr int kMergeCtas = D == 256 ? 4 : 3;
+template <int D> constexpr int kMergeLanes = D <= 64 ? 8 : D <= 128 ? 16 : 32;
 template <bool kHalf, int D>
-// five CTAs per SM (at most 51 registers): more warps to wait for partial rows; six would spill
-__global__ void __launch_bounds__(kMergeThreads, 5)
+__global__ void __launch_bounds__(kMergeThreads, kMergeCtas<D>)
 merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __restrict__ partial_lse,
              const int32_t* __restrict__ status, __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out) {
   pdl_wait();
   pdl_trigger();
-  constexpr int kLanes = D / 8;                  // lanes per partial row
-  constexpr int kGroups = 32 / kLanes;
-  constexpr int kAhead = 4;                      // partial rows a group has in flight
+  constexpr int kW = kMergeLanes<D>;             // lanes per row
+  constexpr int kAhead = kMergeAhead<D>;
+  constexpr int kPieces = D / 8;                 // of which this many hold data (head dim 96: 12 of 16)
+  constexpr int kRowsPerBlock = kMergeThreads / kW;
   const int lane = threadIdx.x & 31;
-  const int grp = lane / kLanes, piece = lane - grp * kLanes;
-  const bool active = grp < kGroups;             // head dim 96: lanes 24-31 idle
+  const int sub = lane & (kW - 1);
+  const unsigned base_lane = lane & ~(kW - 1);
   // a dense stage that gave up on a wait leaves a non-zero status: poison the result
   const bool failed = status != nullptr && *status != 0;
-  const int64_t warps = (int64_t)gridDim.x * (kMergeThreads / 32);
-  // Up to 32 partials per row (top-k up to 32): lane j holds {lse, 1 / scale} of partial j, and the
-  // pair of the warp's next row is requested before this row is worked on, so that a row starts
-  // with its partial rows as the only loads it has to wait for.
-  const bool in_regs = p.NP <= 32;
-  const int64_t row0 = (int64_t)blockIdx.x * (kMergeThreads / 32) + (threadIdx.x >> 5);
-  float2 mine = make_float2(-INFINITY, 0.f);
-  if (in_regs && row0 < p.rows && lane < p.NP) mine = __ldg(partial_lse + row0 * p.NP + lane);
-  for (int64_t row = row0; row < p.rows; row += warps) {
+  const int64_t stride = (int64_t)gridDim.x * kRowsPerBlock;
+  // Up to 2 kW partials per row: lane j holds {lse, 1 / scale} of the partials j and j + kW, and the pairs
+  // of the next row are requested before this row is worked on, so that a row starts with its
+  // partial rows as the only loads it has to wait for.
+  const bool in_regs = p.NP <= 2 * kW;
+  int64_t row = (int64_t)blockIdx.x * kRowsPerBlock + threadIdx.x / kW;
+  const float2 none = make_float2(-INFINITY, 0.f);
+  float2 next0 = none, next1 = none;
+  auto fetch = [&](int64_t r) {
+    next0 = none;
+    next1 = none;
+    if (in_regs && r < p.rows) {
+      if (sub < p.NP) next0 = __ldg(partial_lse + r * p.NP + sub);
+      if (sub + kW < p.NP) next1 = __ldg(partial_lse + r * p.NP + sub + kW);
+    }
+  };
+  fetch(row);
+  // the rows of a warp end together: a row past the end is worked on without loads or stores
+  for (int64_t row0 = row - threadIdx.x / kW + (threadIdx.x >> 5) * (32 / kW); row0 < p.rows; row0 += stride, row += stride) {
+    const bool real = row < p.rows;
     const float2* lse = partial_lse + row * p.NP;
-    const float2 cur = mine;
-    if (in_regs && row + warps < p.rows && lane < p.NP) mine = __ldg(partial_lse + (row + warps) * p.NP + lane);
-    float mx = -INFINITY;
-    if (in_regs) mx = cur.x;
-    else for (int j = lane; j < p.NP; j += 32) mx = fmaxf(mx, lse[j].x);
+    const float2 cur0 = next0, cur1 = next1;
+    fetch(row + stride);
+    float mx = fmaxf(cur0.x, cur1.x);
+    if (!in_regs && real) for (int j = sub; j < p.NP; j += kW) mx = fmaxf(mx, lse[j].x);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    float tot = 0.f;
-    if (in_regs) tot = __expf(cur.x - mx);                    // 0 for lanes past the partials (lse -inf)
-    else for (int j = lane; j < p.NP; j += 32) tot += __expf(lse[j].x - mx);
-    const float wlane = tot * cur.y;                          // in_regs: weight of partial `lane` up to 1 / sum
+    for (int o = kW / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float e0 = __expf(cur0.x - mx), e1 = __expf(cur1.x - mx);      // 0 past the partials (lse -inf)
+    float tot = e0 + e1;
+    if (!in_regs && real) { tot = 0.f; for (int j = sub; j < p.NP; j += kW) tot += __expf(lse[j].x - mx); }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    for (int o = kW / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
     const float inv = failed ? __int_as_float(0x7fc00000) : 1.f / tot;
-    float acc[8];
+    // weights of this lane's partials; the row's power-of-two scale is undone with them
+    const float w0 = e0 * cur0.y * inv, w1 = e1 * cur1.y * inv;
+    float2 acc[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    const uint4* src = reinterpret_cast<const uint4*>(partial_out + row * p.NP * D) + piece;
-    for (int j0 = 0; j0 < p.NP; j0 += kGroups * kAhead) {
+    for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
+    const uint4* src = reinterpret_cast<const uint4*>(partial_out + row * p.NP * D) + sub;
+    for (int j0 = 0; j0 < p.NP; j0 += kAhead) {
       float w[kAhead];
       uint4 o[kAhead];
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
-        const int j = j0 + u * kGroups + grp;
-        w[u] = 0.f;
+        const int j = j0 + u;
         o[u] = make_uint4(0u, 0u, 0u, 0u);
-        // the row's power-of-two scale is undone with the weight
-        const float wj = __shfl_sync(0xffffffffu, wlane, j & 31) * inv;
         if (in_regs) {
-          if (active && j < p.NP && wj != 0.f) {
-            w[u] = wj;
-            o[u] = __ldg(src + j * kLanes);
-          }
-        } else if (active && j < p.NP) {
-          const float2 lj = lse[j];
-          if (lj.x != -INFINITY) {
-            w[u] = __expf(lj.x - mx) * inv * lj.y;
-            o[u] = __ldg(src + j * kLanes);
-          }
+          w[u] = __shfl_sync(0xffffffffu, j < kW ? w0 : w1, base_lane + (j & (kW - 1)));
+        } else {
+          const float2 lj = real && j < p.NP ? __ldg(lse + j) : none;
+          w[u] = lj.x != -INFINITY ? __expf(lj.x - mx) * inv * lj.y : 0.f;
         }
+        // (a weight of NaN marks a failed dense stage: it must reach the sum, but the row is not read)
+        if (real && j < p.NP && sub < kPieces && w[u] != 0.f && !failed) o[u] = __ldg(src + j * kPieces);
       }
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
@@ -192,34 +204,29 @@ merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __r
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&words[i]));
-          acc[2 * i] += w[u] * a.x;
-          acc[2 * i + 1] += w[u] * a.y;
+          acc[i].x += w[u] * a.x;
+          acc[i].y += w[u] * a.y;
         }
       }
     }
-    // sum of the groups into group 0
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      if (kGroups == 4) acc[i] += __shfl_down_sync(0xffffffffu, acc[i], 2 * kLanes);
-      if (kGroups >= 2) acc[i] += __shfl_down_sync(0xffffffffu, acc[i], kLanes);
-    }
     const int64_t t = row / p.Hq;
     const int h = (int)(row - t * p.Hq);
-    if (grp == 0) {
+    if (real && sub < kPieces) {
       uint4 pk;
-      pk.x = pack2_16<kHalf>(acc[0], acc[1]);
-      pk.y = pack2_16<kHalf>(acc[2], acc[3]);
-      pk.z = pack2_16<kHalf>(acc[4], acc[5]);
-      pk.w = pack2_16<kHalf>(acc[6], acc[7]);
-      *reinterpret_cast<uint4*>(out + t * p.so_t + (int64_t)h * p.so_h + piece * 8) = pk;
+      pk.x = pack2_16<kHalf>(acc[0].x, acc[0].y);
+      pk.y = pack2_16<kHalf>(acc[1].x, acc[1].y);
+      pk.z = pack2_16<kHalf>(acc[2].x, acc[2].y);
+      pk.w = pack2_16<kHalf>(acc[3].x, acc[3].y);
+      *reinterpret_cast<uint4*>(out + t * p.so_t + (int64_t)h * p.so_h + sub * 8) = pk;
     }
-    if (lse_out != nullptr && lane == 0) lse_out[(int64_t)h * p.Tq + t] = logf(tot) + mx;
+    if (real && lse_out != nullptr && sub == 0) lse_out[(int64_t)h * p.Tq + t] = logf(tot) + mx;
   }
 }
 
 cudaError_t launch_merge(const Params& p, const __half* partial_out, const float2* partial_lse,
                          const int32_t* status, __nv_bfloat16* out, float* lse_out, cudaStream_t st) {
-  int64_t blocks = (p.rows + (kMergeThreads / 32) - 1) / (kMergeThreads / 32);
+  const int rows_per_block = kMergeThreads / (p.D <= 64 ? 8 : p.D <= 128 ? 16 : 32);
+  int64_t blocks = (p.rows + rows_per_block - 1) / rows_per_block;
   if (blocks > 148 * 64) blocks = 148 * 64;
 #define MOBA_MERGE(HALF, DIM) \
   return launch_pdl(merge_kernel<HALF, DIM>, dim3((unsigned)blocks), kMergeThreads, 0, st, p, partial_out, partial_lse, \
