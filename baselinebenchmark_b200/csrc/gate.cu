@@ -50,43 +50,47 @@ cudaError_t launch_chunk_metadata(const Params& p, const int32_t* cu, int32_t* c
 }
 
 // ---------------------------------------------------------------------------
-// chunk means: one CTA per (slot, kv head), 32 row lanes x D/8 dim lanes
-// (16-byte loads).
+// chunk means: one CTA per (slot, kv head), 32 row lanes x D/8 dim lanes (16-byte loads), or, when
+// that leaves the chip mostly idle (few long chunks, or the one chunk a decode step completes), one
+// CTA per 32 dims of it with four times the rows in flight.  A row lane adds its C / 32 rows
+// one after the other (the order is the contract's), so what a long chunk waits for is the latency of that
+// chain: kAhead rows of it are in flight.  Measured: one 4096-key chunk x 8 heads of a decode step 50 -> 20 us; the
+// seven of a 32768-token sequence 58 -> 54 us, where 56 CTAs were enough to half fill HBM.
 // ---------------------------------------------------------------------------
-template <bool kHalf, int D>
-__global__ void __launch_bounds__(kMeanLanes * (D / 8))
+template <bool kHalf, int D, int kDims, int kAhead>
+__global__ void __launch_bounds__(kMeanLanes * (kDims / 8))
 chunk_mean_kernel(Params p, int slot_begin, const __nv_bfloat16* __restrict__ k, const int32_t* __restrict__ cu,
                   __nv_bfloat16* __restrict__ means, int32_t* __restrict__ zero, int64_t zero_words) {
   pdl_wait();
   pdl_trigger();
   // the counters that the kernels behind this one add to
-  for (int64_t i = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < zero_words;
-       i += (int64_t)gridDim.x * gridDim.y * blockDim.x)
+  for (int64_t i = (((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+       i < zero_words; i += (int64_t)gridDim.x * gridDim.y * gridDim.z * blockDim.x)
     zero[i] = 0;
-  const int slot = slot_begin + blockIdx.x, hk = blockIdx.y;
+  const int slot = slot_begin + blockIdx.x, hk = blockIdx.y, dim0 = blockIdx.z * kDims;
   const int b = slot / p.mc, j = slot - b * p.mc;
   const Slot sl = slot_of(cu, b, j, p.C);
-  constexpr int kDimLanes = D / 8;
-  const int dl = threadIdx.x % kDimLanes;  // dims 8*dl .. 8*dl+7
+  constexpr int kDimLanes = kDims / 8;
+  const int dl = threadIdx.x % kDimLanes;  // dims dim0 + 8*dl .. + 7
   const int rl = threadIdx.x / kDimLanes;  // row lane 0..31
-  __nv_bfloat16* dst = means + ((int64_t)slot * p.Hkv + hk) * D;
+  __nv_bfloat16* dst = means + ((int64_t)slot * p.Hkv + hk) * D + dim0;
 
-  __shared__ float part[kMeanLanes][D + 4];
+  __shared__ float part[kMeanLanes][kDims + 4];
   float acc[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
 
   if (sl.historical) {                     // historical chunks are always full: C rows
-    const __nv_bfloat16* base = k + (int64_t)sl.start * p.sk_t + (int64_t)hk * p.sk_h + dl * 8;
+    const __nv_bfloat16* base = k + (int64_t)sl.start * p.sk_t + (int64_t)hk * p.sk_h + dim0 + dl * 8;
     int r = rl;
-    // four rows in flight per thread, accumulated in increasing r
-    for (; r + 3 * kMeanLanes < p.C; r += 4 * kMeanLanes) {
-      uint4 x[4];
+    // kAhead rows in flight per thread, accumulated in increasing r
+    for (; r + (kAhead - 1) * kMeanLanes < p.C; r += kAhead * kMeanLanes) {
+      uint4 x[kAhead];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
+      for (int u = 0; u < kAhead; ++u)
         x[u] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)(r + u * kMeanLanes) * p.sk_t));
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+      for (int u = 0; u < kAhead; ++u) {
         float f[8];
         unpack8<kHalf>(x[u], f);
 #pragma unroll
@@ -104,7 +108,7 @@ chunk_mean_kernel(Params p, int slot_begin, const __nv_bfloat16* __restrict__ k,
 #pragma unroll
   for (int i = 0; i < 8; ++i) part[rl][dl * 8 + i] = acc[i];
   __syncthreads();
-  if (threadIdx.x < D) {
+  if (threadIdx.x < kDims) {
     float tot = part[0][threadIdx.x];
 #pragma unroll
     for (int a = 1; a < kMeanLanes; ++a) tot += part[a][threadIdx.x];
@@ -120,10 +124,15 @@ cudaError_t launch_chunk_means_range(const Params& p, int slot_begin, int slot_e
                                      int64_t zero_words) {
   if (slot_end <= slot_begin)
     return zero_words > 0 ? cudaMemsetAsync(zero, 0, (size_t)zero_words * sizeof(int32_t), st) : cudaSuccess;
-  dim3 grid(slot_end - slot_begin, p.Hkv);
-#define MOBA_MEANS(HALF, DIM) \
-  return launch_pdl(chunk_mean_kernel<HALF, DIM>, grid, kMeanLanes * (DIM / 8), 0, st, p, slot_begin, k, cu, means, zero, \
-                    zero_words)
+  // Split over the dims when the (slot, head) pairs alone give the SMs fewer than two CTAs each and the
+  // chunk is long enough for several batches of rows.
+  const int64_t pairs = (int64_t)(slot_end - slot_begin) * p.Hkv;
+  const bool split = pairs < 2 * 148 && p.C >= 8 * kMeanLanes;
+#define MOBA_MEANS(HALF, DIM)                                                                                          \
+  return split ? launch_pdl(chunk_mean_kernel<HALF, DIM, 32, 16>, dim3(slot_end - slot_begin, p.Hkv, DIM / 32),        \
+                            kMeanLanes * 4, 0, st, p, slot_begin, k, cu, means, zero, zero_words)                      \
+               : launch_pdl(chunk_mean_kernel<HALF, DIM, DIM, 4>, dim3(slot_end - slot_begin, p.Hkv, 1),               \
+                            kMeanLanes * (DIM / 8), 0, st, p, slot_begin, k, cu, means, zero, zero_words)
   switch (p.D) {
     case 64:  if (p.fp16) MOBA_MEANS(true, 64);  else MOBA_MEANS(false, 64);
     case 96:  if (p.fp16) MOBA_MEANS(true, 96);  else MOBA_MEANS(false, 96);
