@@ -27,11 +27,13 @@
 // No atomics: a key's gradient is written once.  The order of the rows of a routed list is
 // the compaction's (unspecified), so dK and dV vary in their last bits from run to run.
 //
-// Warp roles (384 threads): warp 0 lane 0 loads K/V by TMA, warp 1 issues the MMAs and owns
+// Warp roles (512 threads): warp 0 lane 0 loads K/V by TMA, warp 1 issues the MMAs and owns
 // the TMEM allocation, warps 2-3 describe the rows of the coming steps (LSE, delta, token), warps
 // 4-7 handle the even steps (S buffer 0) and write dK, warps 8-11 the odd steps (S buffer 1) and
-// write dV; after a step the group brings in the Q / dO rows of the step three ahead (one thread
-// requests the boxes, or all 128 gather).
+// write dV, warps 12-15 bring in the Q / dO rows of the steps as far ahead as stages are free (one
+// thread requests the boxes, or all 128 gather).  The copies used to be made by warps 4-11 between their
+// steps: 1010 of the 2300 cycles of a step, now off its path (kernel on 19456 tokens x 32 heads,
+// chunk 512: 1214 -> 989 us; 8191 tokens x 16/4 heads, chunk 128: 220 -> 193 us).
 // TMEM columns: buffer X: S^T 128X..+63 (P^T, 16-bit, over the first 32), dP^T 128X+64..+127
 // (dS^T over its first 32); dK 256.., dV 384...
 // Every wait is bounded; a wait that gives up sets a status word, the CTAs stop drawing units
@@ -50,13 +52,14 @@ namespace {
 
 using namespace ptx;
 
-constexpr int kThreads = 384;
+constexpr int kThreads = 512;
 constexpr int kKeys = 128;                    // keys per unit
 constexpr int kStep = 64;                     // rows per step
 constexpr int kStages = 4;
 // Chunks of at least this many 128-key tiles have their routed rows packed.  Measured backward of
 // 32768 tokens x 32/8 heads, packed against gathered: 4 tiles 21.7 / 20.1 ms, 8 tiles 17.0 / 17.2,
-// 16 tiles 26.1 / 27.3, 32 tiles (config 2) 33.5 / 35.8.
+// 16 tiles 26.1 / 27.3, 32 tiles (config 2) 33.5 / 35.8; with the rows gathered by warps of their own
+// 32 tiles 31.1 / 32.1, 4 tiles the same within 0.1 %.
 constexpr int kPackMinTiles = 8;
 constexpr int kKvBlockBytes = kKeys * 64 * 2; // [128 keys][64 dims]
 constexpr int kKvTileBytes = 2 * kKvBlockBytes;
@@ -123,7 +126,6 @@ __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, bool pr
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
   asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
@@ -165,19 +167,19 @@ constexpr int kPolyPairs = MOBA_BWD_POLY_PAIRS;
 template <bool kMasked, bool kHalf>
 __device__ __forceinline__ void ps_row(uint32_t tS, const float2* meta, const int32_t* tok, int key_tok, bool key_ok,
                                        float sl2) {
-  uint32_t s[64], g[64];
-  tmem_ld64(tS, s);
-  tmem_ld64(tS + 64, g);
-  tmem_wait_ld();
+  // 32 rows at a time: with sixteen warps a thread has 128 registers
   const uint64_t scale2 = pack2(sl2, sl2);
 #pragma unroll
   for (int ch = 0; ch < 2; ++ch) {
-    uint32_t pp[16], pd[16];
+    uint32_t s[32], g[32], pp[16], pd[16];
+    tmem_ld32(tS + ch * 32, s);
+    tmem_ld32(tS + 64 + ch * 32, g);
+    tmem_wait_ld();
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const int e = ch * 32 + 2 * i;
       const float4 m = *reinterpret_cast<const float4*>(meta + e);      // {-lse2, delta} of rows e, e + 1
-      uint64_t x = fma2(pack2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), scale2,
+      uint64_t x = fma2(pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), scale2,
                         pack2(m.x, m.z) ^ 0x8000000080000000ull);
       uint64_t pr;
       if (kMasked) {
@@ -189,7 +191,7 @@ __device__ __forceinline__ void ps_row(uint32_t tS, const float2* meta, const in
       } else {
         pr = pack2(ex2_approx(lo2(x)), ex2_approx(hi2(x)));
       }
-      const uint64_t d = mul2(pr, sub2(pack2(__uint_as_float(g[e]), __uint_as_float(g[e + 1])), pack2(m.y, m.w)));
+      const uint64_t d = mul2(pr, sub2(pack2(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1])), pack2(m.y, m.w)));
       pp[i] = key_ok ? pack2_16<kHalf>(lo2(pr), hi2(pr)) : 0u;
       pd[i] = key_ok ? pack2_16<kHalf>(lo2(d), hi2(d)) : 0u;
     }
@@ -315,7 +317,6 @@ bwd_dkdv_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
   const float sl2 = scale * 1.4426950408889634f;
   TR_T0(t_kernel);
   if (warp < 4) {
-    setmaxnreg_dec<72>();
     uint32_t g0 = 0;                       // steps of the units this CTA has finished
     uint32_t nu = 0;                       // units this CTA has finished
     Unit u;
@@ -453,8 +454,7 @@ bwd_dkdv_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
       g0 += (uint32_t)u.steps;
       ++nu;
     }
-  } else {
-    setmaxnreg_inc<216>();
+  } else if (warp < 12) {
     uint32_t g0 = 0, nu = 0;
     Unit u;
     while (next_unit(p, a, c, key_tiles, n_units, u)) {
@@ -466,11 +466,71 @@ bwd_dkdv_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
       const bool key_ok = key < u.nkeys;
       const int key_tok = u.key0 + key;
       bool ok = true;
-      // The Q and dO rows of step j: 64-row boxes requested by one thread of the group.  It first
-      // waits for the step's description, which the describing warps only write once the stage
-      // is free again.
+      const int first = ((g0 & 1) == (uint32_t)x) ? 0 : 1;
+      for (int i = first; ok && i < u.steps; i += 2) {
+        const uint32_t gi = g0 + i, st = gi & 3;
+        TR_T0(t_s);
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.row_full[st]), (gi >> 2) & 1));   // row data of the stage
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.s_full[x]), (gi >> 1) & 1));
+        if (!ok) break;
+        if (threadIdx.x == 128) TR_ADD(a, 2, t_s);
+        TR_T0(t_x);
+        tc_fence_after();
+        bool masked = false;
+        if (i >= u.routed_steps) {
+          const int o = i - u.routed_steps;
+          const int ot = o - (o / u.own_steps) * u.own_steps;
+          masked = ot * kStep < kKeys - 1;                 // rows whose token lies inside the key tile
+        }
+        if (masked) ps_row<true, kHalf>(tS, c.meta[st], c.tok[st], key_tok, key_ok, sl2);
+        else ps_row<false, kHalf>(tS, c.meta[st], c.tok[st], key_tok, key_ok, sl2);
+        tc_fence_before();
+        mbar_arrive(smem_u32(&c.p_full[x]));
+        if (threadIdx.x == 128) TR_ADD(a, 3, t_x);
+      }
+      TR_T0(t_a);
+      if (ok) ok = mbar_wait(smem_u32(&c.acc_full), nu & 1);
+      ok = __all_sync(0xffffffffu, ok);
+      if (ok) {
+        tc_fence_after();
+        // warps 4-7 write dK (scaled), warps 8-11 dV: a thread owns the D values of its key
+        const uint32_t tA = tmem + lane_base + 256 + x * 128;
+        const float f = x == 0 ? scale : 1.f;
+        __nv_bfloat16* dst = (x == 0 ? a.dk : a.dv) + ((int64_t)key_tok * p.Hkv + u.kvh) * D;
+        uint32_t v[32];
+#pragma unroll
+        for (int ch = 0; ch < D / 32; ++ch) {
+          tmem_ld32(tA + ch * 32, v);
+          tmem_wait_ld();
+          if (key_ok) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint4 o;
+              o.x = pack2_16<kHalf>(__uint_as_float(v[8 * i]) * f, __uint_as_float(v[8 * i + 1]) * f);
+              o.y = pack2_16<kHalf>(__uint_as_float(v[8 * i + 2]) * f, __uint_as_float(v[8 * i + 3]) * f);
+              o.z = pack2_16<kHalf>(__uint_as_float(v[8 * i + 4]) * f, __uint_as_float(v[8 * i + 5]) * f);
+              o.w = pack2_16<kHalf>(__uint_as_float(v[8 * i + 6]) * f, __uint_as_float(v[8 * i + 7]) * f);
+              *reinterpret_cast<uint4*>(dst + ch * 32 + i * 8) = o;
+            }
+          }
+        }
+        tc_fence_before();
+        if (threadIdx.x == 128) TR_ADD(a, 8, t_a);
+      } else {
+        atomicExch(a.status, ST_ROWS);
+        c.abort = 1;
+      }
+      g0 += (uint32_t)u.steps;
+      ++nu;
+    }
+  } else {
+    // ------------------------------------------------ warps 12-15: bring in the rows, as far ahead as stages are free
+    uint32_t g0 = 0;
+    Unit u;
+    while (next_unit(p, a, c, key_tiles, n_units, u)) {
+      // The Q and dO rows of step j.  The group first waits for the step's description, which the
+      // describing warps only write once the stage is free again.
       auto copy_rows = [&](int j) -> bool {
-        if (j >= u.steps) return true;
         const uint32_t gj = g0 + j, sj = gj & 3;
         if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&c.meta_full[sj]), (gj >> 2) & 1))) return false;
         if (!a.packed && j < u.routed_steps) {
@@ -517,72 +577,12 @@ bwd_dkdv_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
         }
         return true;
       };
-      const int first = ((g0 & 1) == (uint32_t)x) ? 0 : 1;
-      {
-        TR_T0(t_w);
-        ok = copy_rows(first);                     // steps 0, 1, 2 before the loop: 0 and 2 by the group of step 0
-        if (ok && first == 0) ok = copy_rows(2);
-        if (threadIdx.x == 128) TR_ADD(a, 10, t_w);
-      }
-      for (int i = first; ok && i < u.steps; i += 2) {
-        const uint32_t gi = g0 + i, st = gi & 3;
-        TR_T0(t_s);
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.row_full[st]), (gi >> 2) & 1));   // row data of the stage
-        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.s_full[x]), (gi >> 1) & 1));
-        if (!ok) break;
-        if (threadIdx.x == 128) TR_ADD(a, 2, t_s);
-        TR_T0(t_x);
-        tc_fence_after();
-        bool masked = false;
-        if (i >= u.routed_steps) {
-          const int o = i - u.routed_steps;
-          const int ot = o - (o / u.own_steps) * u.own_steps;
-          masked = ot * kStep < kKeys - 1;                 // rows whose token lies inside the key tile
-        }
-        if (masked) ps_row<true, kHalf>(tS, c.meta[st], c.tok[st], key_tok, key_ok, sl2);
-        else ps_row<false, kHalf>(tS, c.meta[st], c.tok[st], key_tok, key_ok, sl2);
-        tc_fence_before();
-        mbar_arrive(smem_u32(&c.p_full[x]));
-        if (threadIdx.x == 128) TR_ADD(a, 3, t_x);
-        TR_T0(t_w);
-        ok = copy_rows(i + 3);
-        if (threadIdx.x == 128) TR_ADD(a, 10, t_w);
-      }
-      cp_async_wait_all();
-      TR_T0(t_a);
-      if (ok) ok = mbar_wait(smem_u32(&c.acc_full), nu & 1);
-      ok = __all_sync(0xffffffffu, ok);
-      if (ok) {
-        tc_fence_after();
-        // warps 4-7 write dK (scaled), warps 8-11 dV: a thread owns the D values of its key
-        const uint32_t tA = tmem + lane_base + 256 + x * 128;
-        const float f = x == 0 ? scale : 1.f;
-        __nv_bfloat16* dst = (x == 0 ? a.dk : a.dv) + ((int64_t)key_tok * p.Hkv + u.kvh) * D;
-        uint32_t v[32];
-#pragma unroll
-        for (int ch = 0; ch < D / 32; ++ch) {
-          tmem_ld32(tA + ch * 32, v);
-          tmem_wait_ld();
-          if (key_ok) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint4 o;
-              o.x = pack2_16<kHalf>(__uint_as_float(v[8 * i]) * f, __uint_as_float(v[8 * i + 1]) * f);
-              o.y = pack2_16<kHalf>(__uint_as_float(v[8 * i + 2]) * f, __uint_as_float(v[8 * i + 3]) * f);
-              o.z = pack2_16<kHalf>(__uint_as_float(v[8 * i + 4]) * f, __uint_as_float(v[8 * i + 5]) * f);
-              o.w = pack2_16<kHalf>(__uint_as_float(v[8 * i + 6]) * f, __uint_as_float(v[8 * i + 7]) * f);
-              *reinterpret_cast<uint4*>(dst + ch * 32 + i * 8) = o;
-            }
-          }
-        }
-        tc_fence_before();
-        if (threadIdx.x == 128) TR_ADD(a, 8, t_a);
-      } else {
-        atomicExch(a.status, ST_ROWS);
-        c.abort = 1;
-      }
+      bool ok = true;
+      TR_T0(t_w);
+      for (int i = 0; ok && i < u.steps; ++i) ok = copy_rows(i);
+      if (threadIdx.x == 384) TR_ADD(a, 10, t_w);
+      if (!ok && lane == 0) { atomicExch(a.status, ST_GATHER); c.abort = 1; }
       g0 += (uint32_t)u.steps;
-      ++nu;
     }
   }
 
