@@ -19,7 +19,7 @@ ATTEND_MMA_SYNC = 1
 #: every symbol include/moba_b200.h declares
 SYMBOLS = (
     "moba_b200_abi_version", "moba_b200_strerror", "moba_problem_check", "moba_problem_dims",
-    "moba_workspace_size", "moba_workspace_size_min", "moba_forward", "moba_forward_events", "moba_forward_cached", "moba_workspace_size_host", "moba_forward_host",
+    "moba_workspace_size", "moba_workspace_size_min", "moba_forward", "moba_forward_events", "moba_forward_cached", "moba_append", "moba_workspace_size_host", "moba_forward_host",
     "moba_chunk_metadata", "moba_chunk_means", "moba_gate_topk", "moba_gate_topk_stats", "moba_compact_routes",
     "moba_attend", "moba_merge", "moba_attend_tile_rows", "moba_attend_tile_rows_for", "moba_problem_tile_rows", "moba_route_static",
     "moba_backward_workspace_size", "moba_backward",
@@ -80,6 +80,8 @@ def lib() -> C.CDLL:
         handle.moba_forward.argtypes = [pp, vp, vp, vp, i32p, vp, vp, i32p, vp, sz, vp]
         handle.moba_forward_events.argtypes = [pp, vp, vp, vp, i32p, vp, vp, i32p, vp, sz, vp, C.POINTER(C.c_void_p)]
         handle.moba_forward_cached.argtypes = [pp, vp, vp, vp, i32p, vp, vp, i32p, vp, C.c_int32, vp, sz, vp]
+        handle.moba_append.argtypes = [pp, vp, vp, vp, C.c_int64, C.c_int64, C.c_int64, C.c_int64, vp, vp, i32p, vp, i32p, vp,
+                                       C.c_int32, vp, sz, vp]
         handle.moba_forward_host.argtypes = [pp, vp, vp, vp, i32p, vp, vp, i32p, vp, sz, vp]
         handle.moba_chunk_metadata.argtypes = [pp, i32p, i32p, i32p, vp, vp]
         handle.moba_chunk_means.argtypes = [pp, vp, i32p, vp, vp]

@@ -492,6 +492,35 @@ int moba_forward_cached(const moba_problem_t* p, const void* q, const void* k, c
                       true, opt);
 }
 
+int moba_append(const moba_problem_t* p, const void* q, const void* k_new, const void* v_new, int64_t kn_t, int64_t kn_h,
+                int64_t vn_t, int64_t vn_h, void* k_cache, void* v_cache, int32_t* cu, void* out, int32_t* selected_out,
+                void* means_cache, int32_t cached_slots, void* workspace, size_t workspace_bytes, void* stream) {
+  const int rc = check_problem(p);
+  if (rc != MOBA_OK) return rc;
+  if (!k_new || !v_new || !k_cache || !v_cache || !cu) return MOBA_E_NULL;
+  if (p->batch != 1 || p->q_tokens <= 0 || p->q_token_begin + p->q_tokens != p->total_tokens) return MOBA_E_SHAPE;
+  const int64_t strides[4] = {kn_t, kn_h, vn_t, vn_h};
+  for (int i = 0; i < 4; ++i) {
+    if (strides[i] < 0) return MOBA_E_SHAPE;
+    if (strides[i] % 8 != 0) return MOBA_E_ALIGN;
+  }
+  if (((uintptr_t)k_new | (uintptr_t)v_new | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) return MOBA_E_ALIGN;
+  // everything moba_forward_cached refuses is refused before the caches are touched
+  const Params r = make_params(p);
+  if (!q || !out || !means_cache) return MOBA_E_NULL;
+  if (((uintptr_t)q | (uintptr_t)out | (uintptr_t)means_cache | (uintptr_t)workspace) & 15) return MOBA_E_ALIGN;
+  if (cached_slots < 0 || cached_slots > r.slots) return MOBA_E_SHAPE;
+  if (r.rows * (int64_t)r.NP >= ((int64_t)1 << 31)) return MOBA_E_UNSUPPORTED;
+  if (workspace == nullptr || workspace_bytes < pass_bytes(p, r.Hkv)) return MOBA_E_WORKSPACE;
+  const cudaError_t e = launch_append_rows(r, static_cast<const __nv_bfloat16*>(k_new),
+                                           static_cast<const __nv_bfloat16*>(v_new), kn_t, kn_h, vn_t, vn_h,
+                                           static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), cu,
+                                           (cudaStream_t)stream);
+  if (e != cudaSuccess) return (int)e;
+  return moba_forward_cached(p, q, k_cache, v_cache, cu, out, nullptr, selected_out, means_cache, cached_slots, workspace,
+                             workspace_bytes, stream);
+}
+
 // ---------------------------------------------------------------------------
 // training path: backward of the operator
 // ---------------------------------------------------------------------------

@@ -304,6 +304,10 @@ __device__ __forceinline__ void scan_lists(const ListScan& a, int* scratch) {
 // ---- launchers implemented in the kernel files -----------------------------
 cudaError_t launch_chunk_metadata(const Params& p, const int32_t* cu, int32_t* cu_chunk,
                                   int32_t* chunk_end, int8_t* valid, cudaStream_t st);
+// K and V rows of the query window into the caches (strides of `p`), and cu_seqlens = {0, T}
+cudaError_t launch_append_rows(const Params& p, const __nv_bfloat16* k_new, const __nv_bfloat16* v_new, int64_t kn_t,
+                               int64_t kn_h, int64_t vn_t, int64_t vn_h, __nv_bfloat16* k, __nv_bfloat16* v,
+                               int32_t* cu, cudaStream_t st);
 cudaError_t launch_chunk_means(const Params& p, const __nv_bfloat16* k, const int32_t* cu,
                                __nv_bfloat16* means, cudaStream_t st);
 cudaError_t launch_chunk_means_range(const Params& p, int slot_begin, int slot_end, const __nv_bfloat16* k,

@@ -17,6 +17,41 @@
 namespace moba {
 
 // ---------------------------------------------------------------------------
+// rows of an append: a 16-byte piece of K and of V per thread
+// ---------------------------------------------------------------------------
+constexpr int kAppendThreads = 256;
+
+__global__ void __launch_bounds__(kAppendThreads)
+append_rows_kernel(Params p, const __nv_bfloat16* __restrict__ k_new, const __nv_bfloat16* __restrict__ v_new,
+                   int64_t kn_t, int64_t kn_h, int64_t vn_t, int64_t vn_h, __nv_bfloat16* __restrict__ k,
+                   __nv_bfloat16* __restrict__ v, int32_t* __restrict__ cu) {
+  pdl_wait();
+  pdl_trigger();
+  if (blockIdx.x == 0 && threadIdx.x == 0) { cu[0] = 0; cu[1] = (int32_t)p.T; }
+  const int pieces = p.D / 8;
+  const int64_t total = p.Tq * p.Hkv * pieces;
+  for (int64_t i = (int64_t)blockIdx.x * kAppendThreads + threadIdx.x; i < total; i += (int64_t)gridDim.x * kAppendThreads) {
+    const int64_t r = i / pieces;
+    const int c = (int)(i - r * pieces) * 8;
+    const int64_t t = r / p.Hkv;
+    const int64_t h = r - t * p.Hkv;
+    const uint4 a = __ldg(reinterpret_cast<const uint4*>(k_new + t * kn_t + h * kn_h + c));
+    const uint4 b = __ldg(reinterpret_cast<const uint4*>(v_new + t * vn_t + h * vn_h + c));
+    *reinterpret_cast<uint4*>(k + (p.win_lo + t) * p.sk_t + h * p.sk_h + c) = a;
+    *reinterpret_cast<uint4*>(v + (p.win_lo + t) * p.sv_t + h * p.sv_h + c) = b;
+  }
+}
+
+cudaError_t launch_append_rows(const Params& p, const __nv_bfloat16* k_new, const __nv_bfloat16* v_new, int64_t kn_t,
+                               int64_t kn_h, int64_t vn_t, int64_t vn_h, __nv_bfloat16* k, __nv_bfloat16* v,
+                               int32_t* cu, cudaStream_t st) {
+  int64_t blocks = (p.Tq * p.Hkv * (p.D / 8) + kAppendThreads - 1) / kAppendThreads;
+  if (blocks > 148 * 16) blocks = 148 * 16;
+  return launch_pdl(append_rows_kernel, dim3((unsigned)blocks), kAppendThreads, 0, st, p, k_new, v_new, kn_t, kn_h, vn_t,
+                    vn_h, k, v, cu);
+}
+
+// ---------------------------------------------------------------------------
 // exclusive prefix sums over the lists (single CTA, any number of lists)
 // ---------------------------------------------------------------------------
 constexpr int kScanThreads = 1024;

@@ -7,11 +7,12 @@ appends any number of tokens - a prefill block or a single decode token - and re
 attention rows, which equal the rows of a one-shot run over the final sequence bit for bit
 (a query only sees keys at or before its own position, and a chunk's mean only its own keys).
 """
+import ctypes as C
 from typing import Optional
 
 import torch
 
-from . import parallel
+from . import _lib, parallel
 
 
 class IncrementalMoba:
@@ -49,15 +50,51 @@ class IncrementalMoba:
         if n == 0 or begin + n > self.capacity:
             raise ValueError(f"cannot append {n} tokens at position {begin} of a cache of {self.capacity}")
         end = begin + n
-        self.k[begin:end].copy_(k)
-        self.v[begin:end].copy_(v)
-        self.cu[1:].fill_(end)
         # a call on a prefix of `begin` tokens left final means in the slots of all chunks but the
         # prefix's last one (the last chunk of a sequence is no candidate and is not computed)
         cached = (begin - 1) // self.chunk if begin > 0 else 0
-        out, _, sel = parallel.moba_forward(q, self.k[:end], self.v[:end], self.cu, self.capacity, self.chunk,
-                                            self.topk, attend_impl=self.attend_impl, q_token_begin=begin,
-                                            means_cache=self.means, cached_slots=cached,
-                                            return_selected=return_selected)
+        if self._plain(k, v):
+            out, sel = self._append(q, k, v, begin, end, cached, return_selected)
+        else:
+            self.k[begin:end].copy_(k)
+            self.v[begin:end].copy_(v)
+            self.cu[1:].fill_(end)
+            out, _, sel = parallel.moba_forward(q, self.k[:end], self.v[:end], self.cu, self.capacity, self.chunk,
+                                                self.topk, attend_impl=self.attend_impl, q_token_begin=begin,
+                                                means_cache=self.means, cached_slots=cached,
+                                                return_selected=return_selected)
         self.length = end
         return (out, sel) if return_selected else out
+
+    def _plain(self, k: torch.Tensor, v: torch.Tensor) -> bool:
+        """Rows that moba_append copies as they are: the caches' type, device and row shape, 16-byte pieces, and
+        nothing for autograd to record.  Everything else goes through torch's copy."""
+        row, dtype, device = self.k.shape[1:], self.k.dtype, self.k.device
+        for t, cache in ((k, self.k), (v, self.v)):
+            if cache.data_ptr() <= t.data_ptr() < cache.data_ptr() + cache.nbytes:      # rows of the cache itself
+                return False
+            if (t.shape[1:] != row or t.dtype != dtype or t.device != device or t.stride(2) != 1 or t.stride(0) % 8
+                    or t.stride(1) % 8 or t.data_ptr() % 16 or t.requires_grad):
+                return False
+        return not self.k.requires_grad and not self.v.requires_grad
+
+    def _append(self, q, k, v, begin: int, end: int, cached: int, return_selected: bool):
+        """One native call: rows into the caches, position, attention on the new tokens."""
+        kc, vc = self.k, self.v
+        parallel._validate(q, kc, vc, self.cu, self.capacity, self.chunk, self.topk, windowed=True)
+        out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
+        prob = parallel.make_problem(q, kc, vc, out, self.cu, self.capacity, self.chunk, self.topk, self.attend_impl, begin)
+        prob.total_tokens = end
+        need = parallel.workspace_bytes(prob)
+        ws = parallel._workspace(q.device, need)
+        sel = None
+        if return_selected:
+            hist = parallel._hist(self.capacity, self.chunk, self.topk)
+            sel = torch.empty((hist, q.shape[1], q.shape[0]), dtype=torch.int32, device=q.device)
+        lib = _lib.lib()
+        (kt, kh, _), (vt, vh, _) = k.stride(), v.stride()
+        _lib.check(parallel._on_device(q.device, lambda stream: lib.moba_append(
+            C.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), kt, kh, vt, vh, kc.data_ptr(), vc.data_ptr(),
+            self.cu.data_ptr(), out.data_ptr(), sel.data_ptr() if sel is not None and sel.numel() else None,
+            self.means.data_ptr(), cached, ws.data_ptr(), need, stream)))
+        return out, sel

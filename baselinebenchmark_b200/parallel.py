@@ -28,22 +28,25 @@ HEAD_DIMS = (64, 96, 128, 256)
 def _validate(q, k, v, cu_seqlens, max_seqlen, moba_chunk_size, moba_topk, windowed: bool = False) -> None:
     """parallel.py:410-446, message for message where it matters to callers.
     `windowed`: q holds a window of the packed tokens, so its token count may differ from k's."""
-    if q.ndim != 3 or k.ndim != 3 or v.ndim != 3:
+    qs, ks, vs, dev, dtype = q.shape, k.shape, v.shape, q.device, q.dtype      # each read once: this runs on every call
+    if len(qs) != 3 or len(ks) != 3 or len(vs) != 3:
         raise ValueError("q, k, and v must have shape [tokens, heads, head_dim]")
-    if k.shape != v.shape:
-        raise ValueError(f"k and v must have identical shapes, got {k.shape} and {v.shape}")
-    if (q.shape[0] != k.shape[0] and not windowed) or q.shape[2] != k.shape[2]:
+    tokens, hq, dim = qs
+    hkv = ks[1]
+    if ks != vs:
+        raise ValueError(f"k and v must have identical shapes, got {ks} and {vs}")
+    if (tokens != ks[0] and not windowed) or dim != ks[2]:
         raise ValueError(
-            f"q and k/v must have the same token count and head dimension, got q={q.shape}, k={k.shape}")
-    if q.device != k.device or q.device != v.device or q.device.type != "cuda":
+            f"q and k/v must have the same token count and head dimension, got q={qs}, k={ks}")
+    if dev != k.device or dev != v.device or dev.type != "cuda":
         raise ValueError("q, k, and v must be accelerator tensors on the same device")
-    if q.dtype != k.dtype or q.dtype != v.dtype:
+    if dtype != k.dtype or dtype != v.dtype:
         raise TypeError("q, k, and v must have the same dtype")
-    if q.dtype not in (torch.float16, torch.bfloat16):
-        raise TypeError(f"only float16 and bfloat16 are supported, got {q.dtype}")
+    if dtype not in (torch.float16, torch.bfloat16):
+        raise TypeError(f"only float16 and bfloat16 are supported, got {dtype}")
     if cu_seqlens.ndim != 1 or cu_seqlens.numel() < 2:
         raise ValueError("cu_seqlens must be a one-dimensional tensor of length >= 2")
-    if cu_seqlens.device != q.device or cu_seqlens.dtype != torch.int32:
+    if cu_seqlens.device != dev or cu_seqlens.dtype != torch.int32:
         raise TypeError("cu_seqlens must be an int32 tensor on the q device")
     if not isinstance(max_seqlen, int) or max_seqlen <= 0:
         raise ValueError(f"max_seqlen must be a positive int, got {max_seqlen}")
@@ -53,18 +56,18 @@ def _validate(q, k, v, cu_seqlens, max_seqlen, moba_chunk_size, moba_topk, windo
         raise ValueError(f"moba_topk must be a positive int, got {moba_topk}")
     if moba_topk > 64:
         raise ValueError(f"moba_topk must be <= 64 to match FlashMoBA, got {moba_topk}")
-    if q.shape[0] == 0 or q.shape[1] == 0 or k.shape[1] == 0 or q.shape[2] == 0:
+    if tokens == 0 or hq == 0 or hkv == 0 or dim == 0:
         raise ValueError("q, k, and v dimensions must be non-zero")
-    if q.shape[1] % k.shape[1] != 0:
-        raise ValueError(f"q heads ({q.shape[1]}) must be divisible by kv heads ({k.shape[1]})")
-    if q.shape[2] > 256:
-        raise ValueError(f"head_dim must be <= 256 to match FlashMoBA, got {q.shape[2]}")
+    if hq % hkv != 0:
+        raise ValueError(f"q heads ({hq}) must be divisible by kv heads ({hkv})")
+    if dim > 256:
+        raise ValueError(f"head_dim must be <= 256 to match FlashMoBA, got {dim}")
     # limits of this build (no fallback by design)
-    if q.shape[2] not in HEAD_DIMS:
+    if dim not in HEAD_DIMS:
         raise NotImplementedError(f"this build supports head_dim {HEAD_DIMS} only")
-    for name, t in (("q", q), ("k", k), ("v", v)):
-        if t.stride(2) != 1:
-            raise NotImplementedError(f"{name} must be contiguous in its last dimension")
+    if q.stride(2) != 1 or k.stride(2) != 1 or v.stride(2) != 1:
+        name = "q" if q.stride(2) != 1 else "k" if k.stride(2) != 1 else "v"
+        raise NotImplementedError(f"{name} must be contiguous in its last dimension")
 
 
 def default_attend_impl(head_dim: int) -> int:
@@ -76,16 +79,14 @@ def make_problem(q, k, v, out, cu_seqlens, max_seqlen, chunk, topk, attend_impl=
                  q_token_begin=None):
     """struct moba_problem for these tensors.  With `q_token_begin` set, q/out hold the
     packed tokens [q_token_begin, q_token_begin + q.shape[0]) and k/v all of them."""
+    tokens, hq, dim = q.shape
+    (sq_t, sq_h, _), (sk_t, sk_h, _), (sv_t, sv_h, _), (so_t, so_h, _) = q.stride(), k.stride(), v.stride(), out.stride()
+    # in the order of the struct's fields (filling it by keyword takes twice as long)
     return _lib.Problem(
-        q_token_begin=q_token_begin or 0, q_tokens=q.shape[0] if q_token_begin is not None else 0,
-        dtype=1 if q.dtype == torch.float16 else 0,
-        total_tokens=k.shape[0], batch=cu_seqlens.numel() - 1, num_q_heads=q.shape[1],
-        num_kv_heads=k.shape[1], head_dim=q.shape[2], max_seqlen=max_seqlen, chunk_size=chunk,
-        topk=topk, attend_impl=default_attend_impl(q.shape[2]) if attend_impl is None else attend_impl,
-        q_stride_token=q.stride(0), q_stride_head=q.stride(1),
-        k_stride_token=k.stride(0), k_stride_head=k.stride(1),
-        v_stride_token=v.stride(0), v_stride_head=v.stride(1),
-        o_stride_token=out.stride(0), o_stride_head=out.stride(1))
+        k.shape[0], cu_seqlens.numel() - 1, hq, k.shape[1], dim, max_seqlen, chunk, topk,
+        default_attend_impl(dim) if attend_impl is None else attend_impl,
+        sq_t, sq_h, sk_t, sk_h, sv_t, sv_h, so_t, so_h,
+        q_token_begin or 0, tokens if q_token_begin is not None else 0, 1 if q.dtype == torch.float16 else 0, 0)
 
 
 def workspace_bytes(problem, limit: Optional[int] = None) -> int:
@@ -106,6 +107,20 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     unordered streams never share a buffer, and a buffer allocated while a CUDA graph is
     being captured belongs to that graph's memory pool and stays valid for its replays."""
     return torch.empty(nbytes, dtype=torch.uint8, device=device)
+
+
+def _hist(max_seqlen: int, chunk: int, topk: int) -> int:
+    """Ranks of `selected`: min(topk - 1, chunks per sequence - 1) (parallel.py:303)."""
+    return max(0, min(topk - 1, (max_seqlen + chunk - 1) // chunk - 1))
+
+
+def _on_device(device: torch.device, call):
+    """`call(stream)` with `device` current; the guard is only entered where it changes something."""
+    index = device.index
+    if index is None or index != torch.cuda.current_device():
+        with torch.cuda.device(device):
+            return call(torch.cuda.current_stream(device).cuda_stream)
+    return call(torch._C._cuda_getCurrentRawStream(index))
 
 
 def moba_forward(q, k, v, cu_seqlens, max_seqlen, moba_chunk_size, moba_topk, *,
@@ -132,28 +147,29 @@ def moba_forward(q, k, v, cu_seqlens, max_seqlen, moba_chunk_size, moba_topk, *,
     out = torch.empty(q.shape, dtype=q.dtype, device=q.device)
     prob = make_problem(q, k, v, out, cu_seqlens, max_seqlen, moba_chunk_size, moba_topk, attend_impl,
                         q_token_begin)
-    dims = _lib.Dims()
-    _lib.check(_lib.lib().moba_problem_dims(C.byref(prob), C.byref(dims)))
+    lib, dev = _lib.lib(), q.device
     need = workspace_bytes(prob, workspace_limit)
-    ws = workspace if workspace is not None else _workspace(q.device, need)
-    lse = torch.empty((q.shape[1], q.shape[0]), dtype=torch.float32, device=q.device) if return_lse else None
+    ws = workspace if workspace is not None else _workspace(dev, need)
+    lse = torch.empty((q.shape[1], q.shape[0]), dtype=torch.float32, device=dev) if return_lse else None
     sel = None
     if return_selected:
-        sel = torch.empty((max(dims.hist, 0), q.shape[1], q.shape[0]), dtype=torch.int32, device=q.device)
-    with torch.cuda.device(q.device):
-        stream = torch.cuda.current_stream(q.device).cuda_stream
-        common = (C.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), cu_seqlens.data_ptr(), out.data_ptr(),
-                  lse.data_ptr() if lse is not None else None,
-                  sel.data_ptr() if sel is not None and sel.numel() else None)
-        if means_cache is not None:
-            if means_cache.shape != (dims.slots, k.shape[1], k.shape[2]) or means_cache.dtype != k.dtype \
-                    or not means_cache.is_contiguous():
-                raise ValueError(f"means_cache must be a contiguous {k.dtype} tensor of shape "
-                                 f"{(dims.slots, k.shape[1], k.shape[2])}")
-            rc = _lib.lib().moba_forward_cached(*common, means_cache.data_ptr(), cached_slots,
-                                                ws.data_ptr(), ws.numel() * ws.element_size(), stream)
-        else:
-            rc = _lib.lib().moba_forward(*common, ws.data_ptr(), ws.numel() * ws.element_size(), stream)
+        sel = torch.empty((_hist(max_seqlen, moba_chunk_size, moba_topk), q.shape[1], q.shape[0]), dtype=torch.int32,
+                          device=dev)
+    if means_cache is not None:
+        slots = (cu_seqlens.numel() - 1) * ((max_seqlen + moba_chunk_size - 1) // moba_chunk_size)
+        if means_cache.shape != (slots, k.shape[1], k.shape[2]) or means_cache.dtype != k.dtype \
+                or not means_cache.is_contiguous():
+            raise ValueError(f"means_cache must be a contiguous {k.dtype} tensor of shape "
+                             f"{(slots, k.shape[1], k.shape[2])}")
+    common = (C.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), cu_seqlens.data_ptr(), out.data_ptr(),
+              lse.data_ptr() if lse is not None else None,
+              sel.data_ptr() if sel is not None and sel.numel() else None)
+    ws_args = (ws.data_ptr(), ws.numel() * ws.element_size())
+    if means_cache is not None:
+        rc = _on_device(dev, lambda stream: lib.moba_forward_cached(*common, means_cache.data_ptr(), cached_slots,
+                                                                    *ws_args, stream))
+    else:
+        rc = _on_device(dev, lambda stream: lib.moba_forward(*common, *ws_args, stream))
     _lib.check(rc)
     return out, lse, sel
 

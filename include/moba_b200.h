@@ -162,6 +162,22 @@ int moba_forward_cached(const moba_problem_t* p, const void* q, const void* k, c
                         void* means_cache, int32_t cached_slots, void* workspace, size_t workspace_bytes,
                         void* stream);
 
+/* One append to a growing sequence: stores the K and V rows of the new tokens into caller-held caches, writes
+ * cu_seqlens = {0, total_tokens}, and runs moba_forward_cached on the new tokens' query window, in
+ * one call and with the rows copied by one kernel.  A decode step is a handful of microseconds of
+ * kernels and was bound by the host: one token behind 20011 (16/4 heads, head_dim 64, chunk 512) took 74 us with two
+ * copies, a fill and the forward as operations of their own, 37 us this way.
+ *   p              batch 1; total_tokens = tokens after the append, q_token_begin / q_tokens = the
+ *                  new ones; k_/v_stride_* are those of the caches
+ *   k_new, v_new   [q_tokens, Hkv, D] with the given token and head strides (elements, multiples of
+ *                  8), 16-byte aligned, not overlapping the rows they are stored to
+ *   k_cache, v_cache, cu_seqlens  written here */
+int moba_append(const moba_problem_t* p, const void* q, const void* k_new, const void* v_new,
+                int64_t k_new_stride_token, int64_t k_new_stride_head, int64_t v_new_stride_token,
+                int64_t v_new_stride_head, void* k_cache, void* v_cache, int32_t* cu_seqlens, void* out,
+                int32_t* selected_out, void* means_cache, int32_t cached_slots, void* workspace,
+                size_t workspace_bytes, void* stream);
+
 /* Same call with HOST buffers (pinned memory; cu_seqlens_host is also read by the
  * CPU): copies q, k, v to staging buffers inside `workspace`, runs the operator
  * and copies `out` back.  The caller synchronises `stream`, which completes after
