@@ -36,6 +36,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "short_items.cuh"
 #include "sm100_ptx.cuh"
 
 namespace moba {
@@ -101,39 +102,8 @@ struct KernelArgs {
   float2* partial_lse;                     // {natural-log LSE, 1 / scale}
   int32_t* work_counter;
   int32_t* status;
+  int32_t wide_store;                      // partial_out is 32-byte aligned
 };
-
-// tile_prefix is kept in shared memory sampled every 2^shift entries (shift 0: whole), so that
-// finding the list of a routed item costs `shift` dependent global loads instead of log2(lists).
-__host__ __device__ inline int prefix_shift(int64_t lists, int cache_entries) {
-  int shift = 0;
-  while ((lists >> shift) + 2 > cache_entries) ++shift;
-  return shift;
-}
-template <typename CtrlT>
-__device__ __forceinline__ void fill_prefix_cache(CtrlT& c, const int32_t* __restrict__ tile_prefix, int64_t lists,
-                                                  int nthreads) {
-  const int shift = prefix_shift(lists, CtrlT::kPrefix);
-  const int n = (int)(lists >> shift) + 1;                   // samples 0, 2^shift, ..., the last one <= lists
-  for (int i = threadIdx.x; i < n; i += nthreads) c.prefix_cache[i] = tile_prefix[(int64_t)i << shift];
-}
-// last l in [0, lists) with tile_prefix[l] <= i (i is a routed item: tile_prefix[lists] > i)
-template <typename CtrlT>
-__device__ __forceinline__ int find_list(const CtrlT& c, const int32_t* __restrict__ tile_prefix, int64_t lists, int i) {
-  const int shift = prefix_shift(lists, CtrlT::kPrefix);
-  int lo = 0, hi = (int)(lists >> shift) + 1;                // samples: last k with cache[k] <= i
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (c.prefix_cache[mid] <= i) lo = mid; else hi = mid;
-  }
-  int l = lo << shift;
-  int r = min(l + (1 << shift), (int)lists);                 // tile_prefix[r] > i, or r == lists
-  while (r - l > 1) {
-    const int mid = (l + r) >> 1;
-    if (__ldg(tile_prefix + mid) <= i) l = mid; else r = mid;
-  }
-  return l;
-}
 
 // Runs in one spare warp while the other warps work on the current item: draws the
 // next item from the global queue (skipping empty own-chunk tiles), decodes it and
@@ -259,8 +229,11 @@ __device__ __forceinline__ void softmax_row(uint32_t tS, uint32_t tO, int j, int
   }
   const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
   const float m_new = fmaxf(m_ref, mx * sl2);
-  if (__any_sync(0xffffffffu, m_new > m_ref + 8.f)) {
-    const float alpha = (m_new == -INFINITY) ? 1.f : ex2_approx(m_ref - m_new);
+  // a row's reference moves only when the row itself asks for it: its result does not depend on
+  // the rows it shares a warp with
+  const bool up = m_new > m_ref + 8.f;
+  if (__any_sync(0xffffffffu, up)) {
+    const float alpha = up ? ex2_approx(m_ref - m_new) : 1.f;
     if (j > 0) {
       before_rescale();
       uint32_t o[32];
@@ -274,7 +247,7 @@ __device__ __forceinline__ void softmax_row(uint32_t tS, uint32_t tO, int j, int
       }
     }
     l *= alpha;
-    m_ref = m_new;
+    if (up) m_ref = m_new;
   }
   const uint64_t scale2 = pack2(sl2, sl2);
   const uint64_t negm2 = pack2(-m_ref, -m_ref);
@@ -300,6 +273,131 @@ __device__ __forceinline__ void softmax_row(uint32_t tS, uint32_t tO, int j, int
   const uint64_t sum = add2(sum_a, sum_b);
   l += lo2(sum) + hi2(sum);
   tmem_wait_st();
+}
+
+// The same step with the scores read twice and 32 columns at a time, in loops: for kernels whose items are one or two
+// key tiles.  Unrolled, the step and the epilogue are some 50 KB of straight-line code that such an item
+// runs through once, and fetching it took longer than executing it (4300 cycles a step and 4200 an
+// epilogue, at a quarter of the issue slots); the loops are a few KB.  P of 32 columns never covers
+// scores still to be read.  Same operations in the same order as above: the same bits.
+template <bool kMasked, bool kHalf, int D, typename F>
+__device__ __forceinline__ void softmax_row_rolled(uint32_t tS, uint32_t tO, int j, int key0, int lim, float sl2,
+                                                   float& m_ref, float& l, F&& before_rescale) {
+  float mx = -INFINITY;
+  int rem = lim - key0;                    // visible columns left
+#pragma unroll 1
+  for (int ch = 0; ch < 4; ++ch, rem -= 32) {
+    uint32_t v[32];
+    tmem_ld32(tS + ch * 32, v);
+    tmem_wait_ld();
+    float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      if (kMasked) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[i + u] = i + u < rem ? v[i + u] : 0xff800000u;   // -inf
+      }
+      mx0 = max3(mx0, __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+      mx1 = max3(mx1, __uint_as_float(v[i + 2]), __uint_as_float(v[i + 3]));
+    }
+    mx = max3(mx, mx0, mx1);
+  }
+  const float m_new = fmaxf(m_ref, mx * sl2);
+  const bool up = m_new > m_ref + 8.f;
+  if (__any_sync(0xffffffffu, up)) {
+    const float alpha = up ? ex2_approx(m_ref - m_new) : 1.f;
+    if (j > 0) {
+      before_rescale();
+#pragma unroll 1
+      for (int ch = 0; ch < D / 32; ++ch) {
+        uint32_t o[32];
+        tmem_ld32(tO + ch * 32, o);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+        tmem_st32(tO + ch * 32, o);
+      }
+    }
+    l *= alpha;
+    if (up) m_ref = m_new;
+  }
+  const uint64_t scale2 = pack2(sl2, sl2);
+  const uint64_t negm2 = pack2(-m_ref, -m_ref);
+  uint64_t sum_a = 0, sum_b = 0;           // two packed accumulators = four running sums
+  rem = lim - key0;
+#pragma unroll 1
+  for (int ch = 0; ch < 4; ++ch, rem -= 32) {
+    uint32_t v[32], pk[16];
+    tmem_ld32(tS + ch * 32, v);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      uint32_t e0 = v[2 * i], e1 = v[2 * i + 1];
+      if (kMasked) {
+        e0 = 2 * i < rem ? e0 : 0xff800000u;
+        e1 = 2 * i + 1 < rem ? e1 : 0xff800000u;
+      }
+      const uint64_t x = fma2(pack2(__uint_as_float(e0), __uint_as_float(e1)), scale2, negm2);
+      uint64_t pr;
+      if ((i & 7) < kPolyPairs) {
+        pr = ex2_poly2(x);
+      } else {
+        pr = pack2(ex2_approx(lo2(x)), ex2_approx(hi2(x)));
+      }
+      if (i & 1) sum_b = add2(sum_b, pr); else sum_a = add2(sum_a, pr);
+      pk[i] = pack2_16<kHalf>(lo2(pr), hi2(pr));
+    }
+    tmem_st16(tS + ch * 16, pk);
+  }
+  const uint64_t sum = add2(sum_a, sum_b);
+  l += lo2(sum) + hi2(sum);
+  tmem_wait_st();
+}
+
+// Epilogue of a row in loops over 32 columns: the largest magnitude of the O row, ...
+template <int D>
+__device__ __forceinline__ float amax_row_rolled(uint32_t tO) {
+  float a0 = 0.f, a1 = 0.f;
+#pragma unroll 1
+  for (int ch = 0; ch < D; ch += 32) {
+    uint32_t v[32];
+    tmem_ld32(tO + ch, v);
+    tmem_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 32; i += 4) {
+      a0 = max3(a0, fabsf(__uint_as_float(v[i])), fabsf(__uint_as_float(v[i + 1])));
+      a1 = max3(a1, fabsf(__uint_as_float(v[i + 2])), fabsf(__uint_as_float(v[i + 3])));
+    }
+  }
+  return fmaxf(a0, a1);
+}
+// ... and the row itself, scaled, as fp16 in 32-byte stores (`wide`; 16-byte ones otherwise) for the lanes with a row
+// (`on`).  `drained` runs (warp-uniformly) when the last of O has been read.
+template <int D, typename F>
+__device__ __forceinline__ void store_row_rolled(uint32_t tO, __half* dst, float mul, bool on, bool wide, F&& drained) {
+#pragma unroll 1
+  for (int ch = 0; ch < D; ch += 32) {
+    uint32_t v[32];
+    tmem_ld32(tO + ch, v);
+    tmem_wait_ld();
+    if (ch + 32 == D) drained();
+    if (on) {
+#pragma unroll
+      for (int i = 0; i < 32; i += 16) {
+        uint32_t pk[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          pk[u] = pack2_half(__uint_as_float(v[i + 2 * u]) * mul, __uint_as_float(v[i + 2 * u + 1]) * mul);
+        if (wide) {
+          store32(dst + ch + i, pk);
+        } else {
+          *reinterpret_cast<uint4*>(dst + ch + i) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+          *reinterpret_cast<uint4*>(dst + ch + i + 8) = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+        }
+      }
+    }
+    __syncwarp();
+  }
 }
 
 // Descriptor words.  Low word: start address >> 4 | (leading byte offset >> 4) << 16;
@@ -606,7 +704,7 @@ attend_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
 }
 
 // ---------------------------------------------------------------------------
-// head dim 256
+// head dim 256, chunks of more than kSmallChunk keys
 //
 // One 128-row tile per work item.  Operands keep the shapes of the kernel above: Q, K and V are
 // handled as two 128-dim halves ("lo", "hi"); S = Q_lo.K_lo^T + Q_hi.K_hi^T (16 k-steps into one
@@ -916,61 +1014,88 @@ attend_tc5_wide_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_
 }
 
 // ---------------------------------------------------------------------------
-// small chunks (at most kSmallChunk keys): one 128-row tile per work item, two CTAs per SM
+// short items: chunks of at most kSmallChunk keys, and query windows with at most 128 rows per
+// kv head (decode steps).  One 128-row tile per work item, two CTAs per SM.
 //
-// With one or two key tiles per item the kernels above spend most of an item on its hand-over
-// (description, Q gather, epilogue: 13-19 thousand cycles for 2-3 thousand of MMA), during which the
-// tensor pipe idles.  This variant halves every per-CTA resource - 192 threads (one softmax
-// warpgroup, warps 0-3; warp 4 describes the next item and requests K/V tiles, warp 5 issues the
-// MMAs), one Q tile, one K and one V stage, 256 TMEM columns (S 0-127, O 128-255), about 110 KB
-// of shared memory, 168 registers per thread - so that two CTAs share an SM and one works while
-// the other changes items.  Per tile: QK -> softmax -> PV in sequence (S is single-buffered; P
-// overwrites it), K(j+1) is requested when QK(j) has executed, V(j+1) when PV(j) has.
+// Such an item is one or two key tiles (or, in a decode step, a long chunk for a handful of
+// rows), so what counts is that nothing of its hand-over is waited for.  The roles of a CTA run
+// through one flat stream of key tiles, without a CTA-wide barrier between items:
+//   warp 4     describes the items, up to four ahead (a chain of dependent global loads and divisions as
+//              long as an item: it does nothing else)
+//   warps 6, 7 copy the Q rows of the next item into the swizzled tile (cp.async) as soon as the last
+//              Q.K^T of the item before has executed; warp 6 also requests K/V tiles (TMA).  An item on the
+//              chunk of the item before it (the row tiles of one list are consecutive) finds K and V in
+//              place when the chunk is one tile
+//   warp 5     issues QK(0) PV(0) QK(1) PV(1) ...: QK of the next tile, of the next item
+//              too, directly behind the PV that consumed P, so that S is ready when the softmax
+//              warps return from the epilogue
+//   warps 0-3  softmax, and the epilogue: one thread per row, O from tensor memory through
+//              registers to 32-byte stores (whole sectors, no staging in shared memory)
+// Per CTA: one Q, one K and one V tile (32 KB each), 256 TMEM columns (S 0-127, O 128-255); two CTAs per SM
+// overlap each other's softmax, MMA and stores.
+// Bound by the softmax warps: softmax and epilogue of an item take most of its time (see softmax_row_rolled).
+// Measured against the kernel with CTA-wide barriers between items and unrolled code: dense stage of
+// 2 x 4096 tokens x 16 heads, chunk 128 199 -> 146 us (whole call 347 -> 279); 13311 tokens x 16/4 heads,
+// head_dim 64 233 -> 172; 32768 x 32/8 1651 -> 1094.  A decode step (chunk 4096, 131072-token prefix, 32/8 heads), in
+// place of the 256-row kernel: 132 -> 90.  The rolled loops alone: 205 -> 146 on the first.
 // ---------------------------------------------------------------------------
-constexpr int kSmallThreads = 192;
-constexpr int kSmallPrefix = 2048;
+constexpr int kShortThreads = 256;
 
-struct SmallCtrl {
-  static constexpr int kPrefix = kSmallPrefix;
-  uint64_t k_full, k_empty, v_full, v_empty, s_full, p_full, o_full;
-  uint64_t item_ready[2];
+struct ShortCtrl {
+  static constexpr int kPrefix = kShortPrefix;
+  uint64_t q_full, k_full, v_full;         // tiles landed
+  uint64_t q_free;                         // per item: its last Q.K^T has executed
+  uint64_t k_free;                         // per other key tile of an item: its Q.K^T has executed
+  uint64_t v_free;                         // per key tile that a new V tile follows: its P.V has executed
+  uint64_t s_full, p_full, o_full;
+  uint64_t item_full[kShortSlots], slot_free[kShortSlots];
   uint32_t tmem_slot;
   volatile int32_t abort;
   int32_t n_routed, n_items;
   SlotRange own;
-  Item item[2];
-  int32_t done[2];
-  int64_t qoff[2][kTileM];
-  int32_t entry[2][kTileM];
-  int32_t prefix_cache[kSmallPrefix];
+  ShortItem item[kShortSlots];
+  alignas(16) int32_t entry[kShortSlots][kTileM];
+  alignas(16) int64_t qoff[kShortSlots][kTileM];
+  int32_t prefix_cache[kShortPrefix];
 };
-constexpr size_t kSmallSmemBytes = 1024 + 3 * kTileBytes + sizeof(SmallCtrl);
-static_assert(2 * (kSmallSmemBytes + 1024) <= 232448, "two CTAs per SM");
+constexpr size_t kShortSmemBytes = 1024 + 3 * kTileBytes + sizeof(ShortCtrl);
+static_assert(2 * (kShortSmemBytes + 1024) <= 232448, "two CTAs per SM");
+
+struct ShortArgs {
+  KernelArgs a;
+  ItemQueue iq;
+};
 
 template <bool kHalf, int D>
-__global__ void __launch_bounds__(kSmallThreads, 2)
-attend_tc5_small_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
-                        const __grid_constant__ CUtensorMap tmap_v, const KernelArgs a) {
+__global__ void __launch_bounds__(kShortThreads, 2)
+attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
+                        const __grid_constant__ CUtensorMap tmap_v, const ShortArgs sa) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sQ = smem_u32(smem);
   const uint32_t sK = sQ + kTileBytes;
   const uint32_t sV = sK + kTileBytes;
-  SmallCtrl& c = *reinterpret_cast<SmallCtrl*>(smem + 3 * kTileBytes);
+  ShortCtrl& c = *reinterpret_cast<ShortCtrl*>(smem + 3 * kTileBytes);
+  const KernelArgs& a = sa.a;
   constexpr uint32_t kCols = 256;
+  constexpr int kNBlk = (D + 63) / 64;
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&c.q_full), 64);                        // the copies of two warps' lanes
     mbar_init(smem_u32(&c.k_full), 1);
-    mbar_init(smem_u32(&c.k_empty), 1);
     mbar_init(smem_u32(&c.v_full), 1);
-    mbar_init(smem_u32(&c.v_empty), 1);
+    mbar_init(smem_u32(&c.q_free), 1);
+    mbar_init(smem_u32(&c.k_free), 1);
+    mbar_init(smem_u32(&c.v_free), 1);
     mbar_init(smem_u32(&c.s_full), 1);
     mbar_init(smem_u32(&c.p_full), kTileM);
     mbar_init(smem_u32(&c.o_full), 1);
-    mbar_init(smem_u32(&c.item_ready[0]), 1);
-    mbar_init(smem_u32(&c.item_ready[1]), 1);
+    for (int i = 0; i < kShortSlots; ++i) {
+      mbar_init(smem_u32(&c.item_full[i]), 1);
+      mbar_init(smem_u32(&c.slot_free[i]), 4);                 // the softmax warps
+    }
     c.abort = 0;
     fence_barrier_init();
     prefetch_tmap(&tmap_k);
@@ -985,215 +1110,186 @@ attend_tc5_small_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
   if (threadIdx.x == 0) {
     c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
     c.own = own_slot_range(p, a.cu);
-    c.n_items = c.n_routed + own_item_count(c.own.n, p.Hq, p.C, kTileM);
+    c.n_items = c.n_routed + (sa.iq.grouped ? c.own.n * p.Hkv : own_item_count(c.own.n, p.Hq, p.C, kTileM));
   }
-  if (p.hist > 0) fill_prefix_cache(c, a.tile_prefix, p.lists, kSmallThreads);
+  if (p.hist > 0) fill_prefix_cache(c, a.tile_prefix, p.lists, kShortThreads);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = c.tmem_slot;
 
-  // Head of item n for every thread: the slot filled by warp 4; warps 0-3 gather the Q rows.  Warp 4
-  // does not wait for the gather: it goes on to describe item n + 1 at once (its chain of
-  // dependent global loads is as long as an item).
-  auto next_item = [&](int n, Item& it) -> bool {
-    const int slot = n & 1;
-    __syncthreads();
-    if (c.done[slot]) return false;
-    it = c.item[slot];
-    if (warp < 4) {
-      constexpr int kChunks = D / 8;
-      const int32_t* entry = c.entry[slot];
-      const int64_t* qoff = c.qoff[slot];
-      const int t = threadIdx.x;
-      uint4 val[kChunks];
-#pragma unroll
-      for (int u = 0; u < kChunks; ++u) {
-        const int i = t + u * 128;
-        const int r = i / kChunks, ch = i % kChunks;
-        val[u] = make_uint4(0, 0, 0, 0);
-        if (entry[r] >= 0) val[u] = __ldg(reinterpret_cast<const uint4*>(a.q + qoff[r] + ch * 8));
-      }
-#pragma unroll
-      for (int u = 0; u < kChunks; ++u) {
-        const int i = t + u * 128;
-        const int r = i / kChunks, ch = i % kChunks;
-        const uint32_t dst = (uint32_t)((ch >> 3) * kHalfBytes + r * 128 + (((ch & 7) ^ (r & 7)) << 4));
-        *reinterpret_cast<uint4*>(smem + dst) = val[u];
-      }
-    }
-    fence_proxy_async_smem();
-    if (warp != 4) asm volatile("bar.sync 1, 160;" ::: "memory");
-    return true;
+  bool ok = true;                          // false: a wait of this role gave up
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity));
+    return ok;
   };
-  Item it;
-
-  if (warp >= 4) {
-    uint32_t kt = 0, vt = 0;               // K / V tiles produced (warp 4) or consumed (warp 5) so far
-    uint32_t pph = 0;                      // p_full phase
-    int pre = 0;                           // warp 4: 1 when K(0) and V(0) of the coming item are requested
+  if (warp == 4) {
+    if (p.C <= kBN) ok = describe_items<kShortSlots, 1, true, false>(p, sa.iq, c);
+    else ok = describe_items<kShortSlots, 1, false, false>(p, sa.iq, c);
+    if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
+  } else if (warp >= 6) {
+    // ---- Q rows; K/V tiles
+    uint32_t kt = 0, vt = 0;               // k_free phases waited for, V tiles requested
+    for (int n = 0; ok; ++n) {
+      const int slot = n % kShortSlots;
+      if (!wait(&c.item_full[slot], (n / kShortSlots) & 1)) break;
+      if (c.item[slot].done) break;
+      const int tok0 = c.item[slot].tok0, head = c.item[slot].head;
+      const int ntiles = (c.item[slot].kv_len + kBN - 1) / kBN;
+      const bool fresh = c.item[slot].new_kv != 0;
+      auto load = [&](uint32_t dst, const CUtensorMap* m, uint64_t* full, int j) {
+        if (lane == 0) {
+          const uint32_t bar = smem_u32(full);
+          mbar_expect_tx(bar, kNBlk * kHalfBytes);
+          tma_load_3d(dst, m, bar, 0, head, tok0 + j * kBN);
+          if (D > 64) tma_load_3d(dst + kHalfBytes, m, bar, 64, head, tok0 + j * kBN);
+        }
+      };
+      if (n > 0 && !wait(&c.q_free, (n - 1) & 1)) break;
+      if (warp == 6 && fresh) load(sK, &tmap_k, &c.k_full, 0);
+      copy_rows_async<D / 8, 2>(sQ, a.q, 0, warp - 6, c.item[slot].nrows, [&](int r) { return c.qoff[slot][r]; });
+      cp_async_mbar_arrive(smem_u32(&c.q_full));
+      if (warp == 6)
+        for (int j = 0; j < ntiles; ++j) {
+          if (j > 0) {
+            if (!wait(&c.k_free, kt & 1)) break;
+            ++kt;
+            load(sK, &tmap_k, &c.k_full, j);
+          }
+          if (!fresh) break;                                   // (one tile, in place)
+          if (vt > 0 && !wait(&c.v_free, (vt - 1) & 1)) break;
+          ++vt;
+          load(sV, &tmap_v, &c.v_full, j);
+        }
+    }
+    if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
+  } else if (warp == 5) {
+    // ---- MMA issuer: the whole warp runs this code, one elected lane issues (see above)
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
     const uint32_t dq = __shfl_sync(0xffffffffu, desc_lo(sQ, 16), 0);
     const uint32_t dk = __shfl_sync(0xffffffffu, desc_lo(sK, 16), 0);
     const uint32_t dv = __shfl_sync(0xffffffffu, desc_lo(sV, kHalfBytes), 0);
     const uint32_t el = elect_one();
-    if (warp == 4) prefetch_item<kTileM>(p, a, c, 0);
-    for (int n = 0;; ++n) {
-      if (!next_item(n, it)) break;
-      const int ntiles = (it.kv_len + kBN - 1) / kBN;
-      if (warp == 4) {
-        // K and V tile `j` of item `w`; false after a timeout (lane 0 only)
-        auto load_tile = [&](const Item& w, int j) -> bool {
-          const int tok = w.kv_tok0 + j * kBN;
-          if (!mbar_wait(smem_u32(&c.k_empty), (kt & 1) ^ 1)) return false;
-          uint32_t bar = smem_u32(&c.k_full);
-          mbar_expect_tx(bar, ((D + 63) / 64) * kHalfBytes);
-          tma_load_3d(sK, &tmap_k, bar, 0, w.kv_head, tok);
-          if (D > 64) tma_load_3d(sK + kHalfBytes, &tmap_k, bar, 64, w.kv_head, tok);
-          ++kt;
-          if (!mbar_wait(smem_u32(&c.v_empty), (vt & 1) ^ 1)) return false;
-          bar = smem_u32(&c.v_full);
-          mbar_expect_tx(bar, ((D + 63) / 64) * kHalfBytes);
-          tma_load_3d(sV, &tmap_v, bar, 0, w.kv_head, tok);
-          if (D > 64) tma_load_3d(sV + kHalfBytes, &tmap_v, bar, 64, w.kv_head, tok);
-          ++vt;
-          return true;
-        };
-        bool alive = true;
-        if (lane == 0)
-          for (int j = pre; alive && j < ntiles; ++j) alive = load_tile(it, j);
-        pre = 0;
-        __syncwarp();
-        // the next item: described by the whole warp, its first tiles requested as soon as the
-        // stages free up
-        const int s1 = (n + 1) & 1;
-        prefetch_item<kTileM>(p, a, c, s1);
-        if (lane == 0 && alive && !c.done[s1]) {
-          const Item nx = c.item[s1];
-          alive = load_tile(nx, 0);
-          pre = alive ? 1 : 0;
-        }
-        pre = __shfl_sync(0xffffffffu, pre, 0);
-        if (lane == 0 && !alive) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
-      } else {
-        bool ok = true;
-        tc_fence_after();
-        for (int j = 0; ok && j < ntiles; ++j) {
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.k_full), kt & 1));
-          if (!ok) break;
-          tc_fence_after();
-          if (el) {
-            issue_qk<0, 0, kHalf, D>(tm, dq, dk);
-            tc_commit(smem_u32(&c.s_full));
-            tc_commit(smem_u32(&c.k_empty));
-          }
-          __syncwarp();
-          ++kt;
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.v_full), vt & 1));
-          if (!ok) break;
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.p_full), pph));
-          if (!ok) break;
-          pph ^= 1;
-          tc_fence_after();
-          if (el) {
-            // O in columns 128-255: the P.V of the kernels above with the accumulator moved
-#pragma unroll
-            for (int ks = 0; ks < 8; ++ks)
-              mma_ts(tm + 128, tm + ks * 8, desc64(dv + ks * (2048 >> 4)), kIdescPV<kHalf, D>, j > 0 || ks > 0);
-            tc_commit(smem_u32(&c.v_empty));
-            if (j + 1 == ntiles) tc_commit(smem_u32(&c.o_full));
-          }
-          __syncwarp();
-          ++vt;
-        }
-        if (!ok && lane == 0) { atomicExch(a.status, ST_MMA); c.abort = 1; }
+    uint32_t kt = 0, vt = 0, g = 0;        // K / V tiles consumed, key tiles whose P.V has been issued
+    // Q.K^T of tile j of item n; `fresh`: the K tile is a new one
+    auto qk = [&](int n, int j, int ntiles, bool fresh) {
+      if (j == 0) {
+        if (!wait(&c.q_full, n & 1)) return;
+        fence_proxy_async_smem();                             // rows written by cp.async, read by the tensor core
+      }
+      if (fresh) {
+        if (!wait(&c.k_full, kt & 1)) return;
+        ++kt;
+      }
+      tc_fence_after();
+      if (el) {
+        issue_qk<0, 0, kHalf, D>(tm, dq, dk);
+        tc_commit(smem_u32(&c.s_full));
+        tc_commit(smem_u32(j + 1 == ntiles ? &c.q_free : &c.k_free));
       }
       __syncwarp();
+    };
+    int n = 0;
+    if (wait(&c.item_full[0], 0) && !c.item[0].done) {
+      int ntiles = (c.item[0].kv_len + kBN - 1) / kBN;
+      bool fresh = c.item[0].new_kv != 0;
+      qk(0, 0, ntiles, fresh);
+      while (ok) {
+        int next_tiles = 0;
+        bool next_fresh = false, more = true;
+        for (int j = 0; ok && j < ntiles; ++j, ++g) {
+          if (fresh) {
+            if (!wait(&c.v_full, vt & 1)) break;
+            ++vt;
+          }
+          if (!wait(&c.p_full, g & 1)) break;
+          tc_fence_after();
+          if (el) {
+#pragma unroll
+            for (int ks = 0; ks < 8; ++ks)
+              mma_ts_lo<kDescHi>(tm + 128, tm + ks * 8, dv + ks * (2048 >> 4), kIdescPV<kHalf, D>, j > 0 || ks > 0);
+            tc_commit(smem_u32(j + 1 == ntiles ? &c.o_full : &c.v_free));
+          }
+          __syncwarp();
+          if (j + 1 < ntiles) {
+            qk(n, j + 1, ntiles, true);
+          } else {
+            const int s1 = (n + 1) % kShortSlots;
+            if (!wait(&c.item_full[s1], ((n + 1) / kShortSlots) & 1)) break;
+            more = !c.item[s1].done;
+            next_tiles = (c.item[s1].kv_len + kBN - 1) / kBN;
+            next_fresh = c.item[s1].new_kv != 0;
+            if (more) {
+              if (next_fresh && el) tc_commit(smem_u32(&c.v_free));
+              __syncwarp();
+              qk(n + 1, 0, next_tiles, next_fresh);
+            }
+          }
+        }
+        if (!ok || !more) break;
+        ntiles = next_tiles;
+        fresh = next_fresh;
+        ++n;
+      }
     }
+    if (!ok && lane == 0) { atomicExch(a.status, ST_MMA); c.abort = 1; }
   } else {
+    // ---- softmax + epilogue, one thread per row
     const int row = warp * 32 + lane;
     const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
     const uint32_t tS = tmem + lane_base;
     const uint32_t tO = tmem + lane_base + 128;
     const float sl2 = rsqrtf((float)D) * 1.4426950408889634f;
-    uint32_t sph = 0, oph = 0;
-    for (int n = 0; next_item(n, it); ++n) {
-      const int32_t* entries = c.entry[n & 1];
-      const int ntiles = (it.kv_len + kBN - 1) / kBN;
-      const int qpos = it.tok0 + row;
-      const int lim = it.causal ? min(it.kv_len, qpos - it.kv_tok0 + 1) : it.kv_len;
+    uint32_t g = 0;
+    for (int n = 0; ok; ++n) {
+      const int slot = n % kShortSlots;
+      if (!wait(&c.item_full[slot], (n / kShortSlots) & 1)) break;
+      if (c.item[slot].done) break;
+      const int kv_len = c.item[slot].kv_len, tok_rel = c.item[slot].tok_rel, group = c.item[slot].group;
+      const bool causal = c.item[slot].causal != 0;
+      const bool active = warp * 32 < c.item[slot].nrows;     // warps without rows only keep the barriers going
+      const int32_t e = c.entry[slot][row];
+      const int ntiles = (kv_len + kBN - 1) / kBN;
+      const int qrel = tok_rel + (group == 1 ? row : row / group);              // own chunk: position in the chunk
+      const int lim = causal ? min(kv_len, qrel + 1) : kv_len;                  // keys < lim are visible
       float m_ref = -INFINITY, l = 0.f;
-      bool ok = true;
-      for (int j = 0; ok && j < ntiles; ++j) {
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.s_full), sph));
-        if (!ok) break;
-        sph ^= 1;
-        tc_fence_after();
-        const int key0 = j * kBN;
-        const bool masked = key0 + kBN > it.kv_len || (it.causal && it.kv_tok0 + key0 + kBN - 1 > it.tok0);
-        if (masked) softmax_row<true, kHalf, D>(tS, tO, j, key0, lim, sl2, m_ref, l, [] {});
-        else softmax_row<false, kHalf, D>(tS, tO, j, key0, lim, sl2, m_ref, l, [] {});
-        tc_fence_before();
+      for (int j = 0; j < ntiles; ++j, ++g) {
+        if (!wait(&c.s_full, g & 1)) break;
+        // the item's Q.K^T has run: every role has read its description
+        if (j == 0 && lane == 0) mbar_arrive(smem_u32(&c.slot_free[slot]));
+        if (active) {
+          tc_fence_after();
+          const int key0 = j * kBN;
+          const bool masked = key0 + kBN > kv_len || (causal && key0 + kBN - 1 > tok_rel);
+          // S of the next tile is only computed after this tile's P.V: O is quiet here
+          if (masked) softmax_row_rolled<true, kHalf, D>(tS, tO, j, key0, lim, sl2, m_ref, l, [] {});
+          else softmax_row_rolled<false, kHalf, D>(tS, tO, j, key0, lim, sl2, m_ref, l, [] {});
+          tc_fence_before();
+        }
         mbar_arrive(smem_u32(&c.p_full));
       }
-      if (ok) ok = mbar_wait(smem_u32(&c.o_full), oph);
-      ok = __all_sync(0xffffffffu, ok);
-      if (ok) {
-        oph ^= 1;
+      if (!ok || !wait(&c.o_full, n & 1)) break;
+      if (active) {
         tc_fence_after();
-        const int32_t e = entries[row];
-        uint32_t v0[32], v1[32];
-        float amax = 0.f;
-#pragma unroll
-        for (int ch = 0; ch < D / 32; ++ch) {
-          tmem_ld32(tO + ch * 32, v0);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 32; i += 2)
-            amax = max3(amax, fabsf(__uint_as_float(v0[i])), fabsf(__uint_as_float(v0[i + 1])));
-        }
+        // the row's largest magnitude decides the power of two its fp16 copy is scaled by
+        const float amax = amax_row_rolled<D>(tO);
         const float inv = 1.f / l;
         const PartialScale ps = partial_scale(amax * inv);
-        const float mul = inv * ps.scale;
-        unsigned char* stage = smem + warp * 8192;            // this warp's part of the idle Q tile
-#pragma unroll
-        for (int ch = 0; ch < (D + 63) / 64; ++ch) {
-          constexpr int kLast = D % 64 == 0 ? 64 : D % 64;
-          const int cols = ch == (D + 63) / 64 - 1 ? kLast : 64;
-          tmem_ld32(tO + ch * 64, v0);
-          if (cols > 32) tmem_ld32(tO + ch * 64 + 32, v1);
-          tmem_wait_ld();
-#pragma unroll
-          for (int i = 0; i < 8; ++i)
-            if (i * 8 < cols) {
-              const uint32_t* s8 = i < 4 ? v0 + 8 * i : v1 + 8 * (i - 4);
-              *reinterpret_cast<uint4*>(stage + lane * 144 + i * 16) =
-                  make_uint4(pack2_half(__uint_as_float(s8[0]) * mul, __uint_as_float(s8[1]) * mul),
-                             pack2_half(__uint_as_float(s8[2]) * mul, __uint_as_float(s8[3]) * mul),
-                             pack2_half(__uint_as_float(s8[4]) * mul, __uint_as_float(s8[5]) * mul),
-                             pack2_half(__uint_as_float(s8[6]) * mul, __uint_as_float(s8[7]) * mul));
-            }
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int rl = i * 4 + (lane >> 3), c16 = lane & 7;
-            const int32_t er = __shfl_sync(0xffffffffu, e, rl);
-            const uint4 val = *reinterpret_cast<const uint4*>(stage + rl * 144 + c16 * 16);
-            if (er >= 0 && c16 * 8 < cols)
-              __stcs(reinterpret_cast<uint4*>(a.partial_out + (int64_t)er * D + ch * 64 + c16 * 8), val);
-          }
-          __syncwarp();
-        }
+        store_row_rolled<D>(tO, a.partial_out + (int64_t)(e >= 0 ? e : 0) * D, inv * ps.scale, e >= 0, a.wide_store != 0,
+                            [] { tc_fence_before(); });
         if (e >= 0) a.partial_lse[e] = make_float2((m_ref + log2f(l)) * 0.6931471805599453f, ps.inv);
-        tc_fence_before();
-      } else {
-        atomicExch(a.status, ST_SOFTMAX);
-        c.abort = 1;
       }
+    }
+    if (!ok) {
+      atomicExch(a.status, ST_SOFTMAX);
+      c.abort = 1;
     }
   }
 
-  if (c.abort) {
+  // a role that gave up leaves the others to run into their own bounded waits
+  __syncwarp();
+  __syncthreads();
+  if (c.abort) {                           // copies in flight land before shared memory is given up
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
   }
@@ -1267,25 +1363,33 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
   if (!make_kv_map(&mk, p.fp16 != 0, p.D, k, p.T, p.Hkv, p.sk_t, p.sk_h, kBN) || !make_kv_map(&mv, p.fp16 != 0, p.D, v, p.T, p.Hkv, p.sv_t, p.sv_h, kBN))
     return cudaErrorNotSupported;
   if (p.D != 64 && p.D != 96 && p.D != 128 && p.D != 256) return cudaErrorInvalidValue;
-  auto kernel = p.D == 256 ? (p.fp16 ? attend_tc5_wide_kernel<true> : attend_tc5_wide_kernel<false>)
-              : p.D == 128 ? (p.fp16 ? attend_tc5_kernel<true, 128> : attend_tc5_kernel<false, 128>)
-              : p.D == 96  ? (p.fp16 ? attend_tc5_kernel<true, 96> : attend_tc5_kernel<false, 96>)
-                           : (p.fp16 ? attend_tc5_kernel<true, 64> : attend_tc5_kernel<false, 64>);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-  if (e != cudaSuccess) return e;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const KernelArgs args{q, cu, list_counts, list_offsets, tile_prefix, row_list, partial_out, partial_lse,
-                        work_counter, status};
-  if (tc5_small_items(p.D, p.C)) {
-    auto small = p.D == 128 ? (p.fp16 ? attend_tc5_small_kernel<true, 128> : attend_tc5_small_kernel<false, 128>)
-               : p.D == 96  ? (p.fp16 ? attend_tc5_small_kernel<true, 96> : attend_tc5_small_kernel<false, 96>)
-                            : (p.fp16 ? attend_tc5_small_kernel<true, 64> : attend_tc5_small_kernel<false, 64>);
-    e = cudaFuncSetAttribute(small, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmemBytes);
+                        work_counter, status, ((uintptr_t)partial_out & 31) == 0};
+  cudaError_t e;
+  if (tc5_short_items(p.D, p.C, p.Tq, p.G)) {
+    auto kern = p.D == 128 ? (p.fp16 ? attend_tc5_short_kernel<true, 128> : attend_tc5_short_kernel<false, 128>)
+              : p.D == 96  ? (p.fp16 ? attend_tc5_short_kernel<true, 96> : attend_tc5_short_kernel<false, 96>)
+                           : (p.fp16 ? attend_tc5_short_kernel<true, 64> : attend_tc5_short_kernel<false, 64>);
+    const int threads = kShortThreads, ctas = 2 * sms;
+    const size_t smem = kShortSmemBytes;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    return launch_pdl(small, dim3(2 * sms), kSmallThreads, kSmallSmemBytes, st, p, mk, mv, args);
+    ShortArgs sa;
+    sa.a = args;
+    sa.iq = ItemQueue{cu, list_counts, list_offsets, tile_prefix, row_list, work_counter, 1, 0};
+    sa.iq.grouped = p.Tq * p.G <= kTileM;
+    sa.iq.batch = short_batch(p, ctas, sa.iq.grouped);
+    return launch_pdl(kern, dim3(ctas), threads, smem, st, p, mk, mv, sa);
   }
+  auto kernel = p.D == 256 ? (p.fp16 ? attend_tc5_wide_kernel<true> : attend_tc5_wide_kernel<false>)
+              : p.D == 128 ? (p.fp16 ? attend_tc5_kernel<true, 128> : attend_tc5_kernel<false, 128>)
+              : p.D == 96  ? (p.fp16 ? attend_tc5_kernel<true, 96> : attend_tc5_kernel<false, 96>)
+                           : (p.fp16 ? attend_tc5_kernel<true, 64> : attend_tc5_kernel<false, 64>);
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+  if (e != cudaSuccess) return e;
   return launch_pdl(kernel, dim3(sms), kThreads, kSmemBytes, st, p, mk, mv, args);
 }
 

@@ -1,0 +1,252 @@
+// Work items of one 128-row tile: the description of an item and the walk through the queue of items,
+// shared by the kernels whose roles run through a flat stream of items (the forward's kernels for
+// short items and for head dim 256, and the dq kernel for short chunks).
+#pragma once
+
+#include "common.cuh"
+#include "sm100_ptx.cuh"
+
+namespace moba {
+namespace {
+
+constexpr int kShortPrefix = 2048;         // ints of tile_prefix kept in shared memory
+constexpr int kShortSlots = 4;             // item descriptions in flight
+
+// tile_prefix is kept in shared memory sampled every 2^shift entries (shift 0: whole), so that
+// finding the list of a routed item costs `shift` dependent global loads instead of log2(lists).
+__host__ __device__ inline int prefix_shift(int64_t lists, int cache_entries) {
+  int shift = 0;
+  while ((lists >> shift) + 2 > cache_entries) ++shift;
+  return shift;
+}
+template <typename CtrlT>
+__device__ __forceinline__ void fill_prefix_cache(CtrlT& c, const int32_t* __restrict__ tile_prefix, int64_t lists,
+                                                  int nthreads) {
+  const int shift = prefix_shift(lists, CtrlT::kPrefix);
+  const int n = (int)(lists >> shift) + 1;                   // samples 0, 2^shift, ..., the last one <= lists
+  for (int i = threadIdx.x; i < n; i += nthreads) c.prefix_cache[i] = tile_prefix[(int64_t)i << shift];
+}
+// last l in [0, lists) with tile_prefix[l] <= i (i is a routed item: tile_prefix[lists] > i)
+template <typename CtrlT>
+__device__ __forceinline__ int find_list(const CtrlT& c, const int32_t* __restrict__ tile_prefix, int64_t lists, int i) {
+  const int shift = prefix_shift(lists, CtrlT::kPrefix);
+  int lo = 0, hi = (int)(lists >> shift) + 1;                // samples: last k with cache[k] <= i
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (c.prefix_cache[mid] <= i) lo = mid; else hi = mid;
+  }
+  int l = lo << shift;
+  int r = min(l + (1 << shift), (int)lists);                 // tile_prefix[r] > i, or r == lists
+  while (r - l > 1) {
+    const int mid = (l + r) >> 1;
+    if (__ldg(tile_prefix + mid) <= i) l = mid; else r = mid;
+  }
+  return l;
+}
+
+// Where the items come from.
+struct ItemQueue {
+  const int32_t* cu;
+  const int32_t* list_counts;
+  const int32_t* list_offsets;
+  const int32_t* tile_prefix;
+  const int32_t* row_list;
+  int32_t* work_counter;
+  int32_t batch;                           // items a CTA draws at a time
+  int32_t grouped;                         // own-chunk items cover the heads of a group (short windows)
+};
+// A CTA draws several items at a time, so that row tiles of one list follow one another on it (K and V
+// stay in place), but at most an eighth of its share of the launch, for the balance.
+inline int short_batch(const Params& p, int ctas, bool grouped) {
+  const int64_t items = p.hist * p.rows / kTileRowsWide + (grouped ? 0 : p.rows / kTileRowsWide);
+  const int64_t share = items / (ctas * 8);
+  return share < 1 ? 1 : share > 8 ? 8 : (int)share;
+}
+
+struct ShortItem {
+  int32_t done;                            // 1: the queue is empty
+  int32_t new_kv;                          // 0: K and V of the item before are those of this one (one tile)
+  int32_t nrows, causal;
+  int32_t kv_len;
+  int32_t tok_rel;                         // own chunk: first query token minus first key token
+  int32_t group;                           // own chunk: rows per token (1, or the heads of the group)
+  int32_t tile0;                           // 128-key tiles of the CTA before this item
+  int32_t tok0, head;                      // first key token, kv head
+};
+
+// Walks the items a CTA draws; executed by the whole describing warp.
+struct ShortQueue {
+  int cur, end;                            // items of the current draw left: [cur, end)
+  int list, list_first, list_end;          // list of the last routed item and the items it covers
+  int list_off, list_count, kv_tok0, kv_head;
+};
+
+// The next item: its rows of this lane (4 * lane ... + 3) in `ent` (-1: none, behind the last row), their
+// element offsets in q in `qoff`, its description in `it`.
+template <typename CtrlT>
+__device__ __forceinline__ void short_next(const Params& p, const ItemQueue& a, CtrlT& c, ShortQueue& w, ShortItem& it,
+                                           int& kv_tok0, int& kv_head, int (&ent)[4], int64_t (&qoff)[4]) {
+  const int lane = threadIdx.x & 31;
+  const int n_routed = c.n_routed, n_items = c.n_items;
+  it.done = 1;
+  it.nrows = 0;
+  it.causal = 0;
+  it.kv_len = 0;
+  it.tok_rel = 0;
+  it.group = 1;
+  kv_tok0 = 0;
+  kv_head = 0;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) { ent[u] = -1; qoff[u] = 0; }
+  for (;;) {
+    if (w.cur >= w.end) {
+      int idx = 0;
+      if (lane == 0) idx = c.abort ? 0x7fffffff : atomicAdd(a.work_counter, a.batch);
+      idx = __shfl_sync(0xffffffffu, idx, 0);
+      if (idx >= n_items) return;
+      w.cur = idx;
+      w.end = min(idx + a.batch, n_items);
+    }
+    const int idx = w.cur++;
+    if (idx < n_routed) {
+      if (idx < w.list_first || idx >= w.list_end) {
+        const int l = find_list(c, a.tile_prefix, p.lists, idx);
+        const int slot = l / p.Hkv;
+        const int b = slot / p.mc, j = slot - b * p.mc;
+        w.list = l;
+        w.list_first = __ldg(a.tile_prefix + l);
+        w.list_end = __ldg(a.tile_prefix + l + 1);
+        w.list_off = __ldg(a.list_offsets + l);
+        w.list_count = __ldg(a.list_counts + l);
+        w.kv_tok0 = __ldg(a.cu + b) + j * p.C;
+        w.kv_head = l - slot * p.Hkv;
+      }
+      const int tile = idx - w.list_first;
+      it.nrows = min(w.list_count - tile * kTileRowsWide, kTileRowsWide);
+      it.kv_len = p.C;
+      kv_tok0 = w.kv_tok0;
+      kv_head = w.kv_head;
+      const int32_t* rows = a.row_list + w.list_off + tile * kTileRowsWide + 4 * lane;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (4 * lane + u < it.nrows) ent[u] = __ldg(rows + u);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (ent[u] >= 0) {
+          const uint32_t row = (uint32_t)ent[u] / (uint32_t)p.NP;
+          const uint32_t t = row / (uint32_t)p.Hq;
+          const uint32_t h = row - t * (uint32_t)p.Hq;
+          qoff[u] = (int64_t)t * p.sq_t + (int64_t)h * p.sq_h;
+        }
+      break;
+    }
+    // own chunk: rows are (token, head) pairs, `group` heads per token
+    const int g = a.grouped ? p.G : 1;
+    const int units = p.Hq / g;
+    // grouped: a slot's part of the window is one item
+    const int tiles_per_chunk = a.grouped ? 1 : (p.C + kTileRowsWide - 1) / kTileRowsWide;
+    const int per_tile = c.own.n * units;
+    int i = idx - n_routed;
+    const int ti = tiles_per_chunk - 1 - i / per_tile;        // longest tiles first
+    i -= (i / per_tile) * per_tile;
+    const int slot = c.own.lo + i / units;
+    const int head = (i - (slot - c.own.lo) * units) * g;
+    const int b = slot / p.mc, j = slot - b * p.mc;
+    const Slot s = slot_of(a.cu, b, j, p.C);
+    const int tile0 = s.start + ti * kTileRowsWide;
+    const int lo = max(tile0, p.win_lo);
+    const int hi = min(a.grouped ? s.end : min(tile0 + kTileRowsWide, s.end), p.win_lo + (int)p.Tq);
+    if (lo >= hi) continue;
+    it.nrows = (hi - lo) * g;
+    it.causal = 1;
+    it.group = g;
+    it.tok_rel = lo - s.start;
+    it.kv_len = hi - s.start;
+    kv_tok0 = s.start;
+    kv_head = head / p.G;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int r = 4 * lane + u;
+      if (r < it.nrows) {
+        const int t = lo - p.win_lo + r / g, h = head + r % g;
+        ent[u] = (int32_t)(((int64_t)t * p.Hq + h) * p.NP);
+        qoff[u] = (int64_t)t * p.sq_t + (int64_t)h * p.sq_h;
+      }
+    }
+    break;
+  }
+  it.done = 0;
+}
+
+// Rows [0, nrows) of an item into a 128-byte-swizzled tile of [128][64] blocks, by kWarps warps (this one is number
+// `part`): pieces [piece0, piece0 + kPieces) of 16 bytes of each row, whole rows per instruction.  off(r):
+// element offset of row r from `base`.
+template <int kPieces, int kWarps, typename F>
+__device__ __forceinline__ void copy_rows_async(uint32_t tile, const __nv_bfloat16* base, int piece0, int part, int nrows,
+                                                F&& off) {
+  constexpr int kRowsPerInstr = 32 / kPieces;
+  const int lane = threadIdx.x & 31;
+  const int ch = lane % kPieces, r0 = lane / kPieces;
+  const uint32_t dst = tile + (uint32_t)((ch >> 3) * (128 * 128));
+  const __nv_bfloat16* src = base + (piece0 + ch) * 8;
+  if (r0 < kRowsPerInstr) {                                    // 12 pieces (head dim 96): 24 of the 32 lanes copy
+#pragma unroll 8
+    for (int r = r0 + part * kRowsPerInstr; r < nrows; r += kWarps * kRowsPerInstr)
+      ptx::cp_async_16(dst + (uint32_t)(r * 128 + (((ch & 7) ^ (r & 7)) << 4)), src + off(r));
+  }
+}
+
+// One warp describes the items of the CTA ahead of everybody else: item m goes into slot m % kSlots of the
+// control block once the slot's item before has been let go by its readers (slot_free), and the
+// end of the queue is published `kEnds` times (once per group of threads that takes the items in turn).
+// False when a wait gave up.  kRowIndex: row indices t * Hq + h are kept too.
+template <int kSlots, int kEnds, bool kReuse, bool kRowIndex, typename CtrlT>
+__device__ __forceinline__ bool describe_items(const Params& p, const ItemQueue& iq, CtrlT& c) {
+  const int lane = threadIdx.x & 31;
+  ShortQueue w;
+  w.cur = w.end = 0;
+  w.list = -1;
+  w.list_first = w.list_end = 0;
+  w.list_off = w.list_count = w.kv_tok0 = w.kv_head = 0;
+  ShortItem it;
+  int ent[4], tok0, head, last_tok0 = -1, last_head = -1, ends = 0;
+  int64_t qoff[4];
+  uint32_t tiles = 0;
+  for (int n = 0; ends < kEnds; ++n) {
+    if (ends == 0) short_next(p, iq, c, w, it, tok0, head, ent, qoff);
+    it.new_kv = !(kReuse && tok0 == last_tok0 && head == last_head);
+    it.tok0 = tok0;
+    it.head = head;
+    it.tile0 = (int32_t)tiles;
+    tiles += (uint32_t)(it.kv_len + 127) >> 7;
+    last_tok0 = tok0;
+    last_head = head;
+    ends += it.done;
+    const int slot = n % kSlots;
+    if (n >= kSlots &&
+        !__all_sync(0xffffffffu, ptx::mbar_wait(ptx::smem_u32(&c.slot_free[slot]), ((n / kSlots) - 1) & 1)))
+      return false;
+    *reinterpret_cast<int4*>(&c.entry[slot][4 * lane]) = make_int4(ent[0], ent[1], ent[2], ent[3]);
+    *reinterpret_cast<longlong2*>(&c.qoff[slot][4 * lane]) = make_longlong2(qoff[0], qoff[1]);
+    *reinterpret_cast<longlong2*>(&c.qoff[slot][4 * lane + 2]) = make_longlong2(qoff[2], qoff[3]);
+    if constexpr (kRowIndex) {
+      int row[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) row[u] = ent[u] >= 0 ? (int)((uint32_t)ent[u] / (uint32_t)p.NP) : 0;
+      *reinterpret_cast<int4*>(&c.grow[slot][4 * lane]) = make_int4(row[0], row[1], row[2], row[3]);
+    }
+    if (lane == 0) c.item[slot] = it;
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive(ptx::smem_u32(&c.item_full[slot]));
+  }
+  return true;
+}
+
+__device__ __forceinline__ void store32(void* ptr, const uint32_t* v) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(ptr), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+               "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+               : "memory");
+}
+
+}  // namespace
+}  // namespace moba

@@ -1,0 +1,104 @@
+"""GPU: the dense-stage kernel for short items (chunks of at most 256 keys, and query windows with at
+most 128 rows per kv head) and the row gathers, at the sizes and strides where their branches change.
+
+Outputs are compared with the mma.sync dense stage.  Both round P to 16 bits and a partial row to 11
+significant bits and sum in fp32, so an output element, a weighted mean of values of order one, differs by the
+rounding of P (2^-9 bf16, 2^-11 fp16 relative, averaging out over the keys) and one rounding of the output:
+at most two units of the output type at magnitude 4, 2^-5 in bf16 and 2^-8 in fp16; the mean
+difference is an order of magnitude below one unit at magnitude 1."""
+import pytest
+import torch
+
+from baselinebenchmark_b200 import _lib, parallel
+from oracle import moba_oracle as O
+from tests import gpu_util as G
+
+pytestmark = pytest.mark.gpu
+
+DTYPES = [pytest.param(torch.bfloat16, id="bf16"), pytest.param(torch.float16, id="fp16")]
+
+
+def _inputs(lens, hq, hkv, d, chunk, dtype, seed):
+    q, k, v, cu = O.make_inputs(list(lens), hq, hkv, d, chunk, seed=seed)
+    return (*G.to_dev(q.to(dtype), k.to(dtype), v.to(dtype)), torch.from_numpy(cu).cuda())
+
+
+def _close(out, ref, dtype):
+    mx, mean = G.rel_stats(out, ref)
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert mx <= 8 * unit and mean <= 0.25 * unit, (mx, mean)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d", [64, 96, 128])
+@pytest.mark.parametrize("chunk", [16, 64, 127, 128, 129, 200, 256, 257])
+def test_chunk_sizes_around_the_tiles(chunk, d, dtype):
+    lens, hq, hkv, topk = (1, 130, 1025, 700), 6, 2, 5
+    q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, dtype, seed=chunk + d)
+    out, lse, sel = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True, return_selected=True)
+    ref, ref_lse, ref_sel = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True,
+                                                  return_selected=True, attend_impl=_lib.ATTEND_MMA_SYNC)
+    assert torch.equal(sel, ref_sel)
+    _close(out, ref, dtype)
+    assert (lse - ref_lse).abs().max().item() < 1e-3       # scores in fp32, exponentials to 7.5e-5
+
+
+@pytest.mark.parametrize("hq,hkv", [(4, 4), (8, 2), (16, 1)])
+@pytest.mark.parametrize("chunk", [128, 512, 4096])
+def test_windows_around_the_row_limit_equal_full_run(chunk, hq, hkv):
+    """128 rows per kv head is the largest window of the short kernel; one token more and, with chunks of
+    more than 256 keys, the 256-row kernel runs.  Windows cross chunk and sequence boundaries."""
+    lens, topk = (700, 5000), 4
+    q, k, v, cu = _inputs(lens, hq, hkv, 128, chunk, torch.bfloat16, seed=7)
+    full, lse, sel = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True, return_selected=True)
+    limit = 128 // (hq // hkv)
+    for begin in (0, 690, 700 + 505, 700 + 4096 - 3, 5700 - limit - 1):
+        for n in {1, 2, limit - 1, limit, limit + 1}:
+            if n < 1:
+                continue
+            o, l, s = parallel.moba_forward(q[begin:begin + n], k, v, cu, max(lens), chunk, topk, return_lse=True,
+                                            return_selected=True, q_token_begin=begin)
+            assert torch.equal(s, sel[:, :, begin:begin + n])
+            assert torch.equal(o, full[begin:begin + n]), (begin, n)
+            assert torch.equal(l, lse[:, begin:begin + n]), (begin, n)
+
+
+def _layouts(t, name):
+    """The same values in another memory layout."""
+    n, h, d = t.shape
+    if name == "fused":                                    # heads of a fused projection: gaps between tokens
+        return torch.cat([t, t[:, :1], t[:, :1]], 1)[:, :h]
+    if name == "head_major":                               # [H, T, D] storage
+        return t.permute(1, 0, 2).contiguous().permute(1, 0, 2)
+    if name == "padded_dim":                               # rows longer than head_dim
+        return torch.nn.functional.pad(t, (0, 8))[..., :d]
+    assert name == "odd_token"                             # token stride with no common row grid: the map has no form
+    store = torch.zeros(n * (h * d + 8), dtype=t.dtype, device=t.device)
+    view = store.as_strided((n, h, d), (h * d + 8, d, 1))
+    view.copy_(t)
+    return view
+
+
+@pytest.mark.parametrize("d", [64, 96, 128])
+@pytest.mark.parametrize("layout", ["fused", "head_major", "padded_dim", "odd_token"])
+@pytest.mark.parametrize("chunk", [128, 1024])
+def test_layouts_of_q_give_the_same_bits(chunk, layout, d):
+    """Forward, a decode-sized window and the gradients, with q rows reached through each form of the
+    row map and without one."""
+    lens, hq, hkv, topk = (1500, 2100), 4, 2, 3
+    q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, torch.bfloat16, seed=3)
+    args = (k, v, cu, max(lens), chunk, topk)
+    out, lse, sel = parallel.moba_forward(q, *args, return_lse=True, return_selected=True)
+    ql = _layouts(q, layout)
+    assert torch.equal(ql, q)
+    out2, lse2, sel2 = parallel.moba_forward(ql, *args, return_lse=True, return_selected=True)
+    assert torch.equal(sel2, sel) and torch.equal(out2, out) and torch.equal(lse2, lse)
+    w = parallel.moba_forward(ql[3590:3595], *args, q_token_begin=3590)[0]
+    assert torch.equal(w, out[3590:3595])
+    g = torch.randn_like(out)
+    dq, dk, dv = parallel.moba_backward(q, *args, out, lse, sel, g)
+    dq2, dk2, dv2 = parallel.moba_backward(ql, *args, out, lse, sel, g)
+    assert torch.equal(dq2, dq)
+    # the rows of a list are added in the order of the compaction: fp32 sums, one rounding to bf16
+    for a, b in ((dk2, dk), (dv2, dv)):
+        assert (a.float() - b.float()).abs().max().item() <= 2.0 ** -7 * b.float().abs().max().item()
