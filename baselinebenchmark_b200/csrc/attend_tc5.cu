@@ -1298,6 +1298,321 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
   if (warp == 5) tmem_dealloc(tmem, kCols);
 }
 
+// ---------------------------------------------------------------------------
+// head dim 256, chunks of at most kSmallChunk keys
+//
+// The operands, tensor memory and order of MMAs of attend_tc5_wide_kernel, with the roles of the kernel
+// above: one 128-row tile per work item, one CTA per SM, one flat stream of items and key tiles.  The
+// halves of Q, of K and of V have 32 KB slots of their own, each refilled as soon as the MMAs that read it
+// have executed.  Two softmax warpgroups take the items in turn: one computes the next item's softmax
+// while the other waits for its P.V and writes its rows.  The P.V of a tile can still be executing when
+// the softmax of the item's next tile wants to rescale O: that path waits for it.  Measured against the wide kernel,
+// 2 x 4096 tokens x 16 heads, chunk 128: 446 -> 324 us.  Long chunks stay with the wide kernel: 295 tokens behind
+// 22411, 16 heads, chunk 4096 take 200 us there and 236 here.
+// ---------------------------------------------------------------------------
+// warp 0 describes the items, 1 issues MMAs, 2 copies the lo half of the Q rows and requests K, 3 copies the hi half and
+// requests V; 4-7, 8-11: softmax of the even / odd items
+constexpr int kWideShortThreads = 384;
+
+struct WideShortCtrl {
+  static constexpr int kPrefix = kShortPrefix;
+  uint64_t q_full[2], k_full[2], v_full[2];        // halves landed
+  uint64_t q_free[2];                              // per item: its last Q.K^T has read the halves
+  uint64_t k_free[2];                              // per other key tile of an item: its Q.K^T has read the half of K
+  uint64_t v_free[2];                              // per key tile that a new V follows: its P.V has read the half
+  uint64_t s_full[2][2];                           // [warpgroup][S buffer]
+  uint64_t p_full[2], pv_full[2];                  // [warpgroup], once per key tile
+  uint64_t o_free;                                 // once per item: its rows of O have been read
+  uint64_t item_full[kShortSlots], slot_free[kShortSlots];
+  uint32_t tmem_slot;
+  volatile int32_t abort;
+  int32_t n_routed, n_items;
+  SlotRange own;
+  ShortItem item[kShortSlots];
+  alignas(16) int32_t entry[kShortSlots][kTileM];
+  alignas(16) int64_t qoff[kShortSlots][kTileM];
+  int32_t prefix_cache[kShortPrefix];
+};
+constexpr size_t kWideShortSmemBytes = 1024 + 6 * kTileBytes + sizeof(WideShortCtrl);
+static_assert(kWideShortSmemBytes <= 232448, "shared memory of one CTA");
+
+template <bool kHalf>
+__global__ void __launch_bounds__(kWideShortThreads, 1)
+attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
+                       const __grid_constant__ CUtensorMap tmap_v, const ShortArgs sa) {
+  constexpr int D = 256;
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const uint32_t sQ = smem_u32(smem);                       // lo, hi
+  const uint32_t sK = sQ + 2 * kTileBytes;                  // lo, hi
+  const uint32_t sV = sK + 2 * kTileBytes;                  // lo, hi
+  WideShortCtrl& c = *reinterpret_cast<WideShortCtrl*>(smem + 6 * kTileBytes);
+  const KernelArgs& a = sa.a;
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&c.q_full[i]), 32 + i);              // the copies of a warp's lanes; hi: and warp 2
+      mbar_init(smem_u32(&c.k_full[i]), 1);
+      mbar_init(smem_u32(&c.v_full[i]), 1);
+      mbar_init(smem_u32(&c.q_free[i]), 1);
+      mbar_init(smem_u32(&c.k_free[i]), 1);
+      mbar_init(smem_u32(&c.v_free[i]), 1);
+      mbar_init(smem_u32(&c.s_full[i][0]), 1);
+      mbar_init(smem_u32(&c.s_full[i][1]), 1);
+      mbar_init(smem_u32(&c.p_full[i]), kTileM);
+      mbar_init(smem_u32(&c.pv_full[i]), 1);
+    }
+    mbar_init(smem_u32(&c.o_free), kTileM);
+    for (int i = 0; i < kShortSlots; ++i) {
+      mbar_init(smem_u32(&c.item_full[i]), 1);
+      mbar_init(smem_u32(&c.slot_free[i]), 4);                // the softmax warps of the item
+    }
+    c.abort = 0;
+    fence_barrier_init();
+    prefetch_tmap(&tmap_k);
+    prefetch_tmap(&tmap_v);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&c.tmem_slot), kTmemCols);
+    tmem_relinquish();
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (threadIdx.x == 0) {
+    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
+    c.own = own_slot_range(p, a.cu);
+    c.n_items = c.n_routed + (sa.iq.grouped ? c.own.n * p.Hkv : own_item_count(c.own.n, p.Hq, p.C, kTileM));
+  }
+  if (p.hist > 0) fill_prefix_cache(c, a.tile_prefix, p.lists, kWideShortThreads);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = c.tmem_slot;
+
+  bool ok = true;                          // false: a wait of this role gave up
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity));
+    return ok;
+  };
+  if (warp == 0) {
+    if (p.C <= kBN) ok = describe_items<kShortSlots, 2, true, false>(p, sa.iq, c);
+    else ok = describe_items<kShortSlots, 2, false, false>(p, sa.iq, c);
+    if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
+  } else if (warp == 2 || warp == 3) {
+    // ---- Q rows (a half each); warp 2: K tiles, warp 3: V tiles
+    uint32_t kt = 0, vt = 0;               // k_free phases waited for, V tiles requested
+    const int hq = warp - 2;
+    for (int n = 0; ok; ++n) {
+      const int slot = n % kShortSlots;
+      if (!wait(&c.item_full[slot], (n / kShortSlots) & 1)) break;
+      if (c.item[slot].done) break;
+      const int tok0 = c.item[slot].tok0, head = c.item[slot].head, nrows = c.item[slot].nrows;
+      const int ntiles = (c.item[slot].kv_len + kBN - 1) / kBN;
+      const bool fresh = c.item[slot].new_kv != 0;
+      auto load = [&](uint32_t dst, const CUtensorMap* m, uint64_t* full, int h, int j) {
+        if (lane == 0) {
+          const uint32_t bar = smem_u32(full);
+          mbar_expect_tx(bar, kTileBytes);
+          tma_load_3d(dst, m, bar, h * 128, head, tok0 + j * kBN);
+          tma_load_3d(dst + kHalfBytes, m, bar, h * 128 + 64, head, tok0 + j * kBN);
+        }
+      };
+      if (warp == 2) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          if (n > 0 && !wait(&c.q_free[h], (n - 1) & 1)) break;
+          if (h == 1 && lane == 0) mbar_arrive(smem_u32(&c.q_full[1]));   // (nobody runs past a phase this warp waits for)
+          if (fresh) load(sK + h * kTileBytes, &tmap_k, &c.k_full[h], h, 0);
+          if (h == 0) {
+            copy_rows_async<16, 1>(sQ, a.q, 0, 0, nrows, [&](int r) { return c.qoff[slot][r]; });
+            cp_async_mbar_arrive(smem_u32(&c.q_full[0]));
+          }
+        }
+        for (int j = 1; ok && j < ntiles; ++j, ++kt)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (!wait(&c.k_free[h], kt & 1)) break;
+            load(sK + h * kTileBytes, &tmap_k, &c.k_full[h], h, j);
+          }
+      } else {
+        if (n > 0 && !wait(&c.q_free[1], (n - 1) & 1)) break;
+        copy_rows_async<16, 1>(sQ + hq * kTileBytes, a.q, 16, 0, nrows, [&](int r) { return c.qoff[slot][r]; });
+        cp_async_mbar_arrive(smem_u32(&c.q_full[1]));
+        if (fresh)
+          for (int j = 0; ok && j < ntiles; ++j, ++vt)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              if (vt > 0 && !wait(&c.v_free[h], (vt - 1) & 1)) break;
+              load(sV + h * kTileBytes, &tmap_v, &c.v_full[h], h, j);
+            }
+      }
+    }
+    if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
+  } else if (warp == 1) {
+    // ---- MMA issuer
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t dq = __shfl_sync(0xffffffffu, desc_lo(sQ, 16), 0);
+    const uint32_t dk = __shfl_sync(0xffffffffu, desc_lo(sK, 16), 0);
+    const uint32_t dv = __shfl_sync(0xffffffffu, desc_lo(sV, kHalfBytes), 0);
+    const uint32_t el = elect_one();
+    // the two streams: Q.K^T runs one key tile ahead of P.V
+    uint32_t gq = 0, kt = 0, vt = 0;       // key tiles whose Q.K^T has been issued; K, V tiles consumed
+    int nq = 0, jq = 0, tiles_q = 0;       // item and tile of the next Q.K^T; tiles of that item (0: not looked at yet)
+    bool fresh_q = false, end = false;
+    // Q.K^T of the next key tile; false when there is none (or a wait gave up)
+    auto qk = [&]() -> bool {
+      if (end) return false;
+      if (jq == 0) {
+        const int slot = nq % kShortSlots;
+        if (!wait(&c.item_full[slot], (nq / kShortSlots) & 1)) return false;
+        if (c.item[slot].done) { end = true; return false; }
+        tiles_q = (c.item[slot].kv_len + kBN - 1) / kBN;
+        fresh_q = c.item[slot].new_kv != 0;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (jq == 0) {
+          if (!wait(&c.q_full[h], nq & 1)) return false;
+          fence_proxy_async_smem();                           // rows written by cp.async, read by the tensor core
+        }
+        if (fresh_q && !wait(&c.k_full[h], kt & 1)) return false;
+        tc_fence_after();
+        if (el) {
+          if (h == 0) { if (gq & 1) issue_qk_wide<1, 0, kHalf>(tm, dq, dk); else issue_qk_wide<0, 0, kHalf>(tm, dq, dk); }
+          else        { if (gq & 1) issue_qk_wide<1, 1, kHalf>(tm, dq, dk); else issue_qk_wide<0, 1, kHalf>(tm, dq, dk); }
+          if (h == 1) tc_commit(smem_u32(&c.s_full[nq & 1][gq & 1]));
+          tc_commit(smem_u32(jq + 1 == tiles_q ? &c.q_free[h] : &c.k_free[h]));
+        }
+        __syncwarp();
+      }
+      if (fresh_q) ++kt;
+      ++gq;
+      if (++jq == tiles_q) { jq = 0; ++nq; }
+      return true;
+    };
+    uint32_t pph[2] = {0, 0};              // p_full phases
+    bool have = qk();
+    int np = 0, jp = 0, tiles_p = tiles_q;
+    uint32_t gp = 0;
+    bool fresh_p = fresh_q;
+    while (ok && have) {
+      const bool next = qk();
+      if (!ok) break;
+      const int x = np & 1;
+      if (!wait(&c.p_full[x], x ? pph[1] : pph[0])) break;
+      if (x) pph[1] ^= 1; else pph[0] ^= 1;
+      if (jp == 0 && np > 0 && !wait(&c.o_free, (np - 1) & 1)) break;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        if (fresh_p && !wait(&c.v_full[h], vt & 1)) break;
+        tc_fence_after();
+        if (el) {
+          if (h == 0) { if (gp & 1) issue_pv_wide<1, 0, kHalf>(tm, dv, jp == 0); else issue_pv_wide<0, 0, kHalf>(tm, dv, jp == 0); }
+          else        { if (gp & 1) issue_pv_wide<1, 1, kHalf>(tm, dv, jp == 0); else issue_pv_wide<0, 1, kHalf>(tm, dv, jp == 0); }
+          if (next && fresh_q) tc_commit(smem_u32(&c.v_free[h]));       // (the stream is one tile ahead: fresh_q is the next tile's)
+          if (h == 1) tc_commit(smem_u32(&c.pv_full[x]));
+        }
+        __syncwarp();
+      }
+      if (!ok) break;
+      if (fresh_p) ++vt;
+      ++gp;
+      if (++jp == tiles_p) { jp = 0; ++np; tiles_p = tiles_q; }
+      fresh_p = fresh_q;
+      have = next;
+    }
+    if (!ok && lane == 0) { atomicExch(a.status, ST_MMA); c.abort = 1; }
+  } else {
+    // ---- softmax + epilogue, one thread per row; warpgroup x takes items x, x + 2, ...
+    const int x = (warp >> 2) - 1;
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t tO = tmem + lane_base + 256;
+    const float sl2 = rsqrtf((float)D) * 1.4426950408889634f;
+    uint32_t sph0 = 0, sph1 = 0, pvph = 0;                     // phases of s_full[x][0], [1] and pv_full[x]
+    for (int n = x; ok; n += 2) {
+      const int slot = n % kShortSlots;
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.item_full[slot]), (n / kShortSlots) & 1));
+      if (!ok) break;
+      const ShortItem it = c.item[slot];
+      if (it.done) break;
+      const int32_t e = c.entry[slot][row];
+      const bool active = (warp & 3) * 32 < it.nrows;         // warps without rows only keep the barriers going
+      const int ntiles = (it.kv_len + kBN - 1) / kBN;
+      const int qrel = it.tok_rel + (it.group == 1 ? row : row / it.group);
+      const int lim = it.causal ? min(it.kv_len, qrel + 1) : it.kv_len;
+      float m_ref = -INFINITY, l = 0.f;
+      for (int j = 0; j < ntiles; ++j) {
+        const uint32_t buf = (uint32_t)(it.tile0 + j) & 1;
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.s_full[x][buf]), buf ? sph1 : sph0));
+        if (!ok) break;
+        if (buf) sph1 ^= 1; else sph0 ^= 1;
+        // the item's Q.K^T has run: every role has read its description
+        if (j == 0 && lane == 0) mbar_arrive(smem_u32(&c.slot_free[slot]));
+        // the P.V of the tile before must have executed before O is touched
+        bool waited = j == 0;
+        auto wait_pv = [&] {
+          if (!waited && !mbar_wait(smem_u32(&c.pv_full[x]), pvph)) ok = false;
+          waited = true;
+          tc_fence_after();
+        };
+        if (active) {
+          tc_fence_after();
+          const int key0 = j * kBN;
+          const bool masked = key0 + kBN > it.kv_len || (it.causal && key0 + kBN - 1 > it.tok_rel);
+          const uint32_t tS = tmem + lane_base + buf * kBN;
+          if (masked) softmax_row_rolled<true, kHalf, D>(tS, tO, j, key0, lim, sl2, m_ref, l, wait_pv);
+          else softmax_row_rolled<false, kHalf, D>(tS, tO, j, key0, lim, sl2, m_ref, l, wait_pv);
+        }
+        // every completion of pv_full is waited for before the next P is published, so that a phase is
+        // never passed by
+        if (j > 0) {
+          wait_pv();
+          pvph ^= 1;
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_before();
+        mbar_arrive(smem_u32(&c.p_full[x]));
+      }
+      if (!ok) break;
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.pv_full[x]), pvph));
+      if (!ok) break;
+      pvph ^= 1;
+      if (active) {
+        tc_fence_after();
+        // the row's largest magnitude over all 256 dims decides the power of two of its fp16 copy
+        const float amax = amax_row_rolled<D>(tO);
+        const float inv = 1.f / l;
+        const PartialScale ps = partial_scale(amax * inv);
+        store_row_rolled<D>(tO, a.partial_out + (int64_t)(e >= 0 ? e : 0) * D, inv * ps.scale, e >= 0, a.wide_store != 0, [&] {
+          tc_fence_before();
+          mbar_arrive(smem_u32(&c.o_free));                   // O may be overwritten
+        });
+        if (e >= 0) a.partial_lse[e] = make_float2((m_ref + log2f(l)) * 0.6931471805599453f, ps.inv);
+      } else {
+        mbar_arrive(smem_u32(&c.o_free));
+      }
+    }
+    if (!ok) {
+      atomicExch(a.status, ST_SOFTMAX);
+      c.abort = 1;
+    }
+  }
+
+  __syncwarp();
+  __syncthreads();
+  if (c.abort) {                           // copies in flight land before shared memory is given up
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, kTmemCols);
+}
+
 // One warp waits, with the same bounded wait every role of the dense stage uses, on a barrier
 // nobody ever arrives on: the wait gives up after `limit_ns`, the status word is set like the
 // kernel would set it, and the warp returns.  Lets a test see the give-up path without a fault.
@@ -1369,12 +1684,13 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
   const KernelArgs args{q, cu, list_counts, list_offsets, tile_prefix, row_list, partial_out, partial_lse,
                         work_counter, status, ((uintptr_t)partial_out & 31) == 0};
   cudaError_t e;
-  if (tc5_short_items(p.D, p.C, p.Tq, p.G)) {
-    auto kern = p.D == 128 ? (p.fp16 ? attend_tc5_short_kernel<true, 128> : attend_tc5_short_kernel<false, 128>)
+  if (p.D == 256 ? p.C <= kSmallChunk : tc5_short_items(p.D, p.C, p.Tq, p.G)) {
+    auto kern = p.D == 256 ? (p.fp16 ? attend_tc5_wide_short_kernel<true> : attend_tc5_wide_short_kernel<false>)
+              : p.D == 128 ? (p.fp16 ? attend_tc5_short_kernel<true, 128> : attend_tc5_short_kernel<false, 128>)
               : p.D == 96  ? (p.fp16 ? attend_tc5_short_kernel<true, 96> : attend_tc5_short_kernel<false, 96>)
                            : (p.fp16 ? attend_tc5_short_kernel<true, 64> : attend_tc5_short_kernel<false, 64>);
-    const int threads = kShortThreads, ctas = 2 * sms;
-    const size_t smem = kShortSmemBytes;
+    const int threads = p.D == 256 ? kWideShortThreads : kShortThreads, ctas = p.D == 256 ? sms : 2 * sms;
+    const size_t smem = p.D == 256 ? kWideShortSmemBytes : kShortSmemBytes;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     ShortArgs sa;
