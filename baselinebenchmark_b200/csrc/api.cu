@@ -587,7 +587,7 @@ int moba_backward(const moba_problem_t* p, const void* q, const void* k, const v
   if (r.hist > 0) {
     if ((e = launch_count_lists(r, selected, w.list_counts, st)) != cudaSuccess) return (int)e;
     if ((e = launch_compact(r, cu, selected, w.list_counts, w.list_offsets, w.tile_prefix, w.cursors, w.row_list,
-                            w.partial_lse, dq_tc5 ? kTc5TileRows : kMmaTileRows, st)) != cudaSuccess)
+                            w.partial_lse, !dq_tc5 ? kMmaTileRows : bwd_dq_short_items(r) ? kTileRowsWide : kTc5TileRows, st)) != cudaSuccess)
       return (int)e;
   }
   if ((e = launch_bwd_delta(r, static_cast<const __nv_bfloat16*>(out), gb, qt, hd, lse, delta, lse2, st)) != cudaSuccess)

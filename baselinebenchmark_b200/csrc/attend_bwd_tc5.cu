@@ -18,14 +18,18 @@
 // scale * dQ as an fp32 partial into the row's slot (own chunk = 0, rank r = r + 1); a later
 // kernel adds a row's slots.  No atomics: the result is bit-identical run to run.
 //
-// Warp roles (384 threads) as in the forward kernel: warp 0 TMA producer (K tiles in three
-// stages, V tiles in two), warp 1 MMA issuer and owner of the TMEM allocation, warp 2 draws and resolves
-// the next item, warps 4-7 / 8-11 the rows of tile A / B.
+// Warp roles (512 threads), in one flat stream of items and key tiles without a CTA-wide barrier: warp 0 TMA
+// producer (K tiles in three stages, V tiles in two), warp 1 MMA issuer and owner of the TMEM allocation,
+// warp 2 draws and resolves the next item, warps 4-7 / 8-11 the rows of tile A / B, warps 12-15 copy a tile's Q
+// and dO rows (cp.async) as soon as the last S / dP of the item before has executed.  When the row threads
+// gathered their rows behind a barrier at the item's start the kernel took 950 us on 19456 tokens x 32 heads,
+// chunk 512, 837 us this way.
 // TMEM columns of row tile X: S 128X..128X+63 (dS, 16-bit, overwrites the first 32),
 // dP 128X+64..128X+127, dQ 256+128X..; 512 columns in all, which is why a key step is 64 wide.
 // Every wait is bounded; a wait that gives up sets a status word that the summing kernel
 // turns into NaN results.
 #include "common.cuh"
+#include "short_items.cuh"
 #include "sm100_ptx.cuh"
 
 namespace moba {
@@ -38,7 +42,7 @@ namespace {
 
 using namespace ptx;
 
-constexpr int kThreads = 384;
+constexpr int kThreads = 512;
 constexpr int kTileM = 128;                 // rows per MMA tile
 constexpr int kBN = 64;                     // keys per step
 constexpr int kQBlockBytes = 128 * 64 * 2;  // one [128 rows][64 dims] swizzled block of Q or dO
@@ -57,10 +61,11 @@ enum { ST_OK = 0, ST_PRODUCER = 11, ST_MMA = 12, ST_ROWS = 13 };
 struct Ctrl {
   uint64_t k_full[kKStages], k_empty[kKStages], v_full[2], v_empty[2];
   uint64_t s_full[2], ds_full[2], dq_full[2];
-  uint64_t item_ready[2];
+  uint64_t rows_full[2], rows_free[2];       // per item: Q and dO of tile A / B landed; its last S / dP has executed
+  uint64_t item_full[2], slot_free[2];
   uint32_t tmem_slot;
   volatile int32_t abort;
-  Item item[2];                              // slot (n & 1) holds item n, resolved one item ahead
+  Item item[2];                              // slot (n & 1) holds item n, described an item ahead
   int32_t done[2];
   int64_t qoff[2][2 * kTileM];               // element offset of the row in q
   int32_t grow[2][2 * kTileM];               // row index t * Hq + h (dO, lse and delta are indexed by it)
@@ -84,11 +89,12 @@ struct KernelArgs {
   float* partial_dq;
   int32_t* work_counter;
   int32_t* status;
+  int32_t wide_store;                        // partial_dq is 32-byte aligned
 };
 
-// One spare warp, one item ahead of the others: draws the next item from the global queue,
-// decodes it and resolves its rows into prefetch slot `slot`.
-__device__ __forceinline__ void prefetch_item(const Params& p, const KernelArgs& a, Ctrl& c, int slot,
+// One warp, an item ahead of the others: draws the next item from the global queue, decodes it,
+// resolves its rows into slot `slot` and publishes it.  False when the queue is empty.
+__device__ __forceinline__ bool describe_item(const Params& p, const KernelArgs& a, Ctrl& c, int slot,
                                               int n_routed, int n_items) {
   const int lane = threadIdx.x & 31;
   Item it;
@@ -129,61 +135,11 @@ __device__ __forceinline__ void prefetch_item(const Params& p, const KernelArgs&
       c.entry[slot][r] = e;
       c.qoff[slot][r] = off;
       c.grow[slot][r] = row;
-      if (e >= 0) {                                            // the gather of the next item then hits L2
-        const __nv_bfloat16* g = a.dout + (int64_t)row * p.D;
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(a.q + off));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(g));
-        if (p.D > 64) {
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(a.q + off + 64));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(g + 64));
-        }
-      }
     }
   }
   __syncwarp();
-  if (lane == 0) mbar_arrive(smem_u32(&c.item_ready[slot]));
-}
-
-// Common head of an item, executed by all 384 threads: take the prefetched item of slot
-// `slot`; the 256 row threads (kGather) gather its Q and dO rows into 128-byte-swizzled
-// tiles (Q tile A, Q tile B, dO tile A, dO tile B).  Returns false when the queue is empty.
-template <bool kGather, int D>
-__device__ __forceinline__ bool next_item(const KernelArgs& a, Ctrl& c, unsigned char* smem, int slot, Item& it) {
-  __syncthreads();
-  if (c.done[slot]) return false;
-  it = c.item[slot];
-  if (kGather) {
-    const int32_t* entry = c.entry[slot];
-    const int64_t* qoff = c.qoff[slot];
-    const int32_t* grow = c.grow[slot];
-    constexpr int kChunks = D / 8;                  // 16-byte pieces of a row
-    const int t = threadIdx.x - 128;
-#pragma unroll 1
-    for (int which = 0; which < 2; ++which) {
-      uint4 val[kChunks];
-#pragma unroll
-      for (int u = 0; u < kChunks; ++u) {
-        const int i = t + u * 256;
-        const int r = i / kChunks, ch = i % kChunks;
-        val[u] = make_uint4(0, 0, 0, 0);
-        if (entry[r] >= 0) {
-          const __nv_bfloat16* src = which == 0 ? a.q + qoff[r] : a.dout + (int64_t)grow[r] * D;
-          val[u] = __ldg(reinterpret_cast<const uint4*>(src + ch * 8));
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kChunks; ++u) {
-        const int i = t + u * 256;
-        const int r = i / kChunks, ch = i % kChunks;
-        const uint32_t dst = (uint32_t)(which * 2 * kQTileBytes + (r >> 7) * kQTileBytes + (ch >> 3) * kQBlockBytes +
-                                        (r & 127) * 128 + (((ch & 7) ^ (r & 7)) << 4));
-        *reinterpret_cast<uint4*>(smem + dst) = val[u];
-      }
-    }
-  }
-  fence_proxy_async_smem();
-  __syncthreads();
-  return true;
+  if (lane == 0) mbar_arrive(smem_u32(&c.item_full[slot]));
+  return done == 0;
 }
 
 // Exponentials evaluated with the cubic on the FMA pipe instead of the special-function
@@ -200,23 +156,23 @@ constexpr int kPolyPairs = MOBA_BWD_POLY_PAIRS;
 // Rows that do not exist carry lse = +inf (p = 0) and zero Q / dO rows.
 template <bool kMasked, bool kHalf>
 __device__ __forceinline__ void ds_row(uint32_t tS, int key0, int lim, float sl2, float neg_lse2, float delta) {
-  uint32_t s[64], g[64];
-  tmem_ld64(tS, s);
-  tmem_ld64(tS + 64, g);
-  tmem_wait_ld();
-  if (kMasked) {
-#pragma unroll
-    for (int i = 0; i < 64; ++i) s[i] = (key0 + i < lim) ? s[i] : 0xff800000u;   // -inf: p = 0
-  }
+  // 32 keys at a time: with sixteen warps a thread has 128 registers
   const uint64_t scale2 = pack2(sl2, sl2);
   const uint64_t nl2 = pack2(neg_lse2, neg_lse2);
   const uint64_t dl2 = pack2(delta, delta);
-#pragma unroll
+#pragma unroll 1
   for (int ch = 0; ch < 2; ++ch) {
-    uint32_t pk[16];
+    uint32_t s[32], g[32], pk[16];
+    tmem_ld32(tS + ch * 32, s);
+    tmem_ld32(tS + 64 + ch * 32, g);
+    tmem_wait_ld();
+    if (kMasked) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) s[i] = (i < lim - key0 - ch * 32) ? s[i] : 0xff800000u;   // -inf: p = 0
+    }
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const int e = ch * 32 + 2 * i;
+      const int e = 2 * i;
       const uint64_t x = fma2(pack2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), scale2, nl2);
       uint64_t pr;
       if (!kMasked && (i & 7) < kPolyPairs) pr = ex2_poly2(x);
@@ -291,7 +247,10 @@ bwd_dq_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
       mbar_init(smem_u32(&c.s_full[i]), 1);
       mbar_init(smem_u32(&c.ds_full[i]), kTileM);
       mbar_init(smem_u32(&c.dq_full[i]), 1);
-      mbar_init(smem_u32(&c.item_ready[i]), 1);
+      mbar_init(smem_u32(&c.rows_full[i]), 4 * 32);          // the copies of four warps' lanes
+      mbar_init(smem_u32(&c.rows_free[i]), 1);
+      mbar_init(smem_u32(&c.item_full[i]), 1);
+      mbar_init(smem_u32(&c.slot_free[i]), 8);               // the row warps
     }
     c.abort = 0;
     fence_barrier_init();
@@ -311,14 +270,73 @@ bwd_dq_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
 
   const int n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
   const int n_items = n_routed + own_item_count(p.slots, p.Hq, p.C, 2 * kTileM);
-  Item it;
 
-  if (warp < 4) {
-    // =============================================== warps 0-3: TMA producer, MMA issuer, item prefetch
-    setmaxnreg_dec<72>();
-    uint32_t g = 0;                        // K/V tiles produced (warp 0) or consumed (warp 1) so far
-    uint32_t pph0 = 0, pph1 = 0;           // ds_full phases of tile A / B
-    int pre = 0;                           // producer: tiles of the coming item already requested
+  bool ok = true;                            // false: a wait of this role gave up
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity));
+    return ok;
+  };
+  // item n: slot n & 1, phase n >> 1 of its barriers; false at the end of the queue (or after a wait gave up)
+  auto take = [&](int n) { return wait(&c.item_full[n & 1], (n >> 1) & 1) && !c.done[n & 1]; };
+
+  if (warp == 2) {
+    // =============================================== describes the items
+    for (int n = 0;; ++n) {
+      if (n >= 2 && !wait(&c.slot_free[n & 1], ((n >> 1) - 1) & 1)) break;
+      if (!describe_item(p, a, c, n & 1, n_routed, n_items)) break;
+    }
+    if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
+  } else if (warp == 0) {
+    // =============================================== K / V tiles, as far ahead as stages are free
+    uint32_t g = 0;
+    for (int n = 0; take(n); ++n) {
+      const int ntiles = (c.item[n & 1].kv_len + kBN - 1) / kBN;
+      const int tok0 = c.item[n & 1].kv_tok0, head = c.item[n & 1].kv_head;
+      for (int j = 0; ok && j < ntiles; ++j, ++g) {
+        const int tok = tok0 + j * kBN;
+        {
+          const uint32_t s = g % kKStages, par = ((g / kKStages) & 1) ^ 1;
+          if (!wait(&c.k_empty[s], par)) break;
+          if (lane == 0) {
+            const uint32_t bar = smem_u32(&c.k_full[s]);
+            mbar_expect_tx(bar, ((D + 63) / 64) * kKvBlockBytes);
+            tma_load_3d(sK + s * kKvTileBytes, &tmap_k, bar, 0, head, tok);
+            if (D > 64) tma_load_3d(sK + s * kKvTileBytes + kKvBlockBytes, &tmap_k, bar, 64, head, tok);
+          }
+        }
+        {
+          const uint32_t s = g & 1, par = ((g >> 1) & 1) ^ 1;
+          if (!wait(&c.v_empty[s], par)) break;
+          if (lane == 0) {
+            const uint32_t bar = smem_u32(&c.v_full[s]);
+            mbar_expect_tx(bar, ((D + 63) / 64) * kKvBlockBytes);
+            tma_load_3d(sV + s * kKvTileBytes, &tmap_v, bar, 0, head, tok);
+            if (D > 64) tma_load_3d(sV + s * kKvTileBytes + kKvBlockBytes, &tmap_v, bar, 64, head, tok);
+          }
+        }
+      }
+      if (!ok) break;
+    }
+    if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
+  } else if (warp >= 12) {
+    // =============================================== Q and dO rows: a tile's as soon as the last S / dP of the
+    // item before has executed, while its dQ is still being computed and written
+    for (int n = 0; take(n); ++n) {
+      const int slot = n & 1, nrows = c.item[slot].nrows;
+      for (int x = 0; x < 2; ++x) {
+        if (n > 0 && !wait(&c.rows_free[x], (n - 1) & 1)) break;
+        const int rows = min(max(nrows - x * kTileM, 0), kTileM);
+        copy_rows_async<D / 8, 4>(sQ + x * kQTileBytes, a.q, 0, warp - 12, rows,
+                                  [&](int r) { return c.qoff[slot][x * kTileM + r]; });
+        copy_rows_async<D / 8, 4>(sG + x * kQTileBytes, a.dout, 0, warp - 12, rows,
+                                  [&](int r) { return (int64_t)c.grow[slot][x * kTileM + r] * D; });
+        cp_async_mbar_arrive(smem_u32(&c.rows_full[x]));
+      }
+      if (!ok) break;
+    }
+    if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
+  } else if (warp == 1) {
+    // =============================================== MMA issuer: the whole warp runs convergent, one elected lane issues
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
     const uint32_t dq = __shfl_sync(0xffffffffu, desc_lo(sQ, 16), 0);
     const uint32_t dg = __shfl_sync(0xffffffffu, desc_lo(sG, 16), 0);
@@ -326,113 +344,69 @@ bwd_dq_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
     const uint32_t dv = __shfl_sync(0xffffffffu, desc_lo(sV, 16), 0);
     const uint32_t dkt = __shfl_sync(0xffffffffu, desc_lo(sK, kKvBlockBytes), 0);
     const uint32_t el = elect_one();
-    for (int n = 0;; ++n) {
-      if (warp == 2) prefetch_item(p, a, c, n & 1, n_routed, n_items);
-      if (!next_item<false, D>(a, c, smem, n & 1, it)) break;
-      const int ntiles = (it.kv_len + kBN - 1) / kBN;
-      if (warp == 0 && lane == 0) {
-        // K and V tile `j` of item `w` into the next stage; false after a timeout
-        auto load_tile = [&](const Item& w, int j) -> bool {
-          const int tok = w.kv_tok0 + j * kBN;
-          {
-            const uint32_t s = g % kKStages, par = ((g / kKStages) & 1) ^ 1;
-            if (!mbar_wait(smem_u32(&c.k_empty[s]), par)) return false;
-            const uint32_t bar = smem_u32(&c.k_full[s]);
-            mbar_expect_tx(bar, ((D + 63) / 64) * kKvBlockBytes);
-            tma_load_3d(sK + s * kKvTileBytes, &tmap_k, bar, 0, w.kv_head, tok);
-            if (D > 64) tma_load_3d(sK + s * kKvTileBytes + kKvBlockBytes, &tmap_k, bar, 64, w.kv_head, tok);
-          }
-          {
-            const uint32_t s = g & 1, par = ((g >> 1) & 1) ^ 1;
-            if (!mbar_wait(smem_u32(&c.v_empty[s]), par)) return false;
-            const uint32_t bar = smem_u32(&c.v_full[s]);
-            mbar_expect_tx(bar, ((D + 63) / 64) * kKvBlockBytes);
-            tma_load_3d(sV + s * kKvTileBytes, &tmap_v, bar, 0, w.kv_head, tok);
-            if (D > 64) tma_load_3d(sV + s * kKvTileBytes + kKvBlockBytes, &tmap_v, bar, 64, w.kv_head, tok);
-          }
-          ++g;
-          return true;
-        };
-        bool alive = true;
-        for (int j = pre; alive && j < ntiles; ++j) alive = load_tile(it, j);
-        pre = 0;
-        // first tiles of the next item as soon as stages free up
-        if (alive) {
-          const int s1 = (n + 1) & 1;
-          alive = mbar_wait(smem_u32(&c.item_ready[s1]), ((n + 1) >> 1) & 1);
-          if (alive && !c.done[s1]) {
-            const Item nx = c.item[s1];
-            const int nt = min(2, (nx.kv_len + kBN - 1) / kBN);
-            for (; alive && pre < nt; ++pre) alive = load_tile(nx, pre);
-          }
-        }
-        if (!alive) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
-      } else if (warp == 1) {
-        // MMA issuer: the whole warp runs convergent, one elected lane issues.
-        bool ok = true;
-        constexpr uint32_t kStageDesc = kKvTileBytes >> 4;
-        tc_fence_after();
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.k_full[g % kKStages]), (g / kKStages) & 1));
-        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.v_full[g & 1]), (g >> 1) & 1));
-        if (ok) {
-          tc_fence_after();
-          if (el) {
-            const uint32_t ko = (g % kKStages) * kStageDesc, vo = (g & 1) * kStageDesc;
-            issue_s_dp<0, kHalf, D>(tm, dq, dg, dk + ko, dv + vo);
-            tc_commit(smem_u32(&c.s_full[0]));
-            issue_s_dp<1, kHalf, D>(tm, dq, dg, dk + ko, dv + vo);
-            tc_commit(smem_u32(&c.s_full[1]));
-            tc_commit(smem_u32(&c.v_empty[g & 1]));
-          }
-          __syncwarp();
-        }
-        for (int j = 0; ok && j < ntiles; ++j) {
-          const bool more = j + 1 < ntiles;
-          const uint32_t kcur = g % kKStages, g1 = g + 1, knxt = g1 % kKStages, vnxt = g1 & 1;
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.ds_full[0]), pph0));
-          if (!ok) break;
+    constexpr uint32_t kStageDesc = kKvTileBytes >> 4;
+    uint32_t g = 0;                          // key tiles whose dQ has been issued
+    uint32_t pph0 = 0, pph1 = 0;             // ds_full phases of tile A / B
+    // S and dP of tile x for key tile `gt` of the CTA: step j of `ntiles` of item n
+    auto s_dp = [&](int x, int n, int j, int ntiles, uint32_t gt) {
+      if (j == 0) {
+        if (!wait(&c.rows_full[x], n & 1)) return;
+        fence_proxy_async_smem();                             // rows written by cp.async, read by the tensor core
+      }
+      if (x == 0 && (!wait(&c.k_full[gt % kKStages], (gt / kKStages) & 1) || !wait(&c.v_full[gt & 1], (gt >> 1) & 1))) return;
+      tc_fence_after();
+      if (el) {
+        const uint32_t ko = (gt % kKStages) * kStageDesc, vo = (gt & 1) * kStageDesc;
+        if (x == 0) issue_s_dp<0, kHalf, D>(tm, dq, dg, dk + ko, dv + vo);
+        else issue_s_dp<1, kHalf, D>(tm, dq, dg, dk + ko, dv + vo);
+        tc_commit(smem_u32(&c.s_full[x]));
+        if (j + 1 == ntiles) tc_commit(smem_u32(&c.rows_free[x]));
+        if (x == 1) tc_commit(smem_u32(&c.v_empty[gt & 1]));
+      }
+      __syncwarp();
+    };
+    if (take(0)) {
+      int ntiles = (c.item[0].kv_len + kBN - 1) / kBN;
+      s_dp(0, 0, 0, ntiles, 0);
+      if (ok) s_dp(1, 0, 0, ntiles, 0);
+      for (int n = 0; ok; ++n) {
+        int next_tiles = 0;                  // key tiles of item n + 1 (0: there is none)
+        for (int j = 0; ok && j < ntiles; ++j, ++g) {
+          const bool last = j + 1 == ntiles;
+          const uint32_t kcur = g % kKStages;
+          if (!wait(&c.ds_full[0], pph0)) break;
           pph0 ^= 1;
           tc_fence_after();
-          if (el) issue_dq<0, kHalf, D>(tm, dkt + kcur * kStageDesc, j == 0);
-          __syncwarp();
-          if (more) {
-            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.k_full[knxt]), (g1 / kKStages) & 1));
-            if (ok) ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.v_full[vnxt]), (g1 >> 1) & 1));
-            if (!ok) break;
-            tc_fence_after();
-            if (el) {
-              issue_s_dp<0, kHalf, D>(tm, dq, dg, dk + knxt * kStageDesc, dv + vnxt * kStageDesc);
-              tc_commit(smem_u32(&c.s_full[0]));
-            }
-          } else if (el) {
-            tc_commit(smem_u32(&c.dq_full[0]));
+          if (el) {
+            issue_dq<0, kHalf, D>(tm, dkt + kcur * kStageDesc, j == 0);
+            if (last) tc_commit(smem_u32(&c.dq_full[0]));
           }
           __syncwarp();
-          ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.ds_full[1]), pph1));
-          if (!ok) break;
+          if (last) {
+            if (take(n + 1)) next_tiles = (c.item[(n + 1) & 1].kv_len + kBN - 1) / kBN;
+            if (!ok) break;
+          }
+          if (!last) s_dp(0, n, j + 1, ntiles, g + 1);
+          else if (next_tiles > 0) s_dp(0, n + 1, 0, next_tiles, g + 1);
+          if (!ok || !wait(&c.ds_full[1], pph1)) break;
           pph1 ^= 1;
           tc_fence_after();
           if (el) {
             issue_dq<1, kHalf, D>(tm, dkt + kcur * kStageDesc, j == 0);
             tc_commit(smem_u32(&c.k_empty[kcur]));
-            if (more) {
-              issue_s_dp<1, kHalf, D>(tm, dq, dg, dk + knxt * kStageDesc, dv + vnxt * kStageDesc);
-              tc_commit(smem_u32(&c.s_full[1]));
-              tc_commit(smem_u32(&c.v_empty[vnxt]));
-            } else {
-              tc_commit(smem_u32(&c.dq_full[1]));
-            }
+            if (last) tc_commit(smem_u32(&c.dq_full[1]));
           }
           __syncwarp();
-          ++g;
+          if (!last) s_dp(1, n, j + 1, ntiles, g + 1);
+          else if (next_tiles > 0) s_dp(1, n + 1, 0, next_tiles, g + 1);
         }
-        if (!ok && lane == 0) { atomicExch(a.status, ST_MMA); c.abort = 1; }
+        if (next_tiles == 0) break;
+        ntiles = next_tiles;
       }
-      __syncwarp();
     }
-  } else {
+    if (!ok && lane == 0) { atomicExch(a.status, ST_MMA); c.abort = 1; }
+  } else if (warp >= 4) {
     // =============================================== warps 4-11: one thread per row
-    setmaxnreg_inc<216>();
     const int x = (warp - 4) >> 2;                       // 0: tile A, 1: tile B
     const int row = (warp & 3) * 32 + lane;              // row inside the tile = TMEM lane
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
@@ -440,72 +414,386 @@ bwd_dq_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
     const uint32_t tDQ = tmem + lane_base + 256 + x * 128;
     const float scale = rsqrtf((float)D);
     const float sl2 = scale * 1.4426950408889634f;
-    uint32_t sph = 0, oph = 0;                           // s_full / dq_full phases of this tile
-    for (int n = 0; next_item<true, D>(a, c, smem, n & 1, it); ++n) {
-      const int32_t e = c.entry[n & 1][x * kTileM + row];
+    uint32_t sph = 0;                                    // s_full phase of this tile
+    for (int n = 0; take(n); ++n) {
+      const int slot = n & 1;
+      const int32_t e = c.entry[slot][x * kTileM + row];
+      const int kv_len = c.item[slot].kv_len, causal = c.item[slot].causal;
+      const int rel = c.item[slot].tok0 + x * kTileM - c.item[slot].kv_tok0;   // own chunk: position of the tile's first row
       float neg_lse2 = -INFINITY, delta = 0.f;
       if (e >= 0) {
-        const int32_t gr = c.grow[n & 1][x * kTileM + row];
+        const int32_t gr = c.grow[slot][x * kTileM + row];
         neg_lse2 = -__ldg(a.lse2 + gr);
         delta = __ldg(a.delta + gr);
       }
-      const int ntiles = (it.kv_len + kBN - 1) / kBN;
-      const int qpos = it.tok0 + x * kTileM + row;
-      const int lim = it.causal ? min(it.kv_len, qpos - it.kv_tok0 + 1) : it.kv_len;   // keys < lim are visible
-      bool ok = true;
-      for (int j = 0; ok && j < ntiles; ++j) {
-        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.s_full[x]), sph));   // warp-uniform exit
-        if (!ok) break;
+      const int ntiles = (kv_len + kBN - 1) / kBN;
+      const int lim = causal ? min(kv_len, rel + row + 1) : kv_len;            // keys < lim are visible
+      for (int j = 0; j < ntiles; ++j) {
+        if (!wait(&c.s_full[x], sph)) break;
         sph ^= 1;
+        // the item's S has run: every role but the other tile's row warps has read its description
+        if (j == 0 && lane == 0) mbar_arrive(smem_u32(&c.slot_free[slot]));
         tc_fence_after();
         const int key0 = j * kBN;
-        const bool masked = key0 + kBN > it.kv_len ||
-                            (it.causal && it.kv_tok0 + key0 + kBN - 1 > it.tok0 + x * kTileM);
+        const bool masked = key0 + kBN > kv_len || (causal && key0 + kBN - 1 > rel);
         if (masked) ds_row<true, kHalf>(tS, key0, lim, sl2, neg_lse2, delta);
         else ds_row<false, kHalf>(tS, key0, lim, sl2, neg_lse2, delta);
         tc_fence_before();
         mbar_arrive(smem_u32(&c.ds_full[x]));
       }
-      if (ok) ok = mbar_wait(smem_u32(&c.dq_full[x]), oph);
-      ok = __all_sync(0xffffffffu, ok);
-      if (ok) {
-        oph ^= 1;
-        tc_fence_after();
-        // dQ rows go through this warp's 8 KB of the (now idle) Q tile so that every global
-        // store writes whole 128-byte pieces of four rows: 32 columns at a time, rows 144
-        // bytes apart in shared memory.
-        unsigned char* stage = smem + x * kQTileBytes + (warp & 3) * 8192;
+      if (!ok || !wait(&c.dq_full[x], n & 1)) break;
+      tc_fence_after();
+      float* dst = a.partial_dq + (int64_t)(e >= 0 ? e : 0) * D;
+#pragma unroll
+      for (int ch = 0; ch < D; ch += 32) {
         uint32_t v[32];
+        tmem_ld32(tDQ + ch, v);
+        tmem_wait_ld();
+        if (e >= 0) {
 #pragma unroll
-        for (int ch = 0; ch < D / 32; ++ch) {
-          tmem_ld32(tDQ + ch * 32, v);
-          tmem_wait_ld();
+          for (int i = 0; i < 32; i += 8) {
+            uint32_t o[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
-            *reinterpret_cast<float4*>(stage + lane * 144 + i * 16) =
-                make_float4(__uint_as_float(v[4 * i]) * scale, __uint_as_float(v[4 * i + 1]) * scale,
-                            __uint_as_float(v[4 * i + 2]) * scale, __uint_as_float(v[4 * i + 3]) * scale);
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int rl = i * 4 + (lane >> 3), c16 = lane & 7;
-            const int32_t er = __shfl_sync(0xffffffffu, e, rl);
-            const float4 val = *reinterpret_cast<const float4*>(stage + rl * 144 + c16 * 16);
-            if (er >= 0) *reinterpret_cast<float4*>(a.partial_dq + (int64_t)er * D + ch * 32 + c16 * 4) = val;
+            for (int u = 0; u < 8; ++u) o[u] = __float_as_uint(__uint_as_float(v[i + u]) * scale);
+            if (a.wide_store) {
+              store32(dst + ch + i, o);
+            } else {
+              *reinterpret_cast<uint4*>(dst + ch + i) = make_uint4(o[0], o[1], o[2], o[3]);
+              *reinterpret_cast<uint4*>(dst + ch + i + 4) = make_uint4(o[4], o[5], o[6], o[7]);
+            }
           }
-          __syncwarp();
         }
-        tc_fence_before();
-      } else {
-        atomicExch(a.status, ST_ROWS);
-        c.abort = 1;
+        __syncwarp();
       }
+      tc_fence_before();
     }
+    if (!ok) { atomicExch(a.status, ST_ROWS); c.abort = 1; }
   }
+  __syncwarp();
+  __syncthreads();
 
   // teardown: all roles are past their last wait; give in-flight copies time to land after
   // an abort, then release tensor memory
   if (c.abort) {
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, kTmemCols);
+}
+
+// ---------------------------------------------------------------------------
+// chunks of at most kDqShortChunk keys: one 128-row tile per work item
+//
+// With one chunk tile per item the kernel above spends most of an item on its hand-over (description,
+// gather by the row threads, epilogue, two CTA-wide barriers).  Here the roles run through a flat stream
+// of items without CTA-wide barriers, as in the forward's kernel for short items:
+//   warp 0     describes the items, up to eight ahead
+//   warps 2, 3 copy the Q / dO rows of an item (cp.async) into its slot (two slots, item n uses n & 1) as soon
+//              as the last S / dP of item n - 2 has executed; warp 2 requests K and V of the chunk (TMA)
+//              once per run of items on it
+//   warp 1     issues the MMAs, the two slots in turn: dQ of a step and behind it S / dP of the slot's
+//              next step, of its next item too
+//   warps 4-7, 8-11  the rows of slot 0 / 1: dS of each 64-key step, then dQ from tensor memory to
+//              32-byte stores, while the other slot computes
+// Shared memory: Q and dO of two slots (128 KB), K and V of a chunk (64 KB).  TMEM per slot as above:
+// S 64, dP 64, dQ 128 columns.
+// Measured against the kernel above (as it was with its barriers), 8191 tokens x 16/4 heads, chunk 128: 328 -> 255 us.
+// ---------------------------------------------------------------------------
+constexpr int kSlotBytes = 2 * kQTileBytes;                   // Q tile, dO tile
+constexpr int kChunkBlockBytes = kDqShortChunk * 64 * 2;      // one [128 keys][64 dims] swizzled block
+constexpr int kChunkTileBytes = 2 * kChunkBlockBytes;
+
+constexpr int kDqSlots = 8;                // item descriptions in flight (see the describing warp)
+
+struct DqShortCtrl {
+  static constexpr int kPrefix = kShortPrefix;
+  uint64_t row_full[2];                      // Q and dO of the slot's item landed; once per item
+  uint64_t row_free[2];                      // the last S / dP of the slot's item has executed
+  uint64_t kv_full, kv_free;                 // K and V landed; every MMA that read them has executed (once per chunk followed by another)
+  uint64_t s_full[2], ds_full[2], dq_full[2];
+  uint64_t item_full[kDqSlots], slot_free[kDqSlots];
+  uint32_t tmem_slot;
+  volatile int32_t abort;
+  int32_t n_routed, n_items;
+  SlotRange own;
+  ShortItem item[kDqSlots];
+  alignas(16) int32_t entry[kDqSlots][kTileM];
+  alignas(16) int32_t grow[kDqSlots][kTileM];    // row index t * Hq + h (dO, lse and delta are indexed by it)
+  alignas(16) int64_t qoff[kDqSlots][kTileM];
+  int32_t prefix_cache[kShortPrefix];
+};
+constexpr int kDqShortThreads = 384;
+constexpr size_t kDqShortSmemBytes = 1024 + 2 * kSlotBytes + 2 * kChunkTileBytes + sizeof(DqShortCtrl);
+static_assert(kDqShortSmemBytes <= 232448, "shared memory of one CTA");
+
+struct DqShortArgs {
+  KernelArgs a;
+  ItemQueue iq;
+};
+
+// S_X = Q_X . K^T and dP_X = dO_X . V^T for the 64 keys at row `key0` of the chunk tiles
+template <int X, bool kHalf, int D>
+__device__ __forceinline__ void issue_s_dp_short(uint32_t tmem, uint32_t dq, uint32_t dk, uint32_t dv, int key0) {
+  constexpr int kQBlock = kQBlockBytes >> 4, kSlot = kSlotBytes >> 4, kBlock = kChunkBlockBytes >> 4;
+  const uint32_t rows = (uint32_t)(key0 * 128) >> 4;
+#pragma unroll
+  for (int ks = 0; ks < D / 16; ++ks) {
+    const uint32_t qo = (uint32_t)(X * kSlot + (ks >> 2) * kQBlock + (ks & 3) * 2);
+    const uint32_t ko = (uint32_t)((ks >> 2) * kBlock + (ks & 3) * 2);
+    mma_ss_lo<kDescHi>(tmem + X * 128, dq + qo, dk + rows + ko, kIdescS<kHalf>, ks > 0);
+  }
+#pragma unroll
+  for (int ks = 0; ks < D / 16; ++ks) {
+    const uint32_t qo = (uint32_t)(X * kSlot + (kQTileBytes >> 4) + (ks >> 2) * kQBlock + (ks & 3) * 2);
+    const uint32_t ko = (uint32_t)((ks >> 2) * kBlock + (ks & 3) * 2);
+    mma_ss_lo<kDescHi>(tmem + X * 128 + 64, dq + qo, dv + rows + ko, kIdescS<kHalf>, ks > 0);
+  }
+}
+
+template <bool kHalf, int D>
+__global__ void __launch_bounds__(kDqShortThreads, 1)
+bwd_dq_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
+                    const __grid_constant__ CUtensorMap tmap_v, const DqShortArgs sa) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const uint32_t sQ = smem_u32(smem);                       // slot 0: Q, dO; slot 1: Q, dO
+  const uint32_t sK = sQ + 2 * kSlotBytes;
+  const uint32_t sV = sK + kChunkTileBytes;
+  DqShortCtrl& c = *reinterpret_cast<DqShortCtrl*>(smem + 2 * kSlotBytes + 2 * kChunkTileBytes);
+  const KernelArgs& a = sa.a;
+  constexpr int kNBlk = (D + 63) / 64;
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&c.row_full[i]), 64);               // the copies of two warps' lanes
+      mbar_init(smem_u32(&c.row_free[i]), 1);
+      mbar_init(smem_u32(&c.s_full[i]), 1);
+      mbar_init(smem_u32(&c.ds_full[i]), kTileM);
+      mbar_init(smem_u32(&c.dq_full[i]), 1);
+    }
+    mbar_init(smem_u32(&c.kv_full), 1);
+    mbar_init(smem_u32(&c.kv_free), 1);
+    for (int i = 0; i < kDqSlots; ++i) {
+      mbar_init(smem_u32(&c.item_full[i]), 1);
+      mbar_init(smem_u32(&c.slot_free[i]), 4);               // the row warps of the item
+    }
+    c.abort = 0;
+    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
+    c.own = own_slot_range(p, a.cu);
+    c.n_items = c.n_routed + own_item_count(c.own.n, p.Hq, p.C, kTileM);
+    fence_barrier_init();
+    prefetch_tmap(&tmap_k);
+    prefetch_tmap(&tmap_v);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&c.tmem_slot), kTmemCols);
+    tmem_relinquish();
+  }
+  if (p.hist > 0) fill_prefix_cache(c, a.tile_prefix, p.lists, kDqShortThreads);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = c.tmem_slot;
+
+  bool ok = true;                            // false: a wait of this role gave up
+  auto wait = [&](uint64_t* bar, uint32_t parity) {
+    ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(bar), parity));
+    return ok;
+  };
+  if (warp == 0) {
+    ok = describe_items<kDqSlots, 2, true, true>(p, sa.iq, c);
+    if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
+  } else if (warp == 2 || warp == 3) {
+    // ---- rows: warp 2 copies Q (and requests K and V), warp 3 dO
+    uint32_t kv = 0;                         // chunks requested so far
+    for (int n = 0; ok; ++n) {
+      const int x = n & 1, slot = n % kDqSlots;
+      if (!wait(&c.item_full[slot], (n / kDqSlots) & 1)) break;
+      if (c.item[slot].done) break;
+      const int tok0 = c.item[slot].tok0, head = c.item[slot].head, nrows = c.item[slot].nrows;
+      const bool fresh = c.item[slot].new_kv != 0;
+      if (n >= 2 && !wait(&c.row_free[x], ((n >> 1) - 1) & 1)) break;
+      const uint32_t tile = sQ + x * kSlotBytes;
+      if (warp == 2) copy_rows_async<D / 8, 1>(tile, a.q, 0, 0, nrows, [&](int r) { return c.qoff[slot][r]; });
+      else copy_rows_async<D / 8, 1>(tile + kQTileBytes, a.dout, 0, 0, nrows, [&](int r) { return (int64_t)c.grow[slot][r] * D; });
+      cp_async_mbar_arrive(smem_u32(&c.row_full[x]));
+      if (warp == 2 && fresh) {
+        if (kv > 0 && !wait(&c.kv_free, (kv - 1) & 1)) break;
+        ++kv;
+        if (lane == 0) {
+          const uint32_t bar = smem_u32(&c.kv_full);
+          mbar_expect_tx(bar, 2 * kNBlk * kChunkBlockBytes);
+          tma_load_3d(sK, &tmap_k, bar, 0, head, tok0);
+          if (D > 64) tma_load_3d(sK + kChunkBlockBytes, &tmap_k, bar, 64, head, tok0);
+          tma_load_3d(sV, &tmap_v, bar, 0, head, tok0);
+          if (D > 64) tma_load_3d(sV + kChunkBlockBytes, &tmap_v, bar, 64, head, tok0);
+        }
+      }
+    }
+    if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
+  } else if (warp == 1) {
+    // ---- MMA issuer: the whole warp runs convergent, one elected lane issues.
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t dq = __shfl_sync(0xffffffffu, desc_lo(sQ, 16), 0);
+    const uint32_t dk = __shfl_sync(0xffffffffu, desc_lo(sK, 16), 0);
+    const uint32_t dv = __shfl_sync(0xffffffffu, desc_lo(sV, 16), 0);
+    const uint32_t dkt = __shfl_sync(0xffffffffu, desc_lo(sK, kChunkBlockBytes), 0);
+    const uint32_t el = elect_one();
+    uint32_t kv = 0;                       // chunks consumed
+    int next = 0;                          // the next item to start (item `next` goes to slot next & 1)
+    bool end = false;
+    // per slot: the key step whose dS is due and the steps of its item; 0 steps: empty
+    int step0 = 0, step1 = 0, steps0 = 0, steps1 = 0;
+    uint32_t dph0 = 0, dph1 = 0;           // ds_full phases
+    auto s_dp = [&](int x, int step, int steps) {
+      tc_fence_after();
+      if (el) {
+        if (x) issue_s_dp_short<1, kHalf, D>(tm, dq, dk, dv, step * kBN);
+        else issue_s_dp_short<0, kHalf, D>(tm, dq, dk, dv, step * kBN);
+        tc_commit(smem_u32(&c.s_full[x]));
+        if (step + 1 == steps) tc_commit(smem_u32(&c.row_free[x]));
+      }
+      __syncwarp();
+    };
+    // starts item `next` in its slot, whose item before has issued its last dQ.  An item on another chunk waits
+    // until the other slot has issued its last dQ too (`other_busy` false): K and V are then free.
+    auto start = [&](bool other_busy) {
+      if (end) return;
+      const int slot = next % kDqSlots, x = next & 1;
+      if (!wait(&c.item_full[slot], (next / kDqSlots) & 1)) return;
+      if (c.item[slot].done) { end = true; return; }
+      const bool fresh = c.item[slot].new_kv != 0;
+      if (fresh) {
+        if (other_busy) return;
+        if (kv > 0) {
+          if (el) tc_commit(smem_u32(&c.kv_free));
+          __syncwarp();
+        }
+        if (!wait(&c.kv_full, kv & 1)) return;
+        ++kv;
+      }
+      if (!wait(&c.row_full[x], (next >> 1) & 1)) return;
+      fence_proxy_async_smem();                               // rows written by cp.async, read by the tensor core
+      const int steps = (c.item[slot].kv_len + kBN - 1) / kBN;
+      if (x) { steps1 = steps; step1 = 0; } else { steps0 = steps; step0 = 0; }
+      s_dp(x, 0, steps);
+      ++next;
+    };
+    start(false);
+    if (ok) start(steps0 > 0);
+    // slots in turn; a slot without an item starts the next one when it is that item's slot
+    for (int turn = 0; ok && (steps0 > 0 || steps1 > 0); ++turn) {
+      const int x = turn & 1;
+      const int steps = x ? steps1 : steps0, step = x ? step1 : step0;
+      if (steps > 0) {
+        if (!wait(&c.ds_full[x], x ? dph1 : dph0)) break;
+        if (x) dph1 ^= 1; else dph0 ^= 1;
+        tc_fence_after();
+        if (el) {
+#pragma unroll
+          for (int ks = 0; ks < kBN / 16; ++ks)
+            mma_ts_lo<kDescHi>(tm + 256 + x * 128, tm + x * 128 + ks * 8, dkt + ((step * kBN + ks * 16) * 128 >> 4),
+                               kIdescDQ<kHalf, D>, step > 0 || ks > 0);
+          if (step + 1 == steps) tc_commit(smem_u32(&c.dq_full[x]));
+        }
+        __syncwarp();
+        if (step + 1 < steps) {
+          s_dp(x, step + 1, steps);
+          if (x) ++step1; else ++step0;
+        } else {
+          if (x) steps1 = 0; else steps0 = 0;
+        }
+      }
+      if (ok && (x ? steps1 : steps0) == 0 && (next & 1) == x) start((x ? steps0 : steps1) > 0);
+      // the other slot may have been waiting for this one to let go of K and V
+      if (ok && steps0 == 0 && steps1 == 0) start(false);
+    }
+    if (!ok && lane == 0) { atomicExch(a.status, ST_MMA); c.abort = 1; }
+  } else {
+    // ---- one thread per row; warps 4-7: slot 0, 8-11: slot 1
+    const int x = (warp - 4) >> 2;
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t tS = tmem + lane_base + x * 128;
+    const uint32_t tDQ = tmem + lane_base + 256 + x * 128;
+    const float scale = rsqrtf((float)D);
+    const float sl2 = scale * 1.4426950408889634f;
+    uint32_t sph = 0;
+    for (int n = x; ok; n += 2) {
+      const int slot = n % kDqSlots;
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.item_full[slot]), (n / kDqSlots) & 1));
+      if (!ok) break;
+      const ShortItem it = c.item[slot];
+      if (it.done) break;
+      const int32_t e = c.entry[slot][row];
+      const bool active = (warp & 3) * 32 < it.nrows;
+      float neg_lse2 = -INFINITY, delta = 0.f;
+      if (e >= 0) {
+        const int32_t gr = c.grow[slot][row];
+        neg_lse2 = -__ldg(a.lse2 + gr);
+        delta = __ldg(a.delta + gr);
+      }
+      const int ntiles = (it.kv_len + kBN - 1) / kBN;
+      const int lim = it.causal ? min(it.kv_len, it.tok_rel + row + 1) : it.kv_len;   // keys < lim are visible
+      for (int j = 0; j < ntiles; ++j) {
+        ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.s_full[x]), sph));
+        if (!ok) break;
+        sph ^= 1;
+        // the item's S has run: every role has read its description
+        if (j == 0 && lane == 0) mbar_arrive(smem_u32(&c.slot_free[slot]));
+        if (active) {
+          tc_fence_after();
+          const int key0 = j * kBN;
+          const bool masked = key0 + kBN > it.kv_len || (it.causal && key0 + kBN - 1 > it.tok_rel);
+          if (masked) ds_row<true, kHalf>(tS, key0, lim, sl2, neg_lse2, delta);
+          else ds_row<false, kHalf>(tS, key0, lim, sl2, neg_lse2, delta);
+          tc_fence_before();
+        }
+        mbar_arrive(smem_u32(&c.ds_full[x]));
+      }
+      if (!ok) break;
+      ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.dq_full[x]), (n >> 1) & 1));
+      if (!ok) break;
+      if (active) {
+        tc_fence_after();
+        float* dst = a.partial_dq + (int64_t)(e >= 0 ? e : 0) * D;
+#pragma unroll 1
+        for (int ch = 0; ch < D; ch += 32) {
+          uint32_t v[32];
+          tmem_ld32(tDQ + ch, v);
+          tmem_wait_ld();
+          if (e >= 0) {
+#pragma unroll
+            for (int i = 0; i < 32; i += 8) {
+              uint32_t o[8];
+#pragma unroll
+              for (int u = 0; u < 8; ++u) o[u] = __float_as_uint(__uint_as_float(v[i + u]) * scale);
+              if (a.wide_store) {
+                store32(dst + ch + i, o);
+              } else {
+                *reinterpret_cast<uint4*>(dst + ch + i) = make_uint4(o[0], o[1], o[2], o[3]);
+                *reinterpret_cast<uint4*>(dst + ch + i + 4) = make_uint4(o[4], o[5], o[6], o[7]);
+              }
+            }
+          }
+          __syncwarp();
+        }
+        tc_fence_before();
+      }
+    }
+    if (!ok) {
+      atomicExch(a.status, ST_ROWS);
+      c.abort = 1;
+    }
+  }
+
+  __syncwarp();
+  __syncthreads();
+  if (c.abort) {                           // copies in flight land before shared memory is given up
     const uint64_t t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
   }
@@ -526,16 +814,32 @@ cudaError_t launch_bwd_dq_tc5(const Params& p, const __nv_bfloat16* q, const __n
   if (!make_kv_map(&mk, p.fp16 != 0, p.D, k, p.T, p.Hkv, p.sk_t, p.sk_h, kBN) ||
       !make_kv_map(&mv, p.fp16 != 0, p.D, v, p.T, p.Hkv, p.sv_t, p.sv_h, kBN))
     return cudaErrorNotSupported;
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const KernelArgs args{q, dout, cu, list_counts, list_offsets, tile_prefix, row_list, lse2, delta, partial_dq,
+                        work_counter, status, ((uintptr_t)partial_dq & 31) == 0};
+  if (bwd_dq_short_items(p)) {
+    DqShortArgs sa;
+    sa.a = args;
+    sa.iq = ItemQueue{cu, list_counts, list_offsets, tile_prefix, row_list, work_counter,
+                      short_batch(p, sms, false), 0};
+    if (!make_kv_map(&mk, p.fp16 != 0, p.D, k, p.T, p.Hkv, p.sk_t, p.sk_h, kDqShortChunk) ||
+        !make_kv_map(&mv, p.fp16 != 0, p.D, v, p.T, p.Hkv, p.sv_t, p.sv_h, kDqShortChunk))
+      return cudaErrorNotSupported;
+    auto kern = p.D == 128 ? (p.fp16 ? bwd_dq_short_kernel<true, 128> : bwd_dq_short_kernel<false, 128>)
+              : p.D == 96  ? (p.fp16 ? bwd_dq_short_kernel<true, 96> : bwd_dq_short_kernel<false, 96>)
+                           : (p.fp16 ? bwd_dq_short_kernel<true, 64> : bwd_dq_short_kernel<false, 64>);
+    const cudaError_t se = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDqShortSmemBytes);
+    if (se != cudaSuccess) return se;
+    kern<<<sms, kDqShortThreads, kDqShortSmemBytes, st>>>(p, mk, mv, sa);
+    return cudaGetLastError();
+  }
   auto kernel = p.D == 128 ? (p.fp16 ? bwd_dq_tc5_kernel<true, 128> : bwd_dq_tc5_kernel<false, 128>)
               : p.D == 96  ? (p.fp16 ? bwd_dq_tc5_kernel<true, 96> : bwd_dq_tc5_kernel<false, 96>)
                            : (p.fp16 ? bwd_dq_tc5_kernel<true, 64> : bwd_dq_tc5_kernel<false, 64>);
   cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
   if (e != cudaSuccess) return e;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const KernelArgs args{q, dout, cu, list_counts, list_offsets, tile_prefix, row_list, lse2, delta, partial_dq,
-                        work_counter, status};
   kernel<<<sms, kThreads, kSmemBytes, st>>>(p, mk, mv, args);
   return cudaGetLastError();
 }

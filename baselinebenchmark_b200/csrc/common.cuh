@@ -377,6 +377,11 @@ cudaError_t launch_bwd_dq_tc5(const Params& p, const __nv_bfloat16* q, const __n
                               const int32_t* list_counts, const int32_t* list_offsets, const int32_t* tile_prefix,
                               const int32_t* row_list, const float* lse2, const float* delta, float* partial_dq,
                               int32_t* work_counter, int32_t* status, cudaStream_t st);
+// Chunks of at most this many keys run the dq kernel of one-tile items.
+constexpr int kDqShortChunk = 128;
+inline bool bwd_dq_short_items(const Params& p) {
+  return p.D <= 128 && p.C <= kDqShortChunk;
+}
 cudaError_t launch_bwd_dkdv_tc5(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* k,
                                 const __nv_bfloat16* v, const __nv_bfloat16* dout, const int32_t* cu,
                                 const int32_t* list_counts, const int32_t* list_offsets, const int32_t* row_list,
