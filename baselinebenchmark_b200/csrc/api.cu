@@ -18,17 +18,9 @@ namespace {
 
 // rows per work item of the dense stage: the tcgen05 kernel takes two 128-row tiles per item up to
 // head_dim 128 and one at head_dim 256, the mma.sync kernel one
-int tile_rows_of(int impl, int head_dim) {
+int tile_rows_of(int impl, int head_dim, int chunk = 1 << 30) {
   if (impl == MOBA_ATTEND_MMA_SYNC) return kMmaTileRows;
-  return head_dim > 128 ? kTileRowsWide : kTc5TileRows;
-}
-// for a problem: chunk size and query window may choose the kernel for short items (one tile)
-int tile_rows_of(const moba_problem_t* p) {
-  const int64_t tq = p->q_tokens > 0 ? p->q_tokens : p->total_tokens;
-  if (p->attend_impl == MOBA_ATTEND_TCGEN05 &&
-      tc5_short_items(p->head_dim, p->chunk_size, tq, p->num_q_heads / p->num_kv_heads))
-    return kTileRowsWide;
-  return tile_rows_of(p->attend_impl, p->head_dim);
+  return head_dim > 128 || tc5_small_tiles(head_dim, chunk) ? kTileRowsWide : kTc5TileRows;
 }
 constexpr size_t kAlign = 256;
 inline size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
@@ -72,9 +64,7 @@ int check_problem(const moba_problem_t* p) {
   // tiles = slots * Hq * tiles per chunk, per pass of one kv-head group at least)
   if (p->batch > 65535 || p->num_kv_heads > 65535) return MOBA_E_UNSUPPORTED;
   const int64_t g = p->num_q_heads / p->num_kv_heads;
-  // (by the chunk alone: a window that the kernel for short items takes has one own-chunk item per slot and kv head)
-  const int64_t tile = p->attend_impl == MOBA_ATTEND_TCGEN05 && tc5_short_items(p->head_dim, p->chunk_size, INT32_MAX, 1)
-                           ? kTileRowsWide : tile_rows_of(p->attend_impl, p->head_dim);
+  const int64_t tile = tile_rows_of(p->attend_impl, p->head_dim, p->chunk_size);
   const int64_t own_items = mc * p->batch * g * ((p->chunk_size + tile - 1) / tile);
   const int64_t routed_items = (hist > 0 ? hist : 0) * tq * g / tile + mc * p->batch;
   if (own_items + routed_items >= ((int64_t)1 << 31)) return MOBA_E_UNSUPPORTED;
@@ -264,7 +254,7 @@ int moba_attend_tile_rows(int impl) { return tile_rows_of(impl, 128); }
 int moba_attend_tile_rows_for(int impl, int head_dim) { return tile_rows_of(impl, head_dim); }
 int moba_problem_tile_rows(const moba_problem_t* p) {
   const int rc = check_problem(p);
-  return rc != MOBA_OK ? rc : tile_rows_of(p);
+  return rc != MOBA_OK ? rc : tile_rows_of(p->attend_impl, p->head_dim, p->chunk_size);
 }
 
 int moba_workspace_size(const moba_problem_t* p, size_t* bytes) {
@@ -403,7 +393,8 @@ static int forward_pass(const moba_problem_t* p, int64_t sel_rs, const void* q, 
       return (int)e;
     if (last && (e = mark(1)) != cudaSuccess) return (int)e;
     // the gating kernel ends with the prefix sums over the lists it counted
-    const ListScan scan{w.list_counts, w.list_offsets, w.tile_prefix, w.cursors, r.lists, tile_rows_of(p)};
+    const ListScan scan{w.list_counts, w.list_offsets, w.tile_prefix, w.cursors, r.lists,
+                        tile_rows_of(p->attend_impl, p->head_dim, p->chunk_size)};
     if ((e = launch_gate_topk(r, qb, means, cu, sel, w.list_counts, st, &scan, w.status + 1)) != cudaSuccess) return (int)e;
     if (last && (e = mark(2)) != cudaSuccess) return (int)e;
     if ((e = launch_scatter(r, cu, sel, w.list_offsets, w.cursors, w.row_list, w.partial_lse, st)) != cudaSuccess)

@@ -1014,10 +1014,10 @@ attend_tc5_wide_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_
 }
 
 // ---------------------------------------------------------------------------
-// short items: chunks of at most kSmallChunk keys, and query windows with at most 128 rows per
+// short items: chunks of at most kShortChunk keys, and query windows with at most 128 rows per
 // kv head (decode steps).  One 128-row tile per work item, two CTAs per SM.
 //
-// Such an item is one or two key tiles (or, in a decode step, a long chunk for a handful of
+// Such an item is one to four key tiles (or, in a decode step, a long chunk for a handful of
 // rows), so what counts is that nothing of its hand-over is waited for.  The roles of a CTA run
 // through one flat stream of key tiles, without a CTA-wide barrier between items:
 //   warp 4     describes the items, up to four ahead (a chain of dependent global loads and divisions as
@@ -1108,7 +1108,7 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
   pdl_wait();
   pdl_trigger();
   if (threadIdx.x == 0) {
-    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
+    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] << sa.iq.tile_shift : 0;
     c.own = own_slot_range(p, a.cu);
     c.n_items = c.n_routed + (sa.iq.grouped ? c.own.n * p.Hkv : own_item_count(c.own.n, p.Hq, p.C, kTileM));
   }
@@ -1381,7 +1381,7 @@ attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap
   pdl_wait();
   pdl_trigger();
   if (threadIdx.x == 0) {
-    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;
+    c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] << sa.iq.tile_shift : 0;
     c.own = own_slot_range(p, a.cu);
     c.n_items = c.n_routed + (sa.iq.grouped ? c.own.n * p.Hkv : own_item_count(c.own.n, p.Hq, p.C, kTileM));
   }
@@ -1684,7 +1684,7 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
   const KernelArgs args{q, cu, list_counts, list_offsets, tile_prefix, row_list, partial_out, partial_lse,
                         work_counter, status, ((uintptr_t)partial_out & 31) == 0};
   cudaError_t e;
-  if (p.D == 256 ? p.C <= kSmallChunk : tc5_short_items(p.D, p.C, p.Tq, p.G)) {
+  if (p.D == 256 ? p.C <= kSmallChunk : tc5_short_items(p)) {
     auto kern = p.D == 256 ? (p.fp16 ? attend_tc5_wide_short_kernel<true> : attend_tc5_wide_short_kernel<false>)
               : p.D == 128 ? (p.fp16 ? attend_tc5_short_kernel<true, 128> : attend_tc5_short_kernel<false, 128>)
               : p.D == 96  ? (p.fp16 ? attend_tc5_short_kernel<true, 96> : attend_tc5_short_kernel<false, 96>)
@@ -1695,8 +1695,11 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
     if (e != cudaSuccess) return e;
     ShortArgs sa;
     sa.a = args;
-    sa.iq = ItemQueue{cu, list_counts, list_offsets, tile_prefix, row_list, work_counter, 1, 0};
+    sa.iq = ItemQueue{cu, list_counts, list_offsets, tile_prefix, row_list, work_counter, 1, 0,
+                      0};
     sa.iq.grouped = p.Tq * p.G <= kTileM;
+    // (a window's lists have one tile of either size)
+    sa.iq.tile_shift = p.D == 256 || tc5_small_tiles(p.D, p.C) || sa.iq.grouped ? 0 : 1;
     sa.iq.batch = short_batch(p, ctas, sa.iq.grouped);
     return launch_pdl(kern, dim3(ctas), threads, smem, st, p, mk, mv, sa);
   }

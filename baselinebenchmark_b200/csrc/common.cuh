@@ -340,14 +340,24 @@ cudaError_t launch_merge(const Params& p, const __half* partial_out, const float
 constexpr int kMmaTileRows = 128;        // rows per work item, mma.sync kernel
 constexpr int kTc5TileRows = 256;        // rows per work item, tcgen05 kernel (two 128-row MMA tiles)
 constexpr int kTileRowsWide = 128;       // rows per work item, tcgen05 kernel at head_dim 256 (one tile)
-// Chunks of at most this many keys run the tcgen05 kernel for short items (128-row items, two CTAs per SM),
-// and so do query windows whose rows of one kv head fit its single tile (decode steps): a second row tile would be empty.
+// Row tiles of a list are 128 rows for chunks of at most this many keys (and at head dim 256), 256 otherwise.
 #ifndef MOBA_SMALL_CHUNK
 #define MOBA_SMALL_CHUNK 256
 #endif
 constexpr int kSmallChunk = MOBA_SMALL_CHUNK;
-__host__ __device__ inline bool tc5_short_items(int head_dim, int chunk, int64_t query_tokens, int group) {
-  return head_dim <= 128 && (chunk <= kSmallChunk || query_tokens * group <= kTileRowsWide);
+__host__ __device__ inline bool tc5_small_tiles(int head_dim, int chunk) { return head_dim <= 128 && chunk <= kSmallChunk; }
+// Chunks of at most this many keys run the tcgen05 kernel for short items (one 128-row tile per item, two CTAs per
+// SM; where the lists are cut into 256 rows it takes a half at a time), and so do query windows whose rows of
+// one kv head fit one tile (decode steps): a second row tile would be empty.  Measured against the 256-row kernel,
+// whole call: chunk 512, 32768 tokens x 32/8 heads, top-k 8 3.61 -> 3.27 ms (head_dim 64 2.85 -> 2.42), 2 x 4096 x 16
+// 340 -> 308 us, 19456 x 32 983 -> 888 us; chunk 1024 4.66-5.01 against 5.05 ms on the first (the halves read K and V
+// twice as often), so the line lies at 512.
+constexpr int kShortChunk = 512;
+inline bool tc5_short_items(const Params& p) {
+  if (p.D > 128) return false;
+  if (p.Tq * p.G <= kTileRowsWide) return true;
+  // (own-chunk items are counted in int32; a slot table that large stays with the 256-row kernel)
+  return p.C <= kShortChunk && (int64_t)p.slots * p.Hq * ((p.C + 127) / 128) < ((int64_t)1 << 30);
 }
 
 cudaError_t launch_attend_mma(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* k,

@@ -54,6 +54,7 @@ struct ItemQueue {
   int32_t* work_counter;
   int32_t batch;                           // items a CTA draws at a time
   int32_t grouped;                         // own-chunk items cover the heads of a group (short windows)
+  int32_t tile_shift;                      // 1: the tiles of tile_prefix are 256 rows, two items each
 };
 // A CTA draws several items at a time, so that row tiles of one list follow one another on it (K and V
 // stay in place), but at most an eighth of its share of the launch, for the balance.
@@ -109,8 +110,9 @@ __device__ __forceinline__ void short_next(const Params& p, const ItemQueue& a, 
     }
     const int idx = w.cur++;
     if (idx < n_routed) {
-      if (idx < w.list_first || idx >= w.list_end) {
-        const int l = find_list(c, a.tile_prefix, p.lists, idx);
+      const int cut = idx >> a.tile_shift;                    // tile of tile_prefix
+      if (cut < w.list_first || cut >= w.list_end) {
+        const int l = find_list(c, a.tile_prefix, p.lists, cut);
         const int slot = l / p.Hkv;
         const int b = slot / p.mc, j = slot - b * p.mc;
         w.list = l;
@@ -121,7 +123,8 @@ __device__ __forceinline__ void short_next(const Params& p, const ItemQueue& a, 
         w.kv_tok0 = __ldg(a.cu + b) + j * p.C;
         w.kv_head = l - slot * p.Hkv;
       }
-      const int tile = idx - w.list_first;
+      const int tile = idx - (w.list_first << a.tile_shift);
+      if (tile * kTileRowsWide >= w.list_count) continue;     // the second half of a 256-row tile may be empty
       it.nrows = min(w.list_count - tile * kTileRowsWide, kTileRowsWide);
       it.kv_len = p.C;
       kv_tok0 = w.kv_tok0;

@@ -1,4 +1,4 @@
-"""GPU: the dense-stage kernel for short items (chunks of at most 256 keys, and query windows with at
+"""GPU: the dense-stage kernel for short items (chunks of at most 512 keys, and query windows with at
 most 128 rows per kv head) and the row gathers, at the sizes and strides where their branches change.
 
 Outputs are compared with the mma.sync dense stage.  Both round P to 16 bits and a partial row to 11
@@ -31,7 +31,7 @@ def _close(out, ref, dtype):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("d", [64, 96, 128])
-@pytest.mark.parametrize("chunk", [16, 64, 127, 128, 129, 200, 256, 257])
+@pytest.mark.parametrize("chunk", [16, 64, 127, 128, 129, 200, 256, 257, 512, 513])
 def test_chunk_sizes_around_the_tiles(chunk, d, dtype):
     lens, hq, hkv, topk = (1, 130, 1025, 700), 6, 2, 5
     q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, dtype, seed=chunk + d)
@@ -47,7 +47,7 @@ def test_chunk_sizes_around_the_tiles(chunk, d, dtype):
 @pytest.mark.parametrize("chunk", [128, 512, 4096])
 def test_windows_around_the_row_limit_equal_full_run(chunk, hq, hkv):
     """128 rows per kv head is the largest window of the short kernel; one token more and, with chunks of
-    more than 256 keys, the 256-row kernel runs.  Windows cross chunk and sequence boundaries."""
+    more than 512 keys, the 256-row kernel runs.  Windows cross chunk and sequence boundaries."""
     lens, topk = (700, 5000), 4
     q, k, v, cu = _inputs(lens, hq, hkv, 128, chunk, torch.bfloat16, seed=7)
     full, lse, sel = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True, return_selected=True)
