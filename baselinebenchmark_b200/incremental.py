@@ -67,11 +67,15 @@ class IncrementalMoba:
         return (out, sel) if return_selected else out
 
     def _plain(self, k: torch.Tensor, v: torch.Tensor) -> bool:
-        """Rows that moba_append copies as they are: the caches' type, device and row shape, 16-byte pieces, and
-        nothing for autograd to record.  Everything else goes through torch's copy."""
+        """Rows that moba_append copies as they are: the caches' type, device and row shape, 16-byte pieces, memory
+        of their own, and nothing for autograd to record.  Everything else goes through torch's copy."""
         row, dtype, device = self.k.shape[1:], self.k.dtype, self.k.device
-        for t, cache in ((k, self.k), (v, self.v)):
-            if cache.data_ptr() <= t.data_ptr() < cache.data_ptr() + cache.nbytes:      # rows of the cache itself
+        caches = [(c.untyped_storage().data_ptr(), c.untyped_storage().nbytes()) for c in (self.k, self.v)]
+        for t in (k, v):
+            # One kernel reads the rows and writes both caches: rows that share memory with either of them go
+            # through torch, one cache after the other.
+            mem, size = t.untyped_storage().data_ptr(), t.untyped_storage().nbytes()
+            if any(mem < at + n and at < mem + size for at, n in caches):
                 return False
             if (t.shape[1:] != row or t.dtype != dtype or t.device != device or t.stride(2) != 1 or t.stride(0) % 8
                     or t.stride(1) % 8 or t.data_ptr() % 16 or t.requires_grad):

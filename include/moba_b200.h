@@ -170,7 +170,8 @@ int moba_forward_cached(const moba_problem_t* p, const void* q, const void* k, c
  *   p              batch 1; total_tokens = tokens after the append, q_token_begin / q_tokens = the
  *                  new ones; k_/v_stride_* are those of the caches
  *   k_new, v_new   [q_tokens, Hkv, D] with the given token and head strides (elements, multiples of
- *                  8), 16-byte aligned, not overlapping the rows they are stored to
+ *                  8), 16-byte aligned; one kernel reads both and writes both caches, so neither
+ *                  may overlap the rows stored to in either cache (not checked)
  *   k_cache, v_cache, cu_seqlens  written here */
 int moba_append(const moba_problem_t* p, const void* q, const void* k_new, const void* v_new,
                 int64_t k_new_stride_token, int64_t k_new_stride_head, int64_t v_new_stride_token,
