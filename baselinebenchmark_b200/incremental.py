@@ -80,7 +80,11 @@ class IncrementalMoba:
             if (t.shape[1:] != row or t.dtype != dtype or t.device != device or t.stride(2) != 1 or t.stride(0) % 8
                     or t.stride(1) % 8 or t.data_ptr() % 16 or t.requires_grad):
                 return False
-        return not self.k.requires_grad and not self.v.requires_grad
+        for c in (self.k, self.v, self.cu):
+            # torch refuses to write an inference tensor outside inference mode: leave that to its copy
+            if c.requires_grad or (c.is_inference() and not torch.is_inference_mode_enabled()):
+                return False
+        return True
 
     def _append(self, q, k, v, begin: int, end: int, cached: int, return_selected: bool):
         """One native call: rows into the caches, position, attention on the new tokens."""
@@ -101,4 +105,6 @@ class IncrementalMoba:
             C.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), kt, kh, vt, vh, kc.data_ptr(), vc.data_ptr(),
             self.cu.data_ptr(), out.data_ptr(), sel.data_ptr() if sel is not None and sel.numel() else None,
             self.means.data_ptr(), cached, ws.data_ptr(), need, stream)))
+        # what autograd saved of the caches is stale now, as after an in-place torch operation
+        torch.autograd.graph.increment_version((kc, vc, self.cu))
         return out, sel

@@ -41,3 +41,16 @@ def test_rows_that_start_before_the_cache_and_run_into_it_are_not():
     store = torch.zeros(130, HKV, DIM, dtype=torch.bfloat16)
     inc = _cache(store[2:])
     assert not inc._plain(store[:N], _rows()) and not inc._plain(_rows(), store[:N])
+
+
+@pytest.mark.parametrize("part", ["k", "v", "cu"])
+def test_inference_tensors_outside_inference_mode_are_left_to_torch(part):
+    """torch's in-place copy refuses them there; inside inference mode it does not."""
+    inc = _cache()
+    with torch.inference_mode():
+        setattr(inc, part, torch.zeros_like(getattr(inc, part)))
+        assert inc._plain(_rows(), _rows())
+    assert not inc._plain(_rows(), _rows())
+    with pytest.raises(RuntimeError, match="[Ii]nference"):
+        inc.append(torch.zeros(N, HKV, DIM, dtype=torch.bfloat16), _rows(), _rows())
+    assert inc.length == 0

@@ -44,3 +44,18 @@ def test_rows_of_any_layout_reach_the_cache(how, n):
         assert inc.length == prefix + n
     for a, b in zip(*caches):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_append_counts_as_an_in_place_write(native):
+    """Autograd must notice that what it saved of the caches has been overwritten, whichever way the rows went."""
+    inc = IncrementalMoba(64, 2, 64, 16, 3)
+    rows = torch.randn(4, 2, 64, device="cuda", dtype=torch.bfloat16 if native else torch.float32)
+    q = torch.randn(4, 4, 64, device="cuda", dtype=torch.bfloat16)
+    assert inc._plain(rows, rows) == native
+    scale = torch.ones(1, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    sums = [(scale * c).sum() for c in (inc.k, inc.v)]       # saves the cache for the gradient of `scale`
+    inc.append(q, rows, rows)
+    for s in sums:
+        with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+            s.backward()
