@@ -145,93 +145,98 @@ cudaError_t launch_scatter(const Params& p, const int32_t* cu, const int32_t* se
 }
 
 // ---------------------------------------------------------------------------
-// merge: D / 8 lanes (rounded up to a power of two) per (token, head) row, so a warp combines one row
-// at head dim 256, two at 128 and 96, four at 64.
+// merge: a (token, head) row is combined by D / 8 lanes (rounded up to a power of two: one row a warp at
+// head dim 256, two at 128 and 96, four at 64), or, from top-k 17 on, by a whole warp.
 //   lse_tot = log sum_j exp(lse_j);  out = sum_j O_j * exp(lse_j - lse_tot)
 // (exponentials through ex2.approx: relative error 2^-22, far below the rounding of the output)
-// Bound by HBM by bytes, in practice by issue slots: a whole warp per row spent as many instructions on
-// reducing a handful of LSEs and adding its groups' sums as on the partial rows.  Measured against
-// that: 13311 tokens x 16 heads, head_dim 64, 8 partials 98 -> 60 us; 32768 x 32, head_dim 128 500 -> 417 us;
-// 19456 x 32, 3 partials 277 -> 224 us.
+// Bound by HBM by bytes, with few partials in practice by issue slots: a whole warp per row spends as many
+// instructions on reducing a handful of LSEs and adding its groups' sums as on the partial rows.  With many it
+// reads more of a row in one go, and 64 LSEs fit its registers.  Measured, us, 131072 rows:
+//   partials                  3     8    16    32    64
+//   head dim 128, rows of 16 lanes   34.5  63.6   107     -     -
+//                 rows of a warp     62.9  70.3   105   179   333
+//   head dim 64,  rows of 8 lanes    17.7  35.5  61.3     -     -
+//                 rows of a warp     52.4  64.0  71.4   105   180
+// (reading the LSEs again for each partial where they do not fit the registers: 209 / 812 us at 128 with 32 / 64,
+// 236 / 451 at 64), so the line lies at 16.  It is drawn by top-k, not by the partials of the call: the two add a row's
+// partials in different orders, and a row must come out the same bits however many chunks max_seqlen allows for.
 // ---------------------------------------------------------------------------
 constexpr int kMergeThreads = 256;
+constexpr int kMergeNarrow = 16;                 // largest top-k whose rows are on a part of a warp
 
-// A partial row is D/8 pieces of eight fp16 values (16 bytes), one per lane of the row's lanes, which
-// take the partials of the row in turn, kMergeAhead of them in flight.  No sum crosses the
-// lanes but the two reductions over the LSEs.
-// Two or more rows a warp: eight loads in flight at three CTAs per SM (80 registers); one row a warp: four at four.
-template <int D> constexpr int kMergeAhead = D == 256 ? 4 : 8;
-template <int D> constexpr int kMergeCtas = D == 256 ? 4 : 3;
-template <int D> constexpr int kMergeLanes = D <= 64 ? 8 : D <= 128 ? 16 : 32;
-template <bool kHalf, int D>
-__global__ void __launch_bounds__(kMergeThreads, kMergeCtas<D>)
+// A partial row is D/8 pieces of eight fp16 values (16 bytes), one per lane of a group of lanes.  A row has
+// kW lanes: one group, which takes the partials of the row in turn, or all 32 lanes of a warp, whose groups take
+// every second (head dim 96, 128) or fourth (64) partial and add their sums at the end.
+// kAhead partials of a group are in flight, kPairs LSEs in each lane.
+template <int D> constexpr int kMergeGroup = D <= 64 ? 8 : D <= 128 ? 16 : 32;
+template <bool kHalf, int D, int kW, int kPairs, int kAhead, int kCtas>
+__global__ void __launch_bounds__(kMergeThreads, kCtas)
 merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __restrict__ partial_lse,
              const int32_t* __restrict__ status, __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out) {
   pdl_wait();
   pdl_trigger();
-  constexpr int kW = kMergeLanes<D>;             // lanes per row
-  constexpr int kAhead = kMergeAhead<D>;
-  constexpr int kPieces = D / 8;                 // of which this many hold data (head dim 96: 12 of 16)
+  constexpr int kGroup = kMergeGroup<D>, kGroups = kW / kGroup;
+  constexpr int kPieces = D / 8;                 // lanes of a group that hold data (head dim 96: 12 of 16)
   constexpr int kRowsPerBlock = kMergeThreads / kW;
+  static_assert(kPairs == 1 || kPairs == 2, "LSEs of a lane");
+  static_assert(kW % (kGroups * kAhead) == 0, "the partials of a round lie on one side of kW");
   const int lane = threadIdx.x & 31;
-  const int sub = lane & (kW - 1);
+  const int sub = lane & (kW - 1);               // lane of the row
+  const int grp = sub / kGroup, piece = sub & (kGroup - 1);
   const unsigned base_lane = lane & ~(kW - 1);
   // a dense stage that gave up on a wait leaves a non-zero status: poison the result
   const bool failed = status != nullptr && *status != 0;
   const int64_t stride = (int64_t)gridDim.x * kRowsPerBlock;
-  // Up to 2 kW partials per row: lane j holds {lse, 1 / scale} of the partials j and j + kW, and the pairs
+  // Lane j holds {lse, 1 / scale} of the partials j and j + kW (there are at most kPairs * kW), and the pairs
   // of the next row are requested before this row is worked on, so that a row starts with its
   // partial rows as the only loads it has to wait for.
-  const bool in_regs = p.NP <= 2 * kW;
   int64_t row = (int64_t)blockIdx.x * kRowsPerBlock + threadIdx.x / kW;
   const float2 none = make_float2(-INFINITY, 0.f);
   float2 next0 = none, next1 = none;
   auto fetch = [&](int64_t r) {
     next0 = none;
     next1 = none;
-    if (in_regs && r < p.rows) {
+    if (r < p.rows) {
       if (sub < p.NP) next0 = __ldg(partial_lse + r * p.NP + sub);
-      if (sub + kW < p.NP) next1 = __ldg(partial_lse + r * p.NP + sub + kW);
+      if (kPairs > 1 && sub + kW < p.NP) next1 = __ldg(partial_lse + r * p.NP + sub + kW);
     }
   };
   fetch(row);
   // the rows of a warp end together: a row past the end is worked on without loads or stores
   for (int64_t row0 = row - threadIdx.x / kW + (threadIdx.x >> 5) * (32 / kW); row0 < p.rows; row0 += stride, row += stride) {
     const bool real = row < p.rows;
-    const float2* lse = partial_lse + row * p.NP;
     const float2 cur0 = next0, cur1 = next1;
     fetch(row + stride);
-    float mx = fmaxf(cur0.x, cur1.x);
-    if (!in_regs && real) for (int j = sub; j < p.NP; j += kW) mx = fmaxf(mx, lse[j].x);
+    float mx = kPairs > 1 ? fmaxf(cur0.x, cur1.x) : cur0.x;
 #pragma unroll
     for (int o = kW / 2; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    const float e0 = __expf(cur0.x - mx), e1 = __expf(cur1.x - mx);      // 0 past the partials (lse -inf)
+    const float e0 = __expf(cur0.x - mx), e1 = kPairs > 1 ? __expf(cur1.x - mx) : 0.f;   // 0 past the partials (lse -inf)
     float tot = e0 + e1;
-    if (!in_regs && real) { tot = 0.f; for (int j = sub; j < p.NP; j += kW) tot += __expf(lse[j].x - mx); }
 #pragma unroll
     for (int o = kW / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
     const float inv = failed ? __int_as_float(0x7fc00000) : 1.f / tot;
     // weights of this lane's partials; the row's power-of-two scale is undone with them
-    const float w0 = e0 * cur0.y * inv, w1 = e1 * cur1.y * inv;
+    const float w0 = e0 * cur0.y * inv, w1 = kPairs > 1 ? e1 * cur1.y * inv : 0.f;
     float2 acc[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
-    const uint4* src = reinterpret_cast<const uint4*>(partial_out + row * p.NP * D) + sub;
-    for (int j0 = 0; j0 < p.NP; j0 += kAhead) {
+    const uint4* src = reinterpret_cast<const uint4*>(partial_out + row * p.NP * D) + piece;
+#pragma unroll 1
+    for (int j0 = 0; j0 < p.NP; j0 += kGroups * kAhead) {
       float w[kAhead];
       uint4 o[kAhead];
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
-        const int j = j0 + u;
+        const int j = j0 + u * kGroups + grp;
         o[u] = make_uint4(0u, 0u, 0u, 0u);
-        if (in_regs) {
-          w[u] = __shfl_sync(0xffffffffu, j < kW ? w0 : w1, base_lane + (j & (kW - 1)));
-        } else {
-          const float2 lj = real && j < p.NP ? __ldg(lse + j) : none;
-          w[u] = lj.x != -INFINITY ? __expf(lj.x - mx) * inv * lj.y : 0.f;
+        w[u] = 0.f;
+        // Rows of a warp: a branch, the same for all lanes (head dim 128, 32 partials: 205 us with the loads
+        // predicated only, 179 with it).  Rows of a part of it have no such branch (8 partials: 64 against 85).
+        if (kW < 32 || j0 + u * kGroups < p.NP) {
+          w[u] = __shfl_sync(0xffffffffu, kPairs == 1 || j0 < kW ? w0 : w1, base_lane + (j & (kW - 1)));
+          // (a weight of NaN marks a failed dense stage: it must reach the sum, but the row is not read)
+          if (real && j < p.NP && piece < kPieces && w[u] != 0.f && !failed) o[u] = __ldg(src + j * kPieces);
         }
-        // (a weight of NaN marks a failed dense stage: it must reach the sum, but the row is not read)
-        if (real && j < p.NP && sub < kPieces && w[u] != 0.f && !failed) o[u] = __ldg(src + j * kPieces);
       }
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
@@ -244,33 +249,63 @@ merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __r
         }
       }
     }
+    // the groups' sums
+#pragma unroll
+    for (int o = kW / 2; o >= kGroup; o >>= 1)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        acc[i].x += __shfl_xor_sync(0xffffffffu, acc[i].x, o);
+        acc[i].y += __shfl_xor_sync(0xffffffffu, acc[i].y, o);
+      }
     const int64_t t = row / p.Hq;
     const int h = (int)(row - t * p.Hq);
-    if (real && sub < kPieces) {
+    if (real && grp == 0 && piece < kPieces) {
       uint4 pk;
       pk.x = pack2_16<kHalf>(acc[0].x, acc[0].y);
       pk.y = pack2_16<kHalf>(acc[1].x, acc[1].y);
       pk.z = pack2_16<kHalf>(acc[2].x, acc[2].y);
       pk.w = pack2_16<kHalf>(acc[3].x, acc[3].y);
-      *reinterpret_cast<uint4*>(out + t * p.so_t + (int64_t)h * p.so_h + sub * 8) = pk;
+      *reinterpret_cast<uint4*>(out + t * p.so_t + (int64_t)h * p.so_h + piece * 8) = pk;
     }
     if (real && lse_out != nullptr && sub == 0) lse_out[(int64_t)h * p.Tq + t] = logf(tot) + mx;
   }
 }
 
+template <bool kHalf, int D>
+static cudaError_t launch_merge_dim(const Params& p, const __half* partial_out, const float2* partial_lse,
+                                    const int32_t* status, __nv_bfloat16* out, float* lse_out, cudaStream_t st) {
+  auto launch = [&](auto* kernel, int lanes) {
+    const int rows_per_block = kMergeThreads / lanes;
+    int64_t blocks = (p.rows + rows_per_block - 1) / rows_per_block;
+    if (blocks > 148 * 64) blocks = 148 * 64;
+    return launch_pdl(kernel, dim3((unsigned)blocks), kMergeThreads, 0, st, p, partial_out, partial_lse, status, out, lse_out);
+  };
+  constexpr int kGroup = kMergeGroup<D>;
+  if constexpr (D == 64) {
+    // Eight partials in flight up to three waves of rows, where a row's own latency counts (16 partials: 11200 rows 5.3
+    // against 6.5 us with four), four and more CTAs from there on (131072 rows: 61 against 68).
+    if (p.topk <= kMergeNarrow)
+      return p.rows <= 148 * 3 * 3 * (kMergeThreads / kGroup) ? launch(merge_kernel<kHalf, D, kGroup, 2, 8, 3>, kGroup)
+                                                             : launch(merge_kernel<kHalf, D, kGroup, 2, 4, 5>, kGroup);
+  } else if constexpr (D < 256) {
+    if (p.topk <= kMergeNarrow) return launch(merge_kernel<kHalf, D, kGroup, 1, 4, 5>, kGroup);
+  } else {
+    // one LSE a lane leaves registers for a fifth CTA (131072 rows, 32 partials: 335 -> 323 us)
+    if (p.NP <= 32) return launch(merge_kernel<kHalf, D, 32, 1, 4, 5>, 32);
+  }
+  return launch(merge_kernel<kHalf, D, 32, 2, 4, 4>, 32);
+}
+
 cudaError_t launch_merge(const Params& p, const __half* partial_out, const float2* partial_lse,
                          const int32_t* status, __nv_bfloat16* out, float* lse_out, cudaStream_t st) {
-  const int rows_per_block = kMergeThreads / (p.D <= 64 ? 8 : p.D <= 128 ? 16 : 32);
-  int64_t blocks = (p.rows + rows_per_block - 1) / rows_per_block;
-  if (blocks > 148 * 64) blocks = 148 * 64;
-#define MOBA_MERGE(HALF, DIM) \
-  return launch_pdl(merge_kernel<HALF, DIM>, dim3((unsigned)blocks), kMergeThreads, 0, st, p, partial_out, partial_lse, \
-                    status, out, lse_out)
+#define MOBA_MERGE(DIM)                                                                                          \
+  return p.fp16 ? launch_merge_dim<true, DIM>(p, partial_out, partial_lse, status, out, lse_out, st)             \
+                : launch_merge_dim<false, DIM>(p, partial_out, partial_lse, status, out, lse_out, st)
   switch (p.D) {
-    case 64:  if (p.fp16) MOBA_MERGE(true, 64);  else MOBA_MERGE(false, 64);
-    case 96:  if (p.fp16) MOBA_MERGE(true, 96);  else MOBA_MERGE(false, 96);
-    case 128: if (p.fp16) MOBA_MERGE(true, 128); else MOBA_MERGE(false, 128);
-    case 256: if (p.fp16) MOBA_MERGE(true, 256); else MOBA_MERGE(false, 256);
+    case 64: MOBA_MERGE(64);
+    case 96: MOBA_MERGE(96);
+    case 128: MOBA_MERGE(128);
+    case 256: MOBA_MERGE(256);
     default: return cudaErrorInvalidValue;
   }
 #undef MOBA_MERGE

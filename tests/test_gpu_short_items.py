@@ -6,6 +6,8 @@ significant bits and sum in fp32, so an output element, a weighted mean of value
 rounding of P (2^-9 bf16, 2^-11 fp16 relative, averaging out over the keys) and one rounding of the output:
 at most two units of the output type at magnitude 4, 2^-5 in bf16 and 2^-8 in fp16; the mean
 difference is an order of magnitude below one unit at magnitude 1."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -102,3 +104,48 @@ def test_layouts_of_q_give_the_same_bits(chunk, layout, d):
     # the rows of a list are added in the order of the compaction: fp32 sums, one rounding to bf16
     for a, b in ((dk2, dk), (dv2, dv)):
         assert (a.float() - b.float()).abs().max().item() <= 2.0 ** -7 * b.float().abs().max().item()
+
+
+@pytest.mark.parametrize("d", [64, 96, 128, 256])
+@pytest.mark.parametrize("topk", [1, 9, 16, 17, 33, 64])
+def test_merge_of_few_and_many_partials(topk, d):
+    """The merge has a kernel for rows on a part of a warp (top-k up to 16) and one for rows of a warp, which holds
+    one or two LSEs in a lane: outputs and LSEs against the merge in float64, on rows that fill no
+    block.  A partial is a value of order one at its scale; the result is rounded once to bf16 (2^-9 of values up to 4)
+    and the exponentials are good to 2^-22."""
+    tokens, hq, hkv, chunk = 333, 6, 2, 16
+    rows = tokens * hq
+    g = torch.Generator(device="cuda").manual_seed(topk + d)
+    q = torch.empty(tokens, hq, d, device="cuda", dtype=torch.bfloat16)
+    kv = torch.empty(tokens, hkv, d, device="cuda", dtype=torch.bfloat16)
+    cu = torch.tensor([0, tokens], dtype=torch.int32, device="cuda")
+    out, lse = torch.empty_like(q), torch.empty(hq, tokens, device="cuda")
+    for max_len in (tokens, 16 * 100):                     # 21 chunks, so fewer partials than a top-k of 33 or 64; 100
+        prob = parallel.make_problem(q, kv, kv, out, cu, max_len, chunk, topk)
+        n = G.dims_of(prob).partials
+        assert n == min(topk, -(-max_len // chunk))
+        part = torch.randn(rows, n, d, device="cuda", generator=g).half()
+        pl = torch.randn(rows, n, device="cuda", generator=g) * 3
+        pl[:, 1:][torch.rand(rows, n - 1, device="cuda", generator=g) < 0.3] = -float("inf")    # ranks without a chunk
+        inv_scale = torch.exp2(torch.randint(-2, 3, (rows, n), device="cuda", generator=g).float())
+        pairs = torch.stack([pl, inv_scale], 2).contiguous()
+        _lib.check(_lib.lib().moba_merge(C.byref(prob), part.data_ptr(), pairs.data_ptr(), None, out.data_ptr(),
+                                         lse.data_ptr(), G.stream()))
+        w = torch.softmax(pl.double(), 1)
+        ref = ((w * inv_scale.double())[:, :, None] * part.double()).sum(1)
+        err = (out.view(rows, d).double() - ref).abs()
+        assert (err <= 2.0 ** -8 * ref.abs() + 2.0 ** -16).all(), err.max().item()
+        ref_lse = torch.logsumexp(pl.double(), 1).view(tokens, hq).t()
+        assert (lse.double() - ref_lse).abs().max().item() < 1e-5
+
+
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("topk", [8, 24, 64])
+def test_rows_do_not_depend_on_the_chunks_max_seqlen_allows_for(topk, d):
+    """A longer max_seqlen only adds ranks that hold no chunk: the same bits, also where top-k exceeds the chunks."""
+    lens, hq, hkv, chunk = (700, 150), 4, 2, 64
+    q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, torch.bfloat16, seed=topk)
+    out, lse, _ = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True)
+    for longer in (20 * chunk, 100 * chunk):
+        out2, lse2, _ = parallel.moba_forward(q, k, v, cu, longer, chunk, topk, return_lse=True)
+        assert torch.equal(out2, out) and torch.equal(lse2, lse)
