@@ -351,7 +351,9 @@ __host__ __device__ inline bool tc5_small_tiles(int head_dim, int chunk) { retur
 // one kv head fit one tile (decode steps): a second row tile would be empty.  Measured against the 256-row kernel,
 // whole call: chunk 512, 32768 tokens x 32/8 heads, top-k 8 3.61 -> 3.27 ms (head_dim 64 2.85 -> 2.42), 2 x 4096 x 16
 // 340 -> 308 us, 19456 x 32 983 -> 888 us; chunk 1024 4.66-5.01 against 5.05 ms on the first (the halves read K and V
-// twice as often), so the line lies at 512.
+// twice as often), so the line lies at 512; small launches gain too (700 to 20000 tokens, 1 to 16 heads, chunks 300 and
+// 512: dense stage 0.69 to 1.00 of the other's).  Windows: 1 to 128 rows per kv head, 9000 to 131072 tokens, 1 to 16 kv
+// heads, chunks 1024 to 4096: 0.49 to 1.03 of the other's dense stage, with no more CTAs than items (window_ctas).
 constexpr int kShortChunk = 512;
 inline bool tc5_short_items(const Params& p) {
   if (p.D > 128) return false;
