@@ -392,13 +392,17 @@ static int forward_pass(const moba_problem_t* p, int64_t sel_rs, const void* q, 
                                       (int64_t)(w.zero_bytes / sizeof(int32_t)))) != cudaSuccess)
       return (int)e;
     if (last && (e = mark(1)) != cudaSuccess) return (int)e;
-    // the gating kernel ends with the prefix sums over the lists it counted
+    // with few lists the gating kernel ends with the prefix sums over the lists it counted
+    const bool fused = r.lists <= kGateScanLists;
     const ListScan scan{w.list_counts, w.list_offsets, w.tile_prefix, w.cursors, r.lists,
                         tile_rows_of(p->attend_impl, p->head_dim, p->chunk_size)};
-    if ((e = launch_gate_topk(r, qb, means, cu, sel, w.list_counts, st, &scan, w.status + 1)) != cudaSuccess) return (int)e;
-    if (last && (e = mark(2)) != cudaSuccess) return (int)e;
-    if ((e = launch_scatter(r, cu, sel, w.list_offsets, w.cursors, w.row_list, w.partial_lse, st)) != cudaSuccess)
+    if ((e = launch_gate_topk(r, qb, means, cu, sel, w.list_counts, st, fused ? &scan : nullptr, w.status + 1)) != cudaSuccess)
       return (int)e;
+    if (last && (e = mark(2)) != cudaSuccess) return (int)e;
+    e = fused ? launch_scatter(r, cu, sel, w.list_offsets, w.cursors, w.row_list, w.partial_lse, st)
+              : launch_compact(r, cu, sel, w.list_counts, w.list_offsets, w.tile_prefix, w.cursors, w.row_list,
+                               w.partial_lse, scan.tile_rows, st);
+    if (e != cudaSuccess) return (int)e;
   } else if (last) {
     if ((e = mark(1)) != cudaSuccess || (e = mark(2)) != cudaSuccess) return (int)e;
   }

@@ -149,3 +149,23 @@ def test_rows_do_not_depend_on_the_chunks_max_seqlen_allows_for(topk, d):
     for longer in (20 * chunk, 100 * chunk):
         out2, lse2, _ = parallel.moba_forward(q, k, v, cu, longer, chunk, topk, return_lse=True)
         assert torch.equal(out2, out) and torch.equal(lse2, lse)
+
+
+@pytest.mark.parametrize("chunks", [65, 128])
+def test_prefix_sums_in_the_gating_kernel_and_apart(chunks):
+    """Up to 128 lists (chunks x kv heads of a pass) the gating kernel computes their offsets, beyond a kernel of its
+    own does.  Both heads in one pass have too many for it, one head a pass (a small workspace) has not: the
+    same bits, and the chunk selection and values of the oracle on some rows."""
+    tokens = 16 * chunks - 5
+    q, k, v, cu = _inputs((tokens,), 4, 2, 64, 16, torch.bfloat16, seed=chunks)
+    args = (q, k, v, cu, tokens, 16, 3)
+    out, lse, sel = parallel.moba_forward(*args, return_lse=True, return_selected=True)
+    prob, _ = G.problem_for(q, k, v, cu, tokens, 16, 3)
+    least = C.c_size_t()
+    _lib.check(_lib.lib().moba_workspace_size_min(C.byref(prob), C.byref(least)))
+    out2, lse2, sel2 = parallel.moba_forward(*args, return_lse=True, return_selected=True, workspace_limit=least.value)
+    assert torch.equal(sel2, sel) and torch.equal(out2, out) and torch.equal(lse2, lse)
+    rows = [(t, h) for t in range(0, tokens, 97) for h in (0, 3)]
+    ref, _ = O.attend_rows(q.cpu(), k.cpu(), v.cpu(), cu.cpu().numpy(), tokens, 16, sel.cpu().numpy(), rows)
+    got = torch.stack([out[t, h] for t, h in rows])
+    _close(got.cpu(), ref, torch.bfloat16)
