@@ -55,10 +55,12 @@ cudaError_t launch_chunk_metadata(const Params& p, const int32_t* cu, int32_t* c
 // CTA per 32 dims of it with four times the rows in flight.  A row lane adds its C / 32 rows
 // one after the other (the order is the contract's), so what a long chunk waits for is the latency of that
 // chain: kAhead rows of it are in flight.  Measured: one 4096-key chunk x 8 heads of a decode step 50 -> 20 us; the
-// seven of a 32768-token sequence 58 -> 54 us, where 56 CTAs were enough to half fill HBM.
+// seven of a 32768-token sequence 58 -> 54 us, where 56 CTAs were enough to half fill HBM.  Many short chunks (a
+// CTA adds one or two rows a lane) want all of an SM's threads resident, so up to head dim 128 the registers are held to
+// 32: 42 of them left five CTAs instead of eight (head dim 64, 2048 chunks of 64 keys x 16 heads 107 us, 80 with 32).
 // ---------------------------------------------------------------------------
 template <bool kHalf, int D, int kDims, int kAhead>
-__global__ void __launch_bounds__(kMeanLanes * (kDims / 8))
+__global__ void __launch_bounds__(kMeanLanes * (kDims / 8), kDims == D && D < 256 ? 2048 / (kMeanLanes * (kDims / 8)) : 1)
 chunk_mean_kernel(Params p, int slot_begin, const __nv_bfloat16* __restrict__ k, const int32_t* __restrict__ cu,
                   __nv_bfloat16* __restrict__ means, int32_t* __restrict__ zero, int64_t zero_words) {
   pdl_wait();
