@@ -224,16 +224,29 @@ __host__ __device__ inline int own_item_count(int slots, int Hq, int C, int tile
 // long.  Launched with launch_pdl a kernel may become resident while the one before it drains: it
 // sets up (barriers, tensor memory, descriptors), then pdl_wait() holds it until the grid before it has
 // completed and its writes are visible.  Every kernel so launched calls pdl_wait() in all of its threads before its
-// first access to global memory, and pdl_trigger() behind it, so that at most the next kernel of the
-// stream is resident early.  Both are no-ops in a kernel launched the ordinary way.
+// first access to global memory, and all but the merge call pdl_trigger() behind it, so that at most the next
+// kernel of the stream is resident early.  Both are no-ops in a kernel launched the ordinary way.
 // Measured (B200, events around back-to-back calls), together with the clear of the counters moved into the
 // chunk-mean kernel and the prefix sums into the tail of the gating kernel (seven stream operations
 // become five): one decode token on a 131072-token prefix 224 -> 194 us, 700 tokens behind 50021 245 -> 237 us.
+//
+// A kernel that is resident early is placed where the one before it has left room, not evenly, and runs with the
+// split of L1 and shared memory that it finds.  A few microseconds of launch are not worth that where it runs long:
+//   - the merge triggers nothing: what follows it is the next call, whose chunk means are few long CTAs (268 MB of K
+//     in chunks of 4096, head_dim 64, 700 new tokens, back to back: 375 us with the trigger, 339 without, 369 with
+//     no kernel chained);
+//   - the merge itself is not chained from kChainedMergeBytes of partial rows on (131072 tokens x 16, head_dim 64,
+//     chunk 64, 2.1 GB: 6.83 -> 6.62 ms; 32768 x 32/8, chunk 1024, 1.1 GB 3.98 -> 3.85; 32768 x 32/8, head_dim 128,
+//     chunk 128, 2.1 GB 2.27 -> 2.22; 13311 x 16, 0.22 GB 332 -> 329 us; a decode step's 16 KB: 161 -> 163);
+//   - the gating kernel is not chained behind chunk means of more CTAs than are resident at a time (130859 tokens,
+//     chunk 128, 16 heads, 700 new tokens: 434 -> 413 us; few chunks: 1 to 3 us slower).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+constexpr int64_t kChainedMergeBytes = 64 << 20;
+constexpr int64_t kChainedMeanCtas = 148 * 8;
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st,
-                              Args&&... args) {
+inline cudaError_t launch_chained(bool chained, void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st,
+                                  Args&&... args) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -243,8 +256,12 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, 
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chained ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args&&... args) {
+  return launch_chained(true, kernel, grid, threads, smem, st, std::forward<Args>(args)...);
 }
 
 // Exclusive prefix sums over the lists, by one block of kThreads threads, kPer lists a thread and
@@ -321,7 +338,7 @@ constexpr int kGateScanLists = 128;
 // with `scan`, the last CTA to finish also computes the prefix sums over the lists (`ticket`: a counter at zero)
 cudaError_t launch_gate_topk(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* means,
                              const int32_t* cu, int32_t* selected, int32_t* list_counts,
-                             cudaStream_t st, const ListScan* scan = nullptr, int32_t* ticket = nullptr);
+                             cudaStream_t st, const ListScan* scan = nullptr, int32_t* ticket = nullptr, bool chained = true);
 // The same with optional statistics (int32[4], added to: [0] rows whose near-ties were ranked
 // again in the contract order, [1] largest |estimate - contract score| / eps seen there in
 // units of 2^-16, [2] rows where that ratio exceeded 1, [3] rows ranked over all candidates)
@@ -329,7 +346,7 @@ cudaError_t launch_gate_topk(const Params& p, const __nv_bfloat16* q, const __nv
 cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* means,
                                    const int32_t* cu, int32_t* selected, int32_t* list_counts, int32_t* stats,
                                    int flags, cudaStream_t st, const ListScan* scan = nullptr,
-                                   int32_t* ticket = nullptr);
+                                   int32_t* ticket = nullptr, bool chained = true);
 // false when the shared memory the gating kernel needs for `p` exceeds what an SM offers
 bool gate_topk_fits(const Params& p);
 cudaError_t launch_compact(const Params& p, const int32_t* cu, const int32_t* selected,

@@ -880,7 +880,7 @@ bool gate_topk_fits(const Params& p) { return p.hist <= 0 || gate_launch_config(
 
 cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* means,
                                    const int32_t* cu, int32_t* selected, int32_t* list_counts, int32_t* stats,
-                                   int flags, cudaStream_t st, const ListScan* scan, int32_t* ticket) {
+                                   int flags, cudaStream_t st, const ListScan* scan, int32_t* ticket, bool chained) {
   int tokens_per_cta = kGateRows / p.G;
   if (tokens_per_cta < 1) return cudaErrorInvalidConfiguration;
   const GateLaunch g = gate_launch_config(p);
@@ -926,15 +926,15 @@ cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, cons
   if (resident < 1) resident = 1;
   int64_t grid = (int64_t)sms * resident;
   if (grid > n_tiles) grid = n_tiles;
-  return launch_pdl(kernel, dim3((unsigned)grid), kGateThreads, g.smem, st, p, mq, mm, tokens_per_cta, g.nt, g.list_len,
-                    g.nbuf, g.cnt_in_smem, q, means, cu, selected, list_counts, stats, flags, scan ? *scan : ListScan{},
-                    scan ? ticket : nullptr);
+  return launch_chained(chained, kernel, dim3((unsigned)grid), kGateThreads, g.smem, st, p, mq, mm, tokens_per_cta, g.nt,
+                        g.list_len, g.nbuf, g.cnt_in_smem, q, means, cu, selected, list_counts, stats, flags,
+                        scan ? *scan : ListScan{}, scan ? ticket : nullptr);
 }
 
 cudaError_t launch_gate_topk(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* means,
                              const int32_t* cu, int32_t* selected, int32_t* list_counts,
-                             cudaStream_t st, const ListScan* scan, int32_t* ticket) {
-  return launch_gate_topk_stats(p, q, means, cu, selected, list_counts, nullptr, 0, st, scan, ticket);
+                             cudaStream_t st, const ListScan* scan, int32_t* ticket, bool chained) {
+  return launch_gate_topk_stats(p, q, means, cu, selected, list_counts, nullptr, 0, st, scan, ticket, chained);
 }
 
 }  // namespace moba

@@ -173,8 +173,7 @@ template <bool kHalf, int D, int kW, int kPairs, int kAhead, int kCtas>
 __global__ void __launch_bounds__(kMergeThreads, kCtas)
 merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __restrict__ partial_lse,
              const int32_t* __restrict__ status, __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out) {
-  pdl_wait();
-  pdl_trigger();
+  pdl_wait();                                    // (and no trigger: see launch_chained)
   constexpr int kGroup = kMergeGroup<D>, kGroups = kW / kGroup;
   constexpr int kPieces = D / 8;                 // lanes of a group that hold data (head dim 96: 12 of 16)
   constexpr int kRowsPerBlock = kMergeThreads / kW;
@@ -278,7 +277,9 @@ static cudaError_t launch_merge_dim(const Params& p, const __half* partial_out, 
     const int rows_per_block = kMergeThreads / lanes;
     int64_t blocks = (p.rows + rows_per_block - 1) / rows_per_block;
     if (blocks > 148 * 64) blocks = 148 * 64;
-    return launch_pdl(kernel, dim3((unsigned)blocks), kMergeThreads, 0, st, p, partial_out, partial_lse, status, out, lse_out);
+    const bool chained = p.rows * p.NP * D * (int64_t)sizeof(__half) <= kChainedMergeBytes;
+    return launch_chained(chained, kernel, dim3((unsigned)blocks), kMergeThreads, 0, st, p, partial_out, partial_lse, status,
+                          out, lse_out);
   };
   constexpr int kGroup = kMergeGroup<D>;
   if constexpr (D == 64) {
