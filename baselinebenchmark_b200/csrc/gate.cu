@@ -55,12 +55,15 @@ cudaError_t launch_chunk_metadata(const Params& p, const int32_t* cu, int32_t* c
 // CTA per 32 dims of it with four times the rows in flight.  A row lane adds its C / 32 rows
 // one after the other (the order is the contract's), so what a long chunk waits for is the latency of that
 // chain: kAhead rows of it are in flight.  Measured: one 4096-key chunk x 8 heads of a decode step 50 -> 20 us; the
-// seven of a 32768-token sequence 58 -> 54 us, where 56 CTAs were enough to half fill HBM.  Many short chunks (a
-// CTA adds one or two rows a lane) want all of an SM's threads resident, so up to head dim 128 the registers are held to
-// 32: 42 of them left five CTAs instead of eight (head dim 64, 2048 chunks of 64 keys x 16 heads 107 us, 80 with 32).
+// seven of a 32768-token sequence 58 -> 54 us, where 56 CTAs were enough to half fill HBM.
+// kCtas: CTAs per SM the registers are held to.  Many short chunks (a CTA adds one or two rows a lane) want all of an
+// SM's threads resident: at head dim 64, 42 registers left five CTAs instead of eight (2048 chunks of 64 keys x
+// 16 heads 107 us, 80 with 32).  Few long ones want their loads in flight: with 512 CTAs on chunks of 4096 keys, 268 MB,
+// a call took 340 us with 32 registers, 330 with 54.  So 32 it is where more CTAs come than fit with 48.
+// Split over the dims, 64 registers (eight CTAs) hold ten rows; 106 held sixteen, in four CTAs.
 // ---------------------------------------------------------------------------
-template <bool kHalf, int D, int kDims, int kAhead>
-__global__ void __launch_bounds__(kMeanLanes * (kDims / 8), kDims == D && D < 256 ? 2048 / (kMeanLanes * (kDims / 8)) : 1)
+template <bool kHalf, int D, int kDims, int kAhead, int kCtas>
+__global__ void __launch_bounds__(kMeanLanes * (kDims / 8), kCtas)
 chunk_mean_kernel(Params p, int slot_begin, const __nv_bfloat16* __restrict__ k, const int32_t* __restrict__ cu,
                   __nv_bfloat16* __restrict__ means, int32_t* __restrict__ zero, int64_t zero_words) {
   pdl_wait();
@@ -130,10 +133,12 @@ cudaError_t launch_chunk_means_range(const Params& p, int slot_begin, int slot_e
   // chunk is long enough for several batches of rows.
   const int64_t pairs = (int64_t)(slot_end - slot_begin) * p.Hkv;
   const bool split = pairs < 2 * 148 && p.C >= 8 * kMeanLanes;
+  const bool many = pairs * (kMeanLanes * (p.D / 8)) > 148 * 1280;         // (the same kernel at head dim 256)
 #define MOBA_MEANS(HALF, DIM)                                                                                          \
-  return split ? launch_pdl(chunk_mean_kernel<HALF, DIM, 32, 16>, dim3(slot_end - slot_begin, p.Hkv, DIM / 32),        \
+  return split ? launch_pdl(chunk_mean_kernel<HALF, DIM, 32, 16, 8>, dim3(slot_end - slot_begin, p.Hkv, DIM / 32),     \
                             kMeanLanes * 4, 0, st, p, slot_begin, k, cu, means, zero, zero_words)                      \
-               : launch_pdl(chunk_mean_kernel<HALF, DIM, DIM, 4>, dim3(slot_end - slot_begin, p.Hkv, 1),               \
+               : launch_pdl(many ? chunk_mean_kernel<HALF, DIM, DIM, 4, DIM < 256 ? 2048 / (kMeanLanes * (DIM / 8)) : 1> \
+                                 : chunk_mean_kernel<HALF, DIM, DIM, 4, 1>, dim3(slot_end - slot_begin, p.Hkv, 1),     \
                             kMeanLanes * (DIM / 8), 0, st, p, slot_begin, k, cu, means, zero, zero_words)
   switch (p.D) {
     case 64:  if (p.fp16) MOBA_MEANS(true, 64);  else MOBA_MEANS(false, 64);
