@@ -167,19 +167,19 @@ constexpr int kPolyPairs = MOBA_BWD_POLY_PAIRS;
 template <bool kMasked, bool kHalf>
 __device__ __forceinline__ void ps_row(uint32_t tS, const float2* meta, const int32_t* tok, int key_tok, bool key_ok,
                                        float sl2) {
-  // 32 rows at a time: with sixteen warps a thread has 128 registers
+  uint32_t s[64], g[64];
+  tmem_ld64(tS, s);
+  tmem_ld64(tS + 64, g);
+  tmem_wait_ld();
   const uint64_t scale2 = pack2(sl2, sl2);
 #pragma unroll
   for (int ch = 0; ch < 2; ++ch) {
-    uint32_t s[32], g[32], pp[16], pd[16];
-    tmem_ld32(tS + ch * 32, s);
-    tmem_ld32(tS + 64 + ch * 32, g);
-    tmem_wait_ld();
+    uint32_t pp[16], pd[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const int e = ch * 32 + 2 * i;
       const float4 m = *reinterpret_cast<const float4*>(meta + e);      // {-lse2, delta} of rows e, e + 1
-      uint64_t x = fma2(pack2(__uint_as_float(s[2 * i]), __uint_as_float(s[2 * i + 1])), scale2,
+      uint64_t x = fma2(pack2(__uint_as_float(s[e]), __uint_as_float(s[e + 1])), scale2,
                         pack2(m.x, m.z) ^ 0x8000000080000000ull);
       uint64_t pr;
       if (kMasked) {
@@ -191,7 +191,7 @@ __device__ __forceinline__ void ps_row(uint32_t tS, const float2* meta, const in
       } else {
         pr = pack2(ex2_approx(lo2(x)), ex2_approx(hi2(x)));
       }
-      const uint64_t d = mul2(pr, sub2(pack2(__uint_as_float(g[2 * i]), __uint_as_float(g[2 * i + 1])), pack2(m.y, m.w)));
+      const uint64_t d = mul2(pr, sub2(pack2(__uint_as_float(g[e]), __uint_as_float(g[e + 1])), pack2(m.y, m.w)));
       pp[i] = key_ok ? pack2_16<kHalf>(lo2(pr), hi2(pr)) : 0u;
       pd[i] = key_ok ? pack2_16<kHalf>(lo2(d), hi2(d)) : 0u;
     }
@@ -316,7 +316,12 @@ bwd_dkdv_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
   const float scale = rsqrtf((float)D);
   const float sl2 = scale * 1.4426950408889634f;
   TR_T0(t_kernel);
+  // Registers of a thread in the four warpgroups: 72 + 184 + 184 + 72 = the 4 x 128 of the launch.  The row step keeps S and
+  // dP of its 64 rows in them; with 128 in every warp it had to go through them in two halves and spilled: backward of
+  // 1000 tokens x 16/4 heads at head_dim 64, one chunk, 75 -> 62 us; 32768 x 32/8, chunk 4096 13.6 -> 12.2 ms (head_dim 128
+  // 16.6 -> 16.5).
   if (warp < 4) {
+    setmaxnreg_dec<72>();
     uint32_t g0 = 0;                       // steps of the units this CTA has finished
     uint32_t nu = 0;                       // units this CTA has finished
     Unit u;
@@ -455,6 +460,7 @@ bwd_dkdv_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
       ++nu;
     }
   } else if (warp < 12) {
+    setmaxnreg_inc<184>();
     uint32_t g0 = 0, nu = 0;
     Unit u;
     while (next_unit(p, a, c, key_tiles, n_units, u)) {
@@ -525,6 +531,7 @@ bwd_dkdv_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
     }
   } else {
     // ------------------------------------------------ warps 12-15: bring in the rows, as far ahead as stages are free
+    setmaxnreg_dec<72>();
     uint32_t g0 = 0;
     Unit u;
     while (next_unit(p, a, c, key_tiles, n_units, u)) {
