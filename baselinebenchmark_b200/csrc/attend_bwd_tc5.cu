@@ -431,8 +431,11 @@ bwd_dq_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
       for (int j = 0; j < ntiles; ++j) {
         if (!wait(&c.s_full[x], sph)) break;
         sph ^= 1;
-        // the item's S has run: every role but the other tile's row warps has read its description
-        if (j == 0 && lane == 0) mbar_arrive(smem_u32(&c.slot_free[slot]));
+        // The item's S has run: every role but the other tile's row warps has read its description.  It is let go
+        // four steps before the end, which is time enough to describe the item after the next; at the start of a
+        // long item a CTA would draw two more ahead of CTAs that end before (8192 tokens x 8/2 heads, head_dim 128,
+        // chunk 4096: 270 us, 251 this way).
+        if (j == max(ntiles - 4, 0) && lane == 0) mbar_arrive(smem_u32(&c.slot_free[slot]));
         tc_fence_after();
         const int key0 = j * kBN;
         const bool masked = key0 + kBN > kv_len || (causal && key0 + kBN - 1 > rel);
