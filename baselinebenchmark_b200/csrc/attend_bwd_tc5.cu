@@ -154,13 +154,15 @@ constexpr int kPolyPairs = MOBA_BWD_POLY_PAIRS;
 // the input dtype, written over the first 32 columns of S.
 //   p = 2^(s * scale * log2 e - lse * log2 e),  dS = p * (dP - delta)
 // Rows that do not exist carry lse = +inf (p = 0) and zero Q / dO rows.
-template <bool kMasked, bool kHalf>
+template <bool kMasked, bool kHalf, bool kUnrolled>
 __device__ __forceinline__ void ds_row(uint32_t tS, int key0, int lim, float sl2, float neg_lse2, float delta) {
-  // 32 keys at a time: with sixteen warps a thread has 128 registers
+  // 32 keys at a time: with sixteen warps a thread has 128 registers.  Unrolled, the step is ready a little earlier, which
+  // counts where a step waits for it and for the tensor core in turn (head dim 96, 128, long items: 64 steps 106 -> 105
+  // us); rolled it is less code to fetch, which counts at head dim 64 (16384 tokens x 16/4, chunk 4096 1024 -> 985) and for items of one or two steps.
   const uint64_t scale2 = pack2(sl2, sl2);
   const uint64_t nl2 = pack2(neg_lse2, neg_lse2);
   const uint64_t dl2 = pack2(delta, delta);
-#pragma unroll 1
+#pragma unroll(kUnrolled ? 2 : 1)
   for (int ch = 0; ch < 2; ++ch) {
     uint32_t s[32], g[32], pk[16];
     tmem_ld32(tS + ch * 32, s);
@@ -292,29 +294,22 @@ bwd_dq_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
     for (int n = 0; take(n); ++n) {
       const int ntiles = (c.item[n & 1].kv_len + kBN - 1) / kBN;
       const int tok0 = c.item[n & 1].kv_tok0, head = c.item[n & 1].kv_head;
-      for (int j = 0; ok && j < ntiles; ++j, ++g) {
-        const int tok = tok0 + j * kBN;
-        {
-          const uint32_t s = g % kKStages, par = ((g / kKStages) & 1) ^ 1;
-          if (!wait(&c.k_empty[s], par)) break;
-          if (lane == 0) {
-            const uint32_t bar = smem_u32(&c.k_full[s]);
-            mbar_expect_tx(bar, ((D + 63) / 64) * kKvBlockBytes);
-            tma_load_3d(sK + s * kKvTileBytes, &tmap_k, bar, 0, head, tok);
-            if (D > 64) tma_load_3d(sK + s * kKvTileBytes + kKvBlockBytes, &tmap_k, bar, 64, head, tok);
-          }
+      if (lane == 0)                         // one lane: requests go out a little earlier than behind a vote of the warp
+        for (int j = 0; j < ntiles; ++j, ++g) {
+          const int tok = tok0 + j * kBN;
+          const uint32_t ks = g % kKStages, vs = g & 1;
+          if (!(ok = mbar_wait(smem_u32(&c.k_empty[ks]), ((g / kKStages) & 1) ^ 1))) break;
+          uint32_t bar = smem_u32(&c.k_full[ks]);
+          mbar_expect_tx(bar, ((D + 63) / 64) * kKvBlockBytes);
+          tma_load_3d(sK + ks * kKvTileBytes, &tmap_k, bar, 0, head, tok);
+          if (D > 64) tma_load_3d(sK + ks * kKvTileBytes + kKvBlockBytes, &tmap_k, bar, 64, head, tok);
+          if (!(ok = mbar_wait(smem_u32(&c.v_empty[vs]), ((g >> 1) & 1) ^ 1))) break;
+          bar = smem_u32(&c.v_full[vs]);
+          mbar_expect_tx(bar, ((D + 63) / 64) * kKvBlockBytes);
+          tma_load_3d(sV + vs * kKvTileBytes, &tmap_v, bar, 0, head, tok);
+          if (D > 64) tma_load_3d(sV + vs * kKvTileBytes + kKvBlockBytes, &tmap_v, bar, 64, head, tok);
         }
-        {
-          const uint32_t s = g & 1, par = ((g >> 1) & 1) ^ 1;
-          if (!wait(&c.v_empty[s], par)) break;
-          if (lane == 0) {
-            const uint32_t bar = smem_u32(&c.v_full[s]);
-            mbar_expect_tx(bar, ((D + 63) / 64) * kKvBlockBytes);
-            tma_load_3d(sV + s * kKvTileBytes, &tmap_v, bar, 0, head, tok);
-            if (D > 64) tma_load_3d(sV + s * kKvTileBytes + kKvBlockBytes, &tmap_v, bar, 64, head, tok);
-          }
-        }
-      }
+      ok = __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
       if (!ok) break;
     }
     if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
@@ -347,12 +342,10 @@ bwd_dq_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
     constexpr uint32_t kStageDesc = kKvTileBytes >> 4;
     uint32_t g = 0;                          // key tiles whose dQ has been issued
     uint32_t pph0 = 0, pph1 = 0;             // ds_full phases of tile A / B
-    // S and dP of tile x for key tile `gt` of the CTA: step j of `ntiles` of item n
-    auto s_dp = [&](int x, int n, int j, int ntiles, uint32_t gt) {
-      if (j == 0) {
-        if (!wait(&c.rows_full[x], n & 1)) return;
-        fence_proxy_async_smem();                             // rows written by cp.async, read by the tensor core
-      }
+    // S and dP of tile x for the first step of item n, key tile `gt` of the CTA
+    auto s_dp = [&](int x, int n, int ntiles, uint32_t gt) {
+      if (!wait(&c.rows_full[x], n & 1)) return;
+      fence_proxy_async_smem();                               // rows written by cp.async, read by the tensor core
       if (x == 0 && (!wait(&c.k_full[gt % kKStages], (gt / kKStages) & 1) || !wait(&c.v_full[gt & 1], (gt >> 1) & 1))) return;
       tc_fence_after();
       if (el) {
@@ -360,46 +353,73 @@ bwd_dq_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
         if (x == 0) issue_s_dp<0, kHalf, D>(tm, dq, dg, dk + ko, dv + vo);
         else issue_s_dp<1, kHalf, D>(tm, dq, dg, dk + ko, dv + vo);
         tc_commit(smem_u32(&c.s_full[x]));
-        if (j + 1 == ntiles) tc_commit(smem_u32(&c.rows_free[x]));
+        if (ntiles == 1) tc_commit(smem_u32(&c.rows_free[x]));
         if (x == 1) tc_commit(smem_u32(&c.v_empty[gt & 1]));
       }
       __syncwarp();
     };
     if (take(0)) {
       int ntiles = (c.item[0].kv_len + kBN - 1) / kBN;
-      s_dp(0, 0, 0, ntiles, 0);
-      if (ok) s_dp(1, 0, 0, ntiles, 0);
+      s_dp(0, 0, ntiles, 0);
+      if (ok) s_dp(1, 0, ntiles, 0);
       for (int n = 0; ok; ++n) {
-        int next_tiles = 0;                  // key tiles of item n + 1 (0: there is none)
-        for (int j = 0; ok && j < ntiles; ++j, ++g) {
-          const bool last = j + 1 == ntiles;
-          const uint32_t kcur = g % kKStages;
+        // All steps but the last, whose successor is of the same item.  The issue is part of the chain that a
+        // step waits for, so this loop has nothing in it that depends on where the successor comes from (an item of
+        // 64 steps at head dim 128 112 -> 107 us; one call site for both kinds of successor: 117).
+        for (int j = 0; j + 1 < ntiles; ++j, ++g) {
+          const uint32_t kcur = g % kKStages, g1 = g + 1, knxt = g1 % kKStages, vnxt = g1 & 1;
           if (!wait(&c.ds_full[0], pph0)) break;
           pph0 ^= 1;
           tc_fence_after();
+          if (el) issue_dq<0, kHalf, D>(tm, dkt + kcur * kStageDesc, j == 0);
+          __syncwarp();
+          if (!wait(&c.k_full[knxt], (g1 / kKStages) & 1) || !wait(&c.v_full[vnxt], (g1 >> 1) & 1)) break;
+          tc_fence_after();
           if (el) {
-            issue_dq<0, kHalf, D>(tm, dkt + kcur * kStageDesc, j == 0);
-            if (last) tc_commit(smem_u32(&c.dq_full[0]));
+            issue_s_dp<0, kHalf, D>(tm, dq, dg, dk + knxt * kStageDesc, dv + vnxt * kStageDesc);
+            tc_commit(smem_u32(&c.s_full[0]));
+            if (j + 2 == ntiles) tc_commit(smem_u32(&c.rows_free[0]));
           }
           __syncwarp();
-          if (last) {
-            if (take(n + 1)) next_tiles = (c.item[(n + 1) & 1].kv_len + kBN - 1) / kBN;
-            if (!ok) break;
-          }
-          if (!last) s_dp(0, n, j + 1, ntiles, g + 1);
-          else if (next_tiles > 0) s_dp(0, n + 1, 0, next_tiles, g + 1);
-          if (!ok || !wait(&c.ds_full[1], pph1)) break;
+          if (!wait(&c.ds_full[1], pph1)) break;
           pph1 ^= 1;
           tc_fence_after();
           if (el) {
             issue_dq<1, kHalf, D>(tm, dkt + kcur * kStageDesc, j == 0);
             tc_commit(smem_u32(&c.k_empty[kcur]));
-            if (last) tc_commit(smem_u32(&c.dq_full[1]));
+            issue_s_dp<1, kHalf, D>(tm, dq, dg, dk + knxt * kStageDesc, dv + vnxt * kStageDesc);
+            tc_commit(smem_u32(&c.s_full[1]));
+            if (j + 2 == ntiles) tc_commit(smem_u32(&c.rows_free[1]));
+            tc_commit(smem_u32(&c.v_empty[vnxt]));
           }
           __syncwarp();
-          if (!last) s_dp(1, n, j + 1, ntiles, g + 1);
-          else if (next_tiles > 0) s_dp(1, n + 1, 0, next_tiles, g + 1);
         }
+        if (!ok) break;
+        // the last step, followed by the first of the next item
+        int next_tiles = 0;                  // key tiles of item n + 1 (0: there is none)
+        const uint32_t kcur = g % kKStages;
+        if (!wait(&c.ds_full[0], pph0)) break;
+        pph0 ^= 1;
+        tc_fence_after();
+        if (el) {
+          issue_dq<0, kHalf, D>(tm, dkt + kcur * kStageDesc, ntiles == 1);
+          tc_commit(smem_u32(&c.dq_full[0]));
+        }
+        __syncwarp();
+        if (take(n + 1)) next_tiles = (c.item[(n + 1) & 1].kv_len + kBN - 1) / kBN;
+        if (!ok) break;
+        if (next_tiles > 0) s_dp(0, n + 1, next_tiles, g + 1);
+        if (!ok || !wait(&c.ds_full[1], pph1)) break;
+        pph1 ^= 1;
+        tc_fence_after();
+        if (el) {
+          issue_dq<1, kHalf, D>(tm, dkt + kcur * kStageDesc, ntiles == 1);
+          tc_commit(smem_u32(&c.k_empty[kcur]));
+          tc_commit(smem_u32(&c.dq_full[1]));
+        }
+        __syncwarp();
+        if (next_tiles > 0) s_dp(1, n + 1, next_tiles, g + 1);
+        ++g;
         if (next_tiles == 0) break;
         ntiles = next_tiles;
       }
@@ -439,8 +459,8 @@ bwd_dq_tc5_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
         tc_fence_after();
         const int key0 = j * kBN;
         const bool masked = key0 + kBN > kv_len || (causal && key0 + kBN - 1 > rel);
-        if (masked) ds_row<true, kHalf>(tS, key0, lim, sl2, neg_lse2, delta);
-        else ds_row<false, kHalf>(tS, key0, lim, sl2, neg_lse2, delta);
+        if (masked) ds_row<true, kHalf, (D > 64)>(tS, key0, lim, sl2, neg_lse2, delta);
+        else ds_row<false, kHalf, (D > 64)>(tS, key0, lim, sl2, neg_lse2, delta);
         tc_fence_before();
         mbar_arrive(smem_u32(&c.ds_full[x]));
       }
@@ -752,8 +772,8 @@ bwd_dq_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
           tc_fence_after();
           const int key0 = j * kBN;
           const bool masked = key0 + kBN > it.kv_len || (it.causal && key0 + kBN - 1 > it.tok_rel);
-          if (masked) ds_row<true, kHalf>(tS, key0, lim, sl2, neg_lse2, delta);
-          else ds_row<false, kHalf>(tS, key0, lim, sl2, neg_lse2, delta);
+          if (masked) ds_row<true, kHalf, false>(tS, key0, lim, sl2, neg_lse2, delta);
+          else ds_row<false, kHalf, false>(tS, key0, lim, sl2, neg_lse2, delta);
           tc_fence_before();
         }
         mbar_arrive(smem_u32(&c.ds_full[x]));
