@@ -98,14 +98,16 @@ constexpr int kRowThreads = 256;                 // threads per block of the two
 
 // Both are bound by HBM; what kept them from it was the number of loads in flight.
 // D / 8 lanes (rounded up to a power of two) per row, two rows of a lane in flight (a warp per row, half of its lanes
-// idle at head dim 128: 117 -> 66 us on 19456 tokens x 32 heads, 318 MB).
+// idle at head dim 128: 117 -> 66 us on 19456 tokens x 32 heads, 318 MB).  At head dim 256 a row takes a whole warp
+// anyway, and one row in flight with twice the blocks is faster (8000 x 8: 16.9 -> 14.7 us).
 template <int D> constexpr int kDeltaLanes = D <= 64 ? 8 : D <= 128 ? 16 : 32;
+template <int D> constexpr int kDeltaAhead = D == 256 ? 1 : 2;
 template <bool kHalf, int D>
 __global__ void __launch_bounds__(kRowThreads)
 delta_kernel(Params p, const __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ dout,
              int64_t do_t, int64_t do_h, const float* __restrict__ lse, float* __restrict__ delta,
              float* __restrict__ lse2) {
-  constexpr int kW = kDeltaLanes<D>, kPerBlock = kRowThreads / kW, kAhead = 2;
+  constexpr int kW = kDeltaLanes<D>, kPerBlock = kRowThreads / kW, kAhead = kDeltaAhead<D>;
   const int sub = threadIdx.x & (kW - 1);
   const int64_t stride = (int64_t)gridDim.x * kPerBlock;
   // the loop's bound is the block's: its lanes take part in the shuffles together
@@ -354,10 +356,11 @@ bwd_dq_kernel(Params p, const __nv_bfloat16* __restrict__ q, const __nv_bfloat16
 // order.  D / 4 lanes (rounded up to a power of two, at most 32) per row; which slots hold a
 // contribution is known from one read of the row's selections, so that the slots themselves are read
 // without waiting for one another (a selection read before each slot: 146 -> 83 us on 8191 tokens x 16
-// heads with 8 slots, 570 MB; 293 -> 222 us on 19456 x 32 with 3).
-constexpr int kSumAhead = 8;
+// heads with 8 slots, 570 MB; 293 -> 222 us on 19456 x 32 with 3).  With one or two slots eight loads a lane are
+// loads of slot 0 over and over; two in flight (4096 x 16, head dim 128: one slot 22.3 -> 12.6 us, 15.1 with a loop over
+// the slots; 8192 x 8, two slots 25.3 -> 15.7, 21.4).
 template <int D> constexpr int kSumLanes = D <= 64 ? 16 : 32;
-template <bool kHalf, int D>
+template <bool kHalf, int D, int kSumAhead>
 __global__ void __launch_bounds__(kRowThreads)
 sum_dq_kernel(Params p, const float* __restrict__ partial_dq, const int32_t* __restrict__ selected,
               const int32_t* __restrict__ status, __nv_bfloat16* __restrict__ dq, int64_t dq_t, int64_t dq_h) {
@@ -840,7 +843,8 @@ cudaError_t launch_bwd_delta(const Params& p, const __nv_bfloat16* out, const __
                              int64_t do_h, const float* lse, float* delta, float* lse2, cudaStream_t st) {
   const int per_block = kRowThreads / (p.D <= 64 ? 8 : p.D <= 128 ? 16 : 32);
   int64_t blocks = (p.rows + per_block - 1) / per_block;
-  if (blocks > 148 * 16) blocks = 148 * 16;
+  const int64_t most = 148 * (p.D == 256 ? 32 : 16);
+  if (blocks > most) blocks = most;
 #define MOBA_DELTA(DIM)                                                                                              \
   if (p.fp16) delta_kernel<true, DIM><<<(int)blocks, kRowThreads, 0, st>>>(p, out, dout, do_t, do_h, lse, delta, lse2); \
   else delta_kernel<false, DIM><<<(int)blocks, kRowThreads, 0, st>>>(p, out, dout, do_t, do_h, lse, delta, lse2)
@@ -891,9 +895,11 @@ cudaError_t launch_bwd_sum_dq(const Params& p, const float* partial_dq, const in
   const int per_block = kRowThreads / (p.D <= 64 ? 16 : 32);
   int64_t blocks = (p.rows + per_block - 1) / per_block;
   if (blocks > 148 * 32) blocks = 148 * 32;
-#define MOBA_SUM_DQ(DIM)                                                                                               \
-  if (p.fp16) sum_dq_kernel<true, DIM><<<(int)blocks, kRowThreads, 0, st>>>(p, partial_dq, selected, status, dq, dq_t, dq_h); \
-  else sum_dq_kernel<false, DIM><<<(int)blocks, kRowThreads, 0, st>>>(p, partial_dq, selected, status, dq, dq_t, dq_h)
+#define MOBA_SUM_DQ_HALF(HALF, DIM)                                                                                     \
+  if (p.NP <= 2) sum_dq_kernel<HALF, DIM, 2><<<(int)blocks, kRowThreads, 0, st>>>(p, partial_dq, selected, status, dq, dq_t, dq_h); \
+  else sum_dq_kernel<HALF, DIM, 8><<<(int)blocks, kRowThreads, 0, st>>>(p, partial_dq, selected, status, dq, dq_t, dq_h)
+#define MOBA_SUM_DQ(DIM) \
+  if (p.fp16) { MOBA_SUM_DQ_HALF(true, DIM); } else { MOBA_SUM_DQ_HALF(false, DIM); }
   switch (p.D) {
     case 64: MOBA_SUM_DQ(64); break;
     case 96: MOBA_SUM_DQ(96); break;
@@ -902,6 +908,7 @@ cudaError_t launch_bwd_sum_dq(const Params& p, const float* partial_dq, const in
     default: return cudaErrorInvalidValue;
   }
 #undef MOBA_SUM_DQ
+#undef MOBA_SUM_DQ_HALF
   return cudaGetLastError();
 }
 
