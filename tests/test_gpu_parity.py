@@ -196,17 +196,22 @@ def test_forward_matches_fp32_evaluation(case, impl, dtype):
 @pytest.mark.parametrize("impl", IMPLS)
 @pytest.mark.parametrize("jump", [4.0, 24.0, 140.0])
 @pytest.mark.parametrize("d", [128, 256])
-def test_scores_rising_late_in_a_chunk(impl, dtype, jump, d):
+@pytest.mark.parametrize("chunk,starts", [(256, (150, 460, 700)), (512, (300, 700, 1400)), (1024, (300, 1700, 2900))])
+def test_scores_rising_late_in_a_chunk(impl, dtype, jump, d, chunk, starts):
     """Keys whose scores lie far above everything seen earlier in the same chunk (by `jump`
-    in units of log2 after scaling): the running reference of the softmax has to follow,
-    whatever shortcut a kernel takes on tiles that look ordinary."""
-    t, hq, hkv, chunk, topk = 1536, 4, 2, 512, 3
+    in units of log2 after scaling), after a first rise by half of that: the running reference of the softmax has to
+    follow, whatever shortcut a kernel takes on tiles that look ordinary.  The chunk sizes are those of the
+    kernels: short items at head dim 128 up to 512 and at 256 up to 256, the 256-row kernel and the one
+    for head dim 256 beyond."""
+    t, hq, hkv, topk = 3 * chunk, 4, 2, 3
     g = torch.Generator().manual_seed(int(jump))
     q = torch.ones(t, hq, d) * 0.25
     k = torch.randn(t, hkv, d, generator=g) * 0.05
     v = torch.randn(t, hkv, d, generator=g)
     amp = jump / (0.25 * d * d ** -0.5 * 1.4426950408889634)          # q.k * scale * log2(e) == jump
-    for start in (300, 700, 1400):                                     # late in chunk 0, 1 and 2
+    for start in starts:                                               # late in chunk 0, 1 and 2
+        if start % chunk > 140:
+            k[start - 130:start - 127] = amp / 2                       # in an earlier tile of 128 keys
         k[start:start + 3] = amp
     q, k, v = q.to(dtype), k.to(dtype), v.to(dtype)
     cu = np.array([0, t], dtype=np.int32)
@@ -662,6 +667,17 @@ BACKWARD_CASES = [
     ("bwd_d96_gqa", 96, (900, 257), 8, 2, 128, 4),
     ("bwd_d256", 256, (700, 333), 4, 2, 128, 3),              # mma.sync kernels whichever implementation is asked for
     ("bwd_d256_mqa_c512", 256, (1500,), 4, 1, 512, 3),
+    # chunks of more than 128 keys: two row tiles per item, many key steps; ragged ends, lists that fill one tile only
+    ("bwd_c129", 128, (700, 1, 333), 4, 2, 129, 3),
+    ("bwd_c200_d64", 64, (900, 257, 1), 8, 2, 200, 4),
+    ("bwd_c512", 128, (1500, 130, 520), 8, 2, 512, 2),
+    ("bwd_c512_d64", 64, (1300, 700), 4, 1, 512, 3),
+    ("bwd_c512_d96", 96, (1300, 1, 600), 4, 2, 512, 3),
+    ("bwd_c1000", 128, (2100, 999), 4, 1, 1000, 3),
+    ("bwd_c1000_d64_k2", 64, (2050,), 2, 2, 1000, 2),
+    # chunks between one key step and two: the second is partly masked
+    ("bwd_c100", 128, (700, 333, 1), 4, 2, 100, 4),
+    ("bwd_c100_d64", 64, (450, 270), 4, 4, 100, 9),
 ]
 
 
@@ -906,15 +922,17 @@ def test_config_selection_full_tensor(cfg_id, seed):
     assert counts.sum().item() == (sel_o >= 0).sum()
 
 
-@pytest.mark.parametrize("case", [("long_items", (2048, 900), 8, 2, 128, 512, 4),
+@pytest.mark.parametrize("case", [("long_items", (3000, 900), 8, 2, 128, 1024, 3),
+                                  ("halved_tiles", (2048, 900), 8, 2, 128, 512, 4),
                                   ("short_items", (1500, 700), 8, 2, 128, 128, 5),
+                                  ("d256_long_items", (1700, 300), 4, 2, 256, 512, 3),
                                   ("d256", (1024, 300), 4, 2, 256, 128, 3),
                                   ("mma_sync", (1024, 300), 4, 2, 64, 128, 3)], ids=lambda c: c[0])
 def test_stage_entry_points_chain_to_the_forward_result(case):
     """moba_chunk_means -> moba_gate_topk -> moba_compact_routes -> moba_attend -> moba_merge with
     caller-held buffers (work items of moba_problem_tile_rows rows, fp16 partial rows, {lse,
-    1 / scale} pairs) give bit for bit what moba_forward gives: the three tcgen05 kernels and
-    the mma.sync one."""
+    1 / scale} pairs) give bit for bit what moba_forward gives: the four tcgen05 kernels (the one for short
+    items also on lists cut into 256 rows, half a tile at a time) and the mma.sync one."""
     name, lens, hq, hkv, d, chunk, topk = case
     q, k, v, cu = _case_inputs(lens, hq, hkv, chunk, seed=11, d=d)
     qd, kd, vd = G.to_dev(q, k, v)
@@ -924,7 +942,7 @@ def test_stage_entry_points_chain_to_the_forward_result(case):
     lib = _lib.lib()
     dims = G.dims_of(prob)
     tile_rows = lib.moba_problem_tile_rows(C.byref(prob))
-    assert tile_rows == (256 if name == "long_items" else 128)
+    assert tile_rows == (256 if name in ("long_items", "halved_tiles") else 128)
     m = G.means(prob, kd, cud)
     sel, counts = G.gate(prob, qd, m, cud)
     offsets, tiles, row_list, plse = G.compact(prob, cud, sel, counts, tile_rows)

@@ -1,5 +1,6 @@
-"""GPU: the dense-stage kernel for short items (chunks of at most 512 keys, and query windows with at
-most 128 rows per kv head) and the row gathers, at the sizes and strides where their branches change.
+"""GPU: the dense-stage kernels for short items (chunks of at most 512 keys, at head dim 256 of at most 256, and query
+windows with at most 128 rows per kv head), the row gathers, and the small kernels around them, at the sizes and
+strides where their branches change.
 
 Outputs are compared with the mma.sync dense stage.  Both round P to 16 bits and a partial row to 11
 significant bits and sum in fp32, so an output element, a weighted mean of values of order one, differs by the
@@ -32,7 +33,7 @@ def _close(out, ref, dtype):
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
-@pytest.mark.parametrize("d", [64, 96, 128])
+@pytest.mark.parametrize("d", [64, 96, 128, 256])
 @pytest.mark.parametrize("chunk", [16, 64, 127, 128, 129, 200, 256, 257, 512, 513])
 def test_chunk_sizes_around_the_tiles(chunk, d, dtype):
     lens, hq, hkv, topk = (1, 130, 1025, 700), 6, 2, 5
@@ -46,12 +47,13 @@ def test_chunk_sizes_around_the_tiles(chunk, d, dtype):
 
 
 @pytest.mark.parametrize("hq,hkv", [(4, 4), (8, 2), (16, 1)])
-@pytest.mark.parametrize("chunk", [128, 512, 4096])
-def test_windows_around_the_row_limit_equal_full_run(chunk, hq, hkv):
-    """128 rows per kv head is the largest window of the short kernel; one token more and, with chunks of
-    more than 512 keys, the 256-row kernel runs.  Windows cross chunk and sequence boundaries."""
+@pytest.mark.parametrize("d,chunk", [(128, 128), (128, 512), (128, 4096), (256, 128), (256, 256), (256, 257)])
+def test_windows_around_the_row_limit_equal_full_run(d, chunk, hq, hkv):
+    """128 rows per kv head is the largest window of the short kernel, whose own-chunk items then cover all heads of
+    a group; one token more and, with chunks of more than 512 keys, the 256-row kernel runs.  At head dim 256
+    the chunk alone decides between the kernels (256, 257).  Windows cross chunk and sequence boundaries."""
     lens, topk = (700, 5000), 4
-    q, k, v, cu = _inputs(lens, hq, hkv, 128, chunk, torch.bfloat16, seed=7)
+    q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, torch.bfloat16, seed=7)
     full, lse, sel = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True, return_selected=True)
     limit = 128 // (hq // hkv)
     for begin in (0, 690, 700 + 505, 700 + 4096 - 3, 5700 - limit - 1):
@@ -74,7 +76,7 @@ def _layouts(t, name):
         return t.permute(1, 0, 2).contiguous().permute(1, 0, 2)
     if name == "padded_dim":                               # rows longer than head_dim
         return torch.nn.functional.pad(t, (0, 8))[..., :d]
-    assert name == "odd_token"                             # token stride with no common row grid: the map has no form
+    assert name == "odd_token"                             # a token stride that is no multiple of the head stride
     store = torch.zeros(n * (h * d + 8), dtype=t.dtype, device=t.device)
     view = store.as_strided((n, h, d), (h * d + 8, d, 1))
     view.copy_(t)
@@ -85,8 +87,7 @@ def _layouts(t, name):
 @pytest.mark.parametrize("layout", ["fused", "head_major", "padded_dim", "odd_token"])
 @pytest.mark.parametrize("chunk", [128, 1024])
 def test_layouts_of_q_give_the_same_bits(chunk, layout, d):
-    """Forward, a decode-sized window and the gradients, with q rows reached through each form of the
-    row map and without one."""
+    """Forward, a decode-sized window and the gradients read the rows of q by its token and head strides."""
     lens, hq, hkv, topk = (1500, 2100), 4, 2, 3
     q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, torch.bfloat16, seed=3)
     args = (k, v, cu, max(lens), chunk, topk)
@@ -169,3 +170,62 @@ def test_prefix_sums_in_the_gating_kernel_and_apart(chunks):
     ref, _ = O.attend_rows(q.cpu(), k.cpu(), v.cpu(), cu.cpu().numpy(), tokens, 16, sel.cpu().numpy(), rows)
     got = torch.stack([out[t, h] for t, h in rows])
     _close(got.cpu(), ref, torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d", [64, 96, 128, 256])
+@pytest.mark.parametrize("chunk,chunks", [(16, 400), (100, 400), (300, 5), (300, 160)])
+def test_chunk_means_of_few_and_many_chunks(chunk, chunks, d, dtype):
+    """The mean kernel holds fewer registers when more CTAs come than fit otherwise, and splits long chunks over
+    the dims when few do: bit for bit the oracle's means in every form."""
+    tokens = chunk * chunks + 1
+    _, k, _, cu = _inputs((tokens,), 2, 2, d, chunk, dtype, seed=chunks)
+    prob, _ = G.problem_for(k, k, k, cu, tokens, chunk, 3)
+    cu_chunk, _, valid, _ = O.chunk_slots(cu.cpu().numpy(), tokens, chunk)
+    want = O.chunk_means(k.cpu(), cu_chunk, valid, chunk)
+    assert torch.equal(G.means(prob, k, cu).cpu().view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("topk", [1, 4])
+@pytest.mark.parametrize("chunk", [128, 1024])
+def test_a_call_waits_for_its_inputs_from_another_stream(chunk, topk):
+    """The kernels of a call may become resident before the work in front of them is done.  Inputs written on another
+    stream, behind a kernel that takes milliseconds, must all the same be there when the first of them reads:
+    eagerly behind wait_stream, and captured, where the call follows the join of the two streams."""
+    lens, hq, hkv, d = (1500, 2100), 4, 2, 128
+    src = [_inputs(lens, hq, hkv, d, chunk, torch.bfloat16, seed=s) for s in (1, 2)]
+    want = [parallel.moba_forward(*x, max(lens), chunk, topk)[0] for x in src]
+    bufs = [torch.zeros_like(t) for t in src[0][:3]]
+    stage = [torch.empty_like(t) for t in src[0][:3]]
+    cu = src[0][3]
+    main, side = torch.cuda.Stream(), torch.cuda.Stream()
+
+    def call():
+        side.wait_stream(main)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(6_000_000)                   # about 3 ms
+            for b, t in zip(bufs, stage):
+                b.copy_(t)
+        main.wait_stream(side)
+        return parallel.moba_forward(*bufs, cu, max(lens), chunk, topk)[0]
+
+    main.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(main):
+        for i in (0, 1):
+            for t, x in zip(stage, src[i]):
+                t.copy_(x)
+            out = call()
+            main.synchronize()
+            assert torch.equal(out, want[i])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=main):
+        out = call()
+    with torch.cuda.stream(main):
+        for i in (0, 1):
+            for b in bufs:
+                b.zero_()
+            for t, x in zip(stage, src[i]):
+                t.copy_(x)
+            graph.replay()
+            main.synchronize()
+            assert torch.equal(out, want[i])
