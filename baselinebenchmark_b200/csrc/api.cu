@@ -105,7 +105,7 @@ Params make_params(const moba_problem_t* p) {
 struct Workspace {
   __nv_bfloat16* means;
   int32_t* selected;
-  int32_t* list_counts;      // [lists] + work counter + status, zeroed per call in one memset
+  int32_t* list_counts;      // [lists] + work counter + status, zeroed per call (by the chunk-mean kernel where one runs)
   int32_t* work_counter;
   int32_t* status;
   int32_t* list_offsets;

@@ -153,7 +153,9 @@ constexpr int kPolyPairs = MOBA_BWD_POLY_PAIRS;
 // One step of one row: S and dP (64 fp32 columns each of this thread's TMEM lane) -> dS in
 // the input dtype, written over the first 32 columns of S.
 //   p = 2^(s * scale * log2 e - lse * log2 e),  dS = p * (dP - delta)
-// Rows that do not exist carry lse = +inf (p = 0) and zero Q / dO rows.
+// Rows that do not exist carry lse = +inf, but their Q and dO rows are whatever the tile held before, NaN
+// included: their dS and dQ rows may be anything, are never stored and are added to nothing (a row of the tile only
+// enters its own row of S, dP and dQ).
 template <bool kMasked, bool kHalf, bool kUnrolled>
 __device__ __forceinline__ void ds_row(uint32_t tS, int key0, int lim, float sl2, float neg_lse2, float delta) {
   // 32 keys at a time: with sixteen warps a thread has 128 registers.  Unrolled, the step is ready a little earlier, which

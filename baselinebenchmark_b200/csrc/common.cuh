@@ -12,7 +12,6 @@
 
 namespace moba {
 
-constexpr int kHeadDim = 128;            // largest head dim of the tcgen05 dense stage (64 and 128; others: mma.sync stage)
 constexpr int kMeanLanes = 32;           // row accumulators of a chunk mean
 constexpr int kMaxTopk = 64;             // parallel.py:436
 
@@ -377,6 +376,7 @@ __host__ __device__ inline bool tc5_small_tiles(int head_dim, int chunk) { retur
 // 512: dense stage 0.69 to 1.00 of the other's).  Windows: 1 to 128 rows per kv head, 9000 to 131072 tokens, 1 to 16 kv
 // heads, chunks 1024 to 4096: 0.49 to 1.03 of the other's dense stage, with no more CTAs than items (window_ctas).
 constexpr int kShortChunk = 512;
+static_assert(kSmallChunk <= kShortChunk, "lists cut into 128 rows run the kernel of one-tile items");
 inline bool tc5_short_items(const Params& p) {
   if (p.D > 128) return false;
   if (p.Tq * p.G <= kTileRowsWide) return true;
