@@ -69,20 +69,27 @@ class IncrementalMoba:
     def _plain(self, k: torch.Tensor, v: torch.Tensor) -> bool:
         """Rows that moba_append copies as they are: the caches' type, device and row shape, 16-byte pieces, memory
         of their own, and nothing for autograd to record.  Everything else goes through torch's copy."""
-        row, dtype, device = self.k.shape[1:], self.k.dtype, self.k.device
-        caches = [(c.untyped_storage().data_ptr(), c.untyped_storage().nbytes()) for c in (self.k, self.v)]
+        kc, vc, cu = self.k, self.v, self.cu               # each attribute read once: this runs on every call
+        if kc.requires_grad or vc.requires_grad:
+            return False
+        # torch refuses to write an inference tensor outside inference mode: leave that to its copy
+        if (kc.is_inference() or vc.is_inference() or cu.is_inference()) and not torch.is_inference_mode_enabled():
+            return False
+        (size, heads, dim), dtype, device = kc.shape, kc.dtype, kc.device
+        (k0, k1, _), (v0, v1, _), k_at, v_at = kc.stride(), vc.stride(), kc.data_ptr(), vc.data_ptr()
+        k_end = k_at + 2 * ((size - 1) * k0 + (heads - 1) * k1 + dim)
+        v_end = v_at + 2 * ((size - 1) * v0 + (heads - 1) * v1 + dim)
         for t in (k, v):
+            shape = t.shape
+            if len(shape) != 3 or shape[1] != heads or shape[2] != dim or t.dtype != dtype or t.device != device or t.requires_grad:
+                return False
+            (s0, s1, s2), at = t.stride(), t.data_ptr()
+            if s2 != 1 or s0 % 8 or s1 % 8 or at % 16:
+                return False
             # One kernel reads the rows and writes both caches: rows that share memory with either of them go
             # through torch, one cache after the other.
-            mem, size = t.untyped_storage().data_ptr(), t.untyped_storage().nbytes()
-            if any(mem < at + n and at < mem + size for at, n in caches):
-                return False
-            if (t.shape[1:] != row or t.dtype != dtype or t.device != device or t.stride(2) != 1 or t.stride(0) % 8
-                    or t.stride(1) % 8 or t.data_ptr() % 16 or t.requires_grad):
-                return False
-        for c in (self.k, self.v, self.cu):
-            # torch refuses to write an inference tensor outside inference mode: leave that to its copy
-            if c.requires_grad or (c.is_inference() and not torch.is_inference_mode_enabled()):
+            end = at + 2 * ((shape[0] - 1) * s0 + (heads - 1) * s1 + dim)
+            if at < k_end and k_at < end or at < v_end and v_at < end:
                 return False
         return True
 
