@@ -393,7 +393,7 @@ static int forward_pass(const moba_problem_t* p, int64_t sel_rs, const void* q, 
       return (int)e;
     if (last && (e = mark(1)) != cudaSuccess) return (int)e;
     // with few lists the gating kernel ends with the prefix sums over the lists it counted
-    const bool fused = r.lists <= kGateScanLists;
+    const bool fused = gate_scans_lists(r);
     const ListScan scan{w.list_counts, w.list_offsets, w.tile_prefix, w.cursors, r.lists,
                         tile_rows_of(p->attend_impl, p->head_dim, p->chunk_size)};
     const int64_t mean_ctas = (int64_t)(r.slots - (opt.means_ext ? opt.means_from : 0)) * r.Hkv;

@@ -332,8 +332,10 @@ cudaError_t launch_chunk_means_range(const Params& p, int slot_begin, int slot_e
 // Up to this many lists the gating kernel's last CTA computes the prefix sums over them, which saves a launch; the
 // kernel that does it otherwise takes more lists at a time and leaves the gating CTAs without the ticket.  Whole
 // call, fused / apart: 4 lists 30.3 / 31.2 us, 20 48.1 / 48.8, 128 48.1 / 48.1, 256 107.9 / 105.2 and 198.5 / 189.6,
-// 392 180 / 175, 2048 278.7 / 273.6, 30000 2792 / 2775 (gating alone 90 us longer, scatter 60 shorter).
-constexpr int kGateScanLists = 128;
+// 392 180 / 175, 2048 278.7 / 273.6, 30000 2792 / 2775 (gating alone 90 us longer, scatter 60 shorter).  Calls of few
+// rows are as long as the host takes to issue them, and there a launch counts for more: one decode token, 160
+// lists, 35.0 / 35.0 us with the host ahead, 38.9 / 40.4 through an append; 256 lists 121.5 / 120.4 with the host ahead.
+inline bool gate_scans_lists(const Params& p) { return p.lists <= (p.rows <= 4096 ? 256 : 128); }
 // with `scan`, the last CTA to finish also computes the prefix sums over the lists (`ticket`: a counter at zero)
 cudaError_t launch_gate_topk(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* means,
                              const int32_t* cu, int32_t* selected, int32_t* list_counts,

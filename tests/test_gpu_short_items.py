@@ -154,8 +154,8 @@ def test_rows_do_not_depend_on_the_chunks_max_seqlen_allows_for(topk, d):
 
 @pytest.mark.parametrize("chunks", [65, 128])
 def test_prefix_sums_in_the_gating_kernel_and_apart(chunks):
-    """Up to 128 lists (chunks x kv heads of a pass) the gating kernel computes their offsets, beyond a kernel of its
-    own does.  Both heads in one pass have too many for it, one head a pass (a small workspace) has not: the
+    """Up to 128 lists (chunks x kv heads of a pass) the gating kernel computes their offsets (calls of many rows), beyond a
+    kernel of its own does.  Both heads in one pass have too many for it, one head a pass (a small workspace) has not: the
     same bits, and the chunk selection and values of the oracle on some rows."""
     tokens = 16 * chunks - 5
     q, k, v, cu = _inputs((tokens,), 4, 2, 64, 16, torch.bfloat16, seed=chunks)
@@ -170,6 +170,19 @@ def test_prefix_sums_in_the_gating_kernel_and_apart(chunks):
     ref, _ = O.attend_rows(q.cpu(), k.cpu(), v.cpu(), cu.cpu().numpy(), tokens, 16, sel.cpu().numpy(), rows)
     got = torch.stack([out[t, h] for t, h in rows])
     _close(got.cpu(), ref, torch.bfloat16)
+
+
+@pytest.mark.parametrize("chunks", [256, 257])
+def test_prefix_sums_of_a_window_of_few_rows(chunks):
+    """The line lies at 256 lists for calls of few rows: windows on both sides of it equal the rows of the full run."""
+    tokens = 16 * chunks - 5
+    q, k, v, cu = _inputs((tokens,), 4, 1, 64, 16, torch.bfloat16, seed=chunks)
+    args = (k, v, cu, tokens, 16, 3)
+    full, lse, sel = parallel.moba_forward(q, *args, return_lse=True, return_selected=True)
+    for begin, n in ((tokens - 1, 1), (2000, 3), (7, 1000)):
+        o, l, s = parallel.moba_forward(q[begin:begin + n], *args, return_lse=True, return_selected=True, q_token_begin=begin)
+        assert torch.equal(s, sel[:, :, begin:begin + n]) and torch.equal(o, full[begin:begin + n])
+        assert torch.equal(l, lse[:, begin:begin + n])
 
 
 @pytest.mark.parametrize("dtype", DTYPES)
