@@ -44,7 +44,7 @@ SEQ_LEN = 131072
 NUM_SEQS = 16
 SEQS_PER_CALL = 2         # sequences per operator call (16 units: 18 GB of partial results)
 HQ, HKV, D, CHUNK, TOPK = 32, 8, 128, 4096, 8
-KERNELS_PER_CALL = 5      # chunk_mean, gate_topk, scatter_routes, attend, merge
+KERNELS_PER_CALL = 6      # chunk_mean, gate_topk, scan_lists (512 lists a call), scatter_routes, attend, merge
 # dram__bytes_read.sum + dram__bytes_write.sum of one attend_tc5_kernel launch on configs[2]
 # (32768 tokens x 32 heads, 8 partial results per row), from an ncu capture of that launch
 ATTEND_TRAFFIC_CFG2 = 2.610216e9 + 1.323296e9
