@@ -523,8 +523,11 @@ int moba_append(const moba_problem_t* p, const void* q, const void* k_new, const
                                            static_cast<__nv_bfloat16*>(k_cache), static_cast<__nv_bfloat16*>(v_cache), cu,
                                            (cudaStream_t)stream);
   if (e != cudaSuccess) return (int)e;
-  return moba_forward_cached(p, q, k_cache, v_cache, cu, out, nullptr, selected_out, means_cache, cached_slots, workspace,
-                             workspace_bytes, stream);
+  PassOptions opt;                                           // and checked once: the pass itself, not the entry point
+  opt.means_ext = static_cast<__nv_bfloat16*>(means_cache);
+  opt.means_from = cached_slots;
+  return forward_pass(p, r.sel_rs, q, k_cache, v_cache, cu, out, nullptr, selected_out, workspace, (cudaStream_t)stream,
+                      nullptr, true, true, opt);
 }
 
 // ---------------------------------------------------------------------------
