@@ -166,7 +166,7 @@ int moba_forward_cached(const moba_problem_t* p, const void* q, const void* k, c
  * cu_seqlens = {0, total_tokens}, and runs moba_forward_cached on the new tokens' query window, in
  * one call and with the rows copied by one kernel.  A decode step is a handful of microseconds of
  * kernels and was bound by the host: one token behind 20011 (16/4 heads, head_dim 64, chunk 512) took 74 us with two
- * copies, a fill and the forward as operations of their own, 37 us this way.
+ * copies, a fill and the forward as operations of their own, 38 us this way.
  *   p              batch 1; total_tokens = tokens after the append, q_token_begin / q_tokens = the
  *                  new ones; k_/v_stride_* are those of the caches
  *   k_new, v_new   [q_tokens, Hkv, D] with the given token and head strides (elements, multiples of
