@@ -146,7 +146,7 @@ cudaError_t launch_scatter(const Params& p, const int32_t* cu, const int32_t* se
 
 // ---------------------------------------------------------------------------
 // merge: a (token, head) row is combined by D / 8 lanes (rounded up to a power of two: one row a warp at
-// head dim 256, two at 128 and 96, four at 64), or, from top-k 17 on, by a whole warp.
+// head dim 256, two at 128 and 96, four at 64), or, from 17 partials on, by a whole warp.
 //   lse_tot = log sum_j exp(lse_j);  out = sum_j O_j * exp(lse_j - lse_tot)
 // (exponentials through ex2.approx: relative error 2^-22, far below the rounding of the output)
 // Bound by HBM by bytes, with few partials in practice by issue slots: a whole warp per row spends as many
@@ -158,18 +158,20 @@ cudaError_t launch_scatter(const Params& p, const int32_t* cu, const int32_t* se
 //   head dim 64,  rows of 8 lanes    17.7  35.5  61.3     -     -
 //                 rows of a warp     52.4  64.0  71.4   105   180
 // (reading the LSEs again for each partial where they do not fit the registers: 209 / 812 us at 128 with 32 / 64,
-// 236 / 451 at 64), so the line lies at 16.  It is drawn by top-k, not by the partials of the call: the two add a row's
-// partials in different orders, and a row must come out the same bits however many chunks max_seqlen allows for.
+// 236 / 451 at 64), so the line lies at 16.  A row must come out the same bits however many chunks max_seqlen allows
+// for, and the two add its partials in different orders.  So a top-k above 16 with few partials also runs on a
+// part of a warp, but with the sums of the other's groups (kSums of them, added up in its order).
 // ---------------------------------------------------------------------------
 constexpr int kMergeThreads = 256;
-constexpr int kMergeNarrow = 16;                 // largest top-k whose rows are on a part of a warp
+constexpr int kMergeNarrow = 16;                 // most partials of a row on a part of a warp
 
 // A partial row is D/8 pieces of eight fp16 values (16 bytes), one per lane of a group of lanes.  A row has
 // kW lanes: one group, which takes the partials of the row in turn, or all 32 lanes of a warp, whose groups take
 // every second (head dim 96, 128) or fourth (64) partial and add their sums at the end.
-// kAhead partials of a group are in flight, kPairs LSEs in each lane.
+// kAhead partials of a group are in flight, kPairs LSEs in each lane.  kSums: sums a group keeps, partial j in sum
+// j mod kSums.
 template <int D> constexpr int kMergeGroup = D <= 64 ? 8 : D <= 128 ? 16 : 32;
-template <bool kHalf, int D, int kW, int kPairs, int kAhead, int kCtas>
+template <bool kHalf, int D, int kW, int kPairs, int kAhead, int kCtas, int kSums = 1>
 __global__ void __launch_bounds__(kMergeThreads, kCtas)
 merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __restrict__ partial_lse,
              const int32_t* __restrict__ status, __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out) {
@@ -179,6 +181,7 @@ merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __r
   constexpr int kRowsPerBlock = kMergeThreads / kW;
   static_assert(kPairs == 1 || kPairs == 2, "LSEs of a lane");
   static_assert(kW % (kGroups * kAhead) == 0, "the partials of a round lie on one side of kW");
+  static_assert(kAhead % kSums == 0 && (kSums == 1 || kGroups == 1), "sums by the place in a round");
   const int lane = threadIdx.x & 31;
   const int sub = lane & (kW - 1);               // lane of the row
   const int grp = sub / kGroup, piece = sub & (kGroup - 1);
@@ -216,9 +219,11 @@ merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __r
     const float inv = failed ? __int_as_float(0x7fc00000) : 1.f / tot;
     // weights of this lane's partials; the row's power-of-two scale is undone with them
     const float w0 = e0 * cur0.y * inv, w1 = kPairs > 1 ? e1 * cur1.y * inv : 0.f;
-    float2 acc[4];
+    float2 sums[kSums][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
+    for (int a = 0; a < kSums; ++a)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sums[a][i] = make_float2(0.f, 0.f);
     const uint4* src = reinterpret_cast<const uint4*>(partial_out + row * p.NP * D) + piece;
 #pragma unroll 1
     for (int j0 = 0; j0 < p.NP; j0 += kGroups * kAhead) {
@@ -243,12 +248,22 @@ merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __r
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&words[i]));
-          acc[i].x += w[u] * a.x;
-          acc[i].y += w[u] * a.y;
+          sums[u % kSums][i].x += w[u] * a.x;
+          sums[u % kSums][i].y += w[u] * a.y;
         }
       }
     }
-    // the groups' sums
+    // the sums of a group, and of the groups
+#pragma unroll
+    for (int o = kSums / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int a = 0; a < o; ++a)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          sums[a][i].x += sums[a + o][i].x;
+          sums[a][i].y += sums[a + o][i].y;
+        }
+    float2(&acc)[4] = sums[0];
 #pragma unroll
     for (int o = kW / 2; o >= kGroup; o >>= 1)
 #pragma unroll
@@ -281,15 +296,20 @@ static cudaError_t launch_merge_dim(const Params& p, const __half* partial_out, 
     return launch_chained(chained, kernel, dim3((unsigned)blocks), kMergeThreads, 0, st, p, partial_out, partial_lse, status,
                           out, lse_out);
   };
-  constexpr int kGroup = kMergeGroup<D>;
+  constexpr int kGroup = kMergeGroup<D>, kSums = 32 / kGroup;
+  const bool many = p.topk > kMergeNarrow;                   // (few partials of a top-k whose rows are on a warp elsewhere)
   if constexpr (D == 64) {
     // Eight partials in flight up to three waves of rows, where a row's own latency counts (16 partials: 11200 rows 5.3
     // against 6.5 us with four), four and more CTAs from there on (131072 rows: 61 against 68).
-    if (p.topk <= kMergeNarrow)
-      return p.rows <= 148 * 3 * 3 * (kMergeThreads / kGroup) ? launch(merge_kernel<kHalf, D, kGroup, 2, 8, 3>, kGroup)
-                                                             : launch(merge_kernel<kHalf, D, kGroup, 2, 4, 5>, kGroup);
+    if (p.NP <= kMergeNarrow) {
+      if (p.rows <= 148 * 3 * 3 * (kMergeThreads / kGroup))
+        return many ? launch(merge_kernel<kHalf, D, kGroup, 2, 4, 3, kSums>, kGroup) : launch(merge_kernel<kHalf, D, kGroup, 2, 8, 3>, kGroup);
+      return many ? launch(merge_kernel<kHalf, D, kGroup, 2, 4, 4, kSums>, kGroup) : launch(merge_kernel<kHalf, D, kGroup, 2, 4, 5>, kGroup);
+    }
   } else if constexpr (D < 256) {
-    if (p.topk <= kMergeNarrow) return launch(merge_kernel<kHalf, D, kGroup, 1, 4, 5>, kGroup);
+    // two sums leave four CTAs: ahead of a warp per row up to 8 partials (3: 40 against 63 us, 8: 72 against 70, 16: 117 / 105)
+    if (many && p.NP <= kMergeNarrow / 2) return launch(merge_kernel<kHalf, D, kGroup, 1, 4, 4, kSums>, kGroup);
+    if (!many) return launch(merge_kernel<kHalf, D, kGroup, 1, 4, 5>, kGroup);
   } else {
     // one LSE a lane leaves registers for a fifth CTA (131072 rows, 32 partials: 335 -> 323 us)
     if (p.NP <= 32) return launch(merge_kernel<kHalf, D, 32, 1, 4, 5>, 32);

@@ -110,18 +110,18 @@ def test_layouts_of_q_give_the_same_bits(chunk, layout, d):
 @pytest.mark.parametrize("d", [64, 96, 128, 256])
 @pytest.mark.parametrize("topk", [1, 9, 16, 17, 33, 64])
 def test_merge_of_few_and_many_partials(topk, d):
-    """The merge has a kernel for rows on a part of a warp (top-k up to 16) and one for rows of a warp, which holds
-    one or two LSEs in a lane: outputs and LSEs against the merge in float64, on rows that fill no
+    """The merge has forms for rows on a part of a warp (few partials, with one sum or the sums of the other form) and
+    for rows of a warp, with one or two LSEs in a lane: outputs and LSEs against the merge in float64, on rows that fill no
     block.  A partial is a value of order one at its scale; the result is rounded once to bf16 (2^-9 of values up to 4)
     and the exponentials are good to 2^-22."""
-    tokens, hq, hkv, chunk = 333, 6, 2, 16
+    tokens, hq, hkv, chunk = 333, 6, 2, 16                 # 21 chunks
     rows = tokens * hq
     g = torch.Generator(device="cuda").manual_seed(topk + d)
     q = torch.empty(tokens, hq, d, device="cuda", dtype=torch.bfloat16)
     kv = torch.empty(tokens, hkv, d, device="cuda", dtype=torch.bfloat16)
     cu = torch.tensor([0, tokens], dtype=torch.int32, device="cuda")
     out, lse = torch.empty_like(q), torch.empty(hq, tokens, device="cuda")
-    for max_len in (tokens, 16 * 100):                     # 21 chunks, so fewer partials than a top-k of 33 or 64; 100
+    for max_len in (16 * 3, 16 * 11, tokens, 16 * 100):    # partials: the chunks, where top-k allows for more
         prob = parallel.make_problem(q, kv, kv, out, cu, max_len, chunk, topk)
         n = G.dims_of(prob).partials
         assert n == min(topk, -(-max_len // chunk))
@@ -140,11 +140,13 @@ def test_merge_of_few_and_many_partials(topk, d):
         assert (lse.double() - ref_lse).abs().max().item() < 1e-5
 
 
-@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("d", [64, 96, 128, 256])
 @pytest.mark.parametrize("topk", [8, 24, 64])
-def test_rows_do_not_depend_on_the_chunks_max_seqlen_allows_for(topk, d):
-    """A longer max_seqlen only adds ranks that hold no chunk: the same bits, also where top-k exceeds the chunks."""
-    lens, hq, hkv, chunk = (700, 150), 4, 2, 64
+@pytest.mark.parametrize("tokens", [450, 700, 1100])
+def test_rows_do_not_depend_on_the_chunks_max_seqlen_allows_for(tokens, topk, d):
+    """A longer max_seqlen only adds ranks that hold no chunk: the same bits, also where top-k exceeds the chunks (8, 11
+    and 18 of them here) and the merge adds a row's partials another way."""
+    lens, hq, hkv, chunk = (tokens, 150), 4, 2, 64
     q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, torch.bfloat16, seed=topk)
     out, lse, _ = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True)
     for longer in (20 * chunk, 100 * chunk):
