@@ -414,8 +414,11 @@ static int forward_pass(const moba_problem_t* p, int64_t sel_rs, const void* q, 
                                   static_cast<__half*>(w.partial_out), w.partial_lse, w.work_counter, w.status, st);
   if (arc != 0) return arc;
   if (last && (e = mark(4)) != cudaSuccess) return (int)e;
+  const int64_t mean_slots = opt.means_ready ? 0 : r.slots - (opt.means_ext ? opt.means_from : 0);
+  const int64_t mean_rows = mean_slots * r.C < r.T ? mean_slots * r.C : r.T;
   e = launch_merge(r, static_cast<const __half*>(w.partial_out), w.partial_lse, w.status,
-                   static_cast<__nv_bfloat16*>(out), lse_out, st);
+                   static_cast<__nv_bfloat16*>(out), lse_out, st,
+                   mean_rows * r.Hkv * r.D * (int64_t)sizeof(__nv_bfloat16) <= kTriggerMeanBytes);
   if (e != cudaSuccess) return (int)e;
   return last ? (int)mark(5) : MOBA_OK;
 }

@@ -223,7 +223,7 @@ __host__ __device__ inline int own_item_count(int slots, int Hq, int C, int tile
 // long.  Launched with launch_pdl a kernel may become resident while the one before it drains: it
 // sets up (barriers, tensor memory, descriptors), then pdl_wait() holds it until the grid before it has
 // completed and its writes are visible.  Every kernel so launched calls pdl_wait() in all of its threads before its
-// first access to global memory, and all but the merge call pdl_trigger() behind it, so that at most the next
+// first access to global memory, and pdl_trigger() behind it (the merge: not always), so that at most the next
 // kernel of the stream is resident early.  Both are no-ops in a kernel launched the ordinary way.
 // Measured (B200, events around back-to-back calls), together with the clear of the counters moved into the
 // chunk-mean kernel and the prefix sums into the tail of the gating kernel (seven stream operations
@@ -231,9 +231,10 @@ __host__ __device__ inline int own_item_count(int slots, int Hq, int C, int tile
 //
 // A kernel that is resident early is placed where the one before it has left room, not evenly, and runs with the
 // split of L1 and shared memory that it finds.  A few microseconds of launch are not worth that where it runs long:
-//   - the merge triggers nothing: what follows it is the next call, whose chunk means are few long CTAs (268 MB of K
-//     in chunks of 4096, head_dim 64, 700 new tokens, back to back: 375 us with the trigger, 339 without, 369 with
-//     no kernel chained);
+//   - the merge triggers nothing in a call that averages more than kTriggerMeanBytes of K: what follows it is
+//     likely a call of the same kind, whose chunk means are few long CTAs (268 MB of K in chunks of 4096, head_dim 64, 700
+//     new tokens, back to back: 375 us with the trigger, 339 without, 369 with no kernel chained; one decode token
+//     behind 20011, appended back to back: 37.9 with it, 38.6 without);
 //   - the merge itself is not chained from kChainedMergeBytes of partial rows on (131072 tokens x 16, head_dim 64,
 //     chunk 64, 2.1 GB: 6.83 -> 6.62 ms; 32768 x 32/8, chunk 1024, 1.1 GB 3.98 -> 3.85; 32768 x 32/8, head_dim 128,
 //     chunk 128, 2.1 GB 2.27 -> 2.22; 13311 x 16, 0.22 GB 332 -> 329 us; a decode step's 16 KB: 161 -> 163);
@@ -241,6 +242,7 @@ __host__ __device__ inline int own_item_count(int slots, int Hq, int C, int tile
 //     chunk 128, 16 heads, 700 new tokens: 434 -> 413 us; few chunks: 1 to 3 us slower).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+constexpr int64_t kTriggerMeanBytes = 8 << 20;
 constexpr int64_t kChainedMergeBytes = 64 << 20;
 constexpr int64_t kChainedMeanCtas = 148 * 8;
 template <typename... KArgs, typename... Args>
@@ -358,7 +360,7 @@ cudaError_t launch_compact(const Params& p, const int32_t* cu, const int32_t* se
 cudaError_t launch_scatter(const Params& p, const int32_t* cu, const int32_t* selected, const int32_t* list_offsets,
                            int32_t* cursors, int32_t* row_list, float2* partial_lse, cudaStream_t st);
 cudaError_t launch_merge(const Params& p, const __half* partial_out, const float2* partial_lse,
-                         const int32_t* status, __nv_bfloat16* out, float* lse_out, cudaStream_t st);
+                         const int32_t* status, __nv_bfloat16* out, float* lse_out, cudaStream_t st, bool trigger = false);
 
 constexpr int kMmaTileRows = 128;        // rows per work item, mma.sync kernel
 constexpr int kTc5TileRows = 256;        // rows per work item, tcgen05 kernel (two 128-row MMA tiles)

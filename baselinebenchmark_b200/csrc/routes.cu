@@ -174,8 +174,9 @@ template <int D> constexpr int kMergeGroup = D <= 64 ? 8 : D <= 128 ? 16 : 32;
 template <bool kHalf, int D, int kW, int kPairs, int kAhead, int kCtas, int kSums = 1>
 __global__ void __launch_bounds__(kMergeThreads, kCtas)
 merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __restrict__ partial_lse,
-             const int32_t* __restrict__ status, __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out) {
-  pdl_wait();                                    // (and no trigger: see launch_chained)
+             const int32_t* __restrict__ status, __nv_bfloat16* __restrict__ out, float* __restrict__ lse_out, int trigger) {
+  pdl_wait();
+  if (trigger) pdl_trigger();                    // see launch_chained
   constexpr int kGroup = kMergeGroup<D>, kGroups = kW / kGroup;
   constexpr int kPieces = D / 8;                 // lanes of a group that hold data (head dim 96: 12 of 16)
   constexpr int kRowsPerBlock = kMergeThreads / kW;
@@ -287,14 +288,14 @@ merge_kernel(Params p, const __half* __restrict__ partial_out, const float2* __r
 
 template <bool kHalf, int D>
 static cudaError_t launch_merge_dim(const Params& p, const __half* partial_out, const float2* partial_lse,
-                                    const int32_t* status, __nv_bfloat16* out, float* lse_out, cudaStream_t st) {
+                                    const int32_t* status, __nv_bfloat16* out, float* lse_out, cudaStream_t st, bool trigger) {
   auto launch = [&](auto* kernel, int lanes) {
     const int rows_per_block = kMergeThreads / lanes;
     int64_t blocks = (p.rows + rows_per_block - 1) / rows_per_block;
     if (blocks > 148 * 64) blocks = 148 * 64;
     const bool chained = p.rows * p.NP * D * (int64_t)sizeof(__half) <= kChainedMergeBytes;
     return launch_chained(chained, kernel, dim3((unsigned)blocks), kMergeThreads, 0, st, p, partial_out, partial_lse, status,
-                          out, lse_out);
+                          out, lse_out, (int)trigger);
   };
   constexpr int kGroup = kMergeGroup<D>, kSums = 32 / kGroup;
   const bool many = p.topk > kMergeNarrow;                   // (few partials of a top-k whose rows are on a warp elsewhere)
@@ -318,10 +319,10 @@ static cudaError_t launch_merge_dim(const Params& p, const __half* partial_out, 
 }
 
 cudaError_t launch_merge(const Params& p, const __half* partial_out, const float2* partial_lse,
-                         const int32_t* status, __nv_bfloat16* out, float* lse_out, cudaStream_t st) {
+                         const int32_t* status, __nv_bfloat16* out, float* lse_out, cudaStream_t st, bool trigger) {
 #define MOBA_MERGE(DIM)                                                                                          \
-  return p.fp16 ? launch_merge_dim<true, DIM>(p, partial_out, partial_lse, status, out, lse_out, st)             \
-                : launch_merge_dim<false, DIM>(p, partial_out, partial_lse, status, out, lse_out, st)
+  return p.fp16 ? launch_merge_dim<true, DIM>(p, partial_out, partial_lse, status, out, lse_out, st, trigger)    \
+                : launch_merge_dim<false, DIM>(p, partial_out, partial_lse, status, out, lse_out, st, trigger)
   switch (p.D) {
     case 64: MOBA_MERGE(64);
     case 96: MOBA_MERGE(96);
