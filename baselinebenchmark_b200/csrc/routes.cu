@@ -310,7 +310,10 @@ static cudaError_t launch_merge_dim(const Params& p, const __half* partial_out, 
   } else if constexpr (D < 256) {
     // two sums leave four CTAs: ahead of a warp per row up to 8 partials (3: 40 against 63 us, 8: 72 against 70, 16: 117 / 105)
     if (many && p.NP <= kMergeNarrow / 2) return launch(merge_kernel<kHalf, D, kGroup, 1, 4, 4, kSums>, kGroup);
-    if (!many) return launch(merge_kernel<kHalf, D, kGroup, 1, 4, 5>, kGroup);
+    // (eight in flight for one wave of rows: 16 partials, 256 rows 3.6 against 4.3 us; 8, 11200 rows 6.1 against 5.5)
+    if (!many)
+      return p.rows <= 148 * 3 * (kMergeThreads / kGroup) ? launch(merge_kernel<kHalf, D, kGroup, 1, 8, 3>, kGroup)
+                                                         : launch(merge_kernel<kHalf, D, kGroup, 1, 4, 5>, kGroup);
   } else {
     // one LSE a lane leaves registers for a fifth CTA (131072 rows, 32 partials: 335 -> 323 us)
     if (p.NP <= 32) return launch(merge_kernel<kHalf, D, 32, 1, 4, 5>, 32);
