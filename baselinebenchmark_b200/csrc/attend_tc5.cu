@@ -1027,19 +1027,21 @@ attend_tc5_wide_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_
 //              chunk of the item before it (the row tiles of one list are consecutive) finds K and V in
 //              place when the chunk is one tile
 //   warp 5     issues QK(0) PV(0) QK(1) PV(1) ...: QK of the next tile, of the next item
-//              too, directly behind the PV that consumed P, so that S is ready when the softmax
-//              warps return from the epilogue
-//   warps 0-3  softmax, and the epilogue: one thread per row, O from tensor memory through
-//              registers to 32-byte stores (whole sectors, no staging in shared memory)
+//              too, directly behind the PV that consumed P
+//   warps 0-3, 8-11  softmax, and the epilogue: one thread per row, O from tensor memory through
+//              registers to 32-byte stores (whole sectors, no staging in shared memory).  The two
+//              warpgroups take the items in turn: one computes the softmax of an item while the other
+//              writes the rows of the item before it (o_free: O may be overwritten)
 // Per CTA: one Q, one K and one V tile (32 KB each), 256 TMEM columns (S 0-127, O 128-255); two CTAs per SM
 // overlap each other's softmax, MMA and stores.
-// Bound by the softmax warps: softmax and epilogue of an item take most of its time (see softmax_row_rolled).
+// With one warpgroup for both, softmax and epilogue of an item took most of its time, one after the other (see
+// softmax_row_rolled); with two: length-4096 below 142 -> 134 us, 13311 x 16/4 at head_dim 64 162 -> 145.
 // Measured against the kernel with CTA-wide barriers between items and unrolled code: dense stage of
 // 2 x 4096 tokens x 16 heads, chunk 128 199 -> 146 us (whole call 347 -> 279); 13311 tokens x 16/4 heads,
 // head_dim 64 233 -> 172; 32768 x 32/8 1651 -> 1094.  A decode step (chunk 4096, 131072-token prefix, 32/8 heads), in
 // place of the 256-row kernel: 132 -> 90.  The rolled loops alone: 205 -> 146 on the first.
 // ---------------------------------------------------------------------------
-constexpr int kShortThreads = 256;
+constexpr int kShortThreads = 384;
 
 struct ShortCtrl {
   static constexpr int kPrefix = kShortPrefix;
@@ -1047,7 +1049,8 @@ struct ShortCtrl {
   uint64_t q_free;                         // per item: its last Q.K^T has executed
   uint64_t k_free;                         // per other key tile of an item: its Q.K^T has executed
   uint64_t v_free;                         // per key tile that a new V tile follows: its P.V has executed
-  uint64_t s_full, p_full, o_full;
+  uint64_t s_full[2], p_full[2], o_full[2];  // [softmax warpgroup]
+  uint64_t o_free;                         // per item: its rows of O have been read
   uint64_t item_full[kShortSlots], slot_free[kShortSlots];
   uint32_t tmem_slot;
   volatile int32_t abort;
@@ -1089,12 +1092,15 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
     mbar_init(smem_u32(&c.q_free), 1);
     mbar_init(smem_u32(&c.k_free), 1);
     mbar_init(smem_u32(&c.v_free), 1);
-    mbar_init(smem_u32(&c.s_full), 1);
-    mbar_init(smem_u32(&c.p_full), kTileM);
-    mbar_init(smem_u32(&c.o_full), 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&c.s_full[i]), 1);
+      mbar_init(smem_u32(&c.p_full[i]), kTileM);
+      mbar_init(smem_u32(&c.o_full[i]), 1);
+    }
+    mbar_init(smem_u32(&c.o_free), kTileM);
     for (int i = 0; i < kShortSlots; ++i) {
       mbar_init(smem_u32(&c.item_full[i]), 1);
-      mbar_init(smem_u32(&c.slot_free[i]), 4);                 // the softmax warps
+      mbar_init(smem_u32(&c.slot_free[i]), 4);                 // the softmax warps of the item
     }
     c.abort = 0;
     fence_barrier_init();
@@ -1124,10 +1130,10 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
     return ok;
   };
   if (warp == 4) {
-    if (p.C <= kBN) ok = describe_items<kShortSlots, 1, true, false>(p, sa.iq, c);
-    else ok = describe_items<kShortSlots, 1, false, false>(p, sa.iq, c);
+    if (p.C <= kBN) ok = describe_items<kShortSlots, 2, true, false>(p, sa.iq, c);
+    else ok = describe_items<kShortSlots, 2, false, false>(p, sa.iq, c);
     if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
-  } else if (warp >= 6) {
+  } else if (warp == 6 || warp == 7) {
     // ---- Q rows; K/V tiles
     uint32_t kt = 0, vt = 0;               // k_free phases waited for, V tiles requested
     for (int n = 0; ok; ++n) {
@@ -1170,7 +1176,8 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
     const uint32_t dk = __shfl_sync(0xffffffffu, desc_lo(sK, 16), 0);
     const uint32_t dv = __shfl_sync(0xffffffffu, desc_lo(sV, kHalfBytes), 0);
     const uint32_t el = elect_one();
-    uint32_t kt = 0, vt = 0, g = 0;        // K / V tiles consumed, key tiles whose P.V has been issued
+    uint32_t kt = 0, vt = 0;               // K / V tiles consumed
+    uint32_t pph[2] = {0, 0};              // p_full phases
     // Q.K^T of tile j of item n; `fresh`: the K tile is a new one
     auto qk = [&](int n, int j, int ntiles, bool fresh) {
       if (j == 0) {
@@ -1184,7 +1191,7 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
       tc_fence_after();
       if (el) {
         issue_qk<0, 0, kHalf, D>(tm, dq, dk);
-        tc_commit(smem_u32(&c.s_full));
+        tc_commit(smem_u32(&c.s_full[n & 1]));
         tc_commit(smem_u32(j + 1 == ntiles ? &c.q_free : &c.k_free));
       }
       __syncwarp();
@@ -1197,18 +1204,21 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
       while (ok) {
         int next_tiles = 0;
         bool next_fresh = false, more = true;
-        for (int j = 0; ok && j < ntiles; ++j, ++g) {
+        for (int j = 0; ok && j < ntiles; ++j) {
           if (fresh) {
             if (!wait(&c.v_full, vt & 1)) break;
             ++vt;
           }
-          if (!wait(&c.p_full, g & 1)) break;
+          const int x = n & 1;
+          if (!wait(&c.p_full[x], x ? pph[1] : pph[0])) break;
+          if (x) pph[1] ^= 1; else pph[0] ^= 1;
+          if (j == 0 && n > 0 && !wait(&c.o_free, (n - 1) & 1)) break;
           tc_fence_after();
           if (el) {
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks)
               mma_ts_lo<kDescHi>(tm + 128, tm + ks * 8, dv + ks * (2048 >> 4), kIdescPV<kHalf, D>, j > 0 || ks > 0);
-            tc_commit(smem_u32(j + 1 == ntiles ? &c.o_full : &c.v_free));
+            tc_commit(smem_u32(j + 1 == ntiles ? &c.o_full[x] : &c.v_free));
           }
           __syncwarp();
           if (j + 1 < ntiles) {
@@ -1234,27 +1244,29 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
     }
     if (!ok && lane == 0) { atomicExch(a.status, ST_MMA); c.abort = 1; }
   } else {
-    // ---- softmax + epilogue, one thread per row
-    const int row = warp * 32 + lane;
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+    // ---- softmax + epilogue, one thread per row; warpgroup x takes items x, x + 2, ...
+    const int x = warp >> 3;
+    const int row0 = (warp & 3) * 32, row = row0 + lane;
+    const uint32_t lane_base = (uint32_t)row0 << 16;
     const uint32_t tS = tmem + lane_base;
     const uint32_t tO = tmem + lane_base + 128;
     const float sl2 = rsqrtf((float)D) * 1.4426950408889634f;
-    uint32_t g = 0;
-    for (int n = 0; ok; ++n) {
+    uint32_t sph = 0;                      // phase of s_full[x]
+    for (int n = x; ok; n += 2) {
       const int slot = n % kShortSlots;
       if (!wait(&c.item_full[slot], (n / kShortSlots) & 1)) break;
       if (c.item[slot].done) break;
       const int kv_len = c.item[slot].kv_len, tok_rel = c.item[slot].tok_rel, group = c.item[slot].group;
       const bool causal = c.item[slot].causal != 0;
-      const bool active = warp * 32 < c.item[slot].nrows;     // warps without rows only keep the barriers going
+      const bool active = row0 < c.item[slot].nrows;     // warps without rows only keep the barriers going
       const int32_t e = c.entry[slot][row];
       const int ntiles = (kv_len + kBN - 1) / kBN;
       const int qrel = tok_rel + (group == 1 ? row : row / group);              // own chunk: position in the chunk
       const int lim = causal ? min(kv_len, qrel + 1) : kv_len;                  // keys < lim are visible
       float m_ref = -INFINITY, l = 0.f;
-      for (int j = 0; j < ntiles; ++j, ++g) {
-        if (!wait(&c.s_full, g & 1)) break;
+      for (int j = 0; j < ntiles; ++j) {
+        if (!wait(&c.s_full[x], sph)) break;
+        sph ^= 1;
         // the item's Q.K^T has run: every role has read its description
         if (j == 0 && lane == 0) mbar_arrive(smem_u32(&c.slot_free[slot]));
         if (active) {
@@ -1266,9 +1278,9 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
           else softmax_row_rolled<false, kHalf, D>(tS, tO, j, key0, lim, sl2, m_ref, l, [] {});
           tc_fence_before();
         }
-        mbar_arrive(smem_u32(&c.p_full));
+        mbar_arrive(smem_u32(&c.p_full[x]));
       }
-      if (!ok || !wait(&c.o_full, n & 1)) break;
+      if (!ok || !wait(&c.o_full[x], (n >> 1) & 1)) break;
       if (active) {
         tc_fence_after();
         // the row's largest magnitude decides the power of two its fp16 copy is scaled by
@@ -1276,8 +1288,13 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
         const float inv = 1.f / l;
         const PartialScale ps = partial_scale(amax * inv);
         store_row_rolled<D>(tO, a.partial_out + (int64_t)(e >= 0 ? e : 0) * D, inv * ps.scale, e >= 0, a.wide_store != 0,
-                            [] { tc_fence_before(); });
+                            [&] {
+                              tc_fence_before();
+                              mbar_arrive(smem_u32(&c.o_free));   // O may be overwritten
+                            });
         if (e >= 0) a.partial_lse[e] = make_float2((m_ref + log2f(l)) * 0.6931471805599453f, ps.inv);
+      } else {
+        mbar_arrive(smem_u32(&c.o_free));
       }
     }
     if (!ok) {
