@@ -192,10 +192,23 @@ __device__ __forceinline__ void copy_rows_async(uint32_t tile, const __nv_bfloat
   const int ch = lane % kPieces, r0 = lane / kPieces;
   const uint32_t dst = tile + (uint32_t)((ch >> 3) * (128 * 128));
   const __nv_bfloat16* src = base + (piece0 + ch) * 8;
+  constexpr int kStride = kWarps * kRowsPerInstr, kBatch = 8;
   if (r0 < kRowsPerInstr) {                                    // 12 pieces (head dim 96): 24 of the 32 lanes copy
-#pragma unroll 8
-    for (int r = r0 + part * kRowsPerInstr; r < nrows; r += kWarps * kRowsPerInstr)
-      ptx::cp_async_16(dst + (uint32_t)(r * 128 + (((ch & 7) ^ (r & 7)) << 4)), src + off(r));
+    // The offsets of a batch are read before its first copy: a copy is a barrier to the compiler, and with a shared-memory
+    // read in front of every one of them it took 130 cycles a copy, the longest link of the chain of a one-tile item.
+    // 2 x 4096 tokens x 16 heads, chunk 128: dense stage 133 -> 128 us, at head dim 256 314 -> 291; dq of 8191 tokens x
+    // 16/4 heads 254 -> 238.
+#pragma unroll 1
+    for (int r = r0 + part * kRowsPerInstr; r < nrows; r += kBatch * kStride) {
+      int64_t o[kBatch];
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) o[u] = r + u * kStride < nrows ? off(r + u * kStride) : 0;
+#pragma unroll
+      for (int u = 0; u < kBatch; ++u) {
+        const int x = r + u * kStride;
+        if (x < nrows) ptx::cp_async_16(dst + (uint32_t)(x * 128 + (((ch & 7) ^ (x & 7)) << 4)), src + o[u]);
+      }
+    }
   }
 }
 
