@@ -274,11 +274,12 @@ __device__ __forceinline__ float global_ssq(const __nv_bfloat16* row) {
   return ssq;
 }
 
-// Score of row `r` (Q tile in shared memory) against the mean at `mrow` (global), in the contract order.
-// (not inlined: it is called from the two rarely taken recheck paths, and one copy keeps the
+// Score of the row at `qrow` against the mean at `mrow` (global memory), in the contract order: one
+// candidate per lane.
+// (not inlined: it is called from rarely taken recheck paths, and one copy keeps the
 // kernel's hot loop small in the instruction cache)
 template <bool kHalf, int D>
-__device__ __noinline__ float contract_score(const unsigned char* sQ, int r, const __nv_bfloat16* mrow) {
+__device__ __noinline__ float contract_score(const __nv_bfloat16* qrow, const __nv_bfloat16* mrow) {
   constexpr int kNB = D / 8;
   constexpr int kNBPad = kNB <= 8 ? 8 : (kNB <= 16 ? 16 : 32);
   uint4 mraw[kNB];
@@ -289,7 +290,7 @@ __device__ __noinline__ float contract_score(const unsigned char* sQ, int r, con
   for (int l = 0; l < kNBPad; ++l) {
     if (l < kNB) {
       float qf[8], mf[8];
-      unpack8<kHalf>(*reinterpret_cast<const uint4*>(sQ + swz_piece(r, l, kQBlockBytes)), qf);
+      unpack8<kHalf>(__ldg(reinterpret_cast<const uint4*>(qrow + l * 8)), qf);
       unpack8<kHalf>(mraw[l], mf);
       b[l] = dot8(qf, mf);
     } else {
@@ -301,6 +302,25 @@ __device__ __noinline__ float contract_score(const unsigned char* sQ, int r, con
 #pragma unroll
     for (int l = 0; l < h; ++l) b[l] = __fadd_rn(b[l], b[l + h]);
   return b[0];
+}
+
+// The same score, a block of 8 dims per lane: the groups of kNBPad lanes of a warp each score a candidate, and
+// the first lane of a group has the result.  For the few candidates of a run of near-ties: one load of the mean
+// and eight multiply-adds in a row in place of sixteen and 128 (6200 cycles a row).
+template <int D> constexpr int kScoreLanes = D <= 64 ? 8 : D <= 128 ? 16 : 32;
+template <bool kHalf, int D>
+__device__ __forceinline__ float contract_score_group(const __nv_bfloat16* qrow, const __nv_bfloat16* mrow) {
+  const int l = threadIdx.x & (kScoreLanes<D> - 1);
+  float b = 0.f;
+  if (l < D / 8) {
+    float qf[8], mf[8];
+    unpack8<kHalf>(__ldg(reinterpret_cast<const uint4*>(qrow + l * 8)), qf);
+    unpack8<kHalf>(__ldg(reinterpret_cast<const uint4*>(mrow + l * 8)), mf);
+    b = dot8(qf, mf);
+  }
+#pragma unroll
+  for (int h = kScoreLanes<D> / 2; h >= 1; h >>= 1) b = __fadd_rn(b, __shfl_down_sync(0xffffffffu, b, h));
+  return b;
 }
 
 // Min-heap of {chunk, key} on the key: `heap[0]` is the smallest key kept.  Replaces the
@@ -355,6 +375,415 @@ __device__ __forceinline__ GateTile gate_tile(const Params& p, const int32_t* __
   return t;
 }
 
+// eps of a row is this times |q|_2 max|m|_2 (see the head of this section); kKeys: the estimates went through the keys
+// with the position in their low bits
+template <int D, bool kKeys> constexpr float gate_kappa =
+    ((18.f * (D / 16) + 16.f) / 8388608.f + (kKeys ? 1.f / 262144.f : 0.f)) * 1.001f;
+
+// ---- rows that the estimates alone do not settle ------------------------------------------------------------
+struct GateLists {
+  uint2* lists;                            // [128][lstride] {chunk, key}, largest key first
+  int lstride, list_len;
+  unsigned long long* exact;               // [64] keys, of this warp
+};
+// The warp ranks the rows of its lanes with mode != 0: 1 all n_surv entries of the list, 2 all ncand candidates, 3 the runs of
+// near-ties marked in the list.  The calling lane's row is `row` of the tile, at `qrow` in global memory; eps: its error bound.
+template <bool kHalf, int D>
+__device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, const GateTile& t, const __nv_bfloat16* qrow,
+                                          int row, int mode, int n_surv, int n_keep, int ncand, float eps,
+                                          const __nv_bfloat16* __restrict__ means, int32_t* __restrict__ stats) {
+  const int lane = threadIdx.x & 31;
+  const int hist = p.hist, lstride = g.lstride;
+  const int slot0 = t.b * p.mc;
+  uint2* lists = g.lists;
+  unsigned need = __ballot_sync(0xffffffffu, mode != 0);
+  unsigned long long* lx = g.exact;
+  while (need) {
+    const int src = __ffs(need) - 1;
+    need &= need - 1;
+    const int r = (row & ~31) + src;
+    const int r_mode = __shfl_sync(0xffffffffu, mode, src);
+    const int r_total = r_mode == 2 ? __shfl_sync(0xffffffffu, ncand, src) : __shfl_sync(0xffffffffu, n_surv, src);
+    const int r_keep = __shfl_sync(0xffffffffu, n_keep, src);
+    const float r_eps = __shfl_sync(0xffffffffu, eps, src);
+    const __nv_bfloat16* r_q =
+        reinterpret_cast<const __nv_bfloat16*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(qrow), src));
+    uint2* rlist = lists + (size_t)r * lstride;
+    if (r_mode == 3) {
+      // runs of near-ties: one marked entry per lane (at most 32), exact keys, rank inside the run
+      int cnt = 0, runs = 0, my_e = -1, my_run = 0;
+      for (int e0 = 0; e0 < r_total; e0 += 32) {
+        const int e = e0 + lane;
+        const uint32_t x = e < r_total ? rlist[e].x : 0u;
+        const unsigned bt = __ballot_sync(0xffffffffu, (x & kTied) != 0 && x != 0xFFFFFFFFu);
+        const unsigned bs = __ballot_sync(0xffffffffu, (x & kRunStart) != 0 && x != 0xFFFFFFFFu);
+        if ((bt >> lane) & 1) {
+          const int slot = cnt + __popc(bt & ((1u << lane) - 1));
+          const int run = runs + __popc(bs & ((2u << lane) - 1));
+          lx[slot] = (unsigned long long)e | ((unsigned long long)run << 8);
+        }
+        cnt += __popc(bt);
+        runs += __popc(bs);
+      }
+      __syncwarp();
+      unsigned long long key = 0ull;
+      uint2 ent = make_uint2(0u, 0u);
+      uint32_t cc = 0;
+      if (lane < cnt) {
+        my_e = (int)(lx[lane] & 0xFF);
+        my_run = (int)(lx[lane] >> 8);
+        ent = rlist[my_e];
+        cc = ent.x & kChunkMask;
+      }
+      // as many entries at a time as the warp has groups of lanes; entry i's score goes to lane i
+      float e = 0.f;
+      constexpr int kPer = 32 / kScoreLanes<D>;
+      for (int i0 = 0; i0 < cnt; i0 += kPer) {
+        const int mine = i0 + lane / kScoreLanes<D>;
+        const uint32_t ec = __shfl_sync(0xffffffffu, cc, mine & 31);     // (past the last entry: a chunk scored in vain)
+        const float score = contract_score_group<kHalf, D>(r_q, means + ((int64_t)(slot0 + (int)ec) * p.Hkv + t.hk) * D);
+        const float got = __shfl_sync(0xffffffffu, score, ((lane - i0) * kScoreLanes<D>) & 31);
+        if (lane >= i0 && lane < i0 + kPer) e = got;
+      }
+      if (lane < cnt) {
+        key = ((unsigned long long)float_key(e) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(slot0 + (int)cc));
+        if (stats != nullptr) {
+          const float diff = fabsf(key_float(ent.y) - e);
+          if (!(diff <= r_eps)) atomicAdd(&stats[2], 1);
+          atomicMax(&stats[1], (int)fminf(diff / r_eps * 65536.f, 1.0e9f));
+        }
+      }
+      int rank = 0, first = my_e;
+      for (int t2 = 0; t2 < cnt; ++t2) {
+        const unsigned long long kt = __shfl_sync(0xffffffffu, key, t2);
+        const int rt = __shfl_sync(0xffffffffu, my_run, t2), et = __shfl_sync(0xffffffffu, my_e, t2);
+        if (lane < cnt && rt == my_run) {
+          rank += kt > key;
+          first = min(first, et);
+        }
+      }
+      __syncwarp();
+      if (lane < cnt) rlist[first + rank].x = cc;          // a run occupies consecutive places; marks are cleared
+      __syncwarp();
+      if (stats != nullptr && lane == 0) atomicAdd(&stats[0], 1);
+      continue;
+    }
+    lx[lane] = 0ull;
+    lx[lane + 32] = 0ull;
+    __syncwarp();
+    int viol = 0, ratio = 0;
+    for (int base = 0; base < r_total; base += 32) {
+      const int idx = base + lane;
+      unsigned long long key = 0ull;
+      if (idx < r_total) {
+        const int cc = r_mode == 2 ? idx : (int)rlist[idx].x;
+        const float e = contract_score<kHalf, D>(r_q, means + ((int64_t)(slot0 + cc) * p.Hkv + t.hk) * D);
+        key = ((unsigned long long)float_key(e) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(slot0 + cc));
+        if (r_mode == 1 && stats != nullptr) {
+          const float diff = fabsf(key_float(rlist[idx].y) - e);
+          if (!(diff <= r_eps)) viol = 1;
+          ratio = (int)fminf(diff / r_eps * 65536.f, 1.0e9f);
+        }
+      }
+      // the keys of this batch, in lane order, into the ordered list lx[0, r_keep)
+      unsigned hits = __ballot_sync(0xffffffffu, key > lx[r_keep - 1]);
+      while (hits) {
+        const int l = __ffs(hits) - 1;
+        hits &= hits - 1;
+        const unsigned long long kk = __shfl_sync(0xffffffffu, key, l);
+        const unsigned long long k0 = lane < r_keep ? lx[lane] : 0ull;
+        const unsigned long long k1 = lane + 32 < r_keep ? lx[lane + 32] : 0ull;
+        const int pos = __popc(__ballot_sync(0xffffffffu, k0 > kk)) + __popc(__ballot_sync(0xffffffffu, k1 > kk));
+        if (pos < r_keep) {                                  // uniform; false when the list filled up meanwhile
+          if (lane >= pos && lane + 1 < r_keep) lx[lane + 1] = k0;
+          if (lane + 32 >= pos && lane + 33 < r_keep) lx[lane + 33] = k1;
+          if (lane == 0) lx[pos] = kk;
+        }
+        __syncwarp();
+      }
+    }
+    // the exact ranking replaces the chunk ids of the row's list
+    for (int i = lane; i < hist; i += 32) {
+      const unsigned long long key = i < r_keep ? lx[i] : 0ull;
+      rlist[i].x = key ? (0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFull)) - (uint32_t)slot0 : 0xFFFFFFFFu;
+    }
+    __syncwarp();
+    if (stats != nullptr) {
+      viol = __any_sync(0xffffffffu, viol);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ratio = max(ratio, __shfl_xor_sync(0xffffffffu, ratio, o));
+      if (lane == 0) {
+        atomicAdd(&stats[r_mode == 2 ? 3 : 0], 1);
+        if (r_mode == 1) atomicMax(&stats[1], ratio);
+        if (viol) atomicAdd(&stats[2], 1);
+      }
+    }
+  }
+}
+
+// The CTA that finishes last turns the counts of all into the offsets of the lists.  Executed by the whole CTA.
+template <int kThreads>
+__device__ __forceinline__ void finish_scan(const ListScan& scan, int32_t* __restrict__ ticket, int* scratch) {
+  __threadfence();
+  __syncthreads();                                            // (`scratch` is free from here on)
+  if (threadIdx.x == 0) scratch[0] = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+  __syncthreads();
+  const bool last = scratch[0] != 0;
+  __syncthreads();
+  if (last) {
+    __threadfence();
+    scan_lists<kThreads, 8>(scan, scratch);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// rows with at most 32 candidates
+//
+// One tile of means, one network a row, so what counts is the latency of a tile of rows: 25 000 cycles of it were
+// spent waiting for Q, on norms, on walks through lists in shared memory and at a barrier behind the warp with
+// the most near-ties, 2400 in the network.  Here
+//   warp 4     walks the row tiles of the CTA: requests Q and means as soon as the tensor core and the norms of the
+//              tile before have read theirs, and issues the MMA into the other half of 64 tensor memory columns
+//   warps 0-3  a thread per row.  The sorted keys stay in registers, and what they settle is decided there; a row with
+//              near-ties goes through a list in shared memory.  Every warp counts for itself: no barrier of
+//              the CTA in the loop, a warp may be a tile behind another.
+// Measured against the kernel below for these shapes, gating behind its chunk means: 2 x 4096 tokens x 16 heads, 31 candidates
+// 34 -> 30 us, at head dim 256 83 -> 69; 32768 x 32/8, 7 candidates 159 -> 131; a decode token on 32 chunks 10 -> 4.
+// (The few-lane score of near-ties alone, which the kernel below has too: 32768 x 32/8, 255 candidates 620 -> 573.)
+// ---------------------------------------------------------------------------
+constexpr int kOneThreads = 160;
+constexpr int kOneMeans = 32;              // rows of the tile of means
+constexpr int kOneCols = 2 * kOneMeans;
+
+struct OneCtrl {
+  uint64_t full;                           // per row tile: Q and means landed
+  uint64_t read;                           // ... and have been read by everybody
+  uint64_t mma_done;
+  uint32_t tmem_slot;
+  GateTile tile[2];
+  int32_t mean_ssq[2][kGateRows / 32];     // largest squared norm of a mean, by the warps
+  int32_t cnt[kGateRows / 32][kOneMeans];  // rows of a warp's tile that selected a chunk
+  unsigned long long exact[kGateRows / 32][64];
+};
+
+template <bool kHalf, int D, int kW>
+__global__ void __launch_bounds__(kOneThreads, kGateMinCtas<kW>)
+gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_m,
+                int tokens_per_cta, int nt, int list_len, int, int, const __nv_bfloat16* __restrict__ q,
+                const __nv_bfloat16* __restrict__ means, const int32_t* __restrict__ cu, int32_t* __restrict__ selected,
+                int32_t* __restrict__ list_counts, int32_t* __restrict__ stats, int flags, const ListScan scan,
+                int32_t* __restrict__ ticket) {
+  extern __shared__ unsigned char gate_smem_raw[];
+  constexpr int kNBlk = (D + 63) / 64;
+  const int hist = p.hist;
+  const int lstride = list_len | 1;
+  unsigned char* sQ = reinterpret_cast<unsigned char*>(((uintptr_t)gate_smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* sB = sQ + (size_t)kNBlk * kQBlockBytes;                 // kNBlk blocks [32][64]
+  uint2* lists = reinterpret_cast<uint2*>(sB + (size_t)kNBlk * kOneMeans * 128);
+  OneCtrl& c = *reinterpret_cast<OneCtrl*>(lists + (size_t)kGateRows * lstride);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tiles_x = window_tiles(p, tokens_per_cta);
+  const int n_tiles = tiles_x * p.Hkv * p.B;
+  const int rows_box = tokens_per_cta * p.G;
+
+  if (tid == 0) {
+    mbar_init(smem_u32(&c.full), 1);
+    mbar_init(smem_u32(&c.read), kGateRows);
+    mbar_init(smem_u32(&c.mma_done), 1);
+    fence_barrier_init();
+    prefetch_tmap(&tmap_q);
+    prefetch_tmap(&tmap_m);
+  }
+  if (tid < kGateRows) reinterpret_cast<int32_t*>(c.cnt)[tid] = 0;
+  if (warp == 0) {
+    tmem_alloc(smem_u32(&c.tmem_slot), (uint32_t)kOneCols);
+    tmem_relinquish();
+  }
+  pdl_wait();
+  pdl_trigger();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = c.tmem_slot;
+
+  if (warp == 4) {
+    // row tile n of the CTA is tile blockIdx.x + n * gridDim.x of the grid, valid or not
+    uint32_t n = 0, m = 0;                             // row tiles, tiles with candidates
+    for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x, ++n) {
+      const GateTile t = gate_tile(p, cu, ti, tiles_x, tokens_per_cta);
+      const bool work = t.valid && t.max_cand > 0;
+      // Q, means and half of tensor memory are free once everybody has read the tile before: a thread that has
+      // is through with the one before that
+      bool ok = n == 0 || mbar_wait(smem_u32(&c.read), (n - 1) & 1);
+      if (lane == 0) {
+        c.tile[n & 1] = t;
+        const uint32_t bar = smem_u32(&c.full);
+        if (work) {
+          mbar_expect_tx(bar, (uint32_t)(kNBlk * (rows_box + kOneMeans) * 128));
+#pragma unroll
+          for (int blk = 0; blk < kNBlk; ++blk) {
+            tma_load_3d(smem_u32(sQ + (size_t)blk * kQBlockBytes), &tmap_q, bar, blk * 64, t.hk * p.G, t.tok_lo - p.win_lo);
+            tma_load_3d(smem_u32(sB + (size_t)blk * kOneMeans * 128), &tmap_m, bar, blk * 64, t.hk, t.b * p.mc);
+          }
+        } else {
+          mbar_arrive(bar);
+        }
+      }
+      __syncwarp();
+      ok = mbar_wait(smem_u32(&c.full), n & 1) && ok;
+      if (work && __all_sync(0xffffffffu, ok)) {
+        if (lane == 0) {
+          tc_fence_after();
+          const uint32_t idesc = idesc_16_f32(kHalf, 128, kOneMeans, 0, 0);
+          const uint32_t aQ = smem_u32(sQ), aB = smem_u32(sB);
+#pragma unroll
+          for (int ks = 0; ks < D / 16; ++ks)
+            mma_ss(tmem + (m & 1) * kOneMeans, gate_desc(aQ + (ks >> 2) * kQBlockBytes + (ks & 3) * 32),
+                   gate_desc(aB + (ks >> 2) * kOneMeans * 128 + (ks & 3) * 32), idesc, ks > 0);
+          tc_commit(smem_u32(&c.mma_done));
+        }
+        __syncwarp();
+      }
+      m += work;
+      if (!__all_sync(0xffffffffu, ok)) break;         // the rows' threads run into their own bounded waits
+    }
+  } else {
+    const int row = tid;
+    uint2* mylist = lists + (size_t)row * lstride;
+    uint32_t n = 0, m = 0;
+    for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x, ++n) {
+      bool failed = !mbar_wait(smem_u32(&c.full), n & 1);
+      failed = __any_sync(0xffffffffu, failed);
+      const GateTile t = failed ? gate_tile(p, cu, ti, tiles_x, tokens_per_cta) : c.tile[n & 1];
+      const int nrows = t.valid ? t.ntok * p.G : 0;
+      const int slot0 = t.b * p.mc;
+      const int tl = row / p.G, hl = row - tl * p.G;   // token and head of the row in the tile
+      int32_t* dst = selected + (int64_t)(t.hk * p.G + hl) * p.Tq + (t.tok_lo - p.win_lo) + tl;
+      if (!t.valid || t.max_cand <= 0) {               // nothing, or the first chunk of a sequence: nothing to select
+        mbar_arrive(smem_u32(&c.read));
+        if (row < nrows)
+          for (int r = 0; r < hist; ++r) dst[(int64_t)r * p.sel_rs] = -1;
+        continue;
+      }
+      const int ncand = row < nrows ? (t.tok_lo + tl - t.s0) / p.C : 0;     // chunks before the row's own chunk
+      // squared norms: of the row, and of the means (four lanes a mean, eight means a warp)
+      float q_ssq = 0.f;
+      if (!failed) {
+        q_ssq = row_ssq<kHalf, D>(sQ, row, kQBlockBytes);
+        const int mrow = tid >> 2;
+        float s = 0.f;
+#pragma unroll
+        for (int ch = 0; ch < D / 32; ++ch) {
+          float f[8];
+          unpack8<kHalf>(*reinterpret_cast<const uint4*>(sB + swz_piece(mrow, 4 * ch + (lane & 3), kOneMeans * 128)), f);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) s = __fmaf_rn(f[e], f[e], s);
+        }
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        // floats >= 0 order like their bit patterns; +inf and NaN have the largest patterns
+        int ssq = mrow < t.max_cand ? __float_as_int(s) & 0x7FFFFFFF : 0;
+#pragma unroll
+        for (int o = 16; o >= 4; o >>= 1) ssq = max(ssq, __shfl_xor_sync(0xffffffffu, ssq, o));
+        if (lane == 0) c.mean_ssq[m & 1][warp] = ssq;
+        if (!mbar_wait(smem_u32(&c.mma_done), m & 1)) failed = true;
+      } else if (lane == 0) {
+        c.mean_ssq[m & 1][warp] = 0x7F800000;          // no bound: the other warps' rows are ranked exactly too
+      }
+      tc_fence_after();
+      uint32_t v[32];
+      __syncwarp();
+      tmem_ld32(tmem + (m & 1) * kOneMeans + ((uint32_t)(warp * 32) << 16), v);
+      tmem_wait_ld();
+      tc_fence_before();
+      mbar_arrive(smem_u32(&c.read));                  // Q, means and the estimates have been read
+#pragma unroll
+      for (int i = 0; i < 32; ++i)                     // order-preserving keys, position in the low bits: earlier wins ties
+        v[i] = i < ncand ? (float_key(__uint_as_float(v[i])) & ~31u) | (uint32_t)(31 - i) : 0u;
+      topk::top_of_32<kW>(v);
+      // the norms of the other warps: complete once all threads have arrived on `read`
+      if (!failed && !mbar_wait(smem_u32(&c.read), n & 1)) failed = true;
+      int ssq_max = 0;
+#pragma unroll
+      for (int w = 0; w < kGateRows / 32; ++w) ssq_max = max(ssq_max, c.mean_ssq[m & 1][w]);
+      ++m;
+
+      // What the keys settle.  Bit i: entry i is a candidate (real), can be among the n_keep best (surv), is closer to
+      // entry i + 1 than twice the error (tie)
+      const float eps2 = 2.f * (gate_kappa<D, true> * sqrtf(q_ssq) * sqrtf(__int_as_float(ssq_max)) + 7.9e-31f);
+      const int n_keep = min(hist, ncand), n_real = min(ncand, list_len);
+      const bool all = (flags & GATE_FORCE_RECHECK) != 0;
+      int mode = 0, n_surv = 0;                        // as in recheck_mode
+      uint32_t tied = 0, first = 0;
+      if (ncand > 0) {
+        uint32_t close = 0;
+        bool holes = false;
+        float theta = 0.f;
+#pragma unroll
+        for (int i = 0; i < kW; ++i) {
+          if (i < n_real) holes |= v[i] == 0u;
+          if (i + 1 == n_keep) theta = key_float(v[i]) - eps2;
+          if (i + 1 < kW && i + 1 < n_real && (all || !(key_float(v[i]) - key_float(v[i + 1 < kW ? i + 1 : i]) > eps2)))
+            close |= 1u << i;
+        }
+#pragma unroll
+        for (int i = 0; i < kW; ++i) n_surv += i < n_real && key_float(v[i]) >= theta;
+        const bool amb = all || (close & ((1u << n_keep) - 1u)) != 0;       // n_keep < 32
+        if ((flags & GATE_FORCE_EXACT) || failed || holes) {
+          mode = 2;
+        } else if (amb) {
+          if ((n_surv == list_len && ncand > list_len) || !(eps2 < INFINITY) || n_surv < n_keep) {
+            mode = 2;                                  // the near-ties may go on below the list, or eps is not finite
+          } else {
+            const uint32_t runs = n_surv > 0 ? close & ((1u << (n_surv - 1)) - 1u) : 0u;
+            tied = runs | (runs << 1);
+            first = runs & ~(runs << 1);
+            if (all && tied == 0) tied = first = 1u;   // a single survivor, scored again on request
+            mode = tied != 0 ? 3 : 0;                  // (at most 32 entries)
+          }
+        }
+      }
+      const __nv_bfloat16* qrow = q + (int64_t)(t.tok_lo + tl - p.win_lo) * p.sq_t + (int64_t)(t.hk * p.G + hl) * p.sq_h;
+      if (__any_sync(0xffffffffu, mode != 0)) {
+#pragma unroll
+        for (int i = 0; i < kW; ++i)
+          if (i < list_len)
+            mylist[i] = make_uint2(v[i] ? (31u - (v[i] & 31u)) | ((tied >> i) & 1u ? kTied : 0u) | ((first >> i) & 1u ? kRunStart : 0u)
+                                        : 0xFFFFFFFFu, v[i]);
+        __syncwarp();
+        rank_rows<kHalf, D>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand,
+                            0.5f * eps2, means, stats);
+        __syncwarp();
+      }
+      if (row < nrows) {
+#pragma unroll
+        for (int r = 0; r < kW; ++r)
+          if (r < hist) {
+            const uint32_t x = mode != 0 ? mylist[r].x : v[r] ? 31u - (v[r] & 31u) : 0xFFFFFFFFu;
+            const int cc = x == 0xFFFFFFFFu ? -1 : (int)(x & kChunkMask);
+            dst[(int64_t)r * p.sel_rs] = cc >= 0 ? slot0 + cc : -1;
+            if (cc >= 0 && list_counts != nullptr) atomicAdd(&c.cnt[warp][cc], 1);
+          }
+      }
+      __syncwarp();
+      if (list_counts != nullptr) {
+        const int k = c.cnt[warp][lane];
+        if (k > 0) atomicAdd(&list_counts[(int64_t)(slot0 + lane) * p.Hkv + t.hk], k);
+        c.cnt[warp][lane] = 0;
+      }
+      __syncwarp();
+    }
+  }
+
+  __syncwarp();
+  if (ticket != nullptr) finish_scan<kOneThreads>(scan, ticket, reinterpret_cast<int*>(c.exact));
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, (uint32_t)kOneCols);
+}
+
+// rows with more than 32 candidates, or lists longer than 32
 // kW: width of the compare-exchange network (8, 16 or 32 >= list_len), 0: lists longer than 32 (min-heap)
 template <bool kHalf, int D, int kW>
 __global__ void __launch_bounds__(kGateThreads, kGateMinCtas<kW>)
@@ -373,9 +802,8 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
   unsigned char* sQ0 = smem;                                             // nbuf x kNBlk blocks [128][64]
   unsigned char* sB = sQ0 + (size_t)nbuf * kNBlk * kQBlockBytes;        // kNBlk blocks [nt][64]
   uint2* lists = reinterpret_cast<uint2*>(sB + (size_t)kNBlk * nt * 128);   // [128][lstride] {chunk, score bits}
-  float* scratch = reinterpret_cast<float*>(lists + (size_t)kGateRows * lstride);   // [128][36], absent when unused
-  const bool has_scratch = kW == 0 || p.mc - 1 > 32;   // one 32-candidate step per row needs no merge
-  GateCtrl& c = *reinterpret_cast<GateCtrl*>(scratch + (has_scratch ? kGateRows * kScratchStride : 0));
+  float* scratch = reinterpret_cast<float*>(lists + (size_t)kGateRows * lstride);   // [128][36]
+  GateCtrl& c = *reinterpret_cast<GateCtrl*>(scratch + kGateRows * kScratchStride);
   int32_t* cnt_s = reinterpret_cast<int32_t*>(&c + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -612,8 +1040,7 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
 
     // ---- recheck ------------------------------------------------------------------------------
     // eps of this row (see the head of this section); inf or NaN sends the row to the exact ranking
-    constexpr float kKappa = (18.f * (D / 16) + 16.f) / 8388608.f + (kW > 0 ? 1.f / 262144.f : 0.f);
-    const float eps = kKappa * 1.001f * sqrtf(q_ssq) * sqrtf(__int_as_float(c.mean_ssq_max)) + 7.9e-31f;
+    const float eps = gate_kappa<D, (kW > 0)> * sqrtf(q_ssq) * sqrtf(__int_as_float(c.mean_ssq_max)) + 7.9e-31f;
     const int n_keep = min(hist, ncand);
     // 0: list is exact; 3: order the runs of near-ties (marked in the list); 1: rank all survivors;
     // 2: rank all candidates
@@ -678,124 +1105,9 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
       }
     }
     __syncwarp();                                             // the marks are visible to the warp
-    unsigned need = __ballot_sync(0xffffffffu, mode != 0);
-    unsigned long long* lx = c.exact[warp];
-    while (need) {
-      const int src = __ffs(need) - 1;
-      need &= need - 1;
-      const int r = warp * 32 + src;
-      const int r_mode = __shfl_sync(0xffffffffu, mode, src);
-      const int r_total = r_mode == 2 ? __shfl_sync(0xffffffffu, ncand, src) : __shfl_sync(0xffffffffu, n_surv, src);
-      const int r_keep = __shfl_sync(0xffffffffu, n_keep, src);
-      const float r_eps = __shfl_sync(0xffffffffu, eps, src);
-      uint2* rlist = lists + (size_t)r * lstride;
-      if (r_mode == 3) {
-        // runs of near-ties: one marked entry per lane (at most 32), exact keys, rank inside the run
-        int cnt = 0, runs = 0, my_e = -1, my_run = 0;
-        for (int e0 = 0; e0 < r_total; e0 += 32) {
-          const int e = e0 + lane;
-          const uint32_t x = e < r_total ? rlist[e].x : 0u;
-          const unsigned bt = __ballot_sync(0xffffffffu, (x & kTied) != 0 && x != 0xFFFFFFFFu);
-          const unsigned bs = __ballot_sync(0xffffffffu, (x & kRunStart) != 0 && x != 0xFFFFFFFFu);
-          if ((bt >> lane) & 1) {
-            const int slot = cnt + __popc(bt & ((1u << lane) - 1));
-            const int run = runs + __popc(bs & ((2u << lane) - 1));
-            lx[slot] = (unsigned long long)e | ((unsigned long long)run << 8);
-          }
-          cnt += __popc(bt);
-          runs += __popc(bs);
-        }
-        __syncwarp();
-        unsigned long long key = 0ull;
-        uint32_t cc = 0;
-        if (lane < cnt) {
-          my_e = (int)(lx[lane] & 0xFF);
-          my_run = (int)(lx[lane] >> 8);
-          const uint2 ent = rlist[my_e];
-          cc = ent.x & kChunkMask;
-          const float e = contract_score<kHalf, D>(sQ, r, means + ((int64_t)(slot0 + (int)cc) * p.Hkv + t.hk) * D);
-          key = ((unsigned long long)float_key(e) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(slot0 + (int)cc));
-          if (stats != nullptr) {
-            const float diff = fabsf(key_float(ent.y) - e);
-            if (!(diff <= r_eps)) atomicAdd(&stats[2], 1);
-            atomicMax(&stats[1], (int)fminf(diff / r_eps * 65536.f, 1.0e9f));
-          }
-        }
-        int rank = 0, first = my_e;
-        for (int t2 = 0; t2 < cnt; ++t2) {
-          const unsigned long long kt = __shfl_sync(0xffffffffu, key, t2);
-          const int rt = __shfl_sync(0xffffffffu, my_run, t2), et = __shfl_sync(0xffffffffu, my_e, t2);
-          if (lane < cnt && rt == my_run) {
-            rank += kt > key;
-            first = min(first, et);
-          }
-        }
-        __syncwarp();
-        if (lane < cnt) rlist[first + rank].x = cc;          // a run occupies consecutive places; marks are cleared
-        __syncwarp();
-        if (stats != nullptr && lane == 0) atomicAdd(&stats[0], 1);
-        continue;
-      }
-      lx[lane] = 0ull;
-      lx[lane + 32] = 0ull;
-      if (__shfl_sync(0xffffffffu, (int)failed, src)) {
-        // the row's thread gave up waiting for the Q tile: fetch the row with plain loads into its place
-        if (lane < D / 8) {
-          const int tl = r / p.G, hl = r - tl * p.G;
-          const uint4 val = __ldg(reinterpret_cast<const uint4*>(
-              q + (int64_t)(t.tok_lo + tl - p.win_lo) * p.sq_t + (int64_t)(t.hk * p.G + hl) * p.sq_h + lane * 8));
-          *reinterpret_cast<uint4*>(sQ + swz_piece(r, lane, kQBlockBytes)) = val;
-        }
-      }
-      __syncwarp();
-      int viol = 0, ratio = 0;
-      for (int base = 0; base < r_total; base += 32) {
-        const int idx = base + lane;
-        unsigned long long key = 0ull;
-        if (idx < r_total) {
-          const int cc = r_mode == 2 ? idx : (int)rlist[idx].x;
-          const float e = contract_score<kHalf, D>(sQ, r, means + ((int64_t)(slot0 + cc) * p.Hkv + t.hk) * D);
-          key = ((unsigned long long)float_key(e) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(slot0 + cc));
-          if (r_mode == 1 && stats != nullptr) {
-            const float diff = fabsf(key_float(rlist[idx].y) - e);
-            if (!(diff <= r_eps)) viol = 1;
-            ratio = (int)fminf(diff / r_eps * 65536.f, 1.0e9f);
-          }
-        }
-        // the keys of this batch, in lane order, into the ordered list lx[0, r_keep)
-        unsigned hits = __ballot_sync(0xffffffffu, key > lx[r_keep - 1]);
-        while (hits) {
-          const int l = __ffs(hits) - 1;
-          hits &= hits - 1;
-          const unsigned long long kk = __shfl_sync(0xffffffffu, key, l);
-          const unsigned long long k0 = lane < r_keep ? lx[lane] : 0ull;
-          const unsigned long long k1 = lane + 32 < r_keep ? lx[lane + 32] : 0ull;
-          const int pos = __popc(__ballot_sync(0xffffffffu, k0 > kk)) + __popc(__ballot_sync(0xffffffffu, k1 > kk));
-          if (pos < r_keep) {                                  // uniform; false when the list filled up meanwhile
-            if (lane >= pos && lane + 1 < r_keep) lx[lane + 1] = k0;
-            if (lane + 32 >= pos && lane + 33 < r_keep) lx[lane + 33] = k1;
-            if (lane == 0) lx[pos] = kk;
-          }
-          __syncwarp();
-        }
-      }
-      // the exact ranking replaces the chunk ids of the row's list
-      for (int i = lane; i < hist; i += 32) {
-        const unsigned long long key = i < r_keep ? lx[i] : 0ull;
-        rlist[i].x = key ? (0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFull)) - (uint32_t)slot0 : 0xFFFFFFFFu;
-      }
-      __syncwarp();
-      if (stats != nullptr) {
-        viol = __any_sync(0xffffffffu, viol);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ratio = max(ratio, __shfl_xor_sync(0xffffffffu, ratio, o));
-        if (lane == 0) {
-          atomicAdd(&stats[r_mode == 2 ? 3 : 0], 1);
-          if (r_mode == 1) atomicMax(&stats[1], ratio);
-          if (viol) atomicAdd(&stats[2], 1);
-        }
-      }
-    }
+    const __nv_bfloat16* qrow = q + (int64_t)(t.tok_lo + row / p.G - p.win_lo) * p.sq_t + (int64_t)(t.hk * p.G + row % p.G) * p.sq_h;
+    rank_rows<kHalf, D>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand, eps, means,
+                        stats);
     // selected[rank][head][token]: every thread stores the chunks of its own row (its list was
     // written by its own warp); neighbouring lanes are neighbouring heads, then tokens
     if (row < nrows) {
@@ -823,20 +1135,7 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
     ++n;
   }
 
-  // the CTA that finishes last turns the counts of all into the offsets of the lists
-  if (ticket != nullptr) {
-    int* scratch = reinterpret_cast<int*>(c.exact);           // no row is being ranked any more
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) scratch[0] = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
-    __syncthreads();
-    const bool last = scratch[0] != 0;
-    __syncthreads();
-    if (last) {
-      __threadfence();
-      scan_lists<kGateThreads, 8>(scan, scratch);
-    }
-  }
+  if (ticket != nullptr) finish_scan<kGateThreads>(scan, ticket, reinterpret_cast<int*>(c.exact));
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, (uint32_t)nt);
@@ -850,6 +1149,8 @@ struct GateLaunch {
 // Candidate tile, Q buffers, list length and shared memory of a launch: the combination that puts
 // the most CTAs on an SM (more warps hide the latency of the heap updates), then two Q buffers,
 // then the wider candidate tile.  smem == 0: nothing fits.
+// At most 32 candidates a row, and a network for the list.
+inline bool gate_one(const Params& p) { return p.mc - 1 <= kOneMeans && p.hist + 1 <= 32; }
 GateLaunch gate_launch_config(const Params& p) {
   GateLaunch best{};
   const int nblk = (p.D + 63) / 64;
@@ -857,14 +1158,17 @@ GateLaunch gate_launch_config(const Params& p) {
   // fewer is ranked over all of them in one round of the exact path anyway)
   const int list_len = p.hist + 1 + (p.mc - 1 > 32 ? kListExtra : 0);
   const int cnt_in_smem = p.mc <= kCntSmemMax;
+  if (gate_one(p))
+    return GateLaunch{kOneMeans, list_len, 1, 0, 4,
+                      1024 + (size_t)nblk * kQBlockBytes + (size_t)nblk * kOneMeans * 128 +
+                          (size_t)kGateRows * (list_len | 1) * sizeof(uint2) + sizeof(OneCtrl)};
   int want = 32;
   while (want < p.mc - 1 && want < 256) want *= 2;            // a row has at most mc - 1 candidates
   for (int nbuf = 2; nbuf >= 1; --nbuf)
     for (int nt = want; nt >= 32; nt /= 2) {
-      const bool has_scratch = list_len > 32 || p.mc - 1 > 32;
       const size_t smem = 1024 + (size_t)nbuf * nblk * kQBlockBytes + (size_t)nblk * nt * 128 +
                           (size_t)kGateRows * (list_len | 1) * sizeof(uint2) +
-                          (has_scratch ? (size_t)kGateRows * kScratchStride * sizeof(float) : 0) + sizeof(GateCtrl) +
+                          (size_t)kGateRows * kScratchStride * sizeof(float) + sizeof(GateCtrl) +
                           (cnt_in_smem ? (size_t)p.mc * sizeof(int32_t) : 0);
       if (smem > 227 * 1024) continue;
       int ctas = (int)((228 * 1024) / (smem + 1024));         // 1 KB per CTA is reserved by the system
@@ -898,8 +1202,11 @@ cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, cons
                          const __nv_bfloat16*, const int32_t*, int32_t*, int32_t*, int32_t*, int, ListScan, int32_t*);
   Kernel kernel = nullptr;
   const int w = g.list_len <= 8 ? 8 : (g.list_len <= 16 ? 16 : (g.list_len <= 32 ? 32 : 0));
+  const bool one = gate_one(p);
 #define MOBA_GATE_W(HALF, DIM)                                                                       \
-  kernel = w == 8 ? (Kernel)gate_topk_kernel<HALF, DIM, 8> : w == 16 ? (Kernel)gate_topk_kernel<HALF, DIM, 16> \
+  kernel = one ? (w == 8 ? (Kernel)gate_one_kernel<HALF, DIM, 8> : w == 16 ? (Kernel)gate_one_kernel<HALF, DIM, 16>   \
+                                                                   : (Kernel)gate_one_kernel<HALF, DIM, 32>)         \
+         : w == 8 ? (Kernel)gate_topk_kernel<HALF, DIM, 8> : w == 16 ? (Kernel)gate_topk_kernel<HALF, DIM, 16> \
          : w == 32 ? (Kernel)gate_topk_kernel<HALF, DIM, 32> : (Kernel)gate_topk_kernel<HALF, DIM, 0>
   switch (p.D) {
     case 64:  if (p.fp16) MOBA_GATE_W(true, 64);  else MOBA_GATE_W(false, 64);  break;
@@ -925,13 +1232,15 @@ cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, cons
   cudaDeviceGetAttribute(&smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
   cudaDeviceGetAttribute(&regs_per_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
   int resident = (int)(smem_per_sm / (g.smem + 1024));
-  const int regs_per_cta = ((attr.numRegs + 7) / 8 * 8) * kGateThreads;
+  const int threads = one ? kOneThreads : kGateThreads;
+  const int regs_per_cta = ((attr.numRegs + 7) / 8 * 8) * threads;
   if (regs_per_cta > 0 && resident > regs_per_sm / regs_per_cta) resident = regs_per_sm / regs_per_cta;
-  if (resident > 512 / g.nt) resident = 512 / g.nt;
+  const int cols = one ? kOneCols : g.nt;
+  if (resident > 512 / cols) resident = 512 / cols;
   if (resident < 1) resident = 1;
   int64_t grid = (int64_t)sms * resident;
   if (grid > n_tiles) grid = n_tiles;
-  return launch_chained(chained, kernel, dim3((unsigned)grid), kGateThreads, g.smem, st, p, mq, mm, tokens_per_cta, g.nt,
+  return launch_chained(chained, kernel, dim3((unsigned)grid), threads, g.smem, st, p, mq, mm, tokens_per_cta, g.nt,
                         g.list_len, g.nbuf, g.cnt_in_smem, q, means, cu, selected, list_counts, stats, flags,
                         scan ? *scan : ListScan{}, scan ? ticket : nullptr);
 }

@@ -125,6 +125,27 @@ def test_exact_ties_and_one_ulp_near_ties_across_many_candidates(dtype, topk):
     _gate_with_means(q0, bits.view(dtype), lens, chunk, topk, hkv)
 
 
+@pytest.mark.parametrize("nchunks,topk,d,dtype", [
+    (34, 2, 64, torch.float16), (34, 8, 128, torch.bfloat16), (65, 13, 96, torch.bfloat16), (66, 14, 128, torch.float16),
+    (129, 29, 64, torch.bfloat16), (130, 8, 256, torch.bfloat16), (257, 12, 128, torch.bfloat16), (258, 28, 128, torch.bfloat16),
+    (258, 13, 64, torch.float16)])
+def test_more_than_32_candidates_at_the_edges_of_tiles_and_lists(nchunks, topk, d, dtype):
+    """Numbers of candidates around those of a tile (64, 128, 256, and two tiles), list lengths around those of
+    the networks (16, 32).  Random means, and means whose large scores all lie in one 32nd of the columns
+    (more of them reach the threshold than the fast path sorts) or rise with the chunk."""
+    g = torch.Generator().manual_seed(nchunks * 64 + topk)
+    chunk, hq, hkv = 8, 4, 2
+    lens = [chunk * nchunks, 3 * chunk + 5]
+    q = torch.randn(sum(lens), hq, d, generator=g).to(dtype)
+    means = (torch.randn(2 * nchunks, hkv, d, generator=g) * 0.5).to(dtype)
+    _gate_with_means(q, means, lens, chunk, topk, hkv)
+    c = torch.arange(2 * nchunks) % nchunks
+    q = (q.abs() + 0.1).to(dtype)
+    hot = torch.where(c % 32 == 5, 1.0 + c / 1000.0, 0.01 * (c % 7))
+    _gate_with_means(q, (means.float().abs() * hot[:, None, None]).to(dtype), lens, chunk, topk, hkv)
+    _gate_with_means(q, ((0.1 + c / 100.0)[:, None, None] * (1 + means.float().abs())).to(dtype), lens, chunk, topk, hkv)
+
+
 def test_long_candidate_lists_sampled():
     """More candidates than one tensor-core tile holds (625 > 256), top-k 8 and 64, against the
     oracle on sampled tokens; all three decision paths."""
