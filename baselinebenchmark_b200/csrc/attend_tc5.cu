@@ -1323,12 +1323,15 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
 // halves of Q, of K and of V have 32 KB slots of their own, each refilled as soon as the MMAs that read it
 // have executed.  Two softmax warpgroups take the items in turn: one computes the next item's softmax
 // while the other waits for its P.V and writes its rows.  The P.V of a tile can still be executing when
-// the softmax of the item's next tile wants to rescale O: that path waits for it.  Measured against the wide kernel,
-// 2 x 4096 tokens x 16 heads, chunk 128: 446 -> 324 us.  Long chunks stay with the wide kernel: 295 tokens behind
+// the softmax of the item's next tile wants to rescale O: that path waits for it.  The Q rows of the next item are
+// copied by the warpgroup whose item's last Q.K^T has just executed, in front of its last softmax step: with a
+// warp of its own for each half of Q the MMAs waited half of an item's time for 64 copies a lane (281 -> 228 us; one tile
+// of 128 dims waits for softmax instead, and there two warps of their own are better: 126 against 154).  Measured
+// against the wide kernel, 2 x 4096 tokens x 16 heads, chunk 128: 446 -> 228 us.  Long chunks stay with the wide kernel: 295 tokens behind
 // 22411, 16 heads, chunk 4096 take 200 us there and 236 here.
 // ---------------------------------------------------------------------------
-// warp 0 describes the items, 1 issues MMAs, 2 copies the lo half of the Q rows and requests K, 3 copies the hi half and
-// requests V; 4-7, 8-11: softmax of the even / odd items
+// warp 0 describes the items, 1 issues MMAs, 2 requests K, 3 requests V; 4-7, 8-11: softmax of the even / odd items, and the Q rows
+// of the item behind
 constexpr int kWideShortThreads = 384;
 
 struct WideShortCtrl {
@@ -1370,7 +1373,7 @@ attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
-      mbar_init(smem_u32(&c.q_full[i]), 32 + i);              // the copies of a warp's lanes; hi: and warp 2
+      mbar_init(smem_u32(&c.q_full[i]), kTileM + 1);          // the copies of a warpgroup; warp 2
       mbar_init(smem_u32(&c.k_full[i]), 1);
       mbar_init(smem_u32(&c.v_full[i]), 1);
       mbar_init(smem_u32(&c.q_free[i]), 1);
@@ -1418,14 +1421,13 @@ attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap
     else ok = describe_items<kShortSlots, 2, false, false>(p, sa.iq, c);
     if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
   } else if (warp == 2 || warp == 3) {
-    // ---- Q rows (a half each); warp 2: K tiles, warp 3: V tiles
+    // ---- warp 2: K tiles, warp 3: V tiles
     uint32_t kt = 0, vt = 0;               // k_free phases waited for, V tiles requested
-    const int hq = warp - 2;
     for (int n = 0; ok; ++n) {
       const int slot = n % kShortSlots;
       if (!wait(&c.item_full[slot], (n / kShortSlots) & 1)) break;
       if (c.item[slot].done) break;
-      const int tok0 = c.item[slot].tok0, head = c.item[slot].head, nrows = c.item[slot].nrows;
+      const int tok0 = c.item[slot].tok0, head = c.item[slot].head;
       const int ntiles = (c.item[slot].kv_len + kBN - 1) / kBN;
       const bool fresh = c.item[slot].new_kv != 0;
       auto load = [&](uint32_t dst, const CUtensorMap* m, uint64_t* full, int h, int j) {
@@ -1440,12 +1442,8 @@ attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           if (n > 0 && !wait(&c.q_free[h], (n - 1) & 1)) break;
-          if (h == 1 && lane == 0) mbar_arrive(smem_u32(&c.q_full[1]));   // (nobody runs past a phase this warp waits for)
+          if (lane == 0) mbar_arrive(smem_u32(&c.q_full[h]));   // (nobody runs past a phase this warp waits for)
           if (fresh) load(sK + h * kTileBytes, &tmap_k, &c.k_full[h], h, 0);
-          if (h == 0) {
-            copy_rows_async<16, 1>(sQ, a.q, 0, 0, nrows, [&](int r) { return c.qoff[slot][r]; });
-            cp_async_mbar_arrive(smem_u32(&c.q_full[0]));
-          }
         }
         for (int j = 1; ok && j < ntiles; ++j, ++kt)
 #pragma unroll
@@ -1454,9 +1452,6 @@ attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap
             load(sK + h * kTileBytes, &tmap_k, &c.k_full[h], h, j);
           }
       } else {
-        if (n > 0 && !wait(&c.q_free[1], (n - 1) & 1)) break;
-        copy_rows_async<16, 1>(sQ + hq * kTileBytes, a.q, 16, 0, nrows, [&](int r) { return c.qoff[slot][r]; });
-        cp_async_mbar_arrive(smem_u32(&c.q_full[1]));
         if (fresh)
           for (int j = 0; ok && j < ntiles; ++j, ++vt)
 #pragma unroll
@@ -1549,6 +1544,17 @@ attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap
     const uint32_t tO = tmem + lane_base + 256;
     const float sl2 = rsqrtf((float)D) * 1.4426950408889634f;
     uint32_t sph0 = 0, sph1 = 0, pvph = 0;                     // phases of s_full[x][0], [1] and pv_full[x]
+    // Q rows of item m; the last Q.K^T of the item before has executed
+    auto copy_rows = [&](int m) {
+      const int slot = m % kShortSlots;
+      if (!wait(&c.item_full[slot], (m / kShortSlots) & 1) || c.item[slot].done) return;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        copy_rows_async<16, 4>(sQ + h * kTileBytes, a.q, 16 * h, warp & 3, c.item[slot].nrows, [&](int r) { return c.qoff[slot][r]; });
+        cp_async_mbar_arrive(smem_u32(&c.q_full[h]));
+      }
+    };
+    if (x == 1) copy_rows(0);
     for (int n = x; ok; n += 2) {
       const int slot = n % kShortSlots;
       ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.item_full[slot]), (n / kShortSlots) & 1));
@@ -1568,6 +1574,8 @@ attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap
         if (buf) sph1 ^= 1; else sph0 ^= 1;
         // the item's Q.K^T has run: every role has read its description
         if (j == 0 && lane == 0) mbar_arrive(smem_u32(&c.slot_free[slot]));
+        if (j + 1 == ntiles) copy_rows(n + 1);
+        if (!ok) break;
         // the P.V of the tile before must have executed before O is touched
         bool waited = j == 0;
         auto wait_pv = [&] {
