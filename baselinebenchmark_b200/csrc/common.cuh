@@ -375,17 +375,24 @@ __host__ __device__ inline bool tc5_small_tiles(int head_dim, int chunk) { retur
 // SM; where the lists are cut into 256 rows it takes a half at a time), and so do query windows whose rows of
 // one kv head fit one tile (decode steps): a second row tile would be empty.  Measured against the 256-row kernel,
 // whole call: chunk 512, 32768 tokens x 32/8 heads, top-k 8 3.61 -> 3.27 ms (head_dim 64 2.85 -> 2.42), 2 x 4096 x 16
-// 340 -> 308 us, 19456 x 32 983 -> 888 us; chunk 1024 4.66-5.01 against 5.05 ms on the first (the halves read K and V
-// twice as often), so the line lies at 512; small launches gain too (700 to 20000 tokens, 1 to 16 heads, chunks 300 and
+// 340 -> 308 us, 19456 x 32 983 -> 888 us; small launches gain too (700 to 20000 tokens, 1 to 16 heads, chunks 300 and
 // 512: dense stage 0.69 to 1.00 of the other's).  Windows: 1 to 128 rows per kv head, 9000 to 131072 tokens, 1 to 16 kv
 // heads, chunks 1024 to 4096: 0.49 to 1.03 of the other's dense stage, with no more CTAs than items (window_ctas).
-constexpr int kShortChunk = 512;
+// Up to 1024 keys the halves of a 256-row tile still read K and V twice as often for less than the second CTA per SM
+// gives, whole call: 700 tokens behind 50021, 32/8 heads 197 -> 183 us, 64 behind them 120 -> 93, 1500 behind 20000
+// at head_dim 64 153 -> 148; 12001 x 16/2 753 -> 713; 5000 + 3000 x 8/1 164 -> 156; 32768 x 16 at 64 1977 -> 1805, 20000 x 16/4 at
+// 96 1323 -> 1222.  At head_dim 128, where an item's tiles are the largest, long calls lose (8 M partial rows, 32768 x 32/8,
+// top-k 8 4.63 -> 4.72 ms; 6 M, 65536 x 8, top-k 12 3.62 -> 3.66) and 1.9 M still gain (19456 x 32, top-k 3 1018 -> 998 us): the
+// line lies between.  At 2048 and 4096 keys all but a few lose (20000 x 8/4 759 -> 826).
+constexpr int kShortChunk = 512, kShortChunkFew = 1024;
+constexpr int64_t kShortFewRows = (int64_t)4 << 20;
 static_assert(kSmallChunk <= kShortChunk, "lists cut into 128 rows run the kernel of one-tile items");
 inline bool tc5_short_items(const Params& p) {
   if (p.D > 128) return false;
   if (p.Tq * p.G <= kTileRowsWide) return true;
   // (own-chunk items are counted in int32; a slot table that large stays with the 256-row kernel)
-  return p.C <= kShortChunk && (int64_t)p.slots * p.Hq * ((p.C + 127) / 128) < ((int64_t)1 << 30);
+  const bool few = p.C <= kShortChunkFew && (p.D < 128 || p.rows * p.NP <= kShortFewRows);
+  return (p.C <= kShortChunk || few) && (int64_t)p.slots * p.Hq * ((p.C + 127) / 128) < ((int64_t)1 << 30);
 }
 
 cudaError_t launch_attend_mma(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* k,

@@ -46,6 +46,26 @@ def test_chunk_sizes_around_the_tiles(chunk, d, dtype):
     assert (lse - ref_lse).abs().max().item() < 1e-3       # scores in fp32, exponentials to 7.5e-5
 
 
+@pytest.mark.parametrize("d,dtype", [(64, torch.float16), (96, torch.bfloat16), (128, torch.bfloat16)])
+@pytest.mark.parametrize("chunk", [1000, 1024, 1025])
+def test_chunks_of_up_to_1024_keys_on_either_kernel(chunk, d, dtype):
+    """Chunks of 513 to 1024 keys are items of half a 256-row tile (the last half of a list may be empty or ragged); one
+    key more and the 256-row kernel runs."""
+    lens, hq, hkv, topk = (1, 3 * chunk + 77, 1023, 5 * chunk), 6, 2, 4
+    q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, dtype, seed=chunk + d)
+    out, lse, sel = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True, return_selected=True)
+    ref, ref_lse, ref_sel = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True,
+                                                  return_selected=True, attend_impl=_lib.ATTEND_MMA_SYNC)
+    assert torch.equal(sel, ref_sel)
+    _close(out, ref, dtype)
+    assert (lse - ref_lse).abs().max().item() < 1e-3
+    for begin, n in ((100, 200), (3 * chunk - 5, 131)):                       # windows of more rows than one tile
+        o, l, s = parallel.moba_forward(q[begin:begin + n], k, v, cu, max(lens), chunk, topk, return_lse=True,
+                                        return_selected=True, q_token_begin=begin)
+        assert torch.equal(s, sel[:, :, begin:begin + n])
+        assert torch.equal(o, out[begin:begin + n]) and torch.equal(l, lse[:, begin:begin + n])
+
+
 @pytest.mark.parametrize("hq,hkv", [(4, 4), (8, 2), (16, 1)])
 @pytest.mark.parametrize("d,chunk", [(128, 128), (128, 512), (128, 4096), (256, 128), (256, 256), (256, 257)])
 def test_windows_around_the_row_limit_equal_full_run(d, chunk, hq, hkv):
