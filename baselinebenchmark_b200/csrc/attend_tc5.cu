@@ -1014,10 +1014,10 @@ attend_tc5_wide_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_
 }
 
 // ---------------------------------------------------------------------------
-// short items: chunks of at most kShortChunk keys, and query windows with at most 128 rows per
-// kv head (decode steps).  One 128-row tile per work item, two CTAs per SM.
+// short items: chunks of at most kShortChunk keys (kShortChunkFew in all but long calls, see tc5_short_items), and query windows
+// with at most 128 rows per kv head (decode steps).  One 128-row tile per work item, two CTAs per SM.
 //
-// Such an item is one to four key tiles (or, in a decode step, a long chunk for a handful of
+// Such an item is one to eight key tiles (or, in a decode step, a long chunk for a handful of
 // rows), so what counts is that nothing of its hand-over is waited for.  The roles of a CTA run
 // through one flat stream of key tiles, without a CTA-wide barrier between items:
 //   warp 4     describes the items, up to four ahead (a chain of dependent global loads and divisions as
@@ -1035,7 +1035,8 @@ attend_tc5_wide_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_
 // Per CTA: one Q, one K and one V tile (32 KB each), 256 TMEM columns (S 0-127, O 128-255); two CTAs per SM
 // overlap each other's softmax, MMA and stores.
 // With one warpgroup for both, softmax and epilogue of an item took most of its time, one after the other (see
-// softmax_row_rolled); with two: length-4096 below 142 -> 134 us, 13311 x 16/4 at head_dim 64 162 -> 145.
+// softmax_row_rolled); with two, dense stage of 2 x 4096 tokens x 16 heads, chunk 128 142 -> 134 us, 13311 x 16/4 at
+// head_dim 64 162 -> 145.  An item now takes 7000 cycles of a CTA, the chain Q.K^T, S, softmax, P.V and the copy of the next Q rows.
 // Measured against the kernel with CTA-wide barriers between items and unrolled code: dense stage of
 // 2 x 4096 tokens x 16 heads, chunk 128 199 -> 146 us (whole call 347 -> 279); 13311 tokens x 16/4 heads,
 // head_dim 64 233 -> 172; 32768 x 32/8 1651 -> 1094.  A decode step (chunk 4096, 131072-token prefix, 32/8 heads), in
