@@ -211,7 +211,9 @@ constexpr int kGateRows = 128;            // (token, head) rows per tile
 constexpr int kListExtra = 3;             // list places beyond hist + 1 that absorb near-ties at the cut
 constexpr int kCntSmemMax = 4096;         // chunks per sequence up to which the list histogram is kept in shared memory
 constexpr int kQBlockBytes = 128 * 128;   // one [128 rows][64 dims] swizzled block of 16-bit values
-constexpr int kScratchStride = 36;        // floats per row of the score scratch (144 bytes: conflict-free 16-byte stores)
+// floats per row of the score scratch, for the keys a network leaves (w) or, without one (0), all 32 of a step: an odd
+// number of 16-byte pieces, so that 16-byte stores are free of conflicts
+__host__ __device__ constexpr int scratch_stride(int w) { return (w > 0 ? w : 32) + 4; }
 
 __device__ __forceinline__ uint32_t float_key(float x) {      // routing.py:778-784
   const uint32_t b = __float_as_uint(x);
@@ -547,8 +549,8 @@ __device__ __forceinline__ void finish_scan(const ListScan& scan, int32_t* __res
 //   warps 0-3  a thread per row.  The sorted keys stay in registers, and what they settle is decided there; a row with
 //              near-ties goes through a list in shared memory.  Every warp counts for itself: no barrier of
 //              the CTA in the loop, a warp may be a tile behind another.
-// Measured against the kernel below for these shapes, gating behind its chunk means: 2 x 4096 tokens x 16 heads, 31 candidates
-// 34 -> 30 us, at head dim 256 83 -> 69; 32768 x 32/8, 7 candidates 159 -> 131; a decode token on 32 chunks 10 -> 4.
+// Measured against the kernel below for these shapes, with the wait for the chunk means: 2 x 4096 tokens x 16 heads, 31
+// candidates 44 -> 40 us, at head dim 256 105 -> 91; 32768 x 32/8, 7 candidates 179 -> 152; a decode token on 32 chunks 24 -> 17.
 // (The few-lane score of near-ties alone, which the kernel below has too: 32768 x 32/8, 255 candidates 620 -> 573.)
 // ---------------------------------------------------------------------------
 constexpr int kOneThreads = 160;
@@ -802,8 +804,8 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
   unsigned char* sQ0 = smem;                                             // nbuf x kNBlk blocks [128][64]
   unsigned char* sB = sQ0 + (size_t)nbuf * kNBlk * kQBlockBytes;        // kNBlk blocks [nt][64]
   uint2* lists = reinterpret_cast<uint2*>(sB + (size_t)kNBlk * nt * 128);   // [128][lstride] {chunk, score bits}
-  float* scratch = reinterpret_cast<float*>(lists + (size_t)kGateRows * lstride);   // [128][36]
-  GateCtrl& c = *reinterpret_cast<GateCtrl*>(scratch + kGateRows * kScratchStride);
+  float* scratch = reinterpret_cast<float*>(lists + (size_t)kGateRows * lstride);   // [128][scratch_stride]
+  GateCtrl& c = *reinterpret_cast<GateCtrl*>(scratch + kGateRows * scratch_stride(kW));
   int32_t* cnt_s = reinterpret_cast<int32_t*>(&c + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -925,7 +927,7 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
     uint2* mylist = lists + (size_t)row * lstride;
     for (int i = 0; i < list_len; ++i) mylist[i] = make_uint2(0xFFFFFFFFu, 0u);   // chunk -1, key 0: empty place
     uint32_t tau = 0;                                  // smallest key kept (heap root / last place); 0 while places are free
-    uint32_t* myscratch = reinterpret_cast<uint32_t*>(scratch + row * kScratchStride);
+    uint32_t* myscratch = reinterpret_cast<uint32_t*>(scratch + row * scratch_stride(kW));
 
     // A wait that gives up is remembered by the thread: its row is then ranked exactly, from Q rows
     // read with plain loads (see the recheck).
@@ -1149,6 +1151,8 @@ struct GateLaunch {
 // Candidate tile, Q buffers, list length and shared memory of a launch: the combination that puts
 // the most CTAs on an SM (more warps hide the latency of the heap updates), then two Q buffers,
 // then the wider candidate tile.  smem == 0: nothing fits.
+// Width of the network for a list, 0: none.
+inline int gate_network(int list_len) { return list_len <= 8 ? 8 : list_len <= 16 ? 16 : list_len <= 32 ? 32 : 0; }
 // At most 32 candidates a row, and a network for the list.
 inline bool gate_one(const Params& p) { return p.mc - 1 <= kOneMeans && p.hist + 1 <= 32; }
 GateLaunch gate_launch_config(const Params& p) {
@@ -1162,18 +1166,22 @@ GateLaunch gate_launch_config(const Params& p) {
     return GateLaunch{kOneMeans, list_len, 1, 0, 4,
                       1024 + (size_t)nblk * kQBlockBytes + (size_t)nblk * kOneMeans * 128 +
                           (size_t)kGateRows * (list_len | 1) * sizeof(uint2) + sizeof(OneCtrl)};
+  const int w = gate_network(list_len);
+  // No more CTAs than registers allow: counted for a fourth, the kernels of the wider networks had tiles of 32 candidates,
+  // and a round trip of TMA and MMA for each 32 of a row (32768 x 32/8, 255 candidates 577 -> 543 us with 64).
+  const int max_ctas = w == 16 || w == 32 ? kGateMinCtas<16> : 4;
   int want = 32;
   while (want < p.mc - 1 && want < 256) want *= 2;            // a row has at most mc - 1 candidates
   for (int nbuf = 2; nbuf >= 1; --nbuf)
     for (int nt = want; nt >= 32; nt /= 2) {
       const size_t smem = 1024 + (size_t)nbuf * nblk * kQBlockBytes + (size_t)nblk * nt * 128 +
                           (size_t)kGateRows * (list_len | 1) * sizeof(uint2) +
-                          (size_t)kGateRows * kScratchStride * sizeof(float) + sizeof(GateCtrl) +
+                          (size_t)kGateRows * scratch_stride(w) * sizeof(float) + sizeof(GateCtrl) +
                           (cnt_in_smem ? (size_t)p.mc * sizeof(int32_t) : 0);
       if (smem > 227 * 1024) continue;
       int ctas = (int)((228 * 1024) / (smem + 1024));         // 1 KB per CTA is reserved by the system
       if (ctas > 512 / nt) ctas = 512 / nt;                   // tensor memory columns
-      if (ctas > 4) ctas = 4;
+      if (ctas > max_ctas) ctas = max_ctas;
       if (ctas < 1) continue;
       if (ctas > best.ctas_per_sm) best = GateLaunch{nt, list_len, nbuf, cnt_in_smem, ctas, smem};
     }
@@ -1201,7 +1209,7 @@ cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, cons
   typedef void (*Kernel)(Params, CUtensorMap, CUtensorMap, int, int, int, int, int, const __nv_bfloat16*,
                          const __nv_bfloat16*, const int32_t*, int32_t*, int32_t*, int32_t*, int, ListScan, int32_t*);
   Kernel kernel = nullptr;
-  const int w = g.list_len <= 8 ? 8 : (g.list_len <= 16 ? 16 : (g.list_len <= 32 ? 32 : 0));
+  const int w = gate_network(g.list_len);
   const bool one = gate_one(p);
 #define MOBA_GATE_W(HALF, DIM)                                                                       \
   kernel = one ? (w == 8 ? (Kernel)gate_one_kernel<HALF, DIM, 8> : w == 16 ? (Kernel)gate_one_kernel<HALF, DIM, 16>   \
