@@ -1149,8 +1149,8 @@ struct GateLaunch {
 };
 
 // Candidate tile, Q buffers, list length and shared memory of a launch: the combination that puts
-// the most CTAs on an SM (more warps hide the latency of the heap updates), then two Q buffers,
-// then the wider candidate tile.  smem == 0: nothing fits.
+// the most CTAs on an SM (more warps hide the latency of the heap updates), then the wider candidate
+// tile, then two Q buffers.  smem == 0: nothing fits.
 // Width of the network for a list, 0: none.
 inline int gate_network(int list_len) { return list_len <= 8 ? 8 : list_len <= 16 ? 16 : list_len <= 32 ? 32 : 0; }
 // At most 32 candidates a row, and a network for the list.
@@ -1172,8 +1172,8 @@ GateLaunch gate_launch_config(const Params& p) {
   const int max_ctas = w == 16 || w == 32 ? kGateMinCtas<16> : 4;
   int want = 32;
   while (want < p.mc - 1 && want < 256) want *= 2;            // a row has at most mc - 1 candidates
-  for (int nbuf = 2; nbuf >= 1; --nbuf)
-    for (int nt = want; nt >= 32; nt /= 2) {
+  for (int nt = want; nt >= 32; nt /= 2)
+    for (int nbuf = 2; nbuf >= 1; --nbuf) {
       const size_t smem = 1024 + (size_t)nbuf * nblk * kQBlockBytes + (size_t)nblk * nt * 128 +
                           (size_t)kGateRows * (list_len | 1) * sizeof(uint2) +
                           (size_t)kGateRows * scratch_stride(w) * sizeof(float) + sizeof(GateCtrl) +
