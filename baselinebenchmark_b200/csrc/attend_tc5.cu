@@ -1388,7 +1388,11 @@ attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap
     mbar_init(smem_u32(&c.o_free), kTileM);
     for (int i = 0; i < kShortSlots; ++i) {
       mbar_init(smem_u32(&c.item_full[i]), 1);
-      mbar_init(smem_u32(&c.slot_free[i]), 4);                // the softmax warps of the item
+      // The readers of a description and what orders each before the slot's next item: the MMA warp reads it in front of
+      // Q.K^T, warp 2 and the warpgroup that copies the Q rows before they arrive on q_full, which Q.K^T waits for; the
+      // softmax warps of the item arrive here once its first S is there, behind all of these.  Warp 3 requests V, which no
+      // Q.K^T waits for: it arrives here itself.
+      mbar_init(smem_u32(&c.slot_free[i]), 5);
     }
     c.abort = 0;
     fence_barrier_init();
@@ -1431,6 +1435,8 @@ attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap
       const int tok0 = c.item[slot].tok0, head = c.item[slot].head;
       const int ntiles = (c.item[slot].kv_len + kBN - 1) / kBN;
       const bool fresh = c.item[slot].new_kv != 0;
+      __syncwarp();                                             // every lane has read the description
+      if (warp == 3 && lane == 0) mbar_arrive(smem_u32(&c.slot_free[slot]));
       auto load = [&](uint32_t dst, const CUtensorMap* m, uint64_t* full, int h, int j) {
         if (lane == 0) {
           const uint32_t bar = smem_u32(full);
@@ -1573,7 +1579,7 @@ attend_tc5_wide_short_kernel(const Params p, const __grid_constant__ CUtensorMap
         ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&c.s_full[x][buf]), buf ? sph1 : sph0));
         if (!ok) break;
         if (buf) sph1 ^= 1; else sph0 ^= 1;
-        // the item's Q.K^T has run: every role has read its description
+        // the item's Q.K^T has run: every role but warp 3 has read its description
         if (j == 0 && lane == 0) mbar_arrive(smem_u32(&c.slot_free[slot]));
         if (j + 1 == ntiles) copy_rows(n + 1);
         if (!ok) break;
