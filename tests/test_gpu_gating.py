@@ -74,12 +74,15 @@ def _gate_with_means(q, means, lens, chunk, topk, hkv):
     sel_o = O.select_chunks(q, means, cu, max(lens), chunk, hist)
     qd, md = q.cuda(), means.cuda()
     cud = torch.from_numpy(cu).cuda()
+    count_o = np.bincount((sel_o.astype(np.int64) * hkv + (np.arange(q.shape[1]) // (q.shape[1] // hkv))[None, :, None])[sel_o >= 0],
+                          minlength=(len(cu) - 1) * mc * hkv)
     kdummy = torch.zeros(q.shape[0], hkv, q.shape[2], dtype=q.dtype, device="cuda")
     prob, _ = G.problem_for(qd, kdummy, kdummy, cud, max(lens), chunk, topk)
     out = {}
     for flags in (NORMAL, FORCE_EXACT, FORCE_RECHECK):
-        sel, _, stats = G.gate_stats(prob, qd, md, cud, flags)
+        sel, counts, stats = G.gate_stats(prob, qd, md, cud, flags)
         np.testing.assert_array_equal(sel.cpu().numpy(), sel_o, err_msg=f"flags={flags}")
+        np.testing.assert_array_equal(counts.cpu().numpy(), count_o, err_msg=f"flags={flags}")
         assert stats[2] == 0
         out[flags] = stats
     return out
@@ -131,8 +134,8 @@ def test_exact_ties_and_one_ulp_near_ties_across_many_candidates(dtype, topk):
     (258, 13, 64, torch.float16)])
 def test_more_than_32_candidates_at_the_edges_of_tiles_and_lists(nchunks, topk, d, dtype):
     """Numbers of candidates around those of a tile (64, 128, 256, and two tiles), list lengths around those of
-    the networks (16, 32).  Random means, and means whose large scores all lie in one 32nd of the columns
-    (more of them reach the threshold than the fast path sorts) or rise with the chunk."""
+    the networks (16, 32).  Random means, and means whose large scores all lie in one column of each step
+    of 32 (every step replaces a place of the list) or rise with the chunk (every step replaces the whole list)."""
     g = torch.Generator().manual_seed(nchunks * 64 + topk)
     chunk, hq, hkv = 8, 4, 2
     lens = [chunk * nchunks, 3 * chunk + 5]
@@ -144,6 +147,75 @@ def test_more_than_32_candidates_at_the_edges_of_tiles_and_lists(nchunks, topk, 
     hot = torch.where(c % 32 == 5, 1.0 + c / 1000.0, 0.01 * (c % 7))
     _gate_with_means(q, (means.float().abs() * hot[:, None, None]).to(dtype), lens, chunk, topk, hkv)
     _gate_with_means(q, ((0.1 + c / 100.0)[:, None, None] * (1 + means.float().abs())).to(dtype), lens, chunk, topk, hkv)
+
+
+def _adversarial_means(nchunks, hkv, d, dtype, g):
+    """(what the scores of a row do, means of the chunks)."""
+    base = (torch.randn(hkv, d, generator=g) * 0.5).to(dtype)
+    same = base[None].repeat(nchunks, 1, 1).contiguous()
+    yield "all tie", same
+    five = (torch.randn(5, hkv, d, generator=g) * 0.5).to(dtype)
+    yield "tie in groups", five[torch.arange(nchunks) % 5].contiguous()
+    bits = same.clone().view(torch.int16)
+    bits[torch.arange(nchunks), :, torch.randint(0, d, (nchunks,), generator=g)] += \
+        torch.randint(-1, 2, (nchunks, 1), generator=g).to(torch.int16)
+    yield "one ulp of one element apart", bits.view(dtype)
+    half = (torch.randn(nchunks, hkv, d, generator=g) * 0.5).to(dtype)
+    half[::2] = bits.view(dtype)[::2]
+    yield "runs of near-ties between others", half
+    zeros = torch.zeros(nchunks, hkv, d, dtype=dtype)
+    zeros.view(torch.int16)[1::2] = -32768                                    # -0.0
+    yield "zeros of either sign", zeros
+    at = torch.arange(nchunks)
+    for value in (float("inf"), float("nan")):
+        some = (torch.randn(nchunks, hkv, d, generator=g) * 0.5).to(dtype)
+        some[at[2::4], :, torch.randint(0, d, (nchunks,), generator=g)[2::4]] = value
+        if value == float("inf"):
+            some[at[1::4], :, 3] = -value
+        yield f"some {value}", some
+
+
+@pytest.mark.parametrize("d,dtype", [(64, torch.float16), (96, torch.bfloat16), (128, torch.bfloat16), (128, torch.float16),
+                                     (256, torch.bfloat16)])
+@pytest.mark.parametrize("nchunks,topk", [(2, 2), (2, 8), (9, 2), (9, 8), (9, 17), (31, 17), (32, 8), (32, 9), (32, 32),
+                                          (33, 2), (33, 8), (33, 9), (33, 16), (33, 17), (33, 31), (33, 32), (33, 33)])
+def test_at_most_32_candidates_ties_zeros_infinities(nchunks, topk, d, dtype):
+    """The kernel for rows of at most 32 candidates (33 chunks), which decides in registers: every width of its
+    network (lists of 8, 16 and 32) from both sides, and with lists of 33 the other kernel.  Infinite and NaN scores
+    rank by their bits (NaN of positive sign here, above +inf), equal ones by the chunk."""
+    g = torch.Generator().manual_seed(nchunks * 64 + topk)
+    chunk, hq, hkv = 8, 4, 2
+    lens = [chunk * nchunks, chunk - 1, chunk * (nchunks // 2) + 3]
+    q = torch.randn(sum(lens), hq, d, generator=g).to(dtype)
+    q[q == 0] = 1                                                             # (inf * 0)
+    for what, means in _adversarial_means(3 * nchunks, hkv, d, dtype, g):
+        _gate_with_means(q, means, lens, chunk, topk, hkv)
+        if what.startswith("one ulp"):
+            q0 = q.clone()
+            q0[::3] = 0
+            _gate_with_means(q0, means, lens, chunk, topk, hkv)
+    finite = (torch.randn(3 * nchunks, hkv, d, generator=g) * 0.5).to(dtype)
+    finite[finite == 0] = 1
+    _gate_with_means(q, finite, lens, chunk, topk, hkv)
+    for value in (float("inf"), float("nan")):
+        q1 = q.clone()
+        q1[::5, 1, 7] = value
+        _gate_with_means(q1, finite, lens, chunk, topk, hkv)
+
+
+@pytest.mark.parametrize("topk", [5, 12, 24])
+def test_at_most_32_candidates_many_tiles_of_rows(topk):
+    """Enough tiles of rows that every CTA takes several: tiles with and without candidates, tiles beyond the end of their
+    sequence and sequences shorter than a chunk follow one another in it."""
+    g = torch.Generator().manual_seed(topk)
+    chunk, hq, hkv, d = 8, 16, 4, 64
+    lens = [(264, 3, 130, 7, 8, 9, 40, 1)[(i + i // 8) % 8] for i in range(56)]
+    tiles = len(lens) * hkv * -(-264 // (128 // (hq // hkv)))
+    assert tiles >= 3 * 148 * 4
+    q = torch.randn(sum(lens), hq, d, generator=g).to(torch.bfloat16)
+    means = (torch.randn(33 * len(lens), hkv, d, generator=g) * 0.5).to(torch.bfloat16)
+    means[::3] = means[0]                                                     # ties in every sequence
+    _gate_with_means(q, means, lens, chunk, topk, hkv)
 
 
 def test_long_candidate_lists_sampled():
