@@ -196,13 +196,14 @@ def test_forward_matches_fp32_evaluation(case, impl, dtype):
 @pytest.mark.parametrize("impl", IMPLS)
 @pytest.mark.parametrize("jump", [4.0, 24.0, 140.0])
 @pytest.mark.parametrize("d", [128, 256])
-@pytest.mark.parametrize("chunk,starts", [(256, (150, 460, 700)), (512, (300, 700, 1400)), (1024, (300, 1700, 2900))])
+@pytest.mark.parametrize("chunk,starts", [(256, (150, 460, 700)), (512, (300, 700, 1400)), (1024, (300, 1700, 2900)),
+                                          (1100, (300, 1800, 3100))])
 def test_scores_rising_late_in_a_chunk(impl, dtype, jump, d, chunk, starts):
     """Keys whose scores lie far above everything seen earlier in the same chunk (by `jump`
     in units of log2 after scaling), after a first rise by half of that: the running reference of the softmax has to
     follow, whatever shortcut a kernel takes on tiles that look ordinary.  The chunk sizes are those of the
-    kernels: short items at head dim 128 up to 512 and at 256 up to 256, the 256-row kernel and the one
-    for head dim 256 beyond."""
+    kernels: one-tile items at head dim 128 up to 1024 (in a call of so few rows) and at 256 up to 256, the 256-row
+    kernel and the one for head dim 256 beyond."""
     t, hq, hkv, topk = 3 * chunk, 4, 2, 3
     g = torch.Generator().manual_seed(int(jump))
     q = torch.ones(t, hq, d) * 0.25
@@ -922,7 +923,8 @@ def test_config_selection_full_tensor(cfg_id, seed):
     assert counts.sum().item() == (sel_o >= 0).sum()
 
 
-@pytest.mark.parametrize("case", [("long_items", (3000, 900), 8, 2, 128, 1024, 3),
+@pytest.mark.parametrize("case", [("long_items", (3400, 900), 8, 2, 128, 1100, 3),
+                                  ("halved_long_items", (3000, 900), 8, 2, 128, 1024, 3),
                                   ("halved_tiles", (2048, 900), 8, 2, 128, 512, 4),
                                   ("short_items", (1500, 700), 8, 2, 128, 128, 5),
                                   ("d256_long_items", (1700, 300), 4, 2, 256, 512, 3),
@@ -942,7 +944,7 @@ def test_stage_entry_points_chain_to_the_forward_result(case):
     lib = _lib.lib()
     dims = G.dims_of(prob)
     tile_rows = lib.moba_problem_tile_rows(C.byref(prob))
-    assert tile_rows == (256 if name in ("long_items", "halved_tiles") else 128)
+    assert tile_rows == (256 if name in ("long_items", "halved_long_items", "halved_tiles") else 128)
     m = G.means(prob, kd, cud)
     sel, counts = G.gate(prob, qd, m, cud)
     offsets, tiles, row_list, plse = G.compact(prob, cud, sel, counts, tile_rows)

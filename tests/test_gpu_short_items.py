@@ -1,5 +1,5 @@
-"""GPU: the dense-stage kernels for short items (chunks of at most 512 keys, at head dim 256 of at most 256, and query
-windows with at most 128 rows per kv head), the row gathers, and the small kernels around them, at the sizes and
+"""GPU: the dense-stage kernels for one-tile items (chunks of at most 512 keys, in all but long calls of at most 1024, at
+head dim 256 of at most 256, and query windows with at most 128 rows per kv head), the row gathers, and the small kernels around them, at the sizes and
 strides where their branches change.
 
 Outputs are compared with the mma.sync dense stage.  Both round P to 16 bits and a partial row to 11
@@ -34,9 +34,9 @@ def _close(out, ref, dtype):
 
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("d", [64, 96, 128, 256])
-@pytest.mark.parametrize("chunk", [16, 64, 127, 128, 129, 200, 256, 257, 512, 513])
+@pytest.mark.parametrize("chunk", [16, 64, 127, 128, 129, 200, 256, 257, 512, 513, 1025])
 def test_chunk_sizes_around_the_tiles(chunk, d, dtype):
-    lens, hq, hkv, topk = (1, 130, 1025, 700), 6, 2, 5
+    lens, hq, hkv, topk = (1, 130, max(1025, 2 * chunk + 1), 700), 6, 2, 5
     q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, dtype, seed=chunk + d)
     out, lse, sel = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True, return_selected=True)
     ref, ref_lse, ref_sel = parallel.moba_forward(q, k, v, cu, max(lens), chunk, topk, return_lse=True,
@@ -66,11 +66,33 @@ def test_chunks_of_up_to_1024_keys_on_either_kernel(chunk, d, dtype):
         assert torch.equal(o, out[begin:begin + n]) and torch.equal(l, lse[:, begin:begin + n])
 
 
+def test_a_long_call_equals_its_windows_and_its_head_groups():
+    """At head dim 128 and chunks of 513 to 1024 keys a call of more than 2^22 partial rows runs the 256-row kernel; its
+    windows and, in a small workspace, its kv heads one by one are calls of fewer rows and run the kernel for one-tile
+    items.  Large scores, so that the softmax reference of many rows moves inside a chunk."""
+    tokens, hq, hkv, d, chunk, topk = 16400, 32, 8, 128, 1024, 8
+    assert tokens * hq * topk > 1 << 22
+    q, k, v, cu = _inputs((tokens,), hq, hkv, d, chunk, torch.bfloat16, seed=5)
+    q *= 4
+    args = (k, v, cu, tokens, chunk, topk)
+    out, lse, sel = parallel.moba_forward(q, *args, return_lse=True, return_selected=True)
+    prob, _ = G.problem_for(q, k, v, cu, tokens, chunk, topk)
+    assert G.dims_of(prob).rows * G.dims_of(prob).partials == tokens * hq * topk
+    least = C.c_size_t()
+    _lib.check(_lib.lib().moba_workspace_size_min(C.byref(prob), C.byref(least)))
+    out2, lse2, sel2 = parallel.moba_forward(q, *args, return_lse=True, return_selected=True, workspace_limit=least.value)
+    assert torch.equal(sel2, sel) and torch.equal(out2, out) and torch.equal(lse2, lse)
+    for begin, n in ((0, 700), (5 * chunk - 3, 2000), (tokens - 33, 33), (tokens - 32, 32), (tokens - 1, 1)):
+        o, l, s = parallel.moba_forward(q[begin:begin + n], *args, return_lse=True, return_selected=True, q_token_begin=begin)
+        assert torch.equal(s, sel[:, :, begin:begin + n])
+        assert torch.equal(o, out[begin:begin + n]) and torch.equal(l, lse[:, begin:begin + n]), (begin, n)
+
+
 @pytest.mark.parametrize("hq,hkv", [(4, 4), (8, 2), (16, 1)])
 @pytest.mark.parametrize("d,chunk", [(128, 128), (128, 512), (128, 4096), (256, 128), (256, 256), (256, 257)])
 def test_windows_around_the_row_limit_equal_full_run(d, chunk, hq, hkv):
     """128 rows per kv head is the largest window of the short kernel, whose own-chunk items then cover all heads of
-    a group; one token more and, with chunks of more than 512 keys, the 256-row kernel runs.  At head dim 256
+    a group; one token more and, with chunks of more than 1024 keys, the 256-row kernel runs.  At head dim 256
     the chunk alone decides between the kernels (256, 257).  Windows cross chunk and sequence boundaries."""
     lens, topk = (700, 5000), 4
     q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, torch.bfloat16, seed=7)
@@ -105,7 +127,7 @@ def _layouts(t, name):
 
 @pytest.mark.parametrize("d", [64, 96, 128])
 @pytest.mark.parametrize("layout", ["fused", "head_major", "padded_dim", "odd_token"])
-@pytest.mark.parametrize("chunk", [128, 1024])
+@pytest.mark.parametrize("chunk", [128, 1024, 1025])
 def test_layouts_of_q_give_the_same_bits(chunk, layout, d):
     """Forward, a decode-sized window and the gradients read the rows of q by its token and head strides."""
     lens, hq, hkv, topk = (1500, 2100), 4, 2, 3
@@ -222,7 +244,7 @@ def test_chunk_means_of_few_and_many_chunks(chunk, chunks, d, dtype):
 
 
 @pytest.mark.parametrize("topk", [1, 4])
-@pytest.mark.parametrize("chunk", [128, 1024])
+@pytest.mark.parametrize("chunk", [128, 1024, 1025])
 def test_a_call_waits_for_its_inputs_from_another_stream(chunk, topk):
     """The kernels of a call may become resident before the work in front of them is done.  Inputs written on another
     stream, behind a kernel that takes milliseconds, must all the same be there when the first of them reads:
