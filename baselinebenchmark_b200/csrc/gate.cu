@@ -1148,13 +1148,13 @@ struct GateLaunch {
   size_t smem;
 };
 
-// Candidate tile, Q buffers, list length and shared memory of a launch: the combination that puts
-// the most CTAs on an SM (more warps hide the latency of the heap updates), then the wider candidate
-// tile, then two Q buffers.  smem == 0: nothing fits.
 // Width of the network for a list, 0: none.
 inline int gate_network(int list_len) { return list_len <= 8 ? 8 : list_len <= 16 ? 16 : list_len <= 32 ? 32 : 0; }
 // At most 32 candidates a row, and a network for the list.
 inline bool gate_one(const Params& p) { return p.mc - 1 <= kOneMeans && p.hist + 1 <= 32; }
+// Candidate tile, Q buffers, list length and shared memory of a launch: the combination that puts
+// the most CTAs on an SM (more warps hide the latency of the list updates), then the wider candidate
+// tile, then two Q buffers.  smem == 0: nothing fits.
 GateLaunch gate_launch_config(const Params& p) {
   GateLaunch best{};
   const int nblk = (p.D + 63) / 64;
@@ -1167,9 +1167,10 @@ GateLaunch gate_launch_config(const Params& p) {
                       1024 + (size_t)nblk * kQBlockBytes + (size_t)nblk * kOneMeans * 128 +
                           (size_t)kGateRows * (list_len | 1) * sizeof(uint2) + sizeof(OneCtrl)};
   const int w = gate_network(list_len);
-  // No more CTAs than registers allow: counted for a fourth, the kernels of the wider networks had tiles of 32 candidates,
-  // and a round trip of TMA and MMA for each 32 of a row (32768 x 32/8, 255 candidates 577 -> 543 us with 64).
-  const int max_ctas = w == 16 || w == 32 ? kGateMinCtas<16> : 4;
+  // No more CTAs than the register budget is set for: counted for a fourth, the kernels of the wider networks had tiles of
+  // 32 candidates, and a round trip of TMA and MMA for each 32 of a row (32768 x 32/8, 255 candidates 577 -> 543 us
+  // with 64).  (The min-heap's lists leave shared memory for three at most, whatever is counted here.)
+  const int max_ctas = w == 8 ? kGateMinCtas<8> : w == 16 ? kGateMinCtas<16> : w == 32 ? kGateMinCtas<32> : kGateMinCtas<0>;
   int want = 32;
   while (want < p.mc - 1 && want < 256) want *= 2;            // a row has at most mc - 1 candidates
   for (int nt = want; nt >= 32; nt /= 2)
