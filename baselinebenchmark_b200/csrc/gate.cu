@@ -544,8 +544,8 @@ __device__ __forceinline__ void finish_scan(const ListScan& scan, int32_t* __res
 // One tile of means, one network a row, so what counts is the latency of a tile of rows: 25 000 cycles of it were
 // spent waiting for Q, on norms, on walks through lists in shared memory and at a barrier behind the warp with
 // the most near-ties, 2400 in the network.  Here
-//   warp 4     walks the row tiles of the CTA: requests Q and means as soon as the tensor core and the norms of the
-//              tile before have read theirs, and issues the MMA into the other half of 64 tensor memory columns
+//   warp 4     walks the row tiles of the CTA: requests Q and means and issues the MMA as soon as every row has its
+//              norms and its estimates of the tile before in registers, while networks, decisions and stores go on
 //   warps 0-3  a thread per row.  The sorted keys stay in registers, and what they settle is decided there; a row with
 //              near-ties goes through a list in shared memory.  Every warp counts for itself: no barrier of
 //              the CTA in the loop, a warp may be a tile behind another.
@@ -554,8 +554,7 @@ __device__ __forceinline__ void finish_scan(const ListScan& scan, int32_t* __res
 // (The few-lane score of near-ties alone, which the kernel below has too: 32768 x 32/8, 255 candidates 620 -> 573.)
 // ---------------------------------------------------------------------------
 constexpr int kOneThreads = 160;
-constexpr int kOneMeans = 32;              // rows of the tile of means
-constexpr int kOneCols = 2 * kOneMeans;
+constexpr int kOneMeans = 32;              // rows of the tile of means, columns of tensor memory
 
 struct OneCtrl {
   uint64_t full;                           // per row tile: Q and means landed
@@ -599,7 +598,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
   }
   if (tid < kGateRows) reinterpret_cast<int32_t*>(c.cnt)[tid] = 0;
   if (warp == 0) {
-    tmem_alloc(smem_u32(&c.tmem_slot), (uint32_t)kOneCols);
+    tmem_alloc(smem_u32(&c.tmem_slot), (uint32_t)kOneMeans);
     tmem_relinquish();
   }
   pdl_wait();
@@ -611,12 +610,12 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
 
   if (warp == 4) {
     // row tile n of the CTA is tile blockIdx.x + n * gridDim.x of the grid, valid or not
-    uint32_t n = 0, m = 0;                             // row tiles, tiles with candidates
+    uint32_t n = 0;                                    // row tiles
     for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x, ++n) {
       const GateTile t = gate_tile(p, cu, ti, tiles_x, tokens_per_cta);
       const bool work = t.valid && t.max_cand > 0;
-      // Q, means and half of tensor memory are free once everybody has read the tile before: a thread that has
-      // is through with the one before that
+      // Q, means and tensor memory are free once everybody has read the tile before (c.tile and c.mean_ssq have two
+      // places: a thread that has read it is through with the tile before that)
       bool ok = n == 0 || mbar_wait(smem_u32(&c.read), (n - 1) & 1);
       if (lane == 0) {
         c.tile[n & 1] = t;
@@ -641,13 +640,12 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
           const uint32_t aQ = smem_u32(sQ), aB = smem_u32(sB);
 #pragma unroll
           for (int ks = 0; ks < D / 16; ++ks)
-            mma_ss(tmem + (m & 1) * kOneMeans, gate_desc(aQ + (ks >> 2) * kQBlockBytes + (ks & 3) * 32),
+            mma_ss(tmem, gate_desc(aQ + (ks >> 2) * kQBlockBytes + (ks & 3) * 32),
                    gate_desc(aB + (ks >> 2) * kOneMeans * 128 + (ks & 3) * 32), idesc, ks > 0);
           tc_commit(smem_u32(&c.mma_done));
         }
         __syncwarp();
       }
-      m += work;
       if (!__all_sync(0xffffffffu, ok)) break;         // the rows' threads run into their own bounded waits
     }
   } else {
@@ -696,7 +694,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
       tc_fence_after();
       uint32_t v[32];
       __syncwarp();
-      tmem_ld32(tmem + (m & 1) * kOneMeans + ((uint32_t)(warp * 32) << 16), v);
+      tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16), v);
       tmem_wait_ld();
       tc_fence_before();
       mbar_arrive(smem_u32(&c.read));                  // Q, means and the estimates have been read
@@ -782,7 +780,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
   if (ticket != nullptr) finish_scan<kOneThreads>(scan, ticket, reinterpret_cast<int*>(c.exact));
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tmem, (uint32_t)kOneCols);
+  if (warp == 0) tmem_dealloc(tmem, (uint32_t)kOneMeans);
 }
 
 // rows with more than 32 candidates, or lists longer than 32
@@ -1244,8 +1242,7 @@ cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, cons
   const int threads = one ? kOneThreads : kGateThreads;
   const int regs_per_cta = ((attr.numRegs + 7) / 8 * 8) * threads;
   if (regs_per_cta > 0 && resident > regs_per_sm / regs_per_cta) resident = regs_per_sm / regs_per_cta;
-  const int cols = one ? kOneCols : g.nt;
-  if (resident > 512 / cols) resident = 512 / cols;
+  if (resident > 512 / g.nt) resident = 512 / g.nt;
   if (resident < 1) resident = 1;
   int64_t grid = (int64_t)sms * resident;
   if (grid > n_tiles) grid = n_tiles;
