@@ -604,7 +604,9 @@ bwd_dq_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k,
     mbar_init(smem_u32(&c.kv_free), 1);
     for (int i = 0; i < kDqSlots; ++i) {
       mbar_init(smem_u32(&c.item_full[i]), 1);
-      mbar_init(smem_u32(&c.slot_free[i]), 4);               // the row warps of the item
+      // The row warps of the item, once its first S is there.  Behind that S are the other readers of the description: the MMA
+      // warp reads it in front of S, warps 2 and 3 before they arrive on row_full, which S waits for.
+      mbar_init(smem_u32(&c.slot_free[i]), 4);
     }
     c.abort = 0;
     c.n_routed = p.hist > 0 ? a.tile_prefix[p.lists] : 0;

@@ -1101,7 +1101,9 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
     mbar_init(smem_u32(&c.o_free), kTileM);
     for (int i = 0; i < kShortSlots; ++i) {
       mbar_init(smem_u32(&c.item_full[i]), 1);
-      mbar_init(smem_u32(&c.slot_free[i]), 4);                 // the softmax warps of the item
+      // The softmax warps of the item, once its first S is there.  Behind that S are the other readers of the description:
+      // the MMA warp reads it in front of Q.K^T, warps 6 and 7 before they arrive on q_full, which Q.K^T waits for.
+      mbar_init(smem_u32(&c.slot_free[i]), 4);
     }
     c.abort = 0;
     fence_barrier_init();

@@ -217,7 +217,8 @@ __device__ __forceinline__ void copy_rows_async(uint32_t tile, const __nv_bfloat
 }
 
 // One warp describes the items of the CTA ahead of everybody else: item m goes into slot m % kSlots of the
-// control block once the slot's item before has been let go by its readers (slot_free), and the
+// control block once the slot's item before has been let go by its readers (slot_free: every reader either arrives on it
+// or is ordered before one that does, which each kernel argues at its mbar_init), and the
 // end of the queue is published `kEnds` times (once per group of threads that takes the items in turn).
 // False when a wait gave up.  kRowIndex: row indices t * Hq + h are kept too.
 template <int kSlots, int kEnds, bool kReuse, bool kRowIndex, typename CtrlT>
