@@ -547,8 +547,11 @@ __device__ __forceinline__ void finish_scan(const ListScan& scan, int32_t* __res
 //   warp 4     walks the row tiles of the CTA: requests Q and means and issues the MMA as soon as every row has its
 //              norms and its estimates of the tile before in registers, while networks, decisions and stores go on
 //   warps 0-3  a thread per row.  The sorted keys stay in registers, and what they settle is decided there; a row with
-//              near-ties goes through a list in shared memory.  Every warp counts for itself: no barrier of
-//              the CTA in the loop, a warp may be a tile behind another.
+//              near-ties goes through a list in shared memory.  Every warp counts for itself and warp 4 adds the
+//              counts of a tile to the lists a tile later: no barrier of the CTA in the loop, a warp may be a tile
+//              behind another.  (Added by every warp for itself, four requests for one, and some 7 ns each for the 128-byte
+//              line of counters that all CTAs are at: 32768 x 32/8, 31 candidates, top-k 4 265 us, 162 this way; head
+//              dim 64, top-k 8 251, 150.)
 // Measured against the kernel below for these shapes, with the wait for the chunk means: 2 x 4096 tokens x 16 heads, 31
 // candidates 44 -> 40 us, at head dim 256 105 -> 91; 32768 x 32/8, 7 candidates 179 -> 152; a decode token on 32 chunks 24 -> 17.
 // (The few-lane score of near-ties alone, which the kernel below has too: 32768 x 32/8, 255 candidates 620 -> 573.)
@@ -563,7 +566,9 @@ struct OneCtrl {
   uint32_t tmem_slot;
   GateTile tile[2];
   int32_t mean_ssq[2][kGateRows / 32];     // largest squared norm of a mean, by the warps
-  int32_t cnt[kGateRows / 32][kOneMeans];  // rows of a warp's tile that selected a chunk
+  int32_t cnt[3][kGateRows / 32][kOneMeans];   // rows of a warp that selected a chunk; row tile n: place n % 3
+  int64_t cnt_list[3];                     // at the end: the list of the first chunk of cnt[place], < 0: nothing to add
+  int32_t cnt_lost[kGateRows / 32][kOneMeans]; // the same of a warp that a wait has given up in
   unsigned long long exact[kGateRows / 32][64];
 };
 
@@ -596,7 +601,8 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
     prefetch_tmap(&tmap_q);
     prefetch_tmap(&tmap_m);
   }
-  if (tid < kGateRows) reinterpret_cast<int32_t*>(c.cnt)[tid] = 0;
+  for (int i = tid; i < 3 * kGateRows; i += kOneThreads) reinterpret_cast<int32_t*>(c.cnt)[i] = 0;
+  if (tid < kGateRows) reinterpret_cast<int32_t*>(c.cnt_lost)[tid] = 0;
   if (warp == 0) {
     tmem_alloc(smem_u32(&c.tmem_slot), (uint32_t)kOneMeans);
     tmem_relinquish();
@@ -608,15 +614,30 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
   tc_fence_after();
   const uint32_t tmem = c.tmem_slot;
 
+  // counts of a tile into those of the lists (warp 4); `list` of its first chunk, < 0: nothing to add
+  auto add_counts = [&](int place, int64_t list) {
+    if (list < 0 || list_counts == nullptr) return;
+    int k = 0;
+#pragma unroll
+    for (int w = 0; w < kGateRows / 32; ++w) {
+      k += c.cnt[place][w][lane];
+      c.cnt[place][w][lane] = 0;
+    }
+    if (k > 0) atomicAdd(&list_counts[list + (int64_t)lane * p.Hkv], k);
+  };
   if (warp == 4) {
     // row tile n of the CTA is tile blockIdx.x + n * gridDim.x of the grid, valid or not
-    uint32_t n = 0;                                    // row tiles
+    uint32_t n = 0;
+    int place = 0;                                     // n % 3
+    int64_t list0 = -1, list1 = -1, list2 = -1;        // of tiles n, n - 1, n - 2: their counts are not added yet
     for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x, ++n) {
       const GateTile t = gate_tile(p, cu, ti, tiles_x, tokens_per_cta);
       const bool work = t.valid && t.max_cand > 0;
       // Q, means and tensor memory are free once everybody has read the tile before (c.tile and c.mean_ssq have two
       // places: a thread that has read it is through with the tile before that)
       bool ok = n == 0 || mbar_wait(smem_u32(&c.read), (n - 1) & 1);
+      if (!__all_sync(0xffffffffu, ok)) break;         // the rows' threads run into their own bounded waits
+      list0 = work ? (int64_t)t.b * p.mc * p.Hkv + t.hk : -1;
       if (lane == 0) {
         c.tile[n & 1] = t;
         const uint32_t bar = smem_u32(&c.full);
@@ -631,8 +652,14 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
           mbar_arrive(bar);
         }
       }
+      // Who has read tile n - 1 has counted tile n - 2.  Its place is that of tile n + 1, which is requested behind this.
+      add_counts(place == 2 ? 0 : place + 1, list2);
+      list2 = list1;
+      list1 = list0;
+      list0 = -1;
+      place = place == 2 ? 0 : place + 1;
       __syncwarp();
-      ok = mbar_wait(smem_u32(&c.full), n & 1) && ok;
+      ok = mbar_wait(smem_u32(&c.full), n & 1);
       if (work && __all_sync(0xffffffffu, ok)) {
         if (lane == 0) {
           tc_fence_after();
@@ -646,22 +673,30 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
         }
         __syncwarp();
       }
-      if (!__all_sync(0xffffffffu, ok)) break;         // the rows' threads run into their own bounded waits
+      if (!__all_sync(0xffffffffu, ok)) break;
+    }
+    if (lane == 0) {                                   // (list1, list2: of the last tile requested and the one before it)
+      c.cnt_list[place] = -1;
+      c.cnt_list[place == 0 ? 2 : place - 1] = list1;
+      c.cnt_list[place == 2 ? 0 : place + 1] = list2;
     }
   } else {
     const int row = tid;
     uint2* mylist = lists + (size_t)row * lstride;
-    uint32_t n = 0, m = 0;
+    uint32_t n = 0, m = 0;                             // row tiles, tiles with candidates
+    int place = 2;                                     // n % 3, from the loop's first statement on
+    bool lost = false;                                 // a wait gave up: the barriers say nothing any more
     for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x, ++n) {
-      bool failed = !mbar_wait(smem_u32(&c.full), n & 1);
-      failed = __any_sync(0xffffffffu, failed);
+      place = place == 2 ? 0 : place + 1;
+      bool failed = lost || !mbar_wait(smem_u32(&c.full), n & 1);
+      failed = lost = __any_sync(0xffffffffu, failed);
       const GateTile t = failed ? gate_tile(p, cu, ti, tiles_x, tokens_per_cta) : c.tile[n & 1];
       const int nrows = t.valid ? t.ntok * p.G : 0;
       const int slot0 = t.b * p.mc;
       const int tl = row / p.G, hl = row - tl * p.G;   // token and head of the row in the tile
       int32_t* dst = selected + (int64_t)(t.hk * p.G + hl) * p.Tq + (t.tok_lo - p.win_lo) + tl;
       if (!t.valid || t.max_cand <= 0) {               // nothing, or the first chunk of a sequence: nothing to select
-        mbar_arrive(smem_u32(&c.read));
+        if (!failed) mbar_arrive(smem_u32(&c.read));
         if (row < nrows)
           for (int r = 0; r < hist; ++r) dst[(int64_t)r * p.sel_rs] = -1;
         continue;
@@ -697,7 +732,9 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
       tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16), v);
       tmem_wait_ld();
       tc_fence_before();
-      mbar_arrive(smem_u32(&c.read));                  // Q, means and the estimates have been read
+      // Q, means and the estimates have been read.  (A thread whose wait gave up arrives no more, so that a phase is
+      // never complete without somebody: the others' waits give up in turn, and all rank the rows of this CTA exactly.)
+      if (!failed) mbar_arrive(smem_u32(&c.read));
 #pragma unroll
       for (int i = 0; i < 32; ++i)                     // order-preserving keys, position in the low bits: earlier wins ties
         v[i] = i < ncand ? (float_key(__uint_as_float(v[i])) & ~31u) | (uint32_t)(31 - i) : 0u;
@@ -756,6 +793,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
                             0.5f * eps2, means, stats);
         __syncwarp();
       }
+      int32_t* cnt = failed ? c.cnt_lost[warp] : c.cnt[place][warp];
       if (row < nrows) {
 #pragma unroll
         for (int r = 0; r < kW; ++r)
@@ -763,20 +801,24 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
             const uint32_t x = mode != 0 ? mylist[r].x : v[r] ? 31u - (v[r] & 31u) : 0xFFFFFFFFu;
             const int cc = x == 0xFFFFFFFFu ? -1 : (int)(x & kChunkMask);
             dst[(int64_t)r * p.sel_rs] = cc >= 0 ? slot0 + cc : -1;
-            if (cc >= 0 && list_counts != nullptr) atomicAdd(&c.cnt[warp][cc], 1);
+            if (cc >= 0 && list_counts != nullptr) atomicAdd(&cnt[cc], 1);
           }
       }
-      __syncwarp();
-      if (list_counts != nullptr) {
-        const int k = c.cnt[warp][lane];
+      lost = __any_sync(0xffffffffu, failed);
+      if (lost && list_counts != nullptr) {            // nobody else is told when these are complete
+        __syncwarp();
+        const int k = c.cnt_lost[warp][lane];
         if (k > 0) atomicAdd(&list_counts[(int64_t)(slot0 + lane) * p.Hkv + t.hk], k);
-        c.cnt[warp][lane] = 0;
+        c.cnt_lost[warp][lane] = 0;
       }
       __syncwarp();
     }
   }
 
   __syncwarp();
+  __syncthreads();                                     // everybody has counted
+  if (warp == 4)
+    for (int i = 0; i < 3; ++i) add_counts(i, c.cnt_list[i]);
   if (ticket != nullptr) finish_scan<kOneThreads>(scan, ticket, reinterpret_cast<int*>(c.exact));
   tc_fence_before();
   __syncthreads();
