@@ -214,6 +214,8 @@ constexpr int kQBlockBytes = 128 * 128;   // one [128 rows][64 dims] swizzled bl
 // floats per row of the score scratch, for the keys a network leaves (w) or, without one (0), all 32 of a step: an odd
 // number of 16-byte pieces, so that 16-byte stores are free of conflicts
 __host__ __device__ constexpr int scratch_stride(int w) { return (w > 0 ? w : 32) + 4; }
+// (rows of one step of 32 candidates have nothing to merge)
+__host__ __device__ constexpr bool has_scratch(int mc, int w) { return w == 0 || mc - 1 > 32; }
 
 __device__ __forceinline__ uint32_t float_key(float x) {      // routing.py:778-784
   const uint32_t b = __float_as_uint(x);
@@ -825,7 +827,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
   if (warp == 0) tmem_dealloc(tmem, (uint32_t)kOneMeans);
 }
 
-// rows with more than 32 candidates, or lists longer than 32
+// rows with more than 32 candidates, lists longer than 32, and what else gate_one() leaves
 // kW: width of the compare-exchange network (8, 16 or 32 >= list_len), 0: lists longer than 32 (min-heap)
 template <bool kHalf, int D, int kW>
 __global__ void __launch_bounds__(kGateThreads, kGateMinCtas<kW>)
@@ -844,8 +846,8 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
   unsigned char* sQ0 = smem;                                             // nbuf x kNBlk blocks [128][64]
   unsigned char* sB = sQ0 + (size_t)nbuf * kNBlk * kQBlockBytes;        // kNBlk blocks [nt][64]
   uint2* lists = reinterpret_cast<uint2*>(sB + (size_t)kNBlk * nt * 128);   // [128][lstride] {chunk, score bits}
-  float* scratch = reinterpret_cast<float*>(lists + (size_t)kGateRows * lstride);   // [128][scratch_stride]
-  GateCtrl& c = *reinterpret_cast<GateCtrl*>(scratch + kGateRows * scratch_stride(kW));
+  float* scratch = reinterpret_cast<float*>(lists + (size_t)kGateRows * lstride);   // [128][scratch_stride], absent when unused
+  GateCtrl& c = *reinterpret_cast<GateCtrl*>(scratch + (has_scratch(p.mc, kW) ? kGateRows * scratch_stride(kW) : 0));
   int32_t* cnt_s = reinterpret_cast<int32_t*>(&c + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1190,8 +1192,19 @@ struct GateLaunch {
 
 // Width of the network for a list, 0: none.
 inline int gate_network(int list_len) { return list_len <= 8 ? 8 : list_len <= 16 ? 16 : list_len <= 32 ? 32 : 0; }
-// At most 32 candidates a row, and a network for the list.
-inline bool gate_one(const Params& p) { return p.mc - 1 <= kOneMeans && p.hist + 1 <= 32; }
+// At most 32 candidates a row and a list of at most 8, or a network for the list and few row tiles.  The kernel for few
+// candidates saves latency of a row tile; with the wider networks it has three CTAs or fewer and keeps a row's whole list in
+// registers (spills), and once every SM has its tiles the other one is ahead.  Gating kernel, this / the other, head dim 128, 31 candidates:
+//   top-k 12  one new token 8.4 / 10.5 us, 700 24.1 / 24.0, 1500 31 / 30; 32768 x 16/4 206 / 163
+//   top-k 24  one new token 12.8 / 14.5 us, 64 24.4 / 24.4, 256 31.5 / 29.6; 32768 x 16/4 350 / 177
+// at head dim 64 the lines cross at 200 row tiles (top-k 24: 700 tokens x 16/4 24.4 / 24.8), at 256 at 12 (top-k 12: 8 tokens x 32/8
+// 21.2 / 22.6, 64 32.9 / 31.0; 32768 x 32/8 745 / 575, top-k 24 1113 / 660).  Lists of 8: 32768 x 16/4 119 / 127, one token 7.6 / 9.5.
+inline bool gate_one(const Params& p) {
+  if (p.mc - 1 > kOneMeans || p.hist + 1 > 32) return false;
+  if (p.hist + 1 <= 8) return true;
+  const int few = p.D == 64 || (p.D <= 128 && p.hist + 1 <= 16) ? 148 : 16;
+  return (int64_t)window_tiles(p, kGateRows / p.G) * p.Hkv * p.B <= few;
+}
 // Candidate tile, Q buffers, list length and shared memory of a launch: the combination that puts
 // the most CTAs on an SM (more warps hide the latency of the list updates), then the wider candidate
 // tile, then two Q buffers.  smem == 0: nothing fits.
@@ -1217,7 +1230,7 @@ GateLaunch gate_launch_config(const Params& p) {
     for (int nbuf = 2; nbuf >= 1; --nbuf) {
       const size_t smem = 1024 + (size_t)nbuf * nblk * kQBlockBytes + (size_t)nblk * nt * 128 +
                           (size_t)kGateRows * (list_len | 1) * sizeof(uint2) +
-                          (size_t)kGateRows * scratch_stride(w) * sizeof(float) + sizeof(GateCtrl) +
+                          (has_scratch(p.mc, w) ? (size_t)kGateRows * scratch_stride(w) * sizeof(float) : 0) + sizeof(GateCtrl) +
                           (cnt_in_smem ? (size_t)p.mc * sizeof(int32_t) : 0);
       if (smem > 227 * 1024) continue;
       int ctas = (int)((228 * 1024) / (smem + 1024));         // 1 KB per CTA is reserved by the system

@@ -181,20 +181,26 @@ def _adversarial_means(nchunks, hkv, d, dtype, g):
                                           (33, 2), (33, 8), (33, 9), (33, 16), (33, 17), (33, 31), (33, 32), (33, 33)])
 def test_at_most_32_candidates_ties_zeros_infinities(nchunks, topk, d, dtype):
     """The kernel for rows of at most 32 candidates (33 chunks), which decides in registers: every width of its
-    network (lists of 8, 16 and 32) from both sides, and with lists of 33 the other kernel.  Infinite and NaN scores
-    rank by their bits (NaN of positive sign here, above +inf), equal ones by the chunk."""
+    network (lists of 8, 16 and 32) from both sides, and with lists of 33 the other kernel.  A call of at most 16 row
+    tiles runs it at every width, a larger one the other kernel at widths where that is ahead.  Infinite and NaN
+    scores rank by their bits (NaN of positive sign here, above +inf), equal ones by the chunk."""
+    chunk = 8
+    _few_candidates([chunk * nchunks], 2, 1, nchunks, topk, d, dtype)
+    _few_candidates([chunk * nchunks, chunk - 1, chunk * (nchunks // 2) + 3], 4, 4, nchunks, topk, d, dtype)
+
+
+def _few_candidates(lens, hq, hkv, nchunks, topk, d, dtype):
+    chunk, slots = 8, len(lens) * nchunks
     g = torch.Generator().manual_seed(nchunks * 64 + topk)
-    chunk, hq, hkv = 8, 4, 2
-    lens = [chunk * nchunks, chunk - 1, chunk * (nchunks // 2) + 3]
     q = torch.randn(sum(lens), hq, d, generator=g).to(dtype)
     q[q == 0] = 1                                                             # (inf * 0)
-    for what, means in _adversarial_means(3 * nchunks, hkv, d, dtype, g):
+    for what, means in _adversarial_means(slots, hkv, d, dtype, g):
         _gate_with_means(q, means, lens, chunk, topk, hkv)
         if what.startswith("one ulp"):
             q0 = q.clone()
             q0[::3] = 0
             _gate_with_means(q0, means, lens, chunk, topk, hkv)
-    finite = (torch.randn(3 * nchunks, hkv, d, generator=g) * 0.5).to(dtype)
+    finite = (torch.randn(slots, hkv, d, generator=g) * 0.5).to(dtype)
     finite[finite == 0] = 1
     _gate_with_means(q, finite, lens, chunk, topk, hkv)
     for value in (float("inf"), float("nan")):
@@ -203,12 +209,14 @@ def test_at_most_32_candidates_ties_zeros_infinities(nchunks, topk, d, dtype):
         _gate_with_means(q1, finite, lens, chunk, topk, hkv)
 
 
-@pytest.mark.parametrize("topk", [5, 12, 24])
-def test_at_most_32_candidates_many_tiles_of_rows(topk):
+@pytest.mark.parametrize("d", [64, 96, 128, 256])
+@pytest.mark.parametrize("topk", [5, 8, 12, 24])
+def test_at_most_32_candidates_many_tiles_of_rows(topk, d):
     """Enough tiles of rows that every CTA takes several: tiles with and without candidates, tiles beyond the end of their
-    sequence and sequences shorter than a chunk follow one another in it."""
+    sequence and sequences shorter than a chunk follow one another in it.  (Lists of more than 8 run the kernel for
+    any number of candidates here, without its scratch for a second step of 32.)"""
     g = torch.Generator().manual_seed(topk)
-    chunk, hq, hkv, d = 8, 16, 4, 64
+    chunk, hq, hkv = 8, 16, 4
     lens = [(264, 3, 130, 7, 8, 9, 40, 1)[(i + i // 8) % 8] for i in range(56)]
     tiles = len(lens) * hkv * -(-264 // (128 // (hq // hkv)))
     assert tiles >= 3 * 148 * 4
