@@ -381,17 +381,25 @@ __host__ __device__ inline bool tc5_small_tiles(int head_dim, int chunk) { retur
 // Up to 1024 keys the halves of a 256-row tile still read K and V twice as often for less than the second CTA per SM
 // gives, whole call: 700 tokens behind 50021, 32/8 heads 197 -> 183 us, 64 behind them 120 -> 93, 1500 behind 20000
 // at head_dim 64 153 -> 148; 12001 x 16/2 753 -> 713; 5000 + 3000 x 8/1 164 -> 156; 32768 x 16 at 64 1977 -> 1805, 20000 x 16/4 at
-// 96 1323 -> 1222.  At head_dim 128, where an item's tiles are the largest, long calls lose (8 M partial rows, 32768 x 32/8,
-// top-k 8 4.63 -> 4.72 ms; 6 M, 65536 x 8, top-k 12 3.62 -> 3.66) and 1.9 M still gain (19456 x 32, top-k 3 1018 -> 998 us): the
-// line lies between.  At 2048 and 4096 keys all but a few lose (20000 x 8/4 759 -> 826).
-constexpr int kShortChunk = 512, kShortChunkFew = 1024;
-constexpr int64_t kShortFewRows = (int64_t)4 << 20;
+// 96 1323 -> 1222.  Long calls are another matter: back to back they run at the power limit, where the tensor work counts and
+// the tiles read twice cost more than the second CTA gives.  By partial rows, calls back to back for a second, chunk 1024:
+//   head_dim 128  1.9 M (19456 x 32) 1018 -> 998 us, 2.1 M (16384 x 16) 1112 -> 1116, 3.1 M (32768 x 32, top-k 3) 2203 -> 2236, 3.8 M
+//                 (20000 x 32, chunk 900) 2467 -> 2538, 4.2 M (16384 x 32/8) 2183 -> 2244, 8.4 M (32768 x 32/8) 4.63 -> 4.72 ms
+//   head_dim 96   4.2 M (32768 x 16) 2362 -> 2335, 8.4 M (65536 x 32/8, top-k 4) 5.10 -> 5.20 ms, 16.8 M 9.85 -> 9.97
+//   head_dim 64   16.8 M (65536 x 32) 8.31 -> 7.99 ms
+// With fewer key tiles an item longer calls gain: head_dim 128, 3.8 M, chunk 640 (30000 x 16/2) 1848 -> 1768 us, 4.2 M, chunk 768
+// (16384 x 32/4) 1962 -> 1963; head_dim 96, 16.8 M, chunk 700 8.63 -> 8.61 ms.  At 2048 and 4096 keys all but a few lose
+// (20000 x 8/4 759 -> 826).
+constexpr int kShortChunk = 512, kShortChunkMid = 768, kShortChunkFew = 1024;
+constexpr int64_t kShortFewRows = (int64_t)2 << 20, kShortMidRows = (int64_t)4 << 20;
 static_assert(kSmallChunk <= kShortChunk, "lists cut into 128 rows run the kernel of one-tile items");
 inline bool tc5_short_items(const Params& p) {
   if (p.D > 128) return false;
   if (p.Tq * p.G <= kTileRowsWide) return true;
   // (own-chunk items are counted in int32; a slot table that large stays with the 256-row kernel)
-  const bool few = p.C <= kShortChunkFew && (p.D < 128 || p.rows * p.NP <= kShortFewRows);
+  const bool mid = p.C <= kShortChunkMid;
+  const int64_t most = p.D == 64 || (mid && p.D == 96) ? INT64_MAX : mid || p.D == 96 ? kShortMidRows : kShortFewRows;
+  const bool few = p.C <= kShortChunkFew && p.rows * p.NP <= most;
   return (p.C <= kShortChunk || few) && (int64_t)p.slots * p.Hq * ((p.C + 127) / 128) < ((int64_t)1 << 30);
 }
 
