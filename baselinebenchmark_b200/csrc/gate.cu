@@ -392,7 +392,10 @@ struct GateLists {
 };
 // The warp ranks the rows of its lanes with mode != 0: 1 all n_surv entries of the list, 2 all ncand candidates, 3 the runs of
 // near-ties marked in the list.  The calling lane's row is `row` of the tile, at `qrow` in global memory; eps: its error bound.
-template <bool kHalf, int D>
+// kUnroll: 1 keeps the code short where few rows come here (32768 tokens, at most 32 candidates, lists of 8: gating kernel 117 -> 112 us,
+// head dim 256 552 -> 499; a decode step with a near-tie 60 -> 57 us, most of the difference the fetch of code that runs
+// once), 4 serves many (top-k 28 of 256 candidates at head dim 256, half of the rows: 1874 us, with 1 2056).
+template <bool kHalf, int D, int kUnroll>
 __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, const GateTile& t, const __nv_bfloat16* qrow,
                                           int row, int mode, int n_surv, int n_keep, int ncand, float eps,
                                           const __nv_bfloat16* __restrict__ means, int32_t* __restrict__ stats) {
@@ -416,6 +419,7 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
     if (r_mode == 3) {
       // runs of near-ties: one marked entry per lane (at most 32), exact keys, rank inside the run
       int cnt = 0, runs = 0, my_e = -1, my_run = 0;
+#pragma unroll kUnroll
       for (int e0 = 0; e0 < r_total; e0 += 32) {
         const int e = e0 + lane;
         const uint32_t x = e < r_total ? rlist[e].x : 0u;
@@ -442,6 +446,7 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
       // as many entries at a time as the warp has groups of lanes; entry i's score goes to lane i
       float e = 0.f;
       constexpr int kPer = 32 / kScoreLanes<D>;
+#pragma unroll kUnroll
       for (int i0 = 0; i0 < cnt; i0 += kPer) {
         const int mine = i0 + lane / kScoreLanes<D>;
         const uint32_t ec = __shfl_sync(0xffffffffu, cc, mine & 31);     // (past the last entry: a chunk scored in vain)
@@ -458,6 +463,7 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
         }
       }
       int rank = 0, first = my_e;
+#pragma unroll kUnroll
       for (int t2 = 0; t2 < cnt; ++t2) {
         const unsigned long long kt = __shfl_sync(0xffffffffu, key, t2);
         const int rt = __shfl_sync(0xffffffffu, my_run, t2), et = __shfl_sync(0xffffffffu, my_e, t2);
@@ -476,6 +482,7 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
     lx[lane + 32] = 0ull;
     __syncwarp();
     int viol = 0, ratio = 0;
+#pragma unroll kUnroll
     for (int base = 0; base < r_total; base += 32) {
       const int idx = base + lane;
       unsigned long long key = 0ull;
@@ -507,6 +514,7 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
       }
     }
     // the exact ranking replaces the chunk ids of the row's list
+#pragma unroll kUnroll
     for (int i = lane; i < hist; i += 32) {
       const unsigned long long key = i < r_keep ? lx[i] : 0ull;
       rlist[i].x = key ? (0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFull)) - (uint32_t)slot0 : 0xFFFFFFFFu;
@@ -552,8 +560,8 @@ __device__ __forceinline__ void finish_scan(const ListScan& scan, int32_t* __res
 //              near-ties goes through a list in shared memory.  Every warp counts for itself and warp 4 adds the
 //              counts of a tile to the lists a tile later: no barrier of the CTA in the loop, a warp may be a tile
 //              behind another.  (Added by every warp for itself, four requests for one, and some 7 ns each for the 128-byte
-//              line of counters that all CTAs are at: 32768 x 32/8, 31 candidates, top-k 4 265 us, 162 this way; head
-//              dim 64, top-k 8 251, 150.)
+//              line of counters that all CTAs are at: 32768 x 32/8, 31 candidates, top-k 4 208-265 us, 157 this way;
+//              head dim 64, top-k 8 195-251, 144.)
 // Measured against the kernel below for these shapes, with the wait for the chunk means: 2 x 4096 tokens x 16 heads, 31
 // candidates 44 -> 40 us, at head dim 256 105 -> 91; 32768 x 32/8, 7 candidates 179 -> 152; a decode token on 32 chunks 24 -> 17.
 // (The few-lane score of near-ties alone, which the kernel below has too: 32768 x 32/8, 255 candidates 620 -> 573.)
@@ -568,9 +576,8 @@ struct OneCtrl {
   uint32_t tmem_slot;
   GateTile tile[2];
   int32_t mean_ssq[2][kGateRows / 32];     // largest squared norm of a mean, by the warps
-  int32_t cnt[3][kGateRows / 32][kOneMeans];   // rows of a warp that selected a chunk; row tile n: place n % 3
-  int64_t cnt_list[3];                     // at the end: the list of the first chunk of cnt[place], < 0: nothing to add
-  int32_t cnt_lost[kGateRows / 32][kOneMeans]; // the same of a warp that a wait has given up in
+  int32_t cnt[4][kGateRows / 32][kOneMeans];   // rows of a warp that selected a chunk; row tile n: place n & 3
+  int64_t cnt_list[4];                     // at the end: the list of the first chunk of cnt[place], < 0: nothing to add
   unsigned long long exact[kGateRows / 32][64];
 };
 
@@ -603,8 +610,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
     prefetch_tmap(&tmap_q);
     prefetch_tmap(&tmap_m);
   }
-  for (int i = tid; i < 3 * kGateRows; i += kOneThreads) reinterpret_cast<int32_t*>(c.cnt)[i] = 0;
-  if (tid < kGateRows) reinterpret_cast<int32_t*>(c.cnt_lost)[tid] = 0;
+  for (int i = tid; i < 4 * kGateRows; i += kOneThreads) reinterpret_cast<int32_t*>(c.cnt)[i] = 0;
   if (warp == 0) {
     tmem_alloc(smem_u32(&c.tmem_slot), (uint32_t)kOneMeans);
     tmem_relinquish();
@@ -616,6 +622,8 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
   tc_fence_after();
   const uint32_t tmem = c.tmem_slot;
 
+  // (With the wider networks, whose calls have a row tile a CTA at most (gate_one), every warp adds its own counts.)
+  constexpr bool kDefer = kW == 8;
   // counts of a tile into those of the lists (warp 4); `list` of its first chunk, < 0: nothing to add
   auto add_counts = [&](int place, int64_t list) {
     if (list < 0 || list_counts == nullptr) return;
@@ -630,8 +638,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
   if (warp == 4) {
     // row tile n of the CTA is tile blockIdx.x + n * gridDim.x of the grid, valid or not
     uint32_t n = 0;
-    int place = 0;                                     // n % 3
-    int64_t list0 = -1, list1 = -1, list2 = -1;        // of tiles n, n - 1, n - 2: their counts are not added yet
+    int64_t list1 = -1, list2 = -1;                    // of tiles n - 1, n - 2: their counts are not added yet
     for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x, ++n) {
       const GateTile t = gate_tile(p, cu, ti, tiles_x, tokens_per_cta);
       const bool work = t.valid && t.max_cand > 0;
@@ -639,7 +646,6 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
       // places: a thread that has read it is through with the tile before that)
       bool ok = n == 0 || mbar_wait(smem_u32(&c.read), (n - 1) & 1);
       if (!__all_sync(0xffffffffu, ok)) break;         // the rows' threads run into their own bounded waits
-      list0 = work ? (int64_t)t.b * p.mc * p.Hkv + t.hk : -1;
       if (lane == 0) {
         c.tile[n & 1] = t;
         const uint32_t bar = smem_u32(&c.full);
@@ -654,12 +660,10 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
           mbar_arrive(bar);
         }
       }
-      // Who has read tile n - 1 has counted tile n - 2.  Its place is that of tile n + 1, which is requested behind this.
-      add_counts(place == 2 ? 0 : place + 1, list2);
+      // Who has read tile n - 1 has counted tile n - 2.  Its place is that of tile n + 2, which is requested behind this.
+      if (kDefer) add_counts((n + 2) & 3, list2);
       list2 = list1;
-      list1 = list0;
-      list0 = -1;
-      place = place == 2 ? 0 : place + 1;
+      list1 = work ? (int64_t)t.b * p.mc * p.Hkv + t.hk : -1;
       __syncwarp();
       ok = mbar_wait(smem_u32(&c.full), n & 1);
       if (work && __all_sync(0xffffffffu, ok)) {
@@ -675,21 +679,16 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
         }
         __syncwarp();
       }
-      if (!__all_sync(0xffffffffu, ok)) break;
+      if (!__all_sync(0xffffffffu, ok)) { ++n; break; }
     }
-    if (lane == 0) {                                   // (list1, list2: of the last tile requested and the one before it)
-      c.cnt_list[place] = -1;
-      c.cnt_list[place == 0 ? 2 : place - 1] = list1;
-      c.cnt_list[place == 2 ? 0 : place + 1] = list2;
-    }
+    if (kDefer && lane < 4)                            // (tile n - 1 is the last one requested)
+      c.cnt_list[(n + lane) & 3] = lane == 3 ? list1 : lane == 2 ? list2 : -1;
   } else {
     const int row = tid;
     uint2* mylist = lists + (size_t)row * lstride;
     uint32_t n = 0, m = 0;                             // row tiles, tiles with candidates
-    int place = 2;                                     // n % 3, from the loop's first statement on
-    bool lost = false;                                 // a wait gave up: the barriers say nothing any more
+    bool lost = false;                                 // a wait gave up: no copies or estimates any more, from this tile on
     for (int ti = blockIdx.x; ti < n_tiles; ti += gridDim.x, ++n) {
-      place = place == 2 ? 0 : place + 1;
       bool failed = lost || !mbar_wait(smem_u32(&c.full), n & 1);
       failed = lost = __any_sync(0xffffffffu, failed);
       const GateTile t = failed ? gate_tile(p, cu, ti, tiles_x, tokens_per_cta) : c.tile[n & 1];
@@ -791,11 +790,11 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
             mylist[i] = make_uint2(v[i] ? (31u - (v[i] & 31u)) | ((tied >> i) & 1u ? kTied : 0u) | ((first >> i) & 1u ? kRunStart : 0u)
                                         : 0xFFFFFFFFu, v[i]);
         __syncwarp();
-        rank_rows<kHalf, D>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand,
-                            0.5f * eps2, means, stats);
+        rank_rows<kHalf, D, 1>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand,
+                               0.5f * eps2, means, stats);
         __syncwarp();
       }
-      int32_t* cnt = failed ? c.cnt_lost[warp] : c.cnt[place][warp];
+      const bool count = list_counts != nullptr && !(kDefer && lost);
       if (row < nrows) {
 #pragma unroll
         for (int r = 0; r < kW; ++r)
@@ -803,24 +802,29 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
             const uint32_t x = mode != 0 ? mylist[r].x : v[r] ? 31u - (v[r] & 31u) : 0xFFFFFFFFu;
             const int cc = x == 0xFFFFFFFFu ? -1 : (int)(x & kChunkMask);
             dst[(int64_t)r * p.sel_rs] = cc >= 0 ? slot0 + cc : -1;
-            if (cc >= 0 && list_counts != nullptr) atomicAdd(&cnt[cc], 1);
+            if (cc >= 0 && count) atomicAdd(&c.cnt[n & 3][warp][cc], 1);
           }
+        // Nobody is told when the counts of a tile that was not seen to land are complete.  (Those of the last two
+        // requested tiles are added at the end, and without this warp's arrivals no more than one is requested.)
+        if (kDefer && lost && list_counts != nullptr && ncand > 0)
+          for (int r = 0; r < n_keep; ++r)
+            atomicAdd(&list_counts[(int64_t)(slot0 + (int)(mylist[r].x & kChunkMask)) * p.Hkv + t.hk], 1);
       }
       lost = __any_sync(0xffffffffu, failed);
-      if (lost && list_counts != nullptr) {            // nobody else is told when these are complete
-        __syncwarp();
-        const int k = c.cnt_lost[warp][lane];
-        if (k > 0) atomicAdd(&list_counts[(int64_t)(slot0 + lane) * p.Hkv + t.hk], k);
-        c.cnt_lost[warp][lane] = 0;
-      }
       __syncwarp();
+      if (!kDefer && list_counts != nullptr) {
+        const int k = c.cnt[n & 3][warp][lane];
+        if (k > 0) atomicAdd(&list_counts[(int64_t)(slot0 + lane) * p.Hkv + t.hk], k);
+        c.cnt[n & 3][warp][lane] = 0;
+        __syncwarp();
+      }
     }
   }
 
   __syncwarp();
-  __syncthreads();                                     // everybody has counted
-  if (warp == 4)
-    for (int i = 0; i < 3; ++i) add_counts(i, c.cnt_list[i]);
+  if (kDefer) __syncthreads();                         // everybody has counted
+  if (kDefer && warp == 4)
+    for (int i = 0; i < 4; ++i) add_counts(i, c.cnt_list[i]);
   if (ticket != nullptr) finish_scan<kOneThreads>(scan, ticket, reinterpret_cast<int*>(c.exact));
   tc_fence_before();
   __syncthreads();
@@ -1150,7 +1154,7 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
     }
     __syncwarp();                                             // the marks are visible to the warp
     const __nv_bfloat16* qrow = q + (int64_t)(t.tok_lo + row / p.G - p.win_lo) * p.sq_t + (int64_t)(t.hk * p.G + row % p.G) * p.sq_h;
-    rank_rows<kHalf, D>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand, eps, means,
+    rank_rows<kHalf, D, 4>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand, eps, means,
                         stats);
     // selected[rank][head][token]: every thread stores the chunks of its own row (its list was
     // written by its own warp); neighbouring lanes are neighbouring heads, then tokens
@@ -1198,7 +1202,7 @@ inline int gate_network(int list_len) { return list_len <= 8 ? 8 : list_len <= 1
 //   top-k 12  one new token 8.4 / 10.5 us, 700 24.1 / 24.0, 1500 31 / 30; 32768 x 16/4 206 / 163
 //   top-k 24  one new token 12.8 / 14.5 us, 64 24.4 / 24.4, 256 31.5 / 29.6; 32768 x 16/4 350 / 177
 // at head dim 64 the lines cross at 200 row tiles (top-k 24: 700 tokens x 16/4 24.4 / 24.8), at 256 at 12 (top-k 12: 8 tokens x 32/8
-// 21.2 / 22.6, 64 32.9 / 31.0; 32768 x 32/8 745 / 575, top-k 24 1113 / 660).  Lists of 8: 32768 x 16/4 119 / 127, one token 7.6 / 9.5.
+// 21.2 / 22.6, 64 32.9 / 31.0; 32768 x 32/8 745 / 575, top-k 24 1113 / 660).  Lists of 8: 32768 x 16/4 112 / 127, one token 7.6 / 9.5.
 inline bool gate_one(const Params& p) {
   if (p.mc - 1 > kOneMeans || p.hist + 1 > 32) return false;
   if (p.hist + 1 <= 8) return true;
