@@ -392,10 +392,10 @@ struct GateLists {
 };
 // The warp ranks the rows of its lanes with mode != 0: 1 all n_surv entries of the list, 2 all ncand candidates, 3 the runs of
 // near-ties marked in the list.  The calling lane's row is `row` of the tile, at `qrow` in global memory; eps: its error bound.
-// kUnroll: 1 keeps the code short where few rows come here (32768 tokens, at most 32 candidates, lists of 8: gating kernel 117 -> 112 us,
-// head dim 256 552 -> 499; a decode step with a near-tie 60 -> 57 us, most of the difference the fetch of code that runs
-// once), 4 serves many (top-k 28 of 256 candidates at head dim 256, half of the rows: 1874 us, with 1 2056).
-template <bool kHalf, int D, int kUnroll>
+// kShort: the loops over the entries of a row are not unrolled.  Code that few rows come to is mostly fetched: 32768 x 32/8, at most 32
+// candidates, lists of 8: gating kernel 218 -> 214 us, head dim 256 552 -> 522, a decode step with a near-tie 60 -> 58.
+// Where many rows do, it costs (top-k 28 of 256 candidates at head dim 256, half of the rows: 1936 -> 2056).
+template <bool kHalf, int D, bool kShort>
 __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, const GateTile& t, const __nv_bfloat16* qrow,
                                           int row, int mode, int n_surv, int n_keep, int ncand, float eps,
                                           const __nv_bfloat16* __restrict__ means, int32_t* __restrict__ stats) {
@@ -419,7 +419,6 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
     if (r_mode == 3) {
       // runs of near-ties: one marked entry per lane (at most 32), exact keys, rank inside the run
       int cnt = 0, runs = 0, my_e = -1, my_run = 0;
-#pragma unroll kUnroll
       for (int e0 = 0; e0 < r_total; e0 += 32) {
         const int e = e0 + lane;
         const uint32_t x = e < r_total ? rlist[e].x : 0u;
@@ -446,13 +445,18 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
       // as many entries at a time as the warp has groups of lanes; entry i's score goes to lane i
       float e = 0.f;
       constexpr int kPer = 32 / kScoreLanes<D>;
-#pragma unroll kUnroll
-      for (int i0 = 0; i0 < cnt; i0 += kPer) {
+      auto score = [&](int i0) {
         const int mine = i0 + lane / kScoreLanes<D>;
         const uint32_t ec = __shfl_sync(0xffffffffu, cc, mine & 31);     // (past the last entry: a chunk scored in vain)
         const float score = contract_score_group<kHalf, D>(r_q, means + ((int64_t)(slot0 + (int)ec) * p.Hkv + t.hk) * D);
         const float got = __shfl_sync(0xffffffffu, score, ((lane - i0) * kScoreLanes<D>) & 31);
         if (lane >= i0 && lane < i0 + kPer) e = got;
+      };
+      if constexpr (kShort) {
+#pragma unroll 1
+        for (int i0 = 0; i0 < cnt; i0 += kPer) score(i0);
+      } else {
+        for (int i0 = 0; i0 < cnt; i0 += kPer) score(i0);
       }
       if (lane < cnt) {
         key = ((unsigned long long)float_key(e) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(slot0 + (int)cc));
@@ -463,14 +467,19 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
         }
       }
       int rank = 0, first = my_e;
-#pragma unroll kUnroll
-      for (int t2 = 0; t2 < cnt; ++t2) {
+      auto compare = [&](int t2) {
         const unsigned long long kt = __shfl_sync(0xffffffffu, key, t2);
         const int rt = __shfl_sync(0xffffffffu, my_run, t2), et = __shfl_sync(0xffffffffu, my_e, t2);
         if (lane < cnt && rt == my_run) {
           rank += kt > key;
           first = min(first, et);
         }
+      };
+      if constexpr (kShort) {
+#pragma unroll 1
+        for (int t2 = 0; t2 < cnt; ++t2) compare(t2);
+      } else {
+        for (int t2 = 0; t2 < cnt; ++t2) compare(t2);
       }
       __syncwarp();
       if (lane < cnt) rlist[first + rank].x = cc;          // a run occupies consecutive places; marks are cleared
@@ -482,7 +491,6 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
     lx[lane + 32] = 0ull;
     __syncwarp();
     int viol = 0, ratio = 0;
-#pragma unroll kUnroll
     for (int base = 0; base < r_total; base += 32) {
       const int idx = base + lane;
       unsigned long long key = 0ull;
@@ -514,7 +522,6 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
       }
     }
     // the exact ranking replaces the chunk ids of the row's list
-#pragma unroll kUnroll
     for (int i = lane; i < hist; i += 32) {
       const unsigned long long key = i < r_keep ? lx[i] : 0ull;
       rlist[i].x = key ? (0xFFFFFFFFu - (uint32_t)(key & 0xFFFFFFFFull)) - (uint32_t)slot0 : 0xFFFFFFFFu;
@@ -560,8 +567,8 @@ __device__ __forceinline__ void finish_scan(const ListScan& scan, int32_t* __res
 //              near-ties goes through a list in shared memory.  Every warp counts for itself and warp 4 adds the
 //              counts of a tile to the lists a tile later: no barrier of the CTA in the loop, a warp may be a tile
 //              behind another.  (Added by every warp for itself, four requests for one, and some 7 ns each for the 128-byte
-//              line of counters that all CTAs are at: 32768 x 32/8, 31 candidates, top-k 4 208-265 us, 157 this way;
-//              head dim 64, top-k 8 195-251, 144.)
+//              line of counters that all CTAs are at: 32768 x 32/8, 31 candidates, top-k 4 203-265 us, 161 this way;
+//              head dim 64, top-k 8 195-251, 149.)
 // Measured against the kernel below for these shapes, with the wait for the chunk means: 2 x 4096 tokens x 16 heads, 31
 // candidates 44 -> 40 us, at head dim 256 105 -> 91; 32768 x 32/8, 7 candidates 179 -> 152; a decode token on 32 chunks 24 -> 17.
 // (The few-lane score of near-ties alone, which the kernel below has too: 32768 x 32/8, 255 candidates 620 -> 573.)
@@ -790,8 +797,8 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
             mylist[i] = make_uint2(v[i] ? (31u - (v[i] & 31u)) | ((tied >> i) & 1u ? kTied : 0u) | ((first >> i) & 1u ? kRunStart : 0u)
                                         : 0xFFFFFFFFu, v[i]);
         __syncwarp();
-        rank_rows<kHalf, D, 1>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand,
-                               0.5f * eps2, means, stats);
+        rank_rows<kHalf, D, true>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand,
+                                  0.5f * eps2, means, stats);
         __syncwarp();
       }
       const bool count = list_counts != nullptr && !(kDefer && lost);
@@ -1154,7 +1161,7 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
     }
     __syncwarp();                                             // the marks are visible to the warp
     const __nv_bfloat16* qrow = q + (int64_t)(t.tok_lo + row / p.G - p.win_lo) * p.sq_t + (int64_t)(t.hk * p.G + row % p.G) * p.sq_h;
-    rank_rows<kHalf, D, 4>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand, eps, means,
+    rank_rows<kHalf, D, false>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand, eps, means,
                         stats);
     // selected[rank][head][token]: every thread stores the chunks of its own row (its list was
     // written by its own warp); neighbouring lanes are neighbouring heads, then tokens
@@ -1202,7 +1209,7 @@ inline int gate_network(int list_len) { return list_len <= 8 ? 8 : list_len <= 1
 //   top-k 12  one new token 8.4 / 10.5 us, 700 24.1 / 24.0, 1500 31 / 30; 32768 x 16/4 206 / 163
 //   top-k 24  one new token 12.8 / 14.5 us, 64 24.4 / 24.4, 256 31.5 / 29.6; 32768 x 16/4 350 / 177
 // at head dim 64 the lines cross at 200 row tiles (top-k 24: 700 tokens x 16/4 24.4 / 24.8), at 256 at 12 (top-k 12: 8 tokens x 32/8
-// 21.2 / 22.6, 64 32.9 / 31.0; 32768 x 32/8 745 / 575, top-k 24 1113 / 660).  Lists of 8: 32768 x 16/4 112 / 127, one token 7.6 / 9.5.
+// 21.2 / 22.6, 64 32.9 / 31.0; 32768 x 32/8 745 / 575, top-k 24 1113 / 660).  Lists of 8: 32768 x 16/4 117 / 127, one token 7.6 / 9.5.
 inline bool gate_one(const Params& p) {
   if (p.mc - 1 > kOneMeans || p.hist + 1 > 32) return false;
   if (p.hist + 1 <= 8) return true;
