@@ -849,8 +849,7 @@ cudaError_t launch_bwd_dq_tc5(const Params& p, const __nv_bfloat16* q, const __n
   if (bwd_dq_short_items(p)) {
     DqShortArgs sa;
     sa.a = args;
-    sa.iq = ItemQueue{cu, list_counts, list_offsets, tile_prefix, row_list, work_counter,
-                      short_batch(p, sms, false), 0, 0};
+    sa.iq = item_queue(p, cu, list_counts, list_offsets, tile_prefix, row_list, work_counter, short_batch(p, sms, false), false, 0);
     if (!make_kv_map(&mk, p.fp16 != 0, p.D, k, p.T, p.Hkv, p.sk_t, p.sk_h, kDqShortChunk) ||
         !make_kv_map(&mv, p.fp16 != 0, p.D, v, p.T, p.Hkv, p.sv_t, p.sv_h, kDqShortChunk))
       return cudaErrorNotSupported;

@@ -403,6 +403,14 @@ inline bool tc5_short_items(const Params& p) {
   return (p.C <= kShortChunk || few) && (int64_t)p.slots * p.Hq * ((p.C + 127) / 128) < ((int64_t)1 << 30);
 }
 
+// Chunks of at most 128 keys, one key tile an item, run a kernel that keeps several items of an SM in flight; windows of at most
+// 128 rows per kv head (few items, whose own-chunk ones cover the heads of a group) stay with the one for short items, and so does
+// a q of more than 64 GB (row offsets are 32 bits there, in 16-byte pieces).
+inline bool tc5_one_tile(const Params& p) {
+  return tc5_short_items(p) && p.C <= 128 && p.Tq * p.G > kTileRowsWide &&
+         (p.Tq - 1) * p.sq_t + (p.Hq - 1) * p.sq_h < ((int64_t)1 << 35);
+}
+
 cudaError_t launch_attend_mma(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* k,
                               const __nv_bfloat16* v, const int32_t* cu, const int32_t* list_counts,
                               const int32_t* list_offsets, const int32_t* tile_prefix,
@@ -413,6 +421,10 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
                               const int32_t* list_offsets, const int32_t* tile_prefix,
                               const int32_t* row_list, __half* partial_out, float2* partial_lse,
                               int32_t* work_counter, int32_t* status, cudaStream_t st);
+cudaError_t launch_attend_one_tc5(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v,
+                                  const int32_t* cu, const int32_t* list_counts, const int32_t* list_offsets,
+                                  const int32_t* tile_prefix, const int32_t* row_list, __half* partial_out,
+                                  float2* partial_lse, int32_t* work_counter, int32_t* status, int sms, cudaStream_t st);
 
 cudaError_t launch_bounded_wait_probe(int32_t* status, unsigned long long limit_ns, cudaStream_t st);
 

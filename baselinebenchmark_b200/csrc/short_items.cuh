@@ -1,6 +1,6 @@
 // Work items of one 128-row tile: the description of an item and the walk through the queue of items,
 // shared by the kernels whose roles run through a flat stream of items (the forward's kernels for
-// short items and for head dim 256, and the dq kernel for short chunks).
+// one-tile and short items and for head dim 256, and the dq kernel for short chunks).
 #pragma once
 
 #include "common.cuh"
@@ -26,23 +26,42 @@ __device__ __forceinline__ void fill_prefix_cache(CtrlT& c, const int32_t* __res
   const int n = (int)(lists >> shift) + 1;                   // samples 0, 2^shift, ..., the last one <= lists
   for (int i = threadIdx.x; i < n; i += nthreads) c.prefix_cache[i] = tile_prefix[(int64_t)i << shift];
 }
-// last l in [0, lists) with tile_prefix[l] <= i (i is a routed item: tile_prefix[lists] > i)
+// last k in [0, n) with at(k) <= i, at rising and at(0) <= i: 32 places a round, one for each lane of the (whole) warp
+template <typename F>
+__device__ __forceinline__ int search_warp(int n, int i, F&& at) {
+  const int lane = threadIdx.x & 31;
+  int lo = 0;
+  while (n > 1) {
+    const int step = (n + 31) >> 5, k = lane * step;
+    const int m = __popc(__ballot_sync(0xffffffffu, k < n && at(lo + k) <= i)) - 1;
+    lo += m * step;
+    n = min(step, n - m * step);
+  }
+  return lo;
+}
+// last l in [0, lists) with tile_prefix[l] <= i (i is a routed item: tile_prefix[lists] > i); executed by a whole warp.
+// (Halving took eleven dependent reads where this takes two or three: with several items of an SM in flight the warp that
+// describes them was what the others waited for.)
 template <typename CtrlT>
 __device__ __forceinline__ int find_list(const CtrlT& c, const int32_t* __restrict__ tile_prefix, int64_t lists, int i) {
   const int shift = prefix_shift(lists, CtrlT::kPrefix);
-  int lo = 0, hi = (int)(lists >> shift) + 1;                // samples: last k with cache[k] <= i
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (c.prefix_cache[mid] <= i) lo = mid; else hi = mid;
-  }
-  int l = lo << shift;
-  int r = min(l + (1 << shift), (int)lists);                 // tile_prefix[r] > i, or r == lists
-  while (r - l > 1) {
-    const int mid = (l + r) >> 1;
-    if (__ldg(tile_prefix + mid) <= i) l = mid; else r = mid;
-  }
-  return l;
+  const int l = search_warp((int)(lists >> shift) + 1, i, [&](int k) { return c.prefix_cache[k]; }) << shift;
+  // tile_prefix[l + 2^shift] > i, or the lists end before
+  return l + search_warp(min(1 << shift, (int)lists - l), i, [&](int k) { return __ldg(tile_prefix + l + k); });
 }
+
+// x / d for x < 2^31 as a product: umulhi(2 x, mul) >> shift, with mul = ceil(2^(31 + shift) / d) and 2^shift >= d.  mul d exceeds
+// 2^(31 + shift) by less than d, and x times that stays below 2^(31 + shift): the quotient is never one too large.
+struct FastDiv {
+  uint32_t mul, shift;
+};
+inline FastDiv fast_div(int64_t d) {
+  FastDiv f{0, 0};
+  while ((1ll << f.shift) < d) ++f.shift;
+  f.mul = (uint32_t)(((1ull << (31 + f.shift)) + (uint64_t)d - 1) / (uint64_t)d);
+  return f;
+}
+__device__ __forceinline__ int operator/(int x, const FastDiv& f) { return (int)(__umulhi(2u * (uint32_t)x, f.mul) >> f.shift); }
 
 // Where the items come from.
 struct ItemQueue {
@@ -55,7 +74,14 @@ struct ItemQueue {
   int32_t batch;                           // items a CTA draws at a time
   int32_t grouped;                         // own-chunk items cover the heads of a group (short windows)
   int32_t tile_shift;                      // 1: the tiles of tile_prefix are 256 rows, two items each
+  FastDiv by_np, by_hq, by_hkv, by_mc, by_g;
 };
+inline ItemQueue item_queue(const Params& p, const int32_t* cu, const int32_t* list_counts, const int32_t* list_offsets,
+                            const int32_t* tile_prefix, const int32_t* row_list, int32_t* work_counter, int batch, bool grouped,
+                            int tile_shift) {
+  return ItemQueue{cu, list_counts, list_offsets, tile_prefix, row_list, work_counter, batch, grouped, tile_shift,
+                   fast_div(p.NP), fast_div(p.Hq), fast_div(p.Hkv), fast_div(p.mc), fast_div(p.G)};
+}
 // A CTA draws several items at a time, so that row tiles of one list follow one another on it (K and V
 // stay in place), but at most an eighth of its share of the launch, for the balance.
 inline int short_batch(const Params& p, int ctas, bool grouped) {
@@ -78,16 +104,21 @@ struct ShortItem {
 // Walks the items a CTA draws; executed by the whole describing warp.
 struct ShortQueue {
   int cur, end;                            // items of the current draw left: [cur, end)
+  int ahead;                               // lane 0: the draw behind it (short_pick<true>)
   int list, list_first, list_end;          // list of the last routed item and the items it covers
   int list_off, list_count, kv_tok0, kv_head;
 };
-
-// The next item: its rows of this lane (4 * lane ... + 3) in `ent` (-1: none, behind the last row), their
-// element offsets in q in `qoff`, its description in `it`.
 template <typename CtrlT>
-__device__ __forceinline__ void short_next(const Params& p, const ItemQueue& a, CtrlT& c, ShortQueue& w, ShortItem& it,
-                                           int& kv_tok0, int& kv_head, int (&ent)[4], int64_t (&qoff)[4]) {
-  const int lane = threadIdx.x & 31;
+__device__ __forceinline__ int short_draw(const ItemQueue& a, const CtrlT& c) {
+  return (threadIdx.x & 31) != 0 ? 0 : c.abort ? 0x3fffffff : atomicAdd(a.work_counter, 1);
+}
+
+// The next item: its description in `it`, its first key token and kv head, and where its rows are: from row_list[rows_at]
+// on, or (own chunk) query tokens of the window from rows_at on, heads from `head` on.
+// kDrawAhead: the draw behind the one in hand is under way (w.ahead is set at the start), so that its latency is not waited for.
+template <bool kDrawAhead, typename CtrlT>
+__device__ __forceinline__ void short_pick(const Params& p, const ItemQueue& a, CtrlT& c, ShortQueue& w, ShortItem& it,
+                                           int& kv_tok0, int& kv_head, int& rows_at, int& head) {
   const int n_routed = c.n_routed, n_items = c.n_items;
   it.done = 1;
   it.nrows = 0;
@@ -97,13 +128,13 @@ __device__ __forceinline__ void short_next(const Params& p, const ItemQueue& a, 
   it.group = 1;
   kv_tok0 = 0;
   kv_head = 0;
-#pragma unroll
-  for (int u = 0; u < 4; ++u) { ent[u] = -1; qoff[u] = 0; }
+  rows_at = 0;
+  head = 0;
   for (;;) {
     if (w.cur >= w.end) {
-      int idx = 0;
-      if (lane == 0) idx = c.abort ? 0x3fffffff : atomicAdd(a.work_counter, 1);
-      idx = __shfl_sync(0xffffffffu, idx, 0);
+      const int mine = kDrawAhead ? w.ahead : short_draw(a, c);
+      if (kDrawAhead) w.ahead = short_draw(a, c);
+      const int idx = __shfl_sync(0xffffffffu, mine, 0);
       // Draws of `batch` items, and of single ones for the last two of every CTA: with a whole batch drawn last, some
       // CTAs worked three items longer than others.  Against batches to the end: dense stage of 2 x 4096 tokens x 16
       // heads 127.3 -> 125.9 us, at head dim 256 290 -> 281; 8191 x 16/4 122.5 -> 118.
@@ -117,8 +148,8 @@ __device__ __forceinline__ void short_next(const Params& p, const ItemQueue& a, 
       const int cut = idx >> a.tile_shift;                    // tile of tile_prefix
       if (cut < w.list_first || cut >= w.list_end) {
         const int l = find_list(c, a.tile_prefix, p.lists, cut);
-        const int slot = l / p.Hkv;
-        const int b = slot / p.mc, j = slot - b * p.mc;
+        const int slot = l / a.by_hkv;
+        const int b = slot / a.by_mc, j = slot - b * p.mc;
         w.list = l;
         w.list_first = __ldg(a.tile_prefix + l);
         w.list_end = __ldg(a.tile_prefix + l + 1);
@@ -133,32 +164,25 @@ __device__ __forceinline__ void short_next(const Params& p, const ItemQueue& a, 
       it.kv_len = p.C;
       kv_tok0 = w.kv_tok0;
       kv_head = w.kv_head;
-      const int32_t* rows = a.row_list + w.list_off + tile * kTileRowsWide + 4 * lane;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (4 * lane + u < it.nrows) ent[u] = __ldg(rows + u);
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (ent[u] >= 0) {
-          const uint32_t row = (uint32_t)ent[u] / (uint32_t)p.NP;
-          const uint32_t t = row / (uint32_t)p.Hq;
-          const uint32_t h = row - t * (uint32_t)p.Hq;
-          qoff[u] = (int64_t)t * p.sq_t + (int64_t)h * p.sq_h;
-        }
+      rows_at = w.list_off + tile * kTileRowsWide;
       break;
     }
     // own chunk: rows are (token, head) pairs, `group` heads per token
     const int g = a.grouped ? p.G : 1;
-    const int units = p.Hq / g;
+    const int units = a.grouped ? p.Hkv : p.Hq;
     // grouped: a slot's part of the window is one item
     const int tiles_per_chunk = a.grouped ? 1 : (p.C + kTileRowsWide - 1) / kTileRowsWide;
     const int per_tile = c.own.n * units;
     int i = idx - n_routed;
-    const int ti = tiles_per_chunk - 1 - i / per_tile;        // longest tiles first
-    i -= (i / per_tile) * per_tile;
-    const int slot = c.own.lo + i / units;
-    const int head = (i - (slot - c.own.lo) * units) * g;
-    const int b = slot / p.mc, j = slot - b * p.mc;
+    int ti = 0;
+    if (tiles_per_chunk > 1) {
+      const int x = i / per_tile;
+      ti = tiles_per_chunk - 1 - x;                           // longest tiles first
+      i -= x * per_tile;
+    }
+    const int unit = i / (a.grouped ? a.by_hkv : a.by_hq), slot = c.own.lo + unit;
+    head = (i - unit * units) * g;
+    const int b = slot / a.by_mc, j = slot - b * p.mc;
     const Slot s = slot_of(a.cu, b, j, p.C);
     const int tile0 = s.start + ti * kTileRowsWide;
     const int lo = max(tile0, p.win_lo);
@@ -170,19 +194,50 @@ __device__ __forceinline__ void short_next(const Params& p, const ItemQueue& a, 
     it.tok_rel = lo - s.start;
     it.kv_len = hi - s.start;
     kv_tok0 = s.start;
-    kv_head = head / p.G;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int r = 4 * lane + u;
-      if (r < it.nrows) {
-        const int t = lo - p.win_lo + r / g, h = head + r % g;
-        ent[u] = (int32_t)(((int64_t)t * p.Hq + h) * p.NP);
-        qoff[u] = (int64_t)t * p.sq_t + (int64_t)h * p.sq_h;
-      }
-    }
+    kv_head = head / a.by_g;
+    rows_at = lo - p.win_lo;
     break;
   }
   it.done = 0;
+}
+
+// Element offset in q of the row of an entry id (t * Hq + h) * NP + rank.
+__device__ __forceinline__ int64_t entry_qoff(const Params& p, const ItemQueue& a, int entry) {
+  const int row = entry / a.by_np, t = row / a.by_hq;
+  return (int64_t)t * p.sq_t + (int64_t)(row - t * p.Hq) * p.sq_h;
+}
+
+// The next item with its rows: those of this lane (4 * lane ... + 3) in `ent` (-1: none, behind the last row), their
+// element offsets in q in `qoff`.
+template <typename CtrlT>
+__device__ __forceinline__ void short_next(const Params& p, const ItemQueue& a, CtrlT& c, ShortQueue& w, ShortItem& it,
+                                           int& kv_tok0, int& kv_head, int (&ent)[4], int64_t (&qoff)[4]) {
+  const int lane = threadIdx.x & 31;
+  int rows_at, head;
+  short_pick<false>(p, a, c, w, it, kv_tok0, kv_head, rows_at, head);
+#pragma unroll
+  for (int u = 0; u < 4; ++u) { ent[u] = -1; qoff[u] = 0; }
+  if (it.done) return;
+  if (!it.causal) {
+    const int32_t* rows = a.row_list + rows_at + 4 * lane;
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (4 * lane + u < it.nrows) ent[u] = __ldg(rows + u);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (ent[u] >= 0) qoff[u] = entry_qoff(p, a, ent[u]);
+    return;
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int r = 4 * lane + u;
+    if (r < it.nrows) {
+      const int x = it.group == 1 ? r : r / a.by_g;           // (a group is the heads of a kv head)
+      const int t = rows_at + x, h = head + r - x * it.group;
+      ent[u] = (int32_t)(((int64_t)t * p.Hq + h) * p.NP);
+      qoff[u] = (int64_t)t * p.sq_t + (int64_t)h * p.sq_h;
+    }
+  }
 }
 
 // Rows [0, nrows) of an item into a 128-byte-swizzled tile of [128][64] blocks, by kWarps warps (this one is number
@@ -253,7 +308,7 @@ __device__ __forceinline__ bool describe_items(const Params& p, const ItemQueue&
     if constexpr (kRowIndex) {
       int row[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) row[u] = ent[u] >= 0 ? (int)((uint32_t)ent[u] / (uint32_t)p.NP) : 0;
+      for (int u = 0; u < 4; ++u) row[u] = ent[u] >= 0 ? ent[u] / iq.by_np : 0;
       *reinterpret_cast<int4*>(&c.grow[slot][4 * lane]) = make_int4(row[0], row[1], row[2], row[3]);
     }
     if (lane == 0) c.item[slot] = it;

@@ -47,6 +47,33 @@ def test_chunk_sizes_around_the_tiles(chunk, d, dtype):
 
 
 @pytest.mark.parametrize("d,dtype", [(64, torch.float16), (96, torch.bfloat16), (128, torch.bfloat16)])
+@pytest.mark.parametrize("chunk", [64, 100, 128])
+@pytest.mark.parametrize("lens,hq,hkv", [((5000,), 16, 1), ((700, 9000), 16, 4), ((4100, 3, 4095), 12, 12), ((33,), 16, 2)])
+def test_streams_of_one_tile_items(lens, hq, hkv, chunk, d, dtype):
+    """Chunks of at most 128 keys: a CTA's items run through a ring of descriptions, of Q, K and V tiles and of places in tensor
+    memory, each many times over in the longer calls; lists of many tiles (few kv heads) and of one, K and V shared by the heads
+    of a group and not.  A window of more rows than one tile runs the same kernel, one of fewer rows the kernel for short
+    items: the same bits."""
+    topk = 6
+    q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, dtype, seed=chunk + d + hq)
+    q *= 3                                                   # a moving softmax reference
+    args = (k, v, cu, max(lens), chunk, topk)
+    out, lse, sel = parallel.moba_forward(q, *args, return_lse=True, return_selected=True)
+    ref, ref_lse, ref_sel = parallel.moba_forward(q, *args, return_lse=True, return_selected=True,
+                                                  attend_impl=_lib.ATTEND_MMA_SYNC)
+    assert torch.equal(sel, ref_sel)
+    _close(out, ref, dtype)
+    assert (lse - ref_lse).abs().max().item() < 1e-3
+    total, few = sum(lens), 128 // (hq // hkv)
+    for begin, n in ((total - few, few), (total // 2, few + 1), (total // 3, min(400, total - total // 3)), (total - 1, 1)):
+        if begin < 0 or begin + n > total:
+            continue
+        o, l, s = parallel.moba_forward(q[begin:begin + n], *args, return_lse=True, return_selected=True, q_token_begin=begin)
+        assert torch.equal(s, sel[:, :, begin:begin + n])
+        assert torch.equal(o, out[begin:begin + n]) and torch.equal(l, lse[:, begin:begin + n]), (begin, n)
+
+
+@pytest.mark.parametrize("d,dtype", [(64, torch.float16), (96, torch.bfloat16), (128, torch.bfloat16)])
 @pytest.mark.parametrize("chunk", [1000, 1024, 1025])
 def test_chunks_of_up_to_1024_keys_on_either_kernel(chunk, d, dtype):
     """Chunks of 513 to 1024 keys are items of half a 256-row tile (the last half of a list may be empty or ragged); one
