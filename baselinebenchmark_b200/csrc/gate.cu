@@ -61,9 +61,24 @@ cudaError_t launch_chunk_metadata(const Params& p, const int32_t* cu, int32_t* c
 // 16 heads 107 us, 80 with 32).  Few long ones want their loads in flight: with 512 CTAs on chunks of 4096 keys, 268 MB,
 // a call took 340 us with 32 registers, 330 with 54.  So 32 it is where more CTAs come than fit with 48.
 // Split over the dims, 64 registers (eight CTAs) hold ten rows; 106 held sixteen, in four CTAs.
+// Where even that leaves most SMs without a CTA (the chunk a decode step completes), 16 dims a CTA, 8 bytes a load and 64 rows in
+// flight: all of a 4096-key chunk is requested in two goes.  One 4096-key chunk x 8
+// heads, whole decode step 114 -> 107 us (kernel 14.3 -> 8.3), x 16 heads 105 -> 98, x 4 heads at head dim 256 113 -> 110; chunks of
+// 1024 (65536 tokens) 56.7 -> 55.5, of 2048 55.7 -> 55.3.  From 16 rows a lane on: shorter chains are one round either way.
+// kVec: dims of a load.
 // ---------------------------------------------------------------------------
-template <bool kHalf, int D, int kDims, int kAhead, int kCtas>
-__global__ void __launch_bounds__(kMeanLanes * (kDims / 8), kCtas)
+template <int kVec> struct MeanLoad;
+template <> struct MeanLoad<8> { using T = uint4; };
+template <> struct MeanLoad<4> { using T = uint2; };
+template <bool kHalf>
+__device__ __forceinline__ void unpack_mean(const uint4 x, float (&f)[8]) { unpack8<kHalf>(x, f); }
+template <bool kHalf>
+__device__ __forceinline__ void unpack_mean(const uint2 x, float (&f)[4]) {
+  const float2 a = unpack2<kHalf>(x.x), b = unpack2<kHalf>(x.y);
+  f[0] = a.x; f[1] = a.y; f[2] = b.x; f[3] = b.y;
+}
+template <bool kHalf, int D, int kDims, int kAhead, int kCtas, int kVec = 8>
+__global__ void __launch_bounds__(kMeanLanes * (kDims / kVec), kCtas)
 chunk_mean_kernel(Params p, int slot_begin, const __nv_bfloat16* __restrict__ k, const int32_t* __restrict__ cu,
                   __nv_bfloat16* __restrict__ means, int32_t* __restrict__ zero, int64_t zero_words) {
   pdl_wait();
@@ -75,43 +90,59 @@ chunk_mean_kernel(Params p, int slot_begin, const __nv_bfloat16* __restrict__ k,
   const int slot = slot_begin + blockIdx.x, hk = blockIdx.y, dim0 = blockIdx.z * kDims;
   const int b = slot / p.mc, j = slot - b * p.mc;
   const Slot sl = slot_of(cu, b, j, p.C);
-  constexpr int kDimLanes = kDims / 8;
-  const int dl = threadIdx.x % kDimLanes;  // dims dim0 + 8*dl .. + 7
+  constexpr int kDimLanes = kDims / kVec;
+  using Load = typename MeanLoad<kVec>::T;
+  const int dl = threadIdx.x % kDimLanes;  // dims dim0 + kVec * dl ...
   const int rl = threadIdx.x / kDimLanes;  // row lane 0..31
   __nv_bfloat16* dst = means + ((int64_t)slot * p.Hkv + hk) * D + dim0;
 
   __shared__ float part[kMeanLanes][kDims + 4];
-  float acc[8];
+  float acc[kVec];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+  for (int i = 0; i < kVec; ++i) acc[i] = 0.f;
 
   if (sl.historical) {                     // historical chunks are always full: C rows
-    const __nv_bfloat16* base = k + (int64_t)sl.start * p.sk_t + (int64_t)hk * p.sk_h + dim0 + dl * 8;
+    const __nv_bfloat16* base = k + (int64_t)sl.start * p.sk_t + (int64_t)hk * p.sk_h + dim0 + dl * kVec;
     int r = rl;
     // kAhead rows in flight per thread, accumulated in increasing r
     for (; r + (kAhead - 1) * kMeanLanes < p.C; r += kAhead * kMeanLanes) {
-      uint4 x[kAhead];
+      Load x[kAhead];
 #pragma unroll
       for (int u = 0; u < kAhead; ++u)
-        x[u] = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)(r + u * kMeanLanes) * p.sk_t));
+        x[u] = __ldg(reinterpret_cast<const Load*>(base + (int64_t)(r + u * kMeanLanes) * p.sk_t));
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
-        float f[8];
-        unpack8<kHalf>(x[u], f);
+        float f[kVec];
+        unpack_mean<kHalf>(x[u], f);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] += f[i];
+        for (int i = 0; i < kVec; ++i) acc[i] += f[i];
+      }
+    }
+    if constexpr (kAhead > 16) {           // a quarter as many for what is left
+      for (; r + (kAhead / 4 - 1) * kMeanLanes < p.C; r += kAhead / 4 * kMeanLanes) {
+        Load x[kAhead / 4];
+#pragma unroll
+        for (int u = 0; u < kAhead / 4; ++u)
+          x[u] = __ldg(reinterpret_cast<const Load*>(base + (int64_t)(r + u * kMeanLanes) * p.sk_t));
+#pragma unroll
+        for (int u = 0; u < kAhead / 4; ++u) {
+          float f[kVec];
+          unpack_mean<kHalf>(x[u], f);
+#pragma unroll
+          for (int i = 0; i < kVec; ++i) acc[i] += f[i];
+        }
       }
     }
     for (; r < p.C; r += kMeanLanes) {
-      const uint4 x = __ldg(reinterpret_cast<const uint4*>(base + (int64_t)r * p.sk_t));
-      float f[8];
-      unpack8<kHalf>(x, f);
+      const Load x = __ldg(reinterpret_cast<const Load*>(base + (int64_t)r * p.sk_t));
+      float f[kVec];
+      unpack_mean<kHalf>(x, f);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] += f[i];
+      for (int i = 0; i < kVec; ++i) acc[i] += f[i];
     }
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) part[rl][dl * 8 + i] = acc[i];
+  for (int i = 0; i < kVec; ++i) part[rl][dl * kVec + i] = acc[i];
   __syncthreads();
   if (threadIdx.x < kDims) {
     float tot = part[0][threadIdx.x];
@@ -134,8 +165,12 @@ cudaError_t launch_chunk_means_range(const Params& p, int slot_begin, int slot_e
   const int64_t pairs = (int64_t)(slot_end - slot_begin) * p.Hkv;
   const bool split = pairs < 2 * 148 && p.C >= 8 * kMeanLanes;
   const bool many = pairs * (kMeanLanes * (p.D / 8)) > 148 * 1280;         // (the same kernel at head dim 256)
+  // The split one again where 16 dims a CTA fit two CTAs per SM.
+  const bool few = pairs * (p.D / 16) <= 2 * 148 && p.C >= 16 * kMeanLanes;
 #define MOBA_MEANS(HALF, DIM)                                                                                          \
-  return split ? launch_pdl(chunk_mean_kernel<HALF, DIM, 32, 16, 8>, dim3(slot_end - slot_begin, p.Hkv, DIM / 32),     \
+  return few ? launch_pdl(chunk_mean_kernel<HALF, DIM, 16, 64, 1, 4>, dim3(slot_end - slot_begin, p.Hkv, DIM / 16),    \
+                          kMeanLanes * 4, 0, st, p, slot_begin, k, cu, means, zero, zero_words)                        \
+       : split ? launch_pdl(chunk_mean_kernel<HALF, DIM, 32, 16, 8>, dim3(slot_end - slot_begin, p.Hkv, DIM / 32),     \
                             kMeanLanes * 4, 0, st, p, slot_begin, k, cu, means, zero, zero_words)                      \
                : launch_pdl(many ? chunk_mean_kernel<HALF, DIM, DIM, 4, DIM < 256 ? 2048 / (kMeanLanes * (DIM / 8)) : 1> \
                                  : chunk_mean_kernel<HALF, DIM, DIM, 4, 1>, dim3(slot_end - slot_begin, p.Hkv, 1),     \

@@ -270,6 +270,19 @@ def test_chunk_means_of_few_and_many_chunks(chunk, chunks, d, dtype):
     assert torch.equal(G.means(prob, k, cu).cpu().view(torch.int16), want.view(torch.int16))
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d", [64, 96, 128, 256])
+@pytest.mark.parametrize("chunk", [511, 512, 1025, 2047, 2048, 2049, 4111])
+def test_chunk_means_of_one_or_two_long_chunks(chunk, d, dtype):
+    """Few long chunks: batches of 64 rows a lane, of 16, then single rows; a chunk whose sequence ends with it has no mean."""
+    lens, hkv = (2 * chunk + 1, chunk), 3
+    _, k, _, cu = _inputs(lens, hkv, hkv, d, chunk, dtype, seed=chunk)
+    prob, _ = G.problem_for(k, k, k, cu, max(lens), chunk, 3)
+    cu_chunk, _, valid, _ = O.chunk_slots(cu.cpu().numpy(), max(lens), chunk)
+    want = O.chunk_means(k.cpu(), cu_chunk, valid, chunk)
+    assert torch.equal(G.means(prob, k, cu).cpu().view(torch.int16), want.view(torch.int16))
+
+
 @pytest.mark.parametrize("topk", [1, 4])
 @pytest.mark.parametrize("chunk", [128, 1024, 1025])
 def test_a_call_waits_for_its_inputs_from_another_stream(chunk, topk):
