@@ -8,7 +8,7 @@ from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
 ROOT = PKG.parent
-SOURCES = ["api.cu", "gate.cu", "routes.cu", "attend_mma.cu", "attend_tc5.cu", "attend_one_tc5.cu", "attend_bwd.cu", "attend_bwd_tc5.cu", "attend_bwd_dkdv_tc5.cu", "route_static.cu", "nccl_dl.cu"]
+SOURCES = ["api.cu", "gate.cu", "routes.cu", "attend_mma.cu", "attend_tc5.cu", "attend_one_tc5.cu", "attend_few_tc5.cu", "attend_bwd.cu", "attend_bwd_tc5.cu", "attend_bwd_dkdv_tc5.cu", "route_static.cu", "nccl_dl.cu"]
 LIB = PKG / "libmoba_b200.so"
 
 

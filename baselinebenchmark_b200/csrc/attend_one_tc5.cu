@@ -163,11 +163,7 @@ attend_tc5_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k
   if (warp == kDescWarp) {
     // ---- descriptions
     ShortQueue w;
-    w.cur = w.end = 0;
-    w.ahead = short_draw(sa.iq, c);
-    w.list = -1;
-    w.list_first = w.list_end = 0;
-    w.list_off = w.list_count = w.kv_tok0 = w.kv_head = 0;
+    short_start(sa.iq, c, w);
     int last_tok0 = -1, last_head = -1;
     for (bool done = false; !done; ++run) {
       ShortItem it;

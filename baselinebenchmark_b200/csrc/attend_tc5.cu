@@ -1534,21 +1534,6 @@ cudaError_t launch_bounded_wait_probe(int32_t* status, unsigned long long limit_
   return cudaGetLastError();
 }
 
-// CTAs for a window of at most 128 rows per kv head: no more than it can have items, one per list its rows can be
-// on and one per kv head and chunk it touches.  With two CTAs per SM waiting for work, few items gathered in pairs on
-// some SMs while others had none.  Dense stage, chunk 4096, top-k 8, against the 256-row kernel with one CTA per SM:
-//   20011 tokens, 16/4 heads, 32 new   74 us there, 86 with all CTAs, 70 with this many
-//   131072, 16/4, 32 new               84           98                76
-//   131072, 8/8, 1 new                 78           83                74
-//   131072, 32/8, 1 new               144           86                86   (more items than SMs)
-static int window_ctas(const Params& p, int ctas) {
-  const int64_t routed = p.hist * p.rows < p.lists ? p.hist * p.rows : p.lists;
-  int64_t chunks = p.Tq / p.C + p.B + 1;                     // every sequence may add a part of a chunk
-  if (chunks > p.Tq) chunks = p.Tq;
-  const int64_t items = routed + chunks * p.Hkv;
-  return items < ctas ? (int)items : ctas;
-}
-
 cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* k,
                               const __nv_bfloat16* v, const int32_t* cu, const int32_t* list_counts,
                               const int32_t* list_offsets, const int32_t* tile_prefix,
@@ -1560,6 +1545,9 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (tc5_one_tile(p))
     return launch_attend_one_tc5(p, q, k, v, cu, list_counts, list_offsets, tile_prefix, row_list, partial_out, partial_lse,
+                                 work_counter, status, sms, st);
+  if (tc5_few_rows(p))
+    return launch_attend_few_tc5(p, q, k, v, cu, list_counts, list_offsets, tile_prefix, row_list, partial_out, partial_lse,
                                  work_counter, status, sms, st);
   CUtensorMap mk, mv;
   if (!make_kv_map(&mk, p.fp16 != 0, p.D, k, p.T, p.Hkv, p.sk_t, p.sk_h, kBN) || !make_kv_map(&mv, p.fp16 != 0, p.D, v, p.T, p.Hkv, p.sv_t, p.sv_h, kBN))

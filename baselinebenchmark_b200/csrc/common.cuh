@@ -411,6 +411,13 @@ inline bool tc5_one_tile(const Params& p) {
          (p.Tq - 1) * p.sq_t + (p.Hq - 1) * p.sq_h < ((int64_t)1 << 35);
 }
 
+// Windows of at most this many rows per kv head (decode steps) run a kernel that has keys, not rows, as the lanes of tensor memory
+// (figures and the reason for eight there; chunks of any length: the shortest make no difference).
+constexpr int kFewRows = 8;
+inline bool tc5_few_rows(const Params& p) {
+  return (p.D == 96 || p.D == 128) && p.Tq * p.G <= kFewRows;
+}
+
 cudaError_t launch_attend_mma(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* k,
                               const __nv_bfloat16* v, const int32_t* cu, const int32_t* list_counts,
                               const int32_t* list_offsets, const int32_t* tile_prefix,
@@ -422,6 +429,10 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
                               const int32_t* row_list, __half* partial_out, float2* partial_lse,
                               int32_t* work_counter, int32_t* status, cudaStream_t st);
 cudaError_t launch_attend_one_tc5(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v,
+                                  const int32_t* cu, const int32_t* list_counts, const int32_t* list_offsets,
+                                  const int32_t* tile_prefix, const int32_t* row_list, __half* partial_out,
+                                  float2* partial_lse, int32_t* work_counter, int32_t* status, int sms, cudaStream_t st);
+cudaError_t launch_attend_few_tc5(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* k, const __nv_bfloat16* v,
                                   const int32_t* cu, const int32_t* list_counts, const int32_t* list_offsets,
                                   const int32_t* tile_prefix, const int32_t* row_list, __half* partial_out,
                                   float2* partial_lse, int32_t* work_counter, int32_t* status, int sms, cudaStream_t st);

@@ -90,6 +90,21 @@ inline int short_batch(const Params& p, int ctas, bool grouped) {
   return share < 1 ? 1 : share > 8 ? 8 : (int)share;
 }
 
+// CTAs for a window of at most 128 rows per kv head: no more than it can have items, one per list its rows can be
+// on and one per kv head and chunk it touches.  With two CTAs per SM waiting for work, few items gathered in pairs on
+// some SMs while others had none.  Dense stage, chunk 4096, top-k 8, against the 256-row kernel with one CTA per SM:
+//   20011 tokens, 16/4 heads, 32 new   74 us there, 86 with all CTAs, 70 with this many
+//   131072, 16/4, 32 new               84           98                76
+//   131072, 8/8, 1 new                 78           83                74
+//   131072, 32/8, 1 new               144           86                86   (more items than SMs)
+inline int window_ctas(const Params& p, int ctas) {
+  const int64_t routed = p.hist * p.rows < p.lists ? p.hist * p.rows : p.lists;
+  int64_t chunks = p.Tq / p.C + p.B + 1;                     // every sequence may add a part of a chunk
+  if (chunks > p.Tq) chunks = p.Tq;
+  const int64_t items = routed + chunks * p.Hkv;
+  return items < ctas ? (int)items : ctas;
+}
+
 struct ShortItem {
   int32_t done;                            // 1: the queue is empty
   int32_t new_kv;                          // 0: K and V of the item before are those of this one (one tile)
@@ -104,7 +119,7 @@ struct ShortItem {
 // Walks the items a CTA draws; executed by the whole describing warp.
 struct ShortQueue {
   int cur, end;                            // items of the current draw left: [cur, end)
-  int ahead;                               // lane 0: the draw behind it (short_pick<true>)
+  int ahead, drawn, dealt;                 // short_pick<true>, see short_start: the draw behind it (lane 0), draws so far, of them without the counter
   int list, list_first, list_end;          // list of the last routed item and the items it covers
   int list_off, list_count, kv_tok0, kv_head;
 };
@@ -112,10 +127,31 @@ template <typename CtrlT>
 __device__ __forceinline__ int short_draw(const ItemQueue& a, const CtrlT& c) {
   return (threadIdx.x & 31) != 0 ? 0 : c.abort ? 0x3fffffff : atomicAdd(a.work_counter, 1);
 }
+// A draw that is asked for before the one in hand is used up.  A CTA that describes its items far ahead would draw several before
+// others have started, so the first kDealt draws of every CTA are dealt out instead: CTA b has draws b, b + CTAs, ... .  One decode
+// step on 131072 tokens (168 items, up to 232 CTAs): dense stage 61 or 92 us from run to run without, 60 with it.
+constexpr int kDealt = 9;
+template <typename CtrlT>
+__device__ __forceinline__ int short_draw_ahead(const ItemQueue& a, const CtrlT& c, ShortQueue& w) {
+  const int d = w.drawn++;
+  if (d < w.dealt) return d * (int)gridDim.x + (int)blockIdx.x;
+  return w.dealt * (int)gridDim.x + short_draw(a, c);
+}
+template <typename CtrlT>
+__device__ __forceinline__ void short_start(const ItemQueue& a, const CtrlT& c, ShortQueue& w) {
+  w.cur = w.end = 0;
+  w.list = -1;
+  w.list_first = w.list_end = 0;
+  w.list_off = w.list_count = w.kv_tok0 = w.kv_head = 0;
+  const int big = max(c.n_items - 2 * (int)gridDim.x, 0) / a.batch, draws = big + c.n_items - big * a.batch;
+  w.drawn = 0;
+  w.dealt = min((draws + (int)gridDim.x - 1) / (int)gridDim.x, kDealt);
+  w.ahead = short_draw_ahead(a, c, w);
+}
 
 // The next item: its description in `it`, its first key token and kv head, and where its rows are: from row_list[rows_at]
 // on, or (own chunk) query tokens of the window from rows_at on, heads from `head` on.
-// kDrawAhead: the draw behind the one in hand is under way (w.ahead is set at the start), so that its latency is not waited for.
+// kDrawAhead: the draw behind the one in hand is under way (short_start), so that its latency is not waited for.
 template <bool kDrawAhead, typename CtrlT>
 __device__ __forceinline__ void short_pick(const Params& p, const ItemQueue& a, CtrlT& c, ShortQueue& w, ShortItem& it,
                                            int& kv_tok0, int& kv_head, int& rows_at, int& head) {
@@ -133,7 +169,7 @@ __device__ __forceinline__ void short_pick(const Params& p, const ItemQueue& a, 
   for (;;) {
     if (w.cur >= w.end) {
       const int mine = kDrawAhead ? w.ahead : short_draw(a, c);
-      if (kDrawAhead) w.ahead = short_draw(a, c);
+      if (kDrawAhead) w.ahead = short_draw_ahead(a, c, w);
       const int idx = __shfl_sync(0xffffffffu, mine, 0);
       // Draws of `batch` items, and of single ones for the last two of every CTA: with a whole batch drawn last, some
       // CTAs worked three items longer than others.  Against batches to the end: dense stage of 2 x 4096 tokens x 16

@@ -136,6 +136,27 @@ def test_windows_around_the_row_limit_equal_full_run(d, chunk, hq, hkv):
             assert torch.equal(l, lse[:, begin:begin + n]), (begin, n)
 
 
+@pytest.mark.parametrize("hq,hkv", [(4, 4), (6, 2), (8, 1)])
+@pytest.mark.parametrize("chunk", [100, 128, 512, 4096])
+@pytest.mark.parametrize("d,dtype", [(96, torch.float16), (128, torch.bfloat16)])
+def test_decode_windows_of_up_to_eight_rows(d, dtype, chunk, hq, hkv):
+    """Windows of at most eight rows per kv head run a kernel with the operands of both products exchanged, one row more the
+    kernel for short items: the bits of the full run on either side.  Scores large enough that the reference of a row
+    moves from tile to tile; ragged tiles, windows across chunk and sequence boundaries, a list of its own for each row and shared ones."""
+    lens, topk = (700, 9001), 6
+    q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, dtype, seed=chunk + d)
+    q *= 4
+    args = (k, v, cu, max(lens), chunk, topk)
+    full, lse, sel = parallel.moba_forward(q, *args, return_lse=True, return_selected=True)
+    limit = 8 // (hq // hkv)
+    for begin in (0, 699, 700 + 505, 700 + 4095, sum(lens) - limit - 1):
+        for n in sorted({1, limit, limit + 1}):
+            o, l, s = parallel.moba_forward(q[begin:begin + n], *args, return_lse=True, return_selected=True, q_token_begin=begin)
+            assert torch.equal(s, sel[:, :, begin:begin + n])
+            assert torch.equal(o, full[begin:begin + n]), (begin, n)
+            assert torch.equal(l, lse[:, begin:begin + n]), (begin, n)
+
+
 def _layouts(t, name):
     """The same values in another memory layout."""
     n, h, d = t.shape
