@@ -1004,7 +1004,9 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
     }
     if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
   } else if (warp == 5) {
-    // ---- MMA issuer: the whole warp runs this code, one elected lane issues (see above)
+    // ---- MMA issuer: the whole warp runs this code, one elected lane issues.  Predicated MMAs instead of a branch around them:
+    // dense stage of 700 tokens behind 50021, 32/8 heads, chunk 1024 139 -> 134.5 us; 20000 x 16/4 at
+    // head dim 64, chunk 1024 887 -> 858; 32768 x 32/8, chunk 512 2.58 -> 2.46 ms
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
     const uint32_t dq = __shfl_sync(0xffffffffu, desc_lo(sQ, 16), 0);
     const uint32_t dk = __shfl_sync(0xffffffffu, desc_lo(sK, 16), 0);
@@ -1023,12 +1025,13 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
         ++kt;
       }
       tc_fence_after();
-      if (el) {
-        issue_qk<0, 0, kHalf, D>(tm, dq, dk);
-        tc_commit(smem_u32(&c.s_full[n & 1]));
-        tc_commit(smem_u32(j + 1 == ntiles ? &c.q_free : &c.k_free));
+#pragma unroll
+      for (int ks = 0; ks < D / 16; ++ks) {
+        const uint32_t koff = (uint32_t)((ks >> 2) * (kHalfBytes >> 4) + (ks & 3) * 2);
+        mma_ss_el<kDescHi>(el, tm, dq + koff, dk + koff, kIdescQK<kHalf>, ks > 0);
       }
-      __syncwarp();
+      tc_commit_el(el, smem_u32(&c.s_full[n & 1]));
+      tc_commit_el(el, smem_u32(j + 1 == ntiles ? &c.q_free : &c.k_free));
     };
     int n = 0;
     if (wait(&c.item_full[0], 0) && !c.item[0].done) {
@@ -1048,13 +1051,10 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
           if (x) pph[1] ^= 1; else pph[0] ^= 1;
           if (j == 0 && n > 0 && !wait(&c.o_free, (n - 1) & 1)) break;
           tc_fence_after();
-          if (el) {
 #pragma unroll
-            for (int ks = 0; ks < 8; ++ks)
-              mma_ts_lo<kDescHi>(tm + 128, tm + ks * 8, dv + ks * (2048 >> 4), kIdescPV<kHalf, D>, j > 0 || ks > 0);
-            tc_commit(smem_u32(j + 1 == ntiles ? &c.o_full[x] : &c.v_free));
-          }
-          __syncwarp();
+          for (int ks = 0; ks < 8; ++ks)
+            mma_ts_el<kDescHi>(el, tm + 128, tm + ks * 8, dv + ks * (2048 >> 4), kIdescPV<kHalf, D>, j > 0 || ks > 0);
+          tc_commit_el(el, smem_u32(j + 1 == ntiles ? &c.o_full[x] : &c.v_free));
           if (j + 1 < ntiles) {
             qk(n, j + 1, ntiles, true);
           } else {
@@ -1064,8 +1064,7 @@ attend_tc5_short_kernel(const Params p, const __grid_constant__ CUtensorMap tmap
             next_tiles = (c.item[s1].kv_len + kBN - 1) / kBN;
             next_fresh = c.item[s1].new_kv != 0;
             if (more) {
-              if (next_fresh && el) tc_commit(smem_u32(&c.v_free));
-              __syncwarp();
+              if (next_fresh) tc_commit_el(el, smem_u32(&c.v_free));
               qk(n + 1, 0, next_tiles, next_fresh);
             }
           }
