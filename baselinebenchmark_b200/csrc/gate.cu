@@ -430,13 +430,15 @@ struct GateLists {
 // kShort: the loops over the entries of a row are not unrolled.  Code that few rows come to is mostly fetched: 32768 x 32/8, at most 32
 // candidates, lists of 8: gating kernel 218 -> 214 us, head dim 256 552 -> 522, a decode step with a near-tie 60 -> 58.
 // Where many rows do, it costs (top-k 28 of 256 candidates at head dim 256, half of the rows: 1936 -> 2056).
-template <bool kHalf, int D, bool kShort>
+// kFloats: the list holds the estimates themselves, not keys.
+template <bool kHalf, int D, bool kShort, bool kFloats>
 __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, const GateTile& t, const __nv_bfloat16* qrow,
                                           int row, int mode, int n_surv, int n_keep, int ncand, float eps,
                                           const __nv_bfloat16* __restrict__ means, int32_t* __restrict__ stats) {
   const int lane = threadIdx.x & 31;
   const int hist = p.hist, lstride = g.lstride;
   const int slot0 = t.b * p.mc;
+  auto estimate = [](uint32_t y) { return kFloats ? __uint_as_float(y) : key_float(y); };
   uint2* lists = g.lists;
   unsigned need = __ballot_sync(0xffffffffu, mode != 0);
   unsigned long long* lx = g.exact;
@@ -496,7 +498,7 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
       if (lane < cnt) {
         key = ((unsigned long long)float_key(e) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(slot0 + (int)cc));
         if (stats != nullptr) {
-          const float diff = fabsf(key_float(ent.y) - e);
+          const float diff = fabsf(estimate(ent.y) - e);
           if (!(diff <= r_eps)) atomicAdd(&stats[2], 1);
           atomicMax(&stats[1], (int)fminf(diff / r_eps * 65536.f, 1.0e9f));
         }
@@ -534,7 +536,7 @@ __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, c
         const float e = contract_score<kHalf, D>(r_q, means + ((int64_t)(slot0 + cc) * p.Hkv + t.hk) * D);
         key = ((unsigned long long)float_key(e) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)(slot0 + cc));
         if (r_mode == 1 && stats != nullptr) {
-          const float diff = fabsf(key_float(rlist[idx].y) - e);
+          const float diff = fabsf(estimate(rlist[idx].y) - e);
           if (!(diff <= r_eps)) viol = 1;
           ratio = (int)fminf(diff / r_eps * 65536.f, 1.0e9f);
         }
@@ -832,7 +834,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
             mylist[i] = make_uint2(v[i] ? (31u - (v[i] & 31u)) | ((tied >> i) & 1u ? kTied : 0u) | ((first >> i) & 1u ? kRunStart : 0u)
                                         : 0xFFFFFFFFu, v[i]);
         __syncwarp();
-        rank_rows<kHalf, D, true>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand,
+        rank_rows<kHalf, D, true, false>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand,
                                   0.5f * eps2, means, stats);
         __syncwarp();
       }
@@ -1013,8 +1015,9 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
     const int row = tid;
     const int ncand = row < nrows ? (t.tok_lo + row / p.G - t.s0) / p.C : 0;     // chunks before the row's own chunk
     uint2* mylist = lists + (size_t)row * lstride;
-    for (int i = 0; i < list_len; ++i) mylist[i] = make_uint2(0xFFFFFFFFu, 0u);   // chunk -1, key 0: empty place
-    uint32_t tau = 0;                                  // smallest key kept (heap root / last place); 0 while places are free
+    for (int i = 0; i < list_len; ++i) mylist[i] = make_uint2(0xFFFFFFFFu, kW > 0 ? 0xff800000u : 0u);   // chunk -1, -inf or key 0: empty place
+    uint32_t tau = 0;                                  // smallest key kept, the heap's root; 0 while places are free
+    float last = -INFINITY;                            // the same of a sorted list, its last place
     uint32_t* myscratch = reinterpret_cast<uint32_t*>(scratch + row * scratch_stride(kW));
 
     // A wait that gives up is remembered by the thread: its row is then ranked exactly, from Q rows
@@ -1049,52 +1052,67 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
         __syncwarp();
         tmem_ld32(trow + col, v);
         tmem_wait_ld();
-        // estimates -> order-preserving keys; places past the row's candidates get key 0
         const int rem = cend - col;
-        uint32_t vmax = 0;
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          uint32_t key = float_key(__uint_as_float(v[i]));
-          if (kW > 0) key = (key & ~31u) | (uint32_t)(31 - i);         // position in the low bits: earlier wins ties
-          v[i] = i < rem ? key : 0u;
-          vmax = max(vmax, v[i]);
-        }
-        if (!__any_sync(0xffffffffu, vmax > tau)) continue;             // nothing here enters any list of the warp
         const uint32_t chunk0 = (uint32_t)(c0 + col);
-        if (kW > 0) {
-          topk::top_of_32<(kW > 0 ? kW : 32)>(v);
+        if constexpr (kW > 0) {
+          // Estimates as they are, with their place in the five low bits; places past the row's candidates get -inf.  (Estimates
+          // this close are near-ties, ranked again whatever their order here, and a row with one that is not finite is ranked over
+          // all its candidates.)  Integer keys in the same order took four more instructions an estimate of a kernel that is bound by
+          // integer and min/max instructions: 32768 x 32/8, 255 candidates, top-k 8 545 -> 508 us, 4 424 -> 388, 24 1313 -> 1267;
+          // 65536 x 16/4, 127 candidates 356 -> 327; head dim 64, up to 63 57.7 -> 54.1; 256 508 -> 489.
+          float f[32];
+#pragma unroll
+          for (int i = 0; i < 32; ++i) f[i] = __uint_as_float((v[i] & ~31u) | (uint32_t)(31 - i));
+          if (!__all_sync(0xffffffffu, rem >= 32)) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) f[i] = i < rem ? f[i] : -INFINITY;
+          }
+          float fmx = -INFINITY;
+#pragma unroll
+          for (int i = 0; i < 32; i += 2) fmx = max3(fmx, f[i], f[i + 1]);
+          if (!__any_sync(0xffffffffu, fmx > last)) continue;           // nothing here enters any list of the warp
+          topk::top_of_32<kW>(f);
+          auto entry = [&](uint32_t bits) { return make_uint2(chunk0 + 31u - (bits & 31u), bits); };
           if (c0 == 0 && col == 0) {
-            // first candidates of the row: the list is the head of the sorted keys
+            // first candidates of the row: the list is the head of the sorted ones
 #pragma unroll
             for (int i = 0; i < kW; ++i)
-              if (i < list_len) mylist[i] = make_uint2(v[i] ? chunk0 + 31u - (v[i] & 31u) : 0xFFFFFFFFu, v[i]);
+              if (i < list_len && f[i] > -INFINITY) mylist[i] = entry(__float_as_uint(f[i]));
           } else {
             // s_t enters the list iff it beats the entry t places from the end (both are sorted)
             int j = 0;
 #pragma unroll
             for (int t2 = 0; t2 < kW; ++t2)
-              if (t2 < list_len) j += v[t2] > mylist[list_len - 1 - t2].y;
+              if (t2 < list_len) j += f[t2] > __uint_as_float(mylist[list_len - 1 - t2].y);
             if (j > 0) {
 #pragma unroll
               for (int i = 0; i < kW; i += 4)
-                *reinterpret_cast<uint4*>(myscratch + i) = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-              // in-place merge from the bottom: the smaller of the two tails goes to `pos`; equal keys
+                *reinterpret_cast<float4*>(myscratch + i) = make_float4(f[i], f[i + 1], f[i + 2], f[i + 3]);
+              // in-place merge from the bottom: the smaller of the two tails goes to `pos`; equal ones
               // keep the list's entry (an earlier chunk) above
               int i = list_len - j - 1, jj = j - 1;
               for (int pos = list_len - 1; jj >= 0; --pos) {
                 const uint32_t sk = myscratch[jj];
-                if (i >= 0 && mylist[i].y < sk) {
+                if (i >= 0 && __uint_as_float(mylist[i].y) < __uint_as_float(sk)) {
                   mylist[pos] = mylist[i];
                   --i;
                 } else {
-                  mylist[pos] = make_uint2(chunk0 + 31u - (sk & 31u), sk);
+                  mylist[pos] = entry(sk);
                   --jj;
                 }
               }
             }
           }
-          tau = mylist[list_len - 1].y;
+          last = __uint_as_float(mylist[list_len - 1].y);
         } else {
+          // order-preserving keys; places past the row's candidates get key 0
+          uint32_t vmax = 0;
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            v[i] = i < rem ? float_key(__uint_as_float(v[i])) : 0u;
+            vmax = max(vmax, v[i]);
+          }
+          if (!__any_sync(0xffffffffu, vmax > tau)) continue;
           uint32_t hits = 0;
 #pragma unroll
           for (int i = 0; i < 32; ++i) hits |= v[i] > tau ? (1u << i) : 0u;
@@ -1132,6 +1150,7 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
     // eps of this row (see the head of this section); inf or NaN sends the row to the exact ranking
     const float eps = gate_kappa<D, (kW > 0)> * sqrtf(q_ssq) * sqrtf(__int_as_float(c.mean_ssq_max)) + 7.9e-31f;
     const int n_keep = min(hist, ncand);
+    auto value = [&](int i) { return kW > 0 ? __uint_as_float(mylist[i].y) : key_float(mylist[i].y); };   // estimate of entry i
     // 0: list is exact; 3: order the runs of near-ties (marked in the list); 1: rank all survivors;
     // 2: rank all candidates
     int mode = 0, n_surv = 0;
@@ -1146,17 +1165,17 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
         // settled by the estimates alone? (the common case: nothing else is computed for the row)
         bool amb = all;
         {
-          float prev = key_float(mylist[0].y);
+          float prev = value(0);
           for (int i = 0; i < n_keep && i + 1 < n_real; ++i) {
-            const float next = key_float(mylist[i + 1].y);
+            const float next = value(i + 1);
             if (!(prev - next > eps2)) amb = true;
             prev = next;
           }
         }
         // survivors: the only candidates that can be among the n_keep best exact scores
         if (amb) {
-          const float theta = key_float(mylist[n_keep - 1].y) - eps2;
-          while (n_surv < n_real && key_float(mylist[n_surv].y) >= theta) ++n_surv;
+          const float theta = value(n_keep - 1) - eps2;
+          while (n_surv < n_real && value(n_surv) >= theta) ++n_surv;
         }
         if (!amb) {
           mode = 0;
@@ -1168,9 +1187,9 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
           // members of a run are marked in the chunk word (kTied, kRunStart on its first member).
           int tied = 0;
           bool in_run = false;
-          float prev = key_float(mylist[0].y);
+          float prev = value(0);
           for (int i = 0; i + 1 < n_surv; ++i) {
-            const float next = key_float(mylist[i + 1].y);
+            const float next = value(i + 1);
             if (all || !(prev - next > eps2)) {
               if (!in_run) { mylist[i].x |= kTied | kRunStart; ++tied; }
               mylist[i + 1].x |= kTied;
@@ -1196,7 +1215,7 @@ gate_topk_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, con
     }
     __syncwarp();                                             // the marks are visible to the warp
     const __nv_bfloat16* qrow = q + (int64_t)(t.tok_lo + row / p.G - p.win_lo) * p.sq_t + (int64_t)(t.hk * p.G + row % p.G) * p.sq_h;
-    rank_rows<kHalf, D, false>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand, eps, means,
+    rank_rows<kHalf, D, false, (kW > 0)>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand, eps, means,
                         stats);
     // selected[rank][head][token]: every thread stores the chunks of its own row (its list was
     // written by its own warp); neighbouring lanes are neighbouring heads, then tokens
