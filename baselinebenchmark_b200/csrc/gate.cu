@@ -204,11 +204,11 @@ cudaError_t launch_chunk_means(const Params& p, const __nv_bfloat16* k, const in
 //      memory, one lane per row), and thread r reads the estimates a_c of its
 //      row 32 at a time and keeps the L = hist + 1 (+ 3 when a row can have
 //      more than 32 candidates) largest, sorted, in shared memory.  For
-//      L <= 32 the 32 estimates become order-preserving integer keys whose
-//      five lowest bits hold the position (a change of less than 2^-18 of
-//      the score, counted in eps), a compare-exchange network over the 32
-//      registers brings the largest 8, 16 or 32 keys to the front, and they
-//      are merged with the list; longer lists are kept as a min-heap.
+//      L <= 32 the five lowest bits of the 32 estimates hold their position
+//      (a change of less than 2^-18 of the score, counted in eps), a
+//      compare-exchange network over the 32 registers brings the largest 8, 16
+//      or 32 to the front, and they are merged with the list; longer
+//      lists are kept as a min-heap of order-preserving integer keys.
 //   2. recheck.  With e_c the score in the contract order, |a_c - e_c| <= eps
 //      for every candidate of the row (bound below).  If neighbours in the
 //      sorted list differ by more than 2 eps down to the entry after the
@@ -609,6 +609,8 @@ __device__ __forceinline__ void finish_scan(const ListScan& scan, int32_t* __res
 // Measured against the kernel below for these shapes, with the wait for the chunk means: 2 x 4096 tokens x 16 heads, 31
 // candidates 44 -> 40 us, at head dim 256 105 -> 91; 32768 x 32/8, 7 candidates 179 -> 152; a decode token on 32 chunks 24 -> 17.
 // (The few-lane score of near-ties alone, which the kernel below has too: 32768 x 32/8, 255 candidates 620 -> 573.)
+// Networks over the estimates instead of integer keys, as there (kernel alone, us): 2 x 4096 x 16 heads 43.0 -> 40.9, at head dim 256
+// 90.2 -> 86.9; 32768 x 32/8, 7 candidates 122.8 -> 108.5; 131072 x 32/8, 31 780 -> 685; 32768 x 16/4, 31 118.8 -> 104.5, head dim 64 86 -> 78.
 // ---------------------------------------------------------------------------
 constexpr int kOneThreads = 160;
 constexpr int kOneMeans = 32;              // rows of the tile of means, columns of tensor memory
@@ -773,6 +775,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
       }
       tc_fence_after();
       uint32_t v[32];
+      float f[32];
       __syncwarp();
       tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16), v);
       tmem_wait_ld();
@@ -781,9 +784,9 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
       // never complete without somebody: the others' waits give up in turn, and all rank the rows of this CTA exactly.)
       if (!failed) mbar_arrive(smem_u32(&c.read));
 #pragma unroll
-      for (int i = 0; i < 32; ++i)                     // order-preserving keys, position in the low bits: earlier wins ties
-        v[i] = i < ncand ? (float_key(__uint_as_float(v[i])) & ~31u) | (uint32_t)(31 - i) : 0u;
-      topk::top_of_32<kW>(v);
+      for (int i = 0; i < 32; ++i)                     // the estimates, position in the low bits, as in the kernel below
+        f[i] = i < ncand ? __uint_as_float((v[i] & ~31u) | (uint32_t)(31 - i)) : -INFINITY;
+      topk::top_of_32<kW>(f);
       // the norms of the other warps: complete once all threads have arrived on `read`
       if (!failed && !mbar_wait(smem_u32(&c.read), n & 1)) failed = true;
       int ssq_max = 0;
@@ -804,13 +807,13 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
         float theta = 0.f;
 #pragma unroll
         for (int i = 0; i < kW; ++i) {
-          if (i < n_real) holes |= v[i] == 0u;
-          if (i + 1 == n_keep) theta = key_float(v[i]) - eps2;
-          if (i + 1 < kW && i + 1 < n_real && (all || !(key_float(v[i]) - key_float(v[i + 1 < kW ? i + 1 : i]) > eps2)))
+          if (i < n_real) holes |= !(f[i] > -INFINITY);
+          if (i + 1 == n_keep) theta = f[i] - eps2;
+          if (i + 1 < kW && i + 1 < n_real && (all || !(f[i] - f[i + 1 < kW ? i + 1 : i] > eps2)))
             close |= 1u << i;
         }
 #pragma unroll
-        for (int i = 0; i < kW; ++i) n_surv += i < n_real && key_float(v[i]) >= theta;
+        for (int i = 0; i < kW; ++i) n_surv += i < n_real && f[i] >= theta;
         const bool amb = all || (close & ((1u << n_keep) - 1u)) != 0;       // n_keep < 32
         if ((flags & GATE_FORCE_EXACT) || failed || holes) {
           mode = 2;
@@ -831,10 +834,11 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
 #pragma unroll
         for (int i = 0; i < kW; ++i)
           if (i < list_len)
-            mylist[i] = make_uint2(v[i] ? (31u - (v[i] & 31u)) | ((tied >> i) & 1u ? kTied : 0u) | ((first >> i) & 1u ? kRunStart : 0u)
-                                        : 0xFFFFFFFFu, v[i]);
+            mylist[i] = make_uint2(f[i] > -INFINITY ? (31u - (__float_as_uint(f[i]) & 31u)) | ((tied >> i) & 1u ? kTied : 0u) |
+                                                          ((first >> i) & 1u ? kRunStart : 0u)
+                                                    : 0xFFFFFFFFu, __float_as_uint(f[i]));
         __syncwarp();
-        rank_rows<kHalf, D, true, false>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand,
+        rank_rows<kHalf, D, true, true>(p, GateLists{lists, lstride, list_len, c.exact[warp]}, t, qrow, row, mode, n_surv, n_keep, ncand,
                                   0.5f * eps2, means, stats);
         __syncwarp();
       }
@@ -843,7 +847,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
 #pragma unroll
         for (int r = 0; r < kW; ++r)
           if (r < hist) {
-            const uint32_t x = mode != 0 ? mylist[r].x : v[r] ? 31u - (v[r] & 31u) : 0xFFFFFFFFu;
+            const uint32_t x = mode != 0 ? mylist[r].x : f[r] > -INFINITY ? 31u - (__float_as_uint(f[r]) & 31u) : 0xFFFFFFFFu;
             const int cc = x == 0xFFFFFFFFu ? -1 : (int)(x & kChunkMask);
             dst[(int64_t)r * p.sel_rs] = cc >= 0 ? slot0 + cc : -1;
             if (cc >= 0 && count) atomicAdd(&c.cnt[n & 3][warp][cc], 1);

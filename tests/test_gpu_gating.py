@@ -189,6 +189,16 @@ def test_at_most_32_candidates_ties_zeros_infinities(nchunks, topk, d, dtype):
     _few_candidates([chunk * nchunks, chunk - 1, chunk * (nchunks // 2) + 3], 4, 4, nchunks, topk, d, dtype)
 
 
+@pytest.mark.parametrize("d,dtype", [(64, torch.float16), (128, torch.bfloat16), (256, torch.bfloat16)])
+@pytest.mark.parametrize("nchunks,topk", [(34, 2), (34, 8), (40, 17), (66, 8), (129, 12), (129, 30), (300, 8)])
+def test_more_than_32_candidates_ties_zeros_infinities(nchunks, topk, d, dtype):
+    """The same where a row's list goes through several steps of 32 candidates: the networks compare the estimates as floats,
+    which drop NaN; rows with a score that is not finite are ranked over all their candidates."""
+    chunk = 8
+    _few_candidates([chunk * nchunks], 2, 1, nchunks, topk, d, dtype)
+    _few_candidates([chunk * nchunks, chunk - 1, chunk * (nchunks // 2) + 3], 4, 4, nchunks, topk, d, dtype)
+
+
 def _few_candidates(lens, hq, hkv, nchunks, topk, d, dtype):
     chunk, slots = 8, len(lens) * nchunks
     g = torch.Generator().manual_seed(nchunks * 64 + topk)
