@@ -65,8 +65,11 @@ cudaError_t launch_chunk_metadata(const Params& p, const int32_t* cu, int32_t* c
 // flight: all of a 4096-key chunk is requested in two goes.  One 4096-key chunk x 8
 // heads, whole decode step 114 -> 107 us (kernel 14.3 -> 8.3), x 16 heads 105 -> 98, x 4 heads at head dim 256 113 -> 110; chunks of
 // 1024 (65536 tokens) 56.7 -> 55.5, of 2048 55.7 -> 55.3.  From 16 rows a lane on: shorter chains are one round either way.
+// Head dim 256: 64 dims a CTA.  With all of them its 1024 threads were two CTAs to an SM, which loaded and added up in step: 8192 tokens x
+// 16 heads, chunk 128 26.6 -> 20.4 us, 40000 x 8, chunk 1024 45.1 -> 41.0 (at 128 dims it makes no difference).
 // kVec: dims of a load.
 // ---------------------------------------------------------------------------
+template <int D> constexpr int kMeanDims = D < 256 ? D : 64;
 template <int kVec> struct MeanLoad;
 template <> struct MeanLoad<8> { using T = uint4; };
 template <> struct MeanLoad<4> { using T = uint2; };
@@ -172,9 +175,10 @@ cudaError_t launch_chunk_means_range(const Params& p, int slot_begin, int slot_e
                           kMeanLanes * 4, 0, st, p, slot_begin, k, cu, means, zero, zero_words)                        \
        : split ? launch_pdl(chunk_mean_kernel<HALF, DIM, 32, 16, 8>, dim3(slot_end - slot_begin, p.Hkv, DIM / 32),     \
                             kMeanLanes * 4, 0, st, p, slot_begin, k, cu, means, zero, zero_words)                      \
-               : launch_pdl(many ? chunk_mean_kernel<HALF, DIM, DIM, 4, DIM < 256 ? 2048 / (kMeanLanes * (DIM / 8)) : 1> \
-                                 : chunk_mean_kernel<HALF, DIM, DIM, 4, 1>, dim3(slot_end - slot_begin, p.Hkv, 1),     \
-                            kMeanLanes * (DIM / 8), 0, st, p, slot_begin, k, cu, means, zero, zero_words)
+               : launch_pdl(many ? chunk_mean_kernel<HALF, DIM, kMeanDims<DIM>, 4, DIM < 256 ? 2048 / (kMeanLanes * (DIM / 8)) : 6>  \
+                                 : chunk_mean_kernel<HALF, DIM, kMeanDims<DIM>, 4, DIM < 256 ? 1 : 6>,                  \
+                            dim3(slot_end - slot_begin, p.Hkv, DIM / kMeanDims<DIM>), kMeanLanes * (kMeanDims<DIM> / 8), 0, st, p, \
+                            slot_begin, k, cu, means, zero, zero_words)
   switch (p.D) {
     case 64:  if (p.fp16) MOBA_MEANS(true, 64);  else MOBA_MEANS(false, 64);
     case 96:  if (p.fp16) MOBA_MEANS(true, 96);  else MOBA_MEANS(false, 96);
