@@ -1,4 +1,4 @@
-// Dense stage for chunks of at most 128 keys (head dim 64, 96 or 128): every work item is one 128-row tile of queries
+// Dense stage for chunks of at most 128 keys (head dim 64, 96 or 128; tc5_one_tile says which): every work item is one 128-row tile of queries
 // against one tile of keys, and one CTA per SM keeps three or four of them in flight.
 //
 // The work of such an item is small (1024 cycles of MMA at head dim 128, about as many of exponentials), its chain is

@@ -851,9 +851,10 @@ attend_tc5_wide_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_
 
 // ---------------------------------------------------------------------------
 // short items: chunks of at most kShortChunk keys (kShortChunkFew in all but long calls, see tc5_short_items), and query windows
-// with at most 128 rows per kv head (decode steps).  One 128-row tile per work item, two CTAs per SM.
+// with at most 128 rows per kv head.  One 128-row tile per work item, two CTAs per SM.  (Most chunks of 96 to 128 keys:
+// attend_one_tc5.cu; windows of at most eight rows at head dims 96 and 128: attend_few_tc5.cu.)
 //
-// Such an item is one to eight key tiles (or, in a decode step, a long chunk for a handful of
+// Such an item is one to eight key tiles (or, in a small window, a long chunk for some
 // rows), so what counts is that nothing of its hand-over is waited for.  The roles of a CTA run
 // through one flat stream of key tiles, without a CTA-wide barrier between items:
 //   warp 4     describes the items, up to four ahead (a chain of dependent global loads and divisions as
@@ -873,7 +874,7 @@ attend_tc5_wide_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_
 // With one warpgroup for both, softmax and epilogue of an item took most of its time, one after the other (see
 // softmax_row_rolled); with two, dense stage of 2 x 4096 tokens x 16 heads, chunk 128 142 -> 134 us, 13311 x 16/4 at
 // head_dim 64 162 -> 145.  An item now takes 7000 cycles of a CTA, the chain Q.K^T, S, softmax, P.V and the copy of the next Q rows.
-// Measured against the kernel with CTA-wide barriers between items and unrolled code: dense stage of
+// Measured (chunk 128 where it ran them, and decode steps where it did) against the kernel with CTA-wide barriers between items and unrolled code: dense stage of
 // 2 x 4096 tokens x 16 heads, chunk 128 199 -> 146 us (whole call 347 -> 279); 13311 tokens x 16/4 heads,
 // head_dim 64 233 -> 172; 32768 x 32/8 1651 -> 1094.  A decode step (chunk 4096, 131072-token prefix, 32/8 heads), in
 // place of the 256-row kernel: 132 -> 90.  The rolled loops alone: 205 -> 146 on the first.

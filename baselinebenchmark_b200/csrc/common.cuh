@@ -403,14 +403,24 @@ inline bool tc5_short_items(const Params& p) {
   return (p.C <= kShortChunk || few) && (int64_t)p.slots * p.Hq * ((p.C + 127) / 128) < ((int64_t)1 << 30);
 }
 
-// Chunks of at most 128 keys, one key tile an item, run a kernel that keeps several items of an SM in flight; windows of at most
-// 128 rows per kv head (few items, whose own-chunk ones cover the heads of a group) stay with the one for short items, and so does
-// a q of more than 64 GB (row offsets are 32 bits there, in 16-byte pieces).
+// Chunks of 96 to 128 keys, one key tile an item, run a kernel that keeps several items of an SM in flight, where the lists are a few tiles
+// long: a list or an own-chunk tile of its own costs the warp that describes them and new K and V, and half-filled tiles (chunks of
+// 64 keys have half of their items that way) cost it as much as full ones.  Dense stage, kernel for short items over this one,
+// 20000 tokens x 16 heads, top-k 2 / 4 / 8, by kv heads:
+//   head dim 128  chunk 128  1: 1.21 / 1.14 / 1.09   4: 1.18 / 1.12 / 1.06   16: 0.83 / 1.01 / 1.07
+//                 chunk 96   1: 1.03 / 1.13 / 1.13   4: 1.05 / 1.09 / 1.12   16: 0.72 / 0.99 / 1.05
+//                 chunk 64   1: 0.73 / 0.85 / 0.99   4: 0.68 / 0.85 / 0.97   16: 0.55 / 0.70 / 0.90
+//   head dim 64   chunk 128  1: 1.19 / 1.17 / 1.22   4: 1.23 / 1.19 / 1.23   16: 1.02 / 1.22 / 1.27
+//                 chunk 96   1: 1.13 / 1.15 / 1.19   4: 1.15 / 1.17 / 1.21   16: 0.92 / 1.10 / 1.18
+//                 chunk 64   1: 0.91 / 1.01 / 1.09   4: 0.90 / 1.01 / 1.10   16: 0.75 / 0.91 / 1.05
+// So: three tiles a list (rows of a list: ranks x chunk x heads of a group), and chunks of 64 to 95 keys at head dim 64 with seven ranks.
+// Windows of at most 128 rows per kv head (few items, whose own-chunk ones cover the heads of a group) stay with the kernel for short items,
+// and so does a q of more than 64 GB (row offsets are 32 bits there, in 16-byte pieces).
 inline bool tc5_one_tile(const Params& p) {
-  return tc5_short_items(p) && p.C <= 128 && p.Tq * p.G > kTileRowsWide &&
-         (p.Tq - 1) * p.sq_t + (p.Hq - 1) * p.sq_h < ((int64_t)1 << 35);
+  const bool keys = p.C >= 96 || (p.D == 64 && p.C >= 64 && p.hist >= 7);
+  return tc5_short_items(p) && p.C <= 128 && keys && (int64_t)p.hist * p.C * p.G >= 3 * kTileRowsWide &&
+         p.Tq * p.G > kTileRowsWide && (p.Tq - 1) * p.sq_t + (p.Hq - 1) * p.sq_h < ((int64_t)1 << 35);
 }
-
 // Windows of at most this many rows per kv head (decode steps) run a kernel that has keys, not rows, as the lanes of tensor memory
 // (figures and the reason for eight there; chunks of any length: the shortest make no difference).
 constexpr int kFewRows = 8;

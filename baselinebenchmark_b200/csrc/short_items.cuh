@@ -13,7 +13,7 @@ constexpr int kShortPrefix = 2048;         // ints of tile_prefix kept in shared
 constexpr int kShortSlots = 4;             // item descriptions in flight
 
 // tile_prefix is kept in shared memory sampled every 2^shift entries (shift 0: whole), so that
-// finding the list of a routed item costs `shift` dependent global loads instead of log2(lists).
+// finding the list of a routed item costs a round or two of global loads (find_list).
 __host__ __device__ inline int prefix_shift(int64_t lists, int cache_entries) {
   int shift = 0;
   while ((lists >> shift) + 2 > cache_entries) ++shift;

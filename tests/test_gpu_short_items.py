@@ -47,14 +47,14 @@ def test_chunk_sizes_around_the_tiles(chunk, d, dtype):
 
 
 @pytest.mark.parametrize("d,dtype", [(64, torch.float16), (96, torch.bfloat16), (128, torch.bfloat16)])
-@pytest.mark.parametrize("chunk", [64, 100, 128])
+@pytest.mark.parametrize("chunk", [63, 64, 95, 96, 128])
 @pytest.mark.parametrize("lens,hq,hkv", [((5000,), 16, 1), ((700, 9000), 16, 4), ((4100, 3, 4095), 12, 12), ((33,), 16, 2)])
 def test_streams_of_one_tile_items(lens, hq, hkv, chunk, d, dtype):
-    """Chunks of at most 128 keys: a CTA's items run through a ring of descriptions, of Q, K and V tiles and of places in tensor
+    """Chunks of at most 128 keys (64 of them at head dim 64, 96 and up at the others): a CTA's items run through a ring of descriptions, of Q, K and V tiles and of places in tensor
     memory, each many times over in the longer calls; lists of many tiles (few kv heads) and of one, K and V shared by the heads
     of a group and not.  A window of more rows than one tile runs the same kernel, one of fewer rows the kernel for short
     items: the same bits."""
-    topk = 6
+    topk = 9
     q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, dtype, seed=chunk + d + hq)
     q *= 3                                                   # a moving softmax reference
     args = (k, v, cu, max(lens), chunk, topk)
