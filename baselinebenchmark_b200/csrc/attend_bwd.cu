@@ -821,13 +821,11 @@ bwd_dkdv_wide_kernel(Params p, const __nv_bfloat16* __restrict__ q, const __nv_b
 
 template <typename K>
 cudaError_t set_smem(K kernel, size_t bytes) {
-  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  return prepare_kernel(kernel, bytes);
 }
 
 int sm_count() {
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = device_info().sms;
   return sms;
 }
 

@@ -646,9 +646,7 @@ cudaError_t launch_bwd_dkdv_tc5(const Params& p, const __nv_bfloat16* q, const _
                                 const float* lse2, const float* delta, __nv_bfloat16* dk, __nv_bfloat16* dv,
                                 __nv_bfloat16* packed, int32_t* work_counter, int32_t* status, cudaStream_t st) {
   if (p.D != 64 && p.D != 96 && p.D != 128) return cudaErrorInvalidValue;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = device_info().sms;
   // packed rows of the routed lists: qp, then gp, each [hist * rows + 64, D]
   const int64_t cap = (int64_t)p.hist * p.rows + kStep;
   __nv_bfloat16* qp = packed;
@@ -674,7 +672,7 @@ cudaError_t launch_bwd_dkdv_tc5(const Params& p, const __nv_bfloat16* q, const _
   auto kernel = p.D == 128 ? (p.fp16 ? bwd_dkdv_tc5_kernel<true, 128> : bwd_dkdv_tc5_kernel<false, 128>)
               : p.D == 96  ? (p.fp16 ? bwd_dkdv_tc5_kernel<true, 96> : bwd_dkdv_tc5_kernel<false, 96>)
                            : (p.fp16 ? bwd_dkdv_tc5_kernel<true, 64> : bwd_dkdv_tc5_kernel<false, 64>);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+  cudaError_t e = prepare_kernel(kernel, kSmemBytes);
   if (e != cudaSuccess) return e;
   const KernelArgs args{q, dout, cu, list_counts, list_offsets, row_list, lse2, delta, dk, dv, work_counter, status,
                         use_packed};

@@ -841,9 +841,7 @@ cudaError_t launch_bwd_dq_tc5(const Params& p, const __nv_bfloat16* q, const __n
   if (!make_kv_map(&mk, p.fp16 != 0, p.D, k, p.T, p.Hkv, p.sk_t, p.sk_h, kBN) ||
       !make_kv_map(&mv, p.fp16 != 0, p.D, v, p.T, p.Hkv, p.sv_t, p.sv_h, kBN))
     return cudaErrorNotSupported;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = device_info().sms;
   const KernelArgs args{q, dout, cu, list_counts, list_offsets, tile_prefix, row_list, lse2, delta, partial_dq,
                         work_counter, status, ((uintptr_t)partial_dq & 31) == 0};
   if (bwd_dq_short_items(p)) {
@@ -856,7 +854,7 @@ cudaError_t launch_bwd_dq_tc5(const Params& p, const __nv_bfloat16* q, const __n
     auto kern = p.D == 128 ? (p.fp16 ? bwd_dq_short_kernel<true, 128> : bwd_dq_short_kernel<false, 128>)
               : p.D == 96  ? (p.fp16 ? bwd_dq_short_kernel<true, 96> : bwd_dq_short_kernel<false, 96>)
                            : (p.fp16 ? bwd_dq_short_kernel<true, 64> : bwd_dq_short_kernel<false, 64>);
-    const cudaError_t se = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDqShortSmemBytes);
+    const cudaError_t se = prepare_kernel(kern, kDqShortSmemBytes);
     if (se != cudaSuccess) return se;
     kern<<<sms, kDqShortThreads, kDqShortSmemBytes, st>>>(p, mk, mv, sa);
     return cudaGetLastError();
@@ -864,7 +862,7 @@ cudaError_t launch_bwd_dq_tc5(const Params& p, const __nv_bfloat16* q, const __n
   auto kernel = p.D == 128 ? (p.fp16 ? bwd_dq_tc5_kernel<true, 128> : bwd_dq_tc5_kernel<false, 128>)
               : p.D == 96  ? (p.fp16 ? bwd_dq_tc5_kernel<true, 96> : bwd_dq_tc5_kernel<false, 96>)
                            : (p.fp16 ? bwd_dq_tc5_kernel<true, 64> : bwd_dq_tc5_kernel<false, 64>);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+  cudaError_t e = prepare_kernel(kernel, kSmemBytes);
   if (e != cudaSuccess) return e;
   kernel<<<sms, kThreads, kSmemBytes, st>>>(p, mk, mv, args);
   return cudaGetLastError();

@@ -490,7 +490,7 @@ cudaError_t launch_attend_few_tc5(const Params& p, const __nv_bfloat16* q, const
                          : (p.fp16 ? (one ? attend_tc5_few_kernel<true, 96, 6> : attend_tc5_few_kernel<true, 96, 3>)
                                    : (one ? attend_tc5_few_kernel<false, 96, 6> : attend_tc5_few_kernel<false, 96, 3>));
   const size_t smem = one ? few_smem_bytes<6>() : few_smem_bytes<3>();
-  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = prepare_kernel(kern, smem);
   if (e != cudaSuccess) return e;
   return launch_pdl(kern, dim3(ctas), kFewThreads, smem, st, p, mk, mv, sa);
 }

@@ -287,11 +287,9 @@ cudaError_t launch_attend_mma(const Params& p, const __nv_bfloat16* q, const __n
     case 256: kernel = p.fp16 ? attend_mma_kernel<true, 256> : attend_mma_kernel<false, 256>; smem = sizeof(Smem<256>); break;
     default: return cudaErrorInvalidValue;
   }
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = prepare_kernel(kernel, smem);
   if (e != cudaSuccess) return e;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = device_info().sms;
   kernel<<<sms * (p.D > 128 ? 1 : 2), kThreads, smem, st>>>(p, q, k, v, cu, list_counts, list_offsets, tile_prefix,
                                                     row_list, partial_out, partial_lse, work_counter);
   return cudaGetLastError();

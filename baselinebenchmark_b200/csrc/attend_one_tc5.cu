@@ -412,7 +412,7 @@ template <bool kHalf, int D>
 cudaError_t launch_one(const Params& p, const CUtensorMap& mk, const CUtensorMap& mv, const ShortArgs& sa, int sms,
                        cudaStream_t st) {
   constexpr size_t smem = one_smem_bytes<D>();
-  const cudaError_t e = cudaFuncSetAttribute(attend_tc5_one_kernel<kHalf, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const cudaError_t e = prepare_kernel(attend_tc5_one_kernel<kHalf, D>, smem);
   if (e != cudaSuccess) return e;
   return launch_pdl(attend_tc5_one_kernel<kHalf, D>, dim3(sms), kOneThreads, smem, st, p, mk, mv, sa);
 }

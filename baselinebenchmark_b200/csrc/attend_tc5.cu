@@ -1540,9 +1540,7 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
                               const int32_t* row_list, __half* partial_out, float2* partial_lse,
                               int32_t* work_counter, int32_t* status, cudaStream_t st) {
   if (p.D != 64 && p.D != 96 && p.D != 128 && p.D != 256) return cudaErrorInvalidValue;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = device_info().sms;
   if (tc5_one_tile(p))
     return launch_attend_one_tc5(p, q, k, v, cu, list_counts, list_offsets, tile_prefix, row_list, partial_out, partial_lse,
                                  work_counter, status, sms, st);
@@ -1562,7 +1560,7 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
                            : (p.fp16 ? attend_tc5_short_kernel<true, 64> : attend_tc5_short_kernel<false, 64>);
     const int threads = p.D == 256 ? kWideShortThreads : kShortThreads, ctas = p.D == 256 ? sms : 2 * sms;
     const size_t smem = p.D == 256 ? kWideShortSmemBytes : kShortSmemBytes;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    e = prepare_kernel(kern, smem);
     if (e != cudaSuccess) return e;
     ShortArgs sa;
     sa.a = args;
@@ -1577,7 +1575,7 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
               : p.D == 128 ? (p.fp16 ? attend_tc5_kernel<true, 128> : attend_tc5_kernel<false, 128>)
               : p.D == 96  ? (p.fp16 ? attend_tc5_kernel<true, 96> : attend_tc5_kernel<false, 96>)
                            : (p.fp16 ? attend_tc5_kernel<true, 64> : attend_tc5_kernel<false, 64>);
-  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+  e = prepare_kernel(kernel, kSmemBytes);
   if (e != cudaSuccess) return e;
   return launch_pdl(kernel, dim3(sms), kThreads, kSmemBytes, st, p, mk, mv, args);
 }

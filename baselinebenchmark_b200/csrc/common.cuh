@@ -8,6 +8,7 @@
 
 #include <utility>
 
+#include "kernel_setup.cuh"
 #include "moba_b200.h"
 
 namespace moba {
@@ -247,7 +248,7 @@ constexpr int64_t kChainedMergeBytes = 64 << 20;
 constexpr int64_t kChainedMeanCtas = 148 * 8;
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(bool chained, void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st,
-                                  Args&&... args) {
+                                  const Args&... args) {
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -258,11 +259,17 @@ inline cudaError_t launch_chained(bool chained, void (*kernel)(KArgs...), dim3 g
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = chained ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e == cudaErrorInvalidValue && smem > 48 * 1024 &&
+      KernelSetup::instance().prepare(reinterpret_cast<const void*>(kernel), smem, nullptr, false, true) == cudaSuccess) {
+    cudaGetLastError();
+    e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  }
+  return e;
 }
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args&&... args) {
-  return launch_chained(true, kernel, grid, threads, smem, st, std::forward<Args>(args)...);
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
+  return launch_chained(true, kernel, grid, threads, smem, st, args...);
 }
 
 // Exclusive prefix sums over the lists, by one block of kThreads threads, kPer lists a thread and

@@ -1351,28 +1351,21 @@ cudaError_t launch_gate_topk_stats(const Params& p, const __nv_bfloat16* q, cons
     default: return cudaErrorInvalidValue;
   }
 #undef MOBA_GATE_W
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);
+  int regs = 0;
+  const cudaError_t e = prepare_kernel(kernel, g.smem, &regs, true);
   if (e != cudaSuccess) return e;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const DeviceInfo dev = device_info();
   const int64_t n_tiles = (int64_t)window_tiles(p, tokens_per_cta) * p.Hkv * p.B;
   if (n_tiles >= ((int64_t)1 << 31)) return cudaErrorInvalidConfiguration;
   // persistent CTAs: as many as are resident at once, by shared memory (1 KB per CTA is reserved),
   // registers (allocated in units of 8 per thread) and tensor memory (512 columns per SM)
-  cudaFuncAttributes attr;
-  if ((e = cudaFuncGetAttributes(&attr, kernel)) != cudaSuccess) return e;
-  if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100)) != cudaSuccess) return e;
-  int smem_per_sm = 0, regs_per_sm = 0;
-  cudaDeviceGetAttribute(&smem_per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-  cudaDeviceGetAttribute(&regs_per_sm, cudaDevAttrMaxRegistersPerMultiprocessor, dev);
-  int resident = (int)(smem_per_sm / (g.smem + 1024));
+  int resident = (int)(dev.smem_per_sm / (g.smem + 1024));
   const int threads = one ? kOneThreads : kGateThreads;
-  const int regs_per_cta = ((attr.numRegs + 7) / 8 * 8) * threads;
-  if (regs_per_cta > 0 && resident > regs_per_sm / regs_per_cta) resident = regs_per_sm / regs_per_cta;
+  const int regs_per_cta = ((regs + 7) / 8 * 8) * threads;
+  if (regs_per_cta > 0 && resident > dev.regs_per_sm / regs_per_cta) resident = dev.regs_per_sm / regs_per_cta;
   if (resident > 512 / g.nt) resident = 512 / g.nt;
   if (resident < 1) resident = 1;
-  int64_t grid = (int64_t)sms * resident;
+  int64_t grid = (int64_t)dev.sms * resident;
   if (grid > n_tiles) grid = n_tiles;
   return launch_chained(chained, kernel, dim3((unsigned)grid), threads, g.smem, st, p, mq, mm, tokens_per_cta, g.nt,
                         g.list_len, g.nbuf, g.cnt_in_smem, q, means, cu, selected, list_counts, stats, flags,

@@ -136,7 +136,7 @@ cudaError_t launch_scatter(const Params& p, const int32_t* cu, const int32_t* se
   const size_t smem = (size_t)p.mc * 2 * sizeof(int32_t);
   if (smem > 200 * 1024) return cudaErrorInvalidConfiguration;
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(scatter_routes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = prepare_kernel(scatter_routes_kernel, smem);
     if (e != cudaSuccess) return e;
   }
   dim3 grid(window_tiles(p, kScatterTokens), p.Hkv, p.B);
