@@ -16,12 +16,15 @@ LIB_PATH = Path(os.environ.get("MOBA_B200_LIB") or Path(__file__).resolve().pare
 ATTEND_TCGEN05 = 0
 ATTEND_MMA_SYNC = 1
 
+#: MOBA_KERNEL_*: what moba_problem_attend_kernel answers
+KERNEL_MMA_SYNC, KERNEL_ROWS_256, KERNEL_SHORT, KERNEL_ONE_TILE, KERNEL_FEW_ROWS, KERNEL_WIDE, KERNEL_WIDE_SHORT = range(7)
+
 #: every symbol include/moba_b200.h declares
 SYMBOLS = (
     "moba_b200_abi_version", "moba_b200_strerror", "moba_problem_check", "moba_problem_dims",
     "moba_workspace_size", "moba_workspace_size_min", "moba_forward", "moba_forward_events", "moba_forward_cached", "moba_append", "moba_workspace_size_host", "moba_forward_host",
     "moba_chunk_metadata", "moba_chunk_means", "moba_gate_topk", "moba_gate_topk_stats", "moba_compact_routes",
-    "moba_attend", "moba_merge", "moba_attend_tile_rows", "moba_attend_tile_rows_for", "moba_problem_tile_rows", "moba_route_static",
+    "moba_attend", "moba_merge", "moba_attend_tile_rows", "moba_attend_tile_rows_for", "moba_problem_tile_rows", "moba_problem_attend_kernel", "moba_route_static",
     "moba_backward_workspace_size", "moba_backward",
     "moba_cp_workspace_size", "moba_cp_forward", "moba_cp_poll", "moba_cp_abort", "moba_selftest_bounded_wait",
 )
@@ -93,6 +96,7 @@ def lib() -> C.CDLL:
         handle.moba_attend_tile_rows.argtypes = [C.c_int]
         handle.moba_attend_tile_rows_for.argtypes = [C.c_int, C.c_int]
         handle.moba_problem_tile_rows.argtypes = [pp]
+        handle.moba_problem_attend_kernel.argtypes = [pp]
         handle.moba_route_static.argtypes = [pp, vp, vp, i32p, i32p, vp]
         handle.moba_backward_workspace_size.argtypes = [pp, C.POINTER(sz)]
         handle.moba_backward.argtypes = [pp, vp, vp, vp, i32p, vp, vp, i32p, vp, vp, vp, vp, vp, sz, vp]

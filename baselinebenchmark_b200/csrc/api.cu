@@ -257,6 +257,12 @@ int moba_problem_tile_rows(const moba_problem_t* p) {
   return rc != MOBA_OK ? rc : tile_rows_of(p->attend_impl, p->head_dim, p->chunk_size);
 }
 
+int moba_problem_attend_kernel(const moba_problem_t* p) {
+  const int rc = check_problem(p);
+  if (rc != MOBA_OK) return rc;
+  return p->attend_impl == MOBA_ATTEND_MMA_SYNC ? (int)MOBA_KERNEL_MMA_SYNC : tc5_kernel(make_params(p));
+}
+
 int moba_workspace_size(const moba_problem_t* p, size_t* bytes) {
   const int rc = check_problem(p);
   if (rc != MOBA_OK) return rc;

@@ -1541,10 +1541,11 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
                               int32_t* work_counter, int32_t* status, cudaStream_t st) {
   if (p.D != 64 && p.D != 96 && p.D != 128 && p.D != 256) return cudaErrorInvalidValue;
   const int sms = device_info().sms;
-  if (tc5_one_tile(p))
+  const int which = tc5_kernel(p);
+  if (which == MOBA_KERNEL_ONE_TILE)
     return launch_attend_one_tc5(p, q, k, v, cu, list_counts, list_offsets, tile_prefix, row_list, partial_out, partial_lse,
                                  work_counter, status, sms, st);
-  if (tc5_few_rows(p))
+  if (which == MOBA_KERNEL_FEW_ROWS)
     return launch_attend_few_tc5(p, q, k, v, cu, list_counts, list_offsets, tile_prefix, row_list, partial_out, partial_lse,
                                  work_counter, status, sms, st);
   CUtensorMap mk, mv;
@@ -1553,7 +1554,7 @@ cudaError_t launch_attend_tc5(const Params& p, const __nv_bfloat16* q, const __n
   const KernelArgs args{q, cu, list_counts, list_offsets, tile_prefix, row_list, partial_out, partial_lse,
                         work_counter, status, ((uintptr_t)partial_out & 31) == 0};
   cudaError_t e;
-  if (p.D == 256 ? p.C <= kSmallChunk : tc5_short_items(p)) {
+  if (which == MOBA_KERNEL_WIDE_SHORT || which == MOBA_KERNEL_SHORT) {
     auto kern = p.D == 256 ? (p.fp16 ? attend_tc5_wide_short_kernel<true> : attend_tc5_wide_short_kernel<false>)
               : p.D == 128 ? (p.fp16 ? attend_tc5_short_kernel<true, 128> : attend_tc5_short_kernel<false, 128>)
               : p.D == 96  ? (p.fp16 ? attend_tc5_short_kernel<true, 96> : attend_tc5_short_kernel<false, 96>)

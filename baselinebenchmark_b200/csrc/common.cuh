@@ -420,19 +420,59 @@ inline bool tc5_short_items(const Params& p) {
 //   head dim 64   chunk 128  1: 1.19 / 1.17 / 1.22   4: 1.23 / 1.19 / 1.23   16: 1.02 / 1.22 / 1.27
 //                 chunk 96   1: 1.13 / 1.15 / 1.19   4: 1.15 / 1.17 / 1.21   16: 0.92 / 1.10 / 1.18
 //                 chunk 64   1: 0.91 / 1.01 / 1.09   4: 0.90 / 1.01 / 1.10   16: 0.75 / 0.91 / 1.05
-// So: three tiles a list (rows of a list: ranks x chunk x heads of a group), and chunks of 64 to 95 keys at head dim 64 with seven ranks.
+// So: three tiles a list (ranks x chunk x heads of a group, in a long sequence whose tokens are all queries), and chunks of 64 to 95 keys
+// at head dim 64 with seven ranks.
+// A window of queries, or short sequences, have the lists of their whole prefix and few rows on each: what counts there is the rows that a
+// list has on average (one_tile_rows), and a call of at most kOneTileFewItems items, where an SM has one or none, takes this
+// kernel whatever they are.  Dense stage, this kernel against the one for short items (us), with the average:
+//   18 rows   1000 tokens behind 50000, 16/16 heads, chunk 128, top-k 8   264 / 104
+//   19        1254 behind 24248, 8/8, chunk 128, top-k 4                   77 / 36
+//   221       50 sequences, 20476 tokens, 16/16, chunk 96, top-k 8        217 / 170
+//   275       42 sequences, 6125 tokens, 32/8, chunk 96, top-k 3           88 / 63
+//   358       3000 tokens, 16/16, chunk 128, top-k 4                     36.9 / 38.9
+//   433       45 sequences, 35790 tokens, 16/16, chunk 96, top-k 12       421 / 439
+//   497       9 sequences, 5068 tokens, 32/16, chunk 128, top-k 4        66.6 / 71.7
+//   300 tokens, 16/4 heads, chunk 128, top-k 8 (46 items)                14.4 / 16.4
+// By rows x keys of a list (chunks of 96 keys want a third more rows), over 380 calls of 130 to 60000 tokens, one sequence, batches and
+// windows: lines of 256 to 448 rows of 128 keys choose within 0.3 % of the faster call on average, without one it was 3.5 %
+// (at worst 1.85 x); at head dim 64 of 160 to 256.
 // Windows of at most 128 rows per kv head (few items, whose own-chunk ones cover the heads of a group) stay with the kernel for short items,
 // and so does a q of more than 64 GB (row offsets are 32 bits there, in 16-byte pieces).
+constexpr int kOneTileFewItems = 64;
+// Rows of a list on average, as far as the host can tell: sequences taken to be of one length, a window to lie at the end of its prefix.
+inline double one_tile_rows(const Params& p) {
+  const double group_chunk = (double)p.G * p.C, hist = p.hist;
+  if (p.Tq < p.T) {
+    int64_t prefix = p.max_seqlen > p.Tq ? p.max_seqlen : p.Tq;
+    if (prefix > p.T) prefix = p.T;
+    return group_chunk * hist * (double)p.Tq / (double)prefix;
+  }
+  const double chunks = (double)p.T / ((double)p.B * p.C);   // of a sequence: the first is nobody's list, its tokens select nothing
+  if (chunks <= 1) return 0;
+  const double ranks = chunks >= hist + 1 ? hist * (chunks - (hist + 1) / 2) : chunks * (chunks - 1) / 2;
+  return group_chunk * ranks / (chunks > 2 ? chunks - 1 : 1);
+}
 inline bool tc5_one_tile(const Params& p) {
   const bool keys = p.C >= 96 || (p.D == 64 && p.C >= 64 && p.hist >= 7);
-  return tc5_short_items(p) && p.C <= 128 && keys && (int64_t)p.hist * p.C * p.G >= 3 * kTileRowsWide &&
-         p.Tq * p.G > kTileRowsWide && (p.Tq - 1) * p.sq_t + (p.Hq - 1) * p.sq_h < ((int64_t)1 << 35);
+  if (!tc5_short_items(p) || p.C > 128 || !keys || (int64_t)p.hist * p.C * p.G < 3 * kTileRowsWide || p.Tq * p.G <= kTileRowsWide ||
+      (p.Tq - 1) * p.sq_t + (p.Hq - 1) * p.sq_h >= ((int64_t)1 << 35))
+    return false;
+  const int64_t items = (p.T * p.Hkv + p.rows) / p.C;
+  return items <= kOneTileFewItems || one_tile_rows(p) * p.C >= (p.D == 64 ? 256 : 288) * 128.0;
 }
 // Windows of at most this many rows per kv head (decode steps) run a kernel that has keys, not rows, as the lanes of tensor memory
 // (figures and the reason for eight there; chunks of any length: the shortest make no difference).
 constexpr int kFewRows = 8;
 inline bool tc5_few_rows(const Params& p) {
   return (p.D == 96 || p.D == 128) && p.Tq * p.G <= kFewRows;
+}
+
+// The kernel of the tcgen05 dense stage that runs a problem (MOBA_KERNEL_* of moba_b200.h).
+inline int tc5_kernel(const Params& p) {
+  if (p.D == 256) return p.C <= kSmallChunk ? MOBA_KERNEL_WIDE_SHORT : MOBA_KERNEL_WIDE;
+  if (tc5_one_tile(p)) return MOBA_KERNEL_ONE_TILE;
+  if (tc5_few_rows(p)) return MOBA_KERNEL_FEW_ROWS;
+  return tc5_short_items(p) ? MOBA_KERNEL_SHORT : MOBA_KERNEL_ROWS_256;
 }
 
 cudaError_t launch_attend_mma(const Params& p, const __nv_bfloat16* q, const __nv_bfloat16* k,

@@ -362,6 +362,19 @@ int moba_attend_tile_rows(int attend_impl);
 int moba_attend_tile_rows_for(int attend_impl, int head_dim);
 int moba_problem_tile_rows(const moba_problem_t* p);
 
+/* Which kernel runs the dense stage of a problem (of each pass, where the kv heads are processed in groups
+ * the query is about the group's problem).  The results do not depend on it. */
+enum {
+  MOBA_KERNEL_MMA_SYNC = 0,
+  MOBA_KERNEL_ROWS_256 = 1,   /* tcgen05, two 128-row tiles an item                        */
+  MOBA_KERNEL_SHORT = 2,      /* short chunks and small query windows, one tile an item    */
+  MOBA_KERNEL_ONE_TILE = 3,   /* chunks of one key tile, several items in flight           */
+  MOBA_KERNEL_FEW_ROWS = 4,   /* decode steps                                              */
+  MOBA_KERNEL_WIDE = 5,       /* head_dim 256                                              */
+  MOBA_KERNEL_WIDE_SHORT = 6  /* head_dim 256, chunks of at most 256 keys                  */
+};
+int moba_problem_attend_kernel(const moba_problem_t* p);
+
 #ifdef __cplusplus
 }
 #endif
