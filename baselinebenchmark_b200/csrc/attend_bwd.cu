@@ -824,10 +824,7 @@ cudaError_t set_smem(K kernel, size_t bytes) {
   return prepare_kernel(kernel, bytes);
 }
 
-int sm_count() {
-  const int sms = device_info().sms;
-  return sms;
-}
+int sm_count() { return device_info().sms; }
 
 }  // namespace
 

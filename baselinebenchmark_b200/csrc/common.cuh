@@ -259,13 +259,7 @@ inline cudaError_t launch_chained(bool chained, void (*kernel)(KArgs...), dim3 g
   cfg.stream = st;
   cfg.attrs = &attr;
   cfg.numAttrs = chained ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
-  if (e == cudaErrorInvalidValue && smem > 48 * 1024 &&
-      KernelSetup::instance().prepare(reinterpret_cast<const void*>(kernel), smem, nullptr, false, true) == cudaSuccess) {
-    cudaGetLastError();
-    e = cudaLaunchKernelEx(&cfg, kernel, args...);
-  }
-  return e;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st, const Args&... args) {
