@@ -170,17 +170,26 @@ attend_tc5_few_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_k
     // ---- descriptions
     ShortQueue w;
     short_start(sa.iq, c, w);
-    for (int n = 0;; ++n) {
+    int n = 0;
+    for (bool done = false; ok && !done;) {
       FewItem o;
       short_pick<true>(p, sa.iq, c, w, o.s, o.s.tok0, o.s.head, o.rows_at, o.qhead);
-      const int slot = n % kFewSlots;
-      if (n >= kFewSlots && !wait(&c.slot_free[slot], (n / kFewSlots - 1) & 1)) break;
-      if (lane == 0) {
-        c.item[slot] = o;
-        mbar_arrive(smem_u32(&c.item_full[slot]));
-      }
-      __syncwarp();
-      if (o.s.done) break;
+      done = o.s.done;
+      // (the lists of a selection that names a chunk for several ranks of a row are longer than the window has rows)
+      int rows = o.s.nrows;
+      do {
+        o.s.nrows = min(rows, kFewRows);
+        const int slot = n % kFewSlots;
+        if (n >= kFewSlots && !wait(&c.slot_free[slot], (n / kFewSlots - 1) & 1)) break;
+        if (lane == 0) {
+          c.item[slot] = o;
+          mbar_arrive(smem_u32(&c.item_full[slot]));
+        }
+        __syncwarp();
+        ++n;
+        o.rows_at += kFewRows;
+        rows -= kFewRows;
+      } while (rows > 0);
     }
     if (!ok && lane == 0) { atomicExch(a.status, ST_PRODUCER); c.abort = 1; }
   } else if (warp == 7) {

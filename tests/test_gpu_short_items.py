@@ -347,3 +347,40 @@ def test_a_call_waits_for_its_inputs_from_another_stream(chunk, topk):
             graph.replay()
             main.synchronize()
             assert torch.equal(out, want[i])
+
+
+@pytest.mark.parametrize("rows,hq,hkv", [(1, 8, 1), (2, 8, 2), (1, 3, 3)])
+@pytest.mark.parametrize("d,dtype", [(96, torch.float16), (128, torch.bfloat16)])
+def test_a_list_with_a_row_several_times(d, dtype, rows, hq, hkv):
+    """The staged entry points take any selection, also one that names a chunk for several ranks of a row: a list of a decode window is
+    then longer than the window has rows per kv head.  Every rank gets its partial result, those of the mma.sync stage."""
+    chunk, topk, total = 200, 5, 1500
+    q, k, v, cu = _inputs((total,), hq, hkv, d, chunk, dtype, seed=rows + d)
+    q = q[-rows:].contiguous()
+    out = torch.empty_like(q)
+    sel = torch.full((topk - 1, hq, rows), 2, dtype=torch.int32, device="cuda")
+    sel[3] = 5                                                # slot 2 three times, slot 5 once
+    parts = []
+    for impl in (_lib.ATTEND_TCGEN05, _lib.ATTEND_MMA_SYNC):
+        prob = parallel.make_problem(q, k, v, out, cu, total, chunk, topk, impl, total - rows)
+        dims = G.dims_of(prob)
+        assert _lib.lib().moba_problem_attend_kernel(C.byref(prob)) == (
+            _lib.KERNEL_FEW_ROWS if impl == _lib.ATTEND_TCGEN05 else _lib.KERNEL_MMA_SYNC)
+        counts = torch.zeros(dims.lists, dtype=torch.int32, device="cuda").view(-1, hkv)
+        counts[2], counts[5] = 3 * rows * hq // hkv, rows * hq // hkv
+        counts = counts.reshape(-1).contiguous()
+        offsets, tiles, row_list, plse = G.compact(prob, cu, sel, counts, _lib.lib().moba_problem_tile_rows(C.byref(prob)))
+        partial = torch.full((dims.rows * dims.partials, d), 7.0, dtype=torch.float16, device="cuda")
+        work = torch.zeros(2, dtype=torch.int32, device="cuda")
+        plse.fill_(-9.0)
+        _lib.check(_lib.lib().moba_attend(C.byref(prob), q.data_ptr(), k.data_ptr(), v.data_ptr(), cu.data_ptr(), counts.data_ptr(),
+                                          offsets.data_ptr(), tiles.data_ptr(), row_list.data_ptr(), partial.data_ptr(),
+                                          plse.data_ptr(), work.data_ptr(), G.stream()))
+        torch.cuda.synchronize()
+        assert work[1].item() == 0
+        parts.append((partial.float() * plse[:, 1:], plse[:, 0].clone()))
+    (a, la), (b, lb) = parts
+    assert (la - lb).abs().max().item() < 1e-3               # scores in fp32, exponentials to 7.5e-5
+    _close(a, b, dtype)
+    by_rank = a.view(rows * hq, topk, d)
+    assert torch.equal(by_rank[:, 1], by_rank[:, 2]) and torch.equal(by_rank[:, 1], by_rank[:, 3])
