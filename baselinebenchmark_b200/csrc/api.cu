@@ -14,6 +14,11 @@
 
 using namespace moba;
 
+KernelSetup& KernelSetup::instance() {
+  static KernelSetup s;
+  return s;
+}
+
 namespace {
 
 // rows per work item of the dense stage: the tcgen05 kernel takes two 128-row tiles per item up to

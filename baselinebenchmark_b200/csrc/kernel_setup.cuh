@@ -21,10 +21,9 @@ struct DeviceInfo {
 
 class KernelSetup {
  public:
-  static KernelSetup& instance() {
-    static KernelSetup s;
-    return s;
-  }
+  // Defined in one source file and not here: the static object of an inline function is one for the whole process, also for two builds
+  // of this library that are loaded side by side and may not agree on what it looks like.
+  static KernelSetup& instance();
   // Of the current device.
   DeviceInfo device() {
     DeviceInfo info{148, 0, 0};

@@ -8,6 +8,8 @@ from pathlib import Path
 
 import pytest
 
+from baselinebenchmark_b200 import build
+
 CSRC = Path(__file__).resolve().parent.parent / "baselinebenchmark_b200" / "csrc"
 CUDA_INCLUDE = Path("/usr/local/cuda/include")
 
@@ -47,6 +49,7 @@ cudaError_t cudaGetDriverEntryPoint(const char* name, void** f, unsigned long lo
 }
 }
 using moba::KernelSetup;
+KernelSetup& KernelSetup::instance() { static KernelSetup s; return s; }
 static const void* kernel(int i) { return (const void*)(uintptr_t)(0x400000 + 48 * i); }
 // a launch may rely on this much: what the call leaves behind is what the current context has
 static void use(int i, size_t smem, bool carve = false) {
@@ -96,3 +99,12 @@ def test_what_is_set_is_set_in_every_context(tmp_path):
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(CSRC), "-I", str(CUDA_INCLUDE), "-x", "c++", str(source), "-o",
                     str(tmp_path / "setup")], check=True)
     assert subprocess.run([str(tmp_path / "setup")], capture_output=True, text=True, check=True).stdout == "ok\n"
+
+
+@pytest.mark.skipif(shutil.which("nm") is None, reason="needs nm")
+def test_the_library_shares_no_object_with_another_build_of_it():
+    """A symbol of type u (STB_GNU_UNIQUE) is one object for the whole process, whichever library it is in: two builds of this one that are
+    loaded side by side would work on one table."""
+    symbols = subprocess.run(["nm", "-D", str(build.build())], capture_output=True, text=True, check=True).stdout
+    assert "moba_forward" in symbols
+    assert [line for line in symbols.splitlines() if line.split()[-2] == "u"] == []
