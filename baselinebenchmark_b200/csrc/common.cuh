@@ -429,7 +429,7 @@ inline bool tc5_short_items(const Params& p) {
 //   300 tokens, 16/4 heads, chunk 128, top-k 8 (46 items)                14.4 / 16.4
 // By rows x keys of a list (chunks of 96 keys want a third more rows), over 380 calls of 130 to 60000 tokens, one sequence, batches and
 // windows: lines of 256 to 448 rows of 128 keys choose within 0.3 % of the faster call on average, without one it was 3.5 %
-// (at worst 1.85 x); at head dim 64 of 160 to 256.
+// (at worst 1.85 x); at head dim 64 of 160 to 256, where 192 keeps the last entry of the table's last row here.
 // Windows of at most 128 rows per kv head (few items, whose own-chunk ones cover the heads of a group) stay with the kernel for short items,
 // and so does a q of more than 64 GB (row offsets are 32 bits there, in 16-byte pieces).
 constexpr int kOneTileFewItems = 64;
@@ -452,7 +452,7 @@ inline bool tc5_one_tile(const Params& p) {
       (p.Tq - 1) * p.sq_t + (p.Hq - 1) * p.sq_h >= ((int64_t)1 << 35))
     return false;
   const int64_t items = (p.T * p.Hkv + p.rows) / p.C;
-  return items <= kOneTileFewItems || one_tile_rows(p) * p.C >= (p.D == 64 ? 256 : 288) * 128.0;
+  return items <= kOneTileFewItems || one_tile_rows(p) * p.C >= (p.D == 64 ? 192 : 288) * 128.0;
 }
 // Windows of at most this many rows per kv head (decode steps) run a kernel that has keys, not rows, as the lanes of tensor memory
 // (figures and the reason for eight there; chunks of any length: the shortest make no difference).

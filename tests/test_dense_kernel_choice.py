@@ -70,6 +70,8 @@ def test_batches_of_short_sequences_have_few_rows_a_list(lib):
     assert _kernel(lib, (563,) * 9, 32, 16, 128, 128, 4) == ONE_TILE
     # so few items that an SM has one or none: whatever the lists
     assert [_kernel(lib, 512, h, h, 128, 128, 4) for h in (4, 8, 9, 16)] == [ONE_TILE, ONE_TILE, SHORT, SHORT]
+    # head dim 64, chunks of 64 keys with seven ranks
+    assert _kernel(lib, 20000, 16, 16, 64, 64, 8) == ONE_TILE and _kernel(lib, (400,) * 50, 16, 16, 64, 64, 8) == SHORT
     # the workloads of the benchmark list
     assert _kernel(lib, (4096, 4096), 16, 16, 128, 128, 8) == ONE_TILE
     assert _kernel(lib, (1023, 4097, 8191), 16, 4, 64, 128, 8) == ONE_TILE
