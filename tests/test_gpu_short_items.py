@@ -32,6 +32,11 @@ def _close(out, ref, dtype):
     assert mx <= 8 * unit and mean <= 0.25 * unit, (mx, mean)
 
 
+def _kernel(q, k, v, cu, max_len, chunk, topk, begin=None):
+    prob = parallel.make_problem(q, k, v, torch.empty_like(q), cu, max_len, chunk, topk, None, begin)
+    return _lib.lib().moba_problem_attend_kernel(C.byref(prob))
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("d", [64, 96, 128, 256])
 @pytest.mark.parametrize("chunk", [16, 64, 127, 128, 129, 200, 256, 257, 512, 513, 1025])
@@ -50,14 +55,16 @@ def test_chunk_sizes_around_the_tiles(chunk, d, dtype):
 @pytest.mark.parametrize("chunk", [63, 64, 95, 96, 128])
 @pytest.mark.parametrize("lens,hq,hkv", [((5000,), 16, 1), ((700, 9000), 16, 4), ((4100, 3, 4095), 12, 12), ((33,), 16, 2)])
 def test_streams_of_one_tile_items(lens, hq, hkv, chunk, d, dtype):
-    """Chunks of at most 128 keys (64 of them at head dim 64, 96 and up at the others): a CTA's items run through a ring of descriptions, of Q, K and V tiles and of places in tensor
-    memory, each many times over in the longer calls; lists of many tiles (few kv heads) and of one, K and V shared by the heads
-    of a group and not.  A window of more rows than one tile runs the same kernel, one of fewer rows the kernel for short
-    items: the same bits."""
+    """Chunks of 96 to 128 keys (64 and up at head dim 64) on the one-tile kernel, below and in small calls the kernel for short items: a CTA's
+    items run through a ring of descriptions, of Q, K and V tiles and of places in tensor memory, each many times over in the
+    longer calls; lists of many tiles (few kv heads) and of one, K and V shared by the heads of a group and not.  Windows, some of
+    more rows than one tile, run either kernel: the same bits."""
     topk = 9
     q, k, v, cu = _inputs(lens, hq, hkv, d, chunk, dtype, seed=chunk + d + hq)
     q *= 3                                                   # a moving softmax reference
     args = (k, v, cu, max(lens), chunk, topk)
+    one_tile = chunk >= (64 if d == 64 else 96) and lens != (33,)
+    assert _kernel(q, *args) == (_lib.KERNEL_ONE_TILE if one_tile else _lib.KERNEL_SHORT)
     out, lse, sel = parallel.moba_forward(q, *args, return_lse=True, return_selected=True)
     ref, ref_lse, ref_sel = parallel.moba_forward(q, *args, return_lse=True, return_selected=True,
                                                   attend_impl=_lib.ATTEND_MMA_SYNC)
@@ -151,6 +158,7 @@ def test_decode_windows_of_up_to_eight_rows(d, dtype, chunk, hq, hkv):
     limit = 8 // (hq // hkv)
     for begin in (0, 699, 700 + 505, 700 + 4095, sum(lens) - limit - 1):
         for n in sorted({1, limit, limit + 1}):
+            assert _kernel(q[begin:begin + n], *args, begin) == (_lib.KERNEL_FEW_ROWS if n <= limit else _lib.KERNEL_SHORT)
             o, l, s = parallel.moba_forward(q[begin:begin + n], *args, return_lse=True, return_selected=True, q_token_begin=begin)
             assert torch.equal(s, sel[:, :, begin:begin + n])
             assert torch.equal(o, full[begin:begin + n]), (begin, n)
@@ -347,6 +355,62 @@ def test_a_call_waits_for_its_inputs_from_another_stream(chunk, topk):
             graph.replay()
             main.synchronize()
             assert torch.equal(out, want[i])
+
+
+@pytest.mark.parametrize("layout", ["fused", "head_major", "padded_dim", "odd_token"])
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d", [96, 128])
+@pytest.mark.parametrize("hq,hkv,topk,n", [(16, 16, 12, 1), (16, 16, 12, 8), (8, 2, 6, 2)])
+def test_decode_windows_over_layouts_and_types(hq, hkv, topk, n, d, dtype, layout):
+    """The kernel for few rows with more items than SMs (two CTAs on one, three K/V tiles each) and with fewer (six), both types, q in other
+    layouts: the bits of the full run on contiguous rows."""
+    chunk, total = 128, 4500
+    q, k, v, cu = _inputs((total,), hq, hkv, d, chunk, dtype, seed=d + topk)
+    args = (k, v, cu, total, chunk, topk)
+    out, lse, sel = parallel.moba_forward(q, *args, return_lse=True, return_selected=True)
+    ql = _layouts(q, layout)
+    assert torch.equal(ql, q)
+    for begin in (total - n, 4352 - n // 2):                  # the end of the sequence; across the boundary of a chunk
+        w = ql[begin:begin + n]
+        assert _kernel(w, *args, begin) == _lib.KERNEL_FEW_ROWS
+        o, l, s = parallel.moba_forward(w, *args, return_lse=True, return_selected=True, q_token_begin=begin)
+        assert torch.equal(s, sel[:, :, begin:begin + n])
+        assert torch.equal(o, out[begin:begin + n]) and torch.equal(l, lse[:, begin:begin + n])
+
+
+def _same(a, b):
+    """Equal, NaN in the same places."""
+    return torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a[~torch.isnan(a)], b[~torch.isnan(b)])
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("d", [64, 96, 128])
+@pytest.mark.parametrize("where", ["q", "k", "v"])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 6e4])
+def test_values_that_are_not_finite_on_every_kernel_of_short_chunks(value, where, d, dtype):
+    """Infinities, NaN and values whose products overflow the partial rows' or the scores' type, in a row in seven of one input: the
+    one-tile kernel, the kernel for short items and (head dims 96 and 128) the one for few rows give the same bits, NaN in the same places."""
+    hq, hkv, chunk, topk, total = 8, 4, 128, 5, 4000
+    q, k, v, cu = _inputs((total,), hq, hkv, d, chunk, dtype, seed=d)
+    g = torch.Generator(device="cuda").manual_seed(d)
+    x = {"q": q, "k": k, "v": v}[where]
+    hit = torch.rand(x.shape[:2], device="cuda", generator=g) < (1 / 7 if where == "q" else 1 / 200)
+    dim = torch.randint(0, d, hit.shape, device="cuda", generator=g)
+    x[hit] = x[hit].scatter(1, dim[hit][:, None], value)
+    args = (k, v, cu, total, chunk, topk)
+    assert _kernel(q, *args) == _lib.KERNEL_ONE_TILE
+    out, lse, sel = parallel.moba_forward(q, *args, return_lse=True, return_selected=True)
+    if value != 6e4:
+        assert not torch.isfinite(out).all()
+    assert torch.isfinite(out).any()
+    ran = set()
+    for begin, n in ((0, 64), (700, 64), (1111, 5), (2048, 4), (2049, 3), (2900, 4), (3991, 2), (3996, 4), (3999, 1)):
+        w = q[begin:begin + n]
+        ran.add(_kernel(w, *args, begin))
+        o, l, s = parallel.moba_forward(w, *args, return_lse=True, return_selected=True, q_token_begin=begin)
+        assert torch.equal(s, sel[:, :, begin:begin + n])
+        assert _same(o, out[begin:begin + n]) and _same(l, lse[:, begin:begin + n]), (begin, n)
+    assert ran == ({_lib.KERNEL_SHORT} if d == 64 else {_lib.KERNEL_SHORT, _lib.KERNEL_FEW_ROWS})
 
 
 @pytest.mark.parametrize("rows,hq,hkv", [(1, 8, 1), (2, 8, 2), (1, 3, 3)])
