@@ -4,6 +4,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "fast_div.cuh"
 #include "sm100_ptx.cuh"
 
 namespace moba {
@@ -49,19 +50,6 @@ __device__ __forceinline__ int find_list(const CtrlT& c, const int32_t* __restri
   // tile_prefix[l + 2^shift] > i, or the lists end before
   return l + search_warp(min(1 << shift, (int)lists - l), i, [&](int k) { return __ldg(tile_prefix + l + k); });
 }
-
-// x / d for x < 2^31 as a product: umulhi(2 x, mul) >> shift, with mul = ceil(2^(31 + shift) / d) and 2^shift >= d.  mul d exceeds
-// 2^(31 + shift) by less than d, and x times that stays below 2^(31 + shift): the quotient is never one too large.
-struct FastDiv {
-  uint32_t mul, shift;
-};
-inline FastDiv fast_div(int64_t d) {
-  FastDiv f{0, 0};
-  while ((1ll << f.shift) < d) ++f.shift;
-  f.mul = (uint32_t)(((1ull << (31 + f.shift)) + (uint64_t)d - 1) / (uint64_t)d);
-  return f;
-}
-__device__ __forceinline__ int operator/(int x, const FastDiv& f) { return (int)(__umulhi(2u * (uint32_t)x, f.mul) >> f.shift); }
 
 // Where the items come from.
 struct ItemQueue {
@@ -128,8 +116,12 @@ __device__ __forceinline__ int short_draw(const ItemQueue& a, const CtrlT& c) {
   return (threadIdx.x & 31) != 0 ? 0 : c.abort ? 0x3fffffff : atomicAdd(a.work_counter, 1);
 }
 // A draw that is asked for before the one in hand is used up.  A CTA that describes its items far ahead would draw several before
-// others have started, so the first kDealt draws of every CTA are dealt out instead: CTA b has draws b, b + CTAs, ... .  One decode
-// step on 131072 tokens (168 items, up to 232 CTAs): dense stage 61 or 92 us from run to run without, 60 with it.
+// others have started, so the first draws of every CTA are dealt out instead: CTA b has draws b, b + CTAs, ... .  Nine is what a CTA can
+// draw before its first item is done (eight descriptions of one-tile items ahead, and the draw ahead).  Dense stage (us) with 0 / 1 / 2 / 9 dealt:
+//   one decode step on 131072 tokens, 8/1 heads, top-k 12 (32 items at most)   86.0 / 51.2 / 51.2 / 51.2
+//   32/8 and 16/16 heads, and behind 20479 and 65536 tokens                  all the same (63.5, 49.2, 16.4, 30.7)
+//   one-tile items: 2 x 4096 x 16 119.8 / 117.8 / 118.8 / 115.7, 32768 x 32/8 1020 / 1014 / 1022 / 1022, 13311 x 16/4 at head dim 64
+//   112 / 112 / 111 / 112: what is dealt in advance costs no balance there (the runs of one side differ by 3 %)
 constexpr int kDealt = 9;
 template <typename CtrlT>
 __device__ __forceinline__ int short_draw_ahead(const ItemQueue& a, const CtrlT& c, ShortQueue& w) {
