@@ -407,9 +407,9 @@ static int forward_pass(const moba_problem_t* p, int64_t sel_rs, const void* q, 
     const bool fused = gate_scans_lists(r);
     const ListScan scan{w.list_counts, w.list_offsets, w.tile_prefix, w.cursors, r.lists,
                         tile_rows_of(p->attend_impl, p->head_dim, p->chunk_size)};
-    const int64_t mean_ctas = (int64_t)(r.slots - (opt.means_ext ? opt.means_from : 0)) * r.Hkv;
+    const int64_t mean_pairs = (int64_t)(r.slots - (opt.means_ext ? opt.means_from : 0)) * r.Hkv;
     if ((e = launch_gate_topk(r, qb, means, cu, sel, w.list_counts, st, fused ? &scan : nullptr, w.status + 1,
-                              mean_ctas <= kChainedMeanCtas)) != cudaSuccess)
+                              mean_pairs <= kChainedMeanPairs)) != cudaSuccess)
       return (int)e;
     if (last && (e = mark(2)) != cudaSuccess) return (int)e;
     e = fused ? launch_scatter(r, cu, sel, w.list_offsets, w.cursors, w.row_list, w.partial_lse, st)

@@ -22,8 +22,10 @@
 //   131072, 8/1, top-k 12       71.5 -> 47.8 (95 -> 70)    few items: the chain of a tile, 2700 cycles
 //   34816, 8/1, chunk 2048, head dim 96   38.2 -> 27.2 (58 -> 46)
 //   65536, 32/8, chunk 1024     30.2 -> 21.0;  20479, chunk 512 19.7 -> 16.3;  5000, chunk 128 12.3 -> 12.0
-// Eight rows, because the exponentials of more do not fit beside three K/V tiles and a second CTA; head dim 64 stays with the
-// kernel for short items (64 dims do not fill the lanes).  Six K/V tiles for one CTA per SM: 16/16 46.6 -> 45.9.
+// Eight rows, because the exponentials of more do not fit beside three K/V tiles and a second CTA.  Head dim 64 stays with the kernel for
+// short items: a form of this one for it (O^T with M = 64, tiles of half the bytes) has not been built.
+// Six K/V tiles instead of three where one CTA per SM has all items, chunk 4096: 131072 and 65536 tokens, 16/16 and 8/8 heads 47.1 -> 45.1 us (whole
+// step 143.4 -> 141.8, 80.9 -> 79.4); 20479 tokens, 16/4 49.2 both; chunk 1024 20.5 both; 8/1, top-k 12 50.2 / 51.2.
 #include "attend_rows.cuh"
 #include "common.cuh"
 #include "short_items.cuh"

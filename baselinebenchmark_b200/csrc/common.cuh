@@ -6,8 +6,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <utility>
-
 #include "kernel_setup.cuh"
 #include "moba_b200.h"
 
@@ -239,13 +237,15 @@ __host__ __device__ inline int own_item_count(int slots, int Hq, int C, int tile
 //   - the merge itself is not chained from kChainedMergeBytes of partial rows on (131072 tokens x 16, head_dim 64,
 //     chunk 64, 2.1 GB: 6.83 -> 6.62 ms; 32768 x 32/8, chunk 1024, 1.1 GB 3.98 -> 3.85; 32768 x 32/8, head_dim 128,
 //     chunk 128, 2.1 GB 2.27 -> 2.22; 13311 x 16, 0.22 GB 332 -> 329 us; a decode step's 16 KB: 161 -> 163);
-//   - the gating kernel is not chained behind chunk means of more CTAs than are resident at a time (130859 tokens,
-//     chunk 128, 16 heads, 700 new tokens: 434 -> 413 us; few chunks: 1 to 3 us slower).
+//   - the gating kernel is not chained behind the means of more (slot, kv head) pairs than have a CTA resident at a time with
+//     one CTA a pair (130859 tokens, chunk 128, 16 heads, 700 new tokens: 434 -> 413 us; few chunks: 1 to 3 us slower).  At head
+//     dim 256 a pair has four CTAs, and chaining is the better way up to there too: 96 pairs 81.2 -> 78.0 us, 384 186 -> 184, 648
+//     84.9 -> 81.2, 1024 449 -> 445.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 constexpr int64_t kTriggerMeanBytes = 8 << 20;
 constexpr int64_t kChainedMergeBytes = 64 << 20;
-constexpr int64_t kChainedMeanCtas = 148 * 8;
+constexpr int64_t kChainedMeanPairs = 148 * 8;
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_chained(bool chained, void (*kernel)(KArgs...), dim3 grid, int threads, size_t smem, cudaStream_t st,
                                   const Args&... args) {

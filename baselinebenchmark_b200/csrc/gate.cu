@@ -250,7 +250,7 @@ constexpr int kGateRows = 128;            // (token, head) rows per tile
 constexpr int kListExtra = 3;             // list places beyond hist + 1 that absorb near-ties at the cut
 constexpr int kCntSmemMax = 4096;         // chunks per sequence up to which the list histogram is kept in shared memory
 constexpr int kQBlockBytes = 128 * 128;   // one [128 rows][64 dims] swizzled block of 16-bit values
-// floats per row of the score scratch, for the keys a network leaves (w) or, without one (0), all 32 of a step: an odd
+// floats per row of the score scratch, for the values a network leaves (w) or, without one (0), all 32 of a step: an odd
 // number of 16-byte pieces, so that 16-byte stores are free of conflicts
 __host__ __device__ constexpr int scratch_stride(int w) { return (w > 0 ? w : 32) + 4; }
 // (rows of one step of 32 candidates have nothing to merge)
@@ -392,7 +392,7 @@ constexpr uint32_t kTied = 1u << 30, kRunStart = 1u << 29, kChunkMask = 0x00FFFF
 
 // Resident CTAs per SM the register budget is set for: four with the narrow network (its
 // working set is small and the kernel is bound by the latency of dependent instructions, which
-// more warps hide), three otherwise (a fourth would spill the 32 keys of the wide network).
+// more warps hide), three otherwise (a fourth would spill the 32 values of the wide network).
 template <int kW> constexpr int kGateMinCtas = kW == 8 ? 4 : 3;
 
 struct GateTile {
@@ -418,14 +418,14 @@ __device__ __forceinline__ GateTile gate_tile(const Params& p, const int32_t* __
   return t;
 }
 
-// eps of a row is this times |q|_2 max|m|_2 (see the head of this section); kKeys: the estimates went through the keys
-// with the position in their low bits
-template <int D, bool kKeys> constexpr float gate_kappa =
-    ((18.f * (D / 16) + 16.f) / 8388608.f + (kKeys ? 1.f / 262144.f : 0.f)) * 1.001f;
+// eps of a row is this times |q|_2 max|m|_2 (see the head of this section); kPosition: the estimates hold their
+// position in their low bits
+template <int D, bool kPosition> constexpr float gate_kappa =
+    ((18.f * (D / 16) + 16.f) / 8388608.f + (kPosition ? 1.f / 262144.f : 0.f)) * 1.001f;
 
 // ---- rows that the estimates alone do not settle ------------------------------------------------------------
 struct GateLists {
-  uint2* lists;                            // [128][lstride] {chunk, key}, largest key first
+  uint2* lists;                            // [128][lstride] {chunk, estimate (kFloats) or its key}, the largest first
   int lstride, list_len;
   unsigned long long* exact;               // [64] keys, of this warp
 };
@@ -434,7 +434,7 @@ struct GateLists {
 // kShort: the loops over the entries of a row are not unrolled.  Code that few rows come to is mostly fetched: 32768 x 32/8, at most 32
 // candidates, lists of 8: gating kernel 218 -> 214 us, head dim 256 552 -> 522, a decode step with a near-tie 60 -> 58.
 // Where many rows do, it costs (top-k 28 of 256 candidates at head dim 256, half of the rows: 1936 -> 2056).
-// kFloats: the list holds the estimates themselves, not keys.
+// kFloats: the list holds the estimates themselves, not order-preserving integer keys.
 template <bool kHalf, int D, bool kShort, bool kFloats>
 __device__ __forceinline__ void rank_rows(const Params& p, const GateLists& g, const GateTile& t, const __nv_bfloat16* qrow,
                                           int row, int mode, int n_surv, int n_keep, int ncand, float eps,
@@ -604,7 +604,7 @@ __device__ __forceinline__ void finish_scan(const ListScan& scan, int32_t* __res
 // the most near-ties, 2400 in the network.  Here
 //   warp 4     walks the row tiles of the CTA: requests Q and means and issues the MMA as soon as every row has its
 //              norms and its estimates of the tile before in registers, while networks, decisions and stores go on
-//   warps 0-3  a thread per row.  The sorted keys stay in registers, and what they settle is decided there; a row with
+//   warps 0-3  a thread per row.  The sorted estimates stay in registers, and what they settle is decided there; a row with
 //              near-ties goes through a list in shared memory.  Every warp counts for itself and warp 4 adds the
 //              counts of a tile to the lists a tile later: no barrier of the CTA in the loop, a warp may be a tile
 //              behind another.  (Added by every warp for itself, four requests for one, and some 7 ns each for the 128-byte
@@ -798,7 +798,7 @@ gate_one_kernel(const Params p, const __grid_constant__ CUtensorMap tmap_q, cons
       for (int w = 0; w < kGateRows / 32; ++w) ssq_max = max(ssq_max, c.mean_ssq[m & 1][w]);
       ++m;
 
-      // What the keys settle.  Bit i: entry i is a candidate (real), can be among the n_keep best (surv), is closer to
+      // What the estimates settle.  Bit i: entry i is a candidate (real), can be among the n_keep best (surv), is closer to
       // entry i + 1 than twice the error (tie)
       const float eps2 = 2.f * (gate_kappa<D, true> * sqrtf(q_ssq) * sqrtf(__int_as_float(ssq_max)) + 7.9e-31f);
       const int n_keep = min(hist, ncand), n_real = min(ncand, list_len);
