@@ -414,6 +414,7 @@ inline bool tc5_short_items(const Params& p) {
 //   head dim 64   chunk 128  1: 1.19 / 1.17 / 1.22   4: 1.23 / 1.19 / 1.23   16: 1.02 / 1.22 / 1.27
 //                 chunk 96   1: 1.13 / 1.15 / 1.19   4: 1.15 / 1.17 / 1.21   16: 0.92 / 1.10 / 1.18
 //                 chunk 64   1: 0.91 / 1.01 / 1.09   4: 0.90 / 1.01 / 1.10   16: 0.75 / 0.91 / 1.05
+//   head dim 96   chunk 128  1: 1.18 / 1.13 /  -     4:  -   /  -   / 1.04   16:  -   / 0.99 / 1.04;   chunk 96  4, top-k 8: 1.08
 // So: three tiles a list (ranks x chunk x heads of a group, in a long sequence whose tokens are all queries), and chunks of 64 to 95 keys
 // at head dim 64 with seven ranks.
 // A window of queries, or short sequences, have the lists of their whole prefix and few rows on each: what counts there is the rows that a
